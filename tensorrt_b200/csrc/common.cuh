@@ -62,20 +62,39 @@ int32_t smCount();
 bool dependentLaunchEnabled();
 
 #ifdef __CUDACC__
+// `cluster`: CTAs per thread-block cluster (1: none; the grid is a multiple of it).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launchDependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args)
+inline cudaError_t launchDependentCluster(
+    void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (dependentLaunchEnabled())
+    {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1)
+    {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(cluster);
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = dependentLaunchEnabled() ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launchDependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args)
+{
+    return launchDependentCluster(kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
 }
 #endif
 
@@ -92,6 +111,29 @@ __device__ __forceinline__ void gridDependencyLaunch()
 __device__ __forceinline__ void gridDependencyWait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// All threads of the cluster arrive; shared-memory writes made before are visible to every CTA of it afterwards.
+__device__ __forceinline__ void clusterBarrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The float at the same shared-memory location in CTA `rank` of this cluster.
+__device__ __forceinline__ float ldSharedCluster(float const* local, int rank)
+{
+    float v;
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %1, %2;\n\t"
+        "ld.shared::cluster.f32 %0, [a];\n\t"
+        "}"
+        : "=f"(v)
+        : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank)
+        : "memory");
+    return v;
 }
 
 __device__ __forceinline__ float warpSum(float v)

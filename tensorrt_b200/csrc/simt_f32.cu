@@ -1,7 +1,7 @@
 // FP32 (type_id 0) fully-connected and attention kernels. FP32 has no tensor-core path that keeps
 // full precision (TF32 would break the 1e-5 tolerance the reference configuration states for FP32,
 // plugin/bertQKVToContextPlugin/CustomQKVToContextPluginDynamic_PluginConfig.yaml:72-76), so these
-// are plain SIMT kernels; the FP16 / INT8 paths live in fc_tcgen05.cu and mha_tcgen05.cu.
+// are SIMT kernels; the FP16 / INT8 paths live in fc_tcgen05.cu and mha_tcgen05.cu.
 // The attention kernel also serves FP16 tensors (FP32 arithmetic) for the shapes the tensor-core kernel does not
 // take - heads wider than 64 or not a multiple of 16, sequences longer than 512 - the shapes the reference sends
 // to its unfused runner as well.
@@ -22,67 +22,196 @@ __device__ __forceinline__ float geluErf(float x)
     return 0.5f * x * (1.f + erff(x * 0.70710678118654752440f));
 }
 
+// ---- fully connected ------------------------------------------------------------------------------------------------
+// C[m,n] = act(alpha * sum_k A[m,k] * Wt[n,k] + bias[n]).
+//
+// Bound by the FP32 FMA pipes (128 per clock and SM). A CTA of two warps computes a 64 x 64 tile, every thread 8 x 8
+// outputs, four CTAs per SM. Both operands are K-contiguous, so they are copied to shared memory as they lie (16-byte
+// cp.async, four stages) and read back as 16-byte pieces along K; rows are padded to 20 floats, which puts the 4 or 8 rows
+// that a warp reads at once into different banks. The sums run on packed fma.rn.f32x2: one half takes the even k, the
+// other the odd ones (no operand has to be duplicated), and the two are added at the end; a packed FMA takes half the
+// issue slots, which leaves room for the 16 shared-memory loads that go with 128 of them.
+// A cluster of `split` CTAs divides the K range of a tile where the tiles alone leave SMs idle or fill the last wave badly;
+// its CTAs exchange partial sums through distributed shared memory, each finishing every split-th row.
+// Measured: 1024 x 2304 x 768 in 106 us (34 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x
+// 3072 in 130 us (700 us).
 constexpr int kTile = 64;
 constexpr int kTileK = 16;
+constexpr int kPitch = kTileK + 4; // floats
+constexpr int kStages = 4;
+constexpr int kFcF32Threads = 64;
+constexpr int kFcF32CtasPerSm = 4;
 
-// C[m,n] = act(alpha * sum_k A[m,k] * Wt[n,k] + bias[n]); 64x64 tile, 256 threads, 4x4 per thread.
-__global__ void __launch_bounds__(256) fcF32Kernel(int64_t const M, int64_t const N, int64_t const K,
-    float const* __restrict__ A, int64_t const lda, float const* __restrict__ Wt, float* __restrict__ C,
-    int64_t const ldc, float const* __restrict__ bias, int32_t const act, float const alpha)
+__device__ __forceinline__ void fma2(uint64_t& c, uint64_t a, uint64_t b)
 {
-    __shared__ float sA[kTileK][kTile + 1];
-    __shared__ float sB[kTileK][kTile + 1];
-    int const tx = threadIdx.x % 16;
-    int const ty = threadIdx.x / 16;
-    int64_t const m0 = static_cast<int64_t>(blockIdx.y) * kTile;
-    int64_t const n0 = static_cast<int64_t>(blockIdx.x) * kTile;
-    float acc[4][4] = {};
-    for (int64_t k0 = 0; k0 < K; k0 += kTileK)
-    {
-        for (int i = threadIdx.x; i < kTile * kTileK; i += 256)
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ float sumPair(uint64_t v)
+{
+    return __uint_as_float(static_cast<uint32_t>(v)) + __uint_as_float(static_cast<uint32_t>(v >> 32));
+}
+
+// kBytes (16 or 4) from global to shared memory, zeros when `valid` is false.
+template <int kBytes>
+__device__ __forceinline__ void cpAsync(uint32_t dst, void const* src, bool valid)
+{
+    int const n = valid ? kBytes : 0;
+    if constexpr (kBytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+__device__ __forceinline__ void cpAsyncCommit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void cpAsyncWait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+struct FcF32Args
+{
+    int64_t M, N, K;
+    float const* A;
+    int64_t lda;
+    float const* Wt;
+    float* C;
+    int64_t ldc;
+    float const* bias;
+    int32_t act;
+    float alpha;
+    int32_t nTiles; // tiles along N
+    int32_t split;  // CTAs per tile = cluster size
+};
+
+__device__ __forceinline__ float fcF32Epilogue(FcF32Args const& p, float v, int64_t n)
+{
+    v = v * p.alpha + (p.bias ? p.bias[n] : 0.f);
+    return p.act == BERT_B200_ACT_GELU_ERF ? geluErf(v) : v;
+}
+
+// kVec: floats per copy (4, or 1 where K, lda or an address is not a multiple of 16 bytes)
+template <int kVec>
+__global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(FcF32Args const p)
+{
+    __shared__ __align__(16) float sm[kStages][2][kTile][kPitch];
+    static_assert(sizeof(sm) >= kTile * kTile * sizeof(float), "partial sums reuse the ring");
+    int const tid = threadIdx.x;
+    int const lane = tid & 31;
+    int const ty = lane >> 3;
+    int const tx = lane & 7;
+    int const row0 = (tid >> 5) * 32 + ty; // rows row0 + 4 i, columns tx + 8 j
+    int const rank = static_cast<int>(blockIdx.x % p.split);
+    int64_t const tile = blockIdx.x / p.split;
+    int64_t const m0 = tile / p.nTiles * kTile;
+    int64_t const n0 = tile % p.nTiles * kTile;
+    int64_t const kBlocks = (p.K + kTileK - 1) / kTileK;
+    int const kbFirst = static_cast<int>(kBlocks * rank / p.split);
+    int const kbEnd = static_cast<int>(kBlocks * (rank + 1) / p.split);
+
+    gridDependencyLaunch();
+    gridDependencyWait();
+
+    uint32_t const smBase = static_cast<uint32_t>(__cvta_generic_to_shared(&sm[0][0][0][0]));
+    auto load = [&](int kb, int stage) {
+        constexpr int kPieces = kTileK / kVec; // per row
+        constexpr int kRowStep = kFcF32Threads / kPieces;
+        int const piece = tid % kPieces;
+        int64_t const k = static_cast<int64_t>(kb) * kTileK + piece * kVec;
+        bool const kOk = k < p.K;
+#pragma unroll
+        for (int r = tid / kPieces; r < 2 * kTile; r += kRowStep)
         {
-            int const r = i / kTileK;
-            int const c = i % kTileK;
-            sA[c][r] = (m0 + r < M && k0 + c < K) ? A[(m0 + r) * lda + k0 + c] : 0.f;
-            sB[c][r] = (n0 + r < N && k0 + c < K) ? Wt[(n0 + r) * K + k0 + c] : 0.f;
+            bool const isA = r < kTile;
+            int64_t const g = isA ? m0 + r : n0 + r - kTile;
+            bool const ok = kOk && g < (isA ? p.M : p.N);
+            float const* const src = isA ? p.A + g * p.lda + k : p.Wt + g * p.K + k;
+            cpAsync<4 * kVec>(smBase + 4u * (static_cast<uint32_t>(stage * 2 * kTile + r) * kPitch + piece * kVec), ok ? src : p.A, ok);
         }
-        __syncthreads();
+    };
+
+    uint64_t acc[8][8] = {};
+    for (int s = 0; s < kStages - 1; ++s)
+    {
+        if (kbFirst + s < kbEnd)
+            load(kbFirst + s, s);
+        cpAsyncCommit();
+    }
+    int stage = 0;
+    for (int kb = kbFirst; kb < kbEnd; ++kb)
+    {
+        cpAsyncWait<kStages - 2>();
+        __syncthreads(); // this stage has landed; everybody is done with the one that is filled next
+        int const ahead = stage == 0 ? kStages - 1 : stage - 1;
+        if (kb + kStages - 1 < kbEnd)
+            load(kb + kStages - 1, ahead);
+        cpAsyncCommit();
+        float const(*const a)[kPitch] = sm[stage][0];
+        float const(*const b)[kPitch] = sm[stage][1];
 #pragma unroll
-        for (int k = 0; k < kTileK; ++k)
+        for (int k = 0; k < kTileK; k += 4)
         {
-            float a[4], b[4];
+            ulonglong2 av[8], bv[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 8; ++i)
+                av[i] = *reinterpret_cast<ulonglong2 const*>(&a[row0 + 4 * i][k]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                bv[j] = *reinterpret_cast<ulonglong2 const*>(&b[tx + 8 * j][k]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    fma2(acc[i][j], av[i].x, bv[j].x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    fma2(acc[i][j], av[i].y, bv[j].y);
+        }
+        stage = stage + 1 == kStages ? 0 : stage + 1;
+    }
+    if (p.split == 1)
+    {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+        {
+            int64_t const m = m0 + row0 + 4 * i;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
             {
-                a[i] = sA[k][ty * 4 + i];
-                b[i] = sB[k][tx * 4 + i];
+                int64_t const n = n0 + tx + 8 * j;
+                if (m < p.M && n < p.N)
+                    p.C[m * p.ldc + n] = fcF32Epilogue(p, sumPair(acc[i][j]), n);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
+        return;
     }
+    cpAsyncWait<0>();
+    __syncthreads();
+    float* const part = &sm[0][0][0][0];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            part[(row0 + 4 * i) * kTile + tx + 8 * j] = sumPair(acc[i][j]);
+    clusterBarrier();
+    int const rows = static_cast<int>(p.M - m0 < kTile ? p.M - m0 : kTile);
+    int64_t const n = n0 + tid; // one column per thread, every split-th row
+    for (int r = rank; r < rows; r += p.split)
     {
-        int64_t const m = m0 + ty * 4 + i;
-        if (m >= M)
-            continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-        {
-            int64_t const n = n0 + tx * 4 + j;
-            if (n >= N)
-                continue;
-            float v = acc[i][j] * alpha + (bias ? bias[n] : 0.f);
-            if (act == BERT_B200_ACT_GELU_ERF)
-                v = geluErf(v);
-            C[m * ldc + n] = v;
-        }
+        float v = 0.f;
+        for (int q = 0; q < p.split; ++q)
+            v += ldSharedCluster(part + r * kTile + tid, q);
+        if (n < p.N)
+            p.C[(m0 + r) * p.ldc + n] = fcF32Epilogue(p, v, n);
     }
+    clusterBarrier(); // nobody leaves while its partial sums are being read
 }
 
 __device__ __forceinline__ float toFloat(float v)
@@ -102,6 +231,218 @@ __device__ __forceinline__ void fromFloat(__half& dst, float v)
     dst = __float2half_rn(v);
 }
 
+// ---- attention ------------------------------------------------------------------------------------------------------
+// Where the rows of one (sequence, head) lie.
+struct SeqRows
+{
+    int rows, len;  // query rows, valid keys
+    int64_t row0, rowStride;
+};
+
+__device__ __forceinline__ SeqRows seqRows(int b, int B, int S, int32_t const* cu, int32_t const* maskIdx)
+{
+    if (cu)
+        return {cu[b + 1] - cu[b], cu[b + 1] - cu[b], cu[b], 1};
+    return {S, maskIdx ? min(max(maskIdx[b], 0), S) : S, b, B};
+}
+
+// Four consecutive elements of a row, as FP32.
+__device__ __forceinline__ float4 load4(float const* p)
+{
+    return __ldg(reinterpret_cast<float4 const*>(p));
+}
+__device__ __forceinline__ float4 load4(__half const* p)
+{
+    uint2 const v = __ldg(reinterpret_cast<uint2 const*>(p));
+    float2 const lo = __half22float2(*reinterpret_cast<__half2 const*>(&v.x));
+    float2 const hi = __half22float2(*reinterpret_cast<__half2 const*>(&v.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void store4(float* p, float4 v)
+{
+    *reinterpret_cast<float4*>(p) = v;
+}
+__device__ __forceinline__ void store4(__half* p, float4 v)
+{
+    __half2 const lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t const*>(&lo), *reinterpret_cast<uint32_t const*>(&hi));
+}
+
+// 64 queries of one (sequence, head) per CTA against blocks of 64 keys, running maximum and sum per row.
+//
+// Bound by the FP32 pipes and the shared-memory loads that feed them. Every warp owns 16 query rows, so its scores,
+// probabilities and row sums are its own business (a warp-level sync between the two products); a thread computes 4 rows x
+// 8 keys of the scores with 16-byte loads along d (packed FMAs, even and odd channels apart, as in the FC above), and 4
+// rows x D / 8 columns of the context. Rows are padded by 4 floats against bank conflicts. Measured: 8 sequences of 128
+// tokens, 12 heads of 64 channels in 26 us (a warp per query row, keys and values from global memory: 509 us).
+constexpr int kAttRows = 64;
+constexpr int kAttKeys = 64;
+constexpr int kAttThreads = 128;
+
+template <int D> // head size rounded up to 32, 64, 96 or 128; channels beyond d are zero
+struct AttSmem
+{
+    float q[kAttRows][D + 4];
+    float k[kAttKeys][D + 4];
+    float v[kAttKeys][D];
+    float p[kAttRows][kAttKeys + 4];
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
+    T const* __restrict__ qkv, T* __restrict__ out, int32_t const* __restrict__ cu, int32_t const* __restrict__ maskIdx, float const scale)
+{
+    extern __shared__ float smRaw[];
+    AttSmem<D>& sm = *reinterpret_cast<AttSmem<D>*>(smRaw);
+    constexpr int kVecs = D / 4;
+    constexpr int kCols = D / 32; // float4 columns of the context per thread
+    int const lane = threadIdx.x & 31;
+    int const ty = lane >> 3;
+    int const tx = lane & 7;
+    int const row0 = (threadIdx.x >> 5) * 16 + ty; // rows row0 + 4 i
+
+    gridDependencyLaunch();
+    gridDependencyWait();
+
+    SeqRows const seq = seqRows(blockIdx.y, B, S, cu, maskIdx);
+    int const q0 = blockIdx.z * kAttRows;
+    if (q0 >= seq.rows)
+        return;
+    int64_t const tokStride = static_cast<int64_t>(3) * N * d;
+    T const* const base = qkv + seq.row0 * tokStride + static_cast<int64_t>(blockIdx.x) * 3 * d;
+    int64_t const rowStep = seq.rowStride * tokStride;
+    float4 const zero = make_float4(0.f, 0.f, 0.f, 0.f);
+
+    for (int i = threadIdx.x; i < kAttRows * kVecs; i += kAttThreads)
+    {
+        int const r = i / kVecs, c = i % kVecs * 4;
+        bool const ok = q0 + r < seq.rows && c < d;
+        *reinterpret_cast<float4*>(&sm.q[r][c]) = ok ? load4(base + (q0 + r) * rowStep + c) : zero;
+    }
+    float4 o[4][kCols];
+    float mx[4], sum[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+        mx[i] = -INFINITY;
+        sum[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j)
+            o[i][j] = zero;
+    }
+    for (int k0 = 0; k0 < seq.len; k0 += kAttKeys)
+    {
+        __syncthreads(); // the previous block of keys is done with
+#pragma unroll 4
+        for (int i = threadIdx.x; i < kAttKeys * kVecs; i += kAttThreads)
+        {
+            int const r = i / kVecs, c = i % kVecs * 4;
+            bool const ok = k0 + r < seq.len && c < d;
+            T const* const src = base + (k0 + r) * rowStep + c;
+            *reinterpret_cast<float4*>(&sm.k[r][c]) = ok ? load4(src + d) : zero;
+            *reinterpret_cast<float4*>(&sm.v[r][c]) = ok ? load4(src + 2 * d) : zero;
+        }
+        __syncthreads();
+        uint64_t acc[4][8] = {};
+#pragma unroll 4
+        for (int c = 0; c < D; c += 4)
+        {
+            ulonglong2 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                a[i] = *reinterpret_cast<ulonglong2 const*>(&sm.q[row0 + 4 * i][c]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                ulonglong2 const b = *reinterpret_cast<ulonglong2 const*>(&sm.k[tx + 8 * j][c]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                    fma2(acc[i][j], a[i].x, b.x);
+                    fma2(acc[i][j], a[i].y, b.y);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            float s[8];
+            float m = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                s[j] = k0 + tx + 8 * j < seq.len ? sumPair(acc[i][j]) * scale : -INFINITY;
+                m = fmaxf(m, s[j]);
+            }
+#pragma unroll
+            for (int x = 1; x < 8; x <<= 1)
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+            float const next = fmaxf(mx[i], m); // finite: every block has a valid key
+            float const rescale = expf(mx[i] - next);
+            mx[i] = next;
+            sum[i] *= rescale;
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+            {
+                o[i][j].x *= rescale;
+                o[i][j].y *= rescale;
+                o[i][j].z *= rescale;
+                o[i][j].w *= rescale;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                float const e = expf(s[j] - next);
+                sum[i] += e;
+                sm.p[row0 + 4 * i][tx + 8 * j] = e;
+            }
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int c = 0; c < kAttKeys; c += 4)
+        {
+            float4 pr[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int j = 0; j < kCols; ++j)
+                {
+                    float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                    {
+                        float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
+                        o[i][j].x = fmaf(w, v.x, o[i][j].x);
+                        o[i][j].y = fmaf(w, v.y, o[i][j].y);
+                        o[i][j].z = fmaf(w, v.z, o[i][j].z);
+                        o[i][j].w = fmaf(w, v.w, o[i][j].w);
+                    }
+                }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+    {
+        float t = sum[i];
+#pragma unroll
+        for (int x = 1; x < 8; x <<= 1)
+            t += __shfl_xor_sync(0xffffffffu, t, x);
+        int const r = q0 + row0 + 4 * i;
+        if (r >= seq.rows)
+            continue;
+        float const inv = seq.len > 0 ? 1.f / t : 0.f;
+        T* const dst = out + (seq.row0 + r * seq.rowStride) * (static_cast<int64_t>(N) * d) + static_cast<int64_t>(blockIdx.x) * d;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j)
+            if (tx * 4 + 32 * j < d)
+                store4(dst + tx * 4 + 32 * j, make_float4(o[i][j].x * inv, o[i][j].y * inv, o[i][j].z * inv, o[i][j].w * inv));
+    }
+}
+
+// Heads wider than 128, of a size that is no multiple of 4, or tensors that are not aligned to four elements.
 // One warp per query row. Scores of the row live in shared memory ([warps][S]); all arithmetic in FP32.
 template <typename T>
 __global__ void __launch_bounds__(128) mhaSimtKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
@@ -116,22 +457,9 @@ __global__ void __launch_bounds__(128) mhaSimtKernel(int32_t const B, int32_t co
     float* scores = sm + warp * (S + d);
     float* qs = scores + S;
 
-    int rows, len;
-    int64_t row0, rowStride;
-    if (cu)
-    {
-        row0 = cu[b];
-        len = cu[b + 1] - cu[b];
-        rows = len;
-        rowStride = 1;
-    }
-    else
-    {
-        row0 = b;
-        rowStride = B;
-        rows = S;
-        len = maskIdx ? min(max(maskIdx[b], 0), S) : S;
-    }
+    SeqRows const seq = seqRows(b, B, S, cu, maskIdx);
+    int const rows = seq.rows, len = seq.len;
+    int64_t const row0 = seq.row0, rowStride = seq.rowStride;
     int64_t const tokStride = static_cast<int64_t>(3) * N * d;
     int64_t const headOff = static_cast<int64_t>(n) * 3 * d;
     for (int s = blockIdx.z * 4 + warp; s < rows; s += gridDim.z * 4)
@@ -176,21 +504,72 @@ __global__ void __launch_bounds__(128) mhaSimtKernel(int32_t const B, int32_t co
 
 } // namespace
 
+// CTAs per tile. A k-block of a tile is 64 x 64 x 16 multiply-adds: 0.5 us on the FMA pipes of half an SM, all that one
+// CTA can use, and twice that once four share an SM. A CTA costs about 1.5 us besides (first loads, result), the exchange
+// of partial sums another 1.5 us.
+static int pickSplitF32(int64_t tiles, int64_t kBlocks)
+{
+    int64_t const sms = smCount();
+    int64_t const slots = sms * kFcF32CtasPerSm;
+    int best = 1;
+    double bestCost = 0.0;
+    for (int s = 1; s <= 8 && s <= kBlocks; ++s)
+    {
+        int64_t const ctas = tiles * s;
+        int64_t const waves = (ctas + slots - 1) / slots;
+        int64_t const perSm = waves > 1 ? kFcF32CtasPerSm : (ctas + sms - 1) / sms;
+        double const block = perSm <= 2 ? 0.53 : 0.265 * static_cast<double>(perSm);
+        double const cost = static_cast<double>(waves) * (static_cast<double>((kBlocks + s - 1) / s) * block + 1.5) + (s > 1 ? 1.5 : 0.0);
+        if (s == 1 || cost < bestCost)
+        {
+            best = s;
+            bestCost = cost;
+        }
+    }
+    return best;
+}
+
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
-    dim3 const grid(static_cast<unsigned>((p.n + kTile - 1) / kTile), static_cast<unsigned>((p.m + kTile - 1) / kTile));
-    B200_REQUIRE(grid.y <= 65535, "fc (FP32): m=%lld too large", static_cast<long long>(p.m));
-    fcF32Kernel<<<grid, 256, 0, stream>>>(p.m, p.n, p.k, static_cast<float const*>(p.a), p.lda,
-        static_cast<float const*>(p.wt), static_cast<float*>(p.c), p.ldc, p.bias, p.activation, p.alpha);
+    int64_t const mTiles = (p.m + kTile - 1) / kTile;
+    int64_t const nTiles = (p.n + kTile - 1) / kTile;
+    bool const vec = p.k % 4 == 0 && p.lda % 4 == 0 && aligned16(p.a) && aligned16(p.wt);
+    int const split = pickSplitF32(mTiles * nTiles, (p.k + kTileK - 1) / kTileK);
+    B200_REQUIRE(mTiles * nTiles * split < (1ll << 31), "fc (FP32): m=%lld, n=%lld too large", static_cast<long long>(p.m), static_cast<long long>(p.n));
+    FcF32Args const args{p.m, p.n, p.k, static_cast<float const*>(p.a), p.lda, static_cast<float const*>(p.wt), static_cast<float*>(p.c), p.ldc,
+        p.bias, p.activation, p.alpha, static_cast<int32_t>(nTiles), split};
+    cudaError_t const e = launchDependentCluster(vec ? fcF32Kernel<4> : fcF32Kernel<1>, dim3(static_cast<unsigned>(mTiles * nTiles * split)),
+        dim3(kFcF32Threads), 0, stream, split, args);
+    if (e != cudaSuccess)
+        B200_FAIL(BERT_B200_CUDA_ERROR, "fcF32Kernel: %s", cudaGetErrorString(e));
     return checkLaunch("fcF32Kernel");
 }
 
 namespace
 {
 
+template <typename T, int D>
+int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
+{
+    auto kernel = mhaTiledKernel<T, D>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(AttSmem<D>)));
+    if (e == cudaSuccess)
+        e = launchDependent(kernel, dim3(p.num_heads, p.B, (p.S + kAttRows - 1) / kAttRows), dim3(kAttThreads), sizeof(AttSmem<D>), stream, p.B, p.S,
+            p.num_heads, p.head_size, static_cast<T const*>(p.qkv), static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
+    if (e != cudaSuccess)
+        B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTiledKernel: %s", cudaGetErrorString(e));
+    return checkLaunch("mhaTiledKernel");
+}
+
 template <typename T>
 int32_t launchMhaSimt(bert_b200_mha_params const& p, cudaStream_t stream)
 {
+    uintptr_t const bits = reinterpret_cast<uintptr_t>(p.qkv) | reinterpret_cast<uintptr_t>(p.out);
+    if (p.head_size % 4 == 0 && p.head_size <= 128 && bits % (4 * sizeof(T)) == 0)
+        return p.head_size <= 32 ? launchMhaTiled<T, 32>(p, stream)
+            : p.head_size <= 64  ? launchMhaTiled<T, 64>(p, stream)
+            : p.head_size <= 96  ? launchMhaTiled<T, 96>(p, stream)
+                                 : launchMhaTiled<T, 128>(p, stream);
     size_t const smem = 4 * static_cast<size_t>(p.S + p.head_size) * sizeof(float);
     B200_REQUIRE(smem <= 200 * 1024, "mha (SIMT): S=%d with head size %d does not fit shared memory", p.S, p.head_size);
     auto kernel = mhaSimtKernel<T>;

@@ -98,6 +98,26 @@ def test_fc_fp32(cuda, m, k, n):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
 
 
+# tile and k-block edges of the FP32 kernel: one row, single column past a 64-wide tile, K below and above a k-block, K and
+# strides that are no multiple of four (element copies), shapes that divide K over a cluster (odd shares included)
+@pytest.mark.parametrize("m,k,n", [(1, 4, 1), (65, 20, 67), (64, 7, 64), (33, 1001, 130), (38, 3072, 768), (200, 784, 96), (1024, 768, 768)])
+@pytest.mark.parametrize("epi", ["none", "bias_gelu"])
+def test_fc_fp32_tile_edges(cuda, m, k, n, epi):
+    """Tolerance: a random walk of k roundings to 2^-24 of sums of size 0.02 sqrt(k) stays below 0.02 k 2^-24 < 4e-6."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(m + k + n)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    w = (0.02 * rng.standard_normal((k, n))).astype(np.float32)
+    bias = (0.02 * rng.standard_normal(n)).astype(np.float32) if epi != "none" else None
+    ref = O.fc(a, w, bias, "gelu" if epi == "bias_gelu" else None)
+    out = torch.full((m + 1, n), 7.0, device=cuda)
+    T.fc(_t(a, cuda), _t(np.ascontiguousarray(w.T), cuda), None if bias is None else _t(bias, cuda),
+         T.ACT_GELU_ERF if epi == "bias_gelu" else T.ACT_NONE, out=out[:m])
+    assert O.close_abs_or_rel(out[:m].cpu().numpy(), ref, 1e-5, 1e-5)[0]
+    assert bool((out[m] == 7.0).all())   # nothing written past the last row
+
+
 def test_fc_linearity_full_size(cuda):
     """BERT-large sizes (24576 x 1024 -> 4096): fc(a1 + a2) == fc(a1) + fc(a2) within FP16 rounding, and a
     checksum of the INT8 product equals the checksum computed from row/column sums."""

@@ -359,6 +359,31 @@ def test_mha_fp32(cuda, d):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
 
 
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("d", [4, 20, 64, 72, 96, 128, 132])
+def test_mha_simt_tile_edges(cuda, d, half):
+    """The FP32-arithmetic kernels around their 64-query / 64-key tiles (one key, a full tile, one past it, several), packed
+    and fixed with an empty sequence; head sizes on both sides of every channel padding and beyond the tiled kernel's 128."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(d)
+    N, lengths = 2, np.array([1, 64, 65, 200, 0, 63], dtype=np.int32)
+    if half and d in (64, 96):
+        d += 2   # FP16 multiples of 16 up to 64 belong to the tensor-core kernel; these take the row kernel
+    kind, tol = (np.float16, 1e-2) if half else (np.float32, 1e-5)
+    cu = O.cu_seqlens(lengths)
+    qkv = rng.standard_normal((int(cu[-1]), 3 * N * d)).astype(kind)
+    ref = O.mha(qkv, len(lengths), 200, N, d, cu=cu)
+    out = T.mha(_t(qkv, cuda), len(lengths), 200, N, head_size=d, cu_seqlens=_t(cu, cuda))
+    assert O.close_abs_or_rel(out.cpu().numpy(), ref, tol, tol)[0]
+    S = 130
+    qkv = rng.standard_normal((S, 3, 3 * N * d)).astype(kind)
+    lens = np.array([130, 0, 65], dtype=np.int32)
+    ref = O.mha(qkv, 3, S, N, d, lengths=lens)
+    out = T.mha(_t(qkv, cuda), 3, S, N, head_size=d, mask_idx=_t(lens, cuda))
+    assert O.close_abs_or_rel(out.cpu().numpy(), ref, tol, tol)[0]
+
+
 def test_mha_full_size_properties(cuda):
     """BERT-large S=384, B=64, N=16: with V = const per head the context equals that constant (rows of the
     softmax sum to one), and attention is invariant to a permutation of the keys."""
