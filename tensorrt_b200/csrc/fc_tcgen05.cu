@@ -596,59 +596,60 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFcThreads, 1)
 
     if (warp == 0)
     {
-        if (lane == 0)
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        // running shared-memory addresses of the stage being filled (see mmaPairLoHi for why)
+        uint32_t const fullAddr0 = smemAddr(full), emptyAddr0 = smemAddr(empty);
+        uint32_t const fullLeader0 = mapaShared(full, 0);
+        uint32_t const aAddr0 = smemAddr(sA), bAddr0 = smemAddr(sB);
+        uint32_t off8 = 0, aAddr = aAddr0, bAddr = bAddr0;
+        for (int64_t tile = firstTile; tile < numTiles && ok; tile += tileStride)
         {
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            // running shared-memory addresses of the stage being filled (see mmaPairLoHi for why)
-            uint32_t const fullAddr0 = smemAddr(full), emptyAddr0 = smemAddr(empty);
-            uint32_t const fullLeader0 = mapaShared(full, 0);
-            uint32_t const aAddr0 = smemAddr(sA), bAddr0 = smemAddr(sB);
-            uint32_t off8 = 0, aAddr = aAddr0, bAddr = bAddr0;
-            for (int64_t tile = firstTile; tile < numTiles && ok; tile += tileStride)
+            int32_t const m0 = static_cast<int32_t>(tile / nBlocks) * kPairM + static_cast<int32_t>(rank) * kBlockM;
+            int32_t const n0 = static_cast<int32_t>(tile % nBlocks) * BLOCK_N + static_cast<int32_t>(rank) * (BLOCK_N / 2);
+            for (int kb = 0; kb < kBlocks; ++kb)
             {
-                int32_t const m0 = static_cast<int32_t>(tile / nBlocks) * kPairM + static_cast<int32_t>(rank) * kBlockM;
-                int32_t const n0 = static_cast<int32_t>(tile % nBlocks) * BLOCK_N + static_cast<int32_t>(rank) * (BLOCK_N / 2);
-                for (int kb = 0; kb < kBlocks; ++kb)
+                if (!mbarWaitWarp(emptyAddr0 + off8, phase ^ 1u, abortFlag, kWaitStageFree))
                 {
-                    if (!mbarWaitAddr(emptyAddr0 + off8, phase ^ 1u, abortFlag, kWaitStageFree))
-                    {
-                        ok = false;
-                        break;
-                    }
+                    ok = false;
+                    break;
+                }
+                if (electOne())
+                {
                     if (leader)
                         mbarArriveExpectTxAddr(fullAddr0 + off8, 2 * L::kStageBytes);
                     tmaLoad2dPairAddr(aAddr, &mapA, fullLeader0 + off8, kb * kBlockK, m0);
                     tmaLoad2dPairAddr(bAddr, &mapB, fullLeader0 + off8, kb * kBlockK, n0);
-                    off8 += 8;
-                    aAddr += L::kABytes;
-                    bAddr += L::kBBytes;
-                    if (++stage == L::kStages)
-                    {
-                        stage = 0;
-                        phase ^= 1u;
-                        off8 = 0;
-                        aAddr = aAddr0;
-                        bAddr = bAddr0;
-                    }
                 }
-            }
-            // Tail: every stage released, i.e. no commit arrival is still on its way to this CTA.
-            for (int i = 0; i < L::kStages && ok; ++i)
-            {
-                ok = mbarWait(&empty[stage], phase ^ 1u, abortFlag, kWaitStageFree);
+                __syncwarp();
+                off8 += 8;
+                aAddr += L::kABytes;
+                bAddr += L::kBBytes;
                 if (++stage == L::kStages)
                 {
                     stage = 0;
                     phase ^= 1u;
+                    off8 = 0;
+                    aAddr = aAddr0;
+                    bAddr = bAddr0;
                 }
+            }
+        }
+        // Tail: every stage released, i.e. no commit arrival is still on its way to this CTA.
+        for (int i = 0; i < L::kStages && ok; ++i)
+        {
+            ok = mbarWaitWarp(smemAddr(&empty[stage]), phase ^ 1u, abortFlag, kWaitStageFree);
+            if (++stage == L::kStages)
+            {
+                stage = 0;
+                phase ^= 1u;
             }
         }
     }
     else if (warp == 1)
     {
-        if (lane == 0 && leader)
+        if (leader)
         {
             int stage = 0;
             uint32_t phase = 0;
@@ -666,26 +667,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFcThreads, 1)
             static_assert(kRowBytes / kUmmaKBytes == 4, "four MMAs per k-block");
             for (int64_t tile = firstTile; tile < numTiles && ok; tile += tileStride)
             {
-                if (!mbarWait(&accEmpty[acc], accPhase ^ 1u, abortFlag, kWaitAccFree))
+                if (!mbarWaitWarp(smemAddr(&accEmpty[acc]), accPhase ^ 1u, abortFlag, kWaitAccFree))
                     break;
                 tcFenceAfter();
                 uint32_t const dTmem = tmemBase + static_cast<uint32_t>(acc * BLOCK_N);
                 for (int kb = 0; kb < kBlocks; ++kb)
                 {
-                    if (!mbarWaitAddr(fullAddr0 + off8, phase, abortFlag, kWaitTmaFull))
+                    if (!mbarWaitWarp(fullAddr0 + off8, phase, abortFlag, kWaitTmaFull))
                     {
                         ok = false;
                         break;
                     }
                     tcFenceAfter();
-                    if (kb == 0)
-                        mmaPairLoHi<kInt8, false>(dTmem, aLo, bLo, descHi, kIdesc);
-                    else
-                        mmaPairLoHi<kInt8, true>(dTmem, aLo, bLo, descHi, kIdesc);
-                    mmaPairLoHi<kInt8, true>(dTmem, aLo + kStep, bLo + kStep, descHi, kIdesc);
-                    mmaPairLoHi<kInt8, true>(dTmem, aLo + 2 * kStep, bLo + 2 * kStep, descHi, kIdesc);
-                    mmaPairLoHi<kInt8, true>(dTmem, aLo + 3 * kStep, bLo + 3 * kStep, descHi, kIdesc);
-                    tcCommitPairAddr(emptyAddr0 + off8, 3);
+                    if (electOne())
+                    {
+                        if (kb == 0)
+                            mmaPairLoHi<kInt8, false>(dTmem, aLo, bLo, descHi, kIdesc);
+                        else
+                            mmaPairLoHi<kInt8, true>(dTmem, aLo, bLo, descHi, kIdesc);
+                        mmaPairLoHi<kInt8, true>(dTmem, aLo + kStep, bLo + kStep, descHi, kIdesc);
+                        mmaPairLoHi<kInt8, true>(dTmem, aLo + 2 * kStep, bLo + 2 * kStep, descHi, kIdesc);
+                        mmaPairLoHi<kInt8, true>(dTmem, aLo + 3 * kStep, bLo + 3 * kStep, descHi, kIdesc);
+                        tcCommitPairAddr(emptyAddr0 + off8, 3);
+                    }
+                    __syncwarp();
                     off8 += 8;
                     aLo += L::kABytes >> 4;
                     bLo += L::kBBytes >> 4;
@@ -700,7 +705,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFcThreads, 1)
                 }
                 if (!ok)
                     break;
-                tcCommitPair(&accFull[acc], 3);
+                if (electOne())
+                    tcCommitPair(&accFull[acc], 3);
+                __syncwarp();
                 acc ^= 1;
                 if (acc == 0)
                     accPhase ^= 1u;

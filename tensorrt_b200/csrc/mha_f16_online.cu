@@ -19,14 +19,14 @@
 //   warp 9          : one lane loads K / V blocks (128 keys x 64 channels, 16 KB) into a ring of 12 stages. The
 //                     blocks of an item stay resident for all its query tiles when they fit (S <= 768); longer
 //                     sequences stream their blocks once per pair of query tiles.
-//   warps 10 / 11   : one lane each, the MMA thread of stream 0 / 1. It issues the stream's scores  S = Q K_j^T
+//   warps 10 / 11   : the MMA warp of stream 0 / 1 (an elected lane issues). It issues the stream's scores  S = Q K_j^T
 //                     (128 x 128, FP32, TMEM columns 128*stream ..) as soon as the softmax threads hold the previous
 //                     block in registers - the first block of the stream's NEXT tile right behind the last block of
 //                     this one -, and the context products  O (+)= P_j V_j  (128 x 64, A operand = P straight from TMEM
 //                     columns 256 + 64*stream .., accumulator in columns 384 + 64*stream ..) as soon as P_j is stored.
-//                     (Every tcgen05.mma / commit keeps its issuing thread busy for 50-120 cycles: the twelve MMAs and
-//                     four commits of a block are a thread's work of its own per stream.) A thread per stream may block
-//                     on its stream's barriers; one thread serving both streams must not - an operand that a loader
+//                     (Every tcgen05.mma / commit keeps its issuing warp busy for 30-60 cycles: the twelve MMAs and
+//                     four commits of a block are a warp's work of its own per stream.) A warp per stream may block
+//                     on its stream's barriers; one warp serving both streams must not - an operand that a loader
 //                     delivers only after the OTHER stream has been served would never arrive.
 // Online softmax: the running maximum m only moves when the block maximum exceeds it by more than 8 in the log2
 // domain (P then stays below 2^8, far inside FP16); when it moves, the softmax threads scale the row sum and the
@@ -306,7 +306,7 @@ struct Walker
     }
 };
 
-// The loads [first, last) of a ring of kStages stages, in load order, for a thread that reads none of them: wait until
+// The loads [first, last) of a ring of kStages stages, in load order, for a warp that reads none of them: wait until
 // each block has landed, hand its stage back. Out of line: it runs once per tile at most and the kernel is sensitive to
 // the size of its hot code.
 static __device__ __noinline__ bool passThroughLoads(
@@ -315,9 +315,11 @@ static __device__ __noinline__ bool passThroughLoads(
     for (uint32_t L = first; L < last; ++L)
     {
         uint32_t const stage = L % kStages;
-        if (!mbarWaitAddr(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull))
+        if (!mbarWaitWarp(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull))
             return false;
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(emptyAddr + 8 * stage) : "memory");
+        if (electOne())
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(emptyAddr + 8 * stage) : "memory");
+        __syncwarp();
     }
     return true;
 }
@@ -406,48 +408,50 @@ __global__ void __maxnreg__(168)
     if (warp == 8)
     {
         // ---- Q tiles: slot n & 1, refilled when the score MMAs of the stream's previous tile have completed ----
-        if (lane == 0)
+        Walker w(args, geoTable);
+        bool ok = true;
+        for (bool more = w.begin(); more && ok; more = w.next())
         {
-            Walker w(args, geoTable);
-            bool ok = true;
-            for (bool more = w.begin(); more && ok; more = w.next())
+            uint32_t const slot = w.n & 1u;
+            if (w.n >= 2)
+                ok = mbarWaitWarp(smemAddr(&qFree[slot]), ((w.n >> 1) - 1) & 1u, abortFlag, kWaitStageFree);
+            if (!ok)
+                break;
+            if (electOne())
             {
-                uint32_t const slot = w.n & 1u;
-                if (w.n >= 2)
-                    ok = mbarWait(&qFree[slot], ((w.n >> 1) - 1) & 1u, abortFlag, kWaitStageFree);
-                if (!ok)
-                    break;
                 mbarArriveExpectTx(&qFull[slot], kStageBytes);
                 load(sQ + slot * kStageBytes, &qFull[slot], 0, w.g, (args.fixedLayout ? 0 : w.g.rowBase) + w.t * kTile);
             }
+            __syncwarp();
         }
     }
     else if (warp == 9)
     {
         // ---- K / V blocks of every sub-item, in the order the MMA threads consume them ----
-        if (lane == 0)
+        Walker w(args, geoTable);
+        bool ok = true;
+        for (bool more = w.begin(); more && ok; more = w.next())
         {
-            Walker w(args, geoTable);
-            bool ok = true;
-            for (bool more = w.begin(); more && ok; more = w.next())
+            if (!w.firstOfSub())
+                continue;
+            int32_t const rowK = args.fixedLayout ? 0 : w.g.rowBase;
+            for (int j = 0; j < w.g.nb && ok; ++j)
             {
-                if (!w.firstOfSub())
-                    continue;
-                int32_t const rowK = args.fixedLayout ? 0 : w.g.rowBase;
-                for (int j = 0; j < w.g.nb && ok; ++j)
+                for (int kv = 0; kv < 2 && ok; ++kv)
                 {
-                    for (int kv = 0; kv < 2 && ok; ++kv)
+                    uint32_t const L = w.loadBase + 2u * j + kv;
+                    uint32_t const s = L % kStages;
+                    uint32_t const fill = L / kStages;
+                    if (fill > 0)
+                        ok = mbarWaitWarp(smemAddr(&empty[s]), (fill - 1) & 1u, abortFlag, kWaitStageFree);
+                    if (!ok)
+                        break;
+                    if (electOne())
                     {
-                        uint32_t const L = w.loadBase + 2u * j + kv;
-                        uint32_t const s = L % kStages;
-                        uint32_t const fill = L / kStages;
-                        if (fill > 0)
-                            ok = mbarWait(&empty[s], (fill - 1) & 1u, abortFlag, kWaitStageFree);
-                        if (!ok)
-                            break;
                         mbarArriveExpectTx(&full[s], kStageBytes);
                         load(sKv + s * kStageBytes, &full[s], 1 + kv, w.g, rowK + j * kTile);
                     }
+                    __syncwarp();
                 }
             }
         }
@@ -458,51 +462,51 @@ __global__ void __maxnreg__(168)
         // The events of one stream come in a fixed order - scores of block j in registers (sFree), P_j written
         // (pReady), scores of block j+1 in registers, ... - so its thread simply waits for them in turn: after sFree it
         // issues the next scores (of this tile or of the stream's next one), after pReady the context product.
-        if (lane == 0)
-        {
-            uint32_t const s = static_cast<uint32_t>(warp - 10);
-            // K-major Q / K tiles (128-byte rows, 128-byte swizzle): SBO = 8 rows = 1024 B. V is MN-major (the head
-            // dimension contiguous): one MMA consumes 16 key rows = 2048 B.
-            uint64_t const dQk = makeSmemDesc(0, 16, 1024, kSwizzle128B);
-            uint64_t const dV = makeSmemDesc(0, 1024, 1024, kSwizzle128B);
-            uint32_t const hiQk = static_cast<uint32_t>(dQk >> 32), hiV = static_cast<uint32_t>(dV >> 32);
-            uint32_t const qLo = static_cast<uint32_t>(dQk) + (smemAddr(sQ) >> 4) + s * (kStageBytes >> 4);
-            uint32_t const kLo = static_cast<uint32_t>(dQk) + (smemAddr(sKv) >> 4);
-            uint32_t const vLo = static_cast<uint32_t>(dV) + (smemAddr(sKv) >> 4);
-            constexpr uint32_t kStage16 = kStageBytes >> 4;
-            uint32_t const fullAddr = smemAddr(full), emptyAddr = smemAddr(empty);
-            uint32_t const sFullAddr = smemAddr(&sFull[s]), sFreeAddr = smemAddr(&sFree[s]), pReadyAddr = smemAddr(&pReady[s]);
-            uint32_t const pvDoneAddr = smemAddr(&pvDone[s]), qFullAddr = smemAddr(&qFull[s]), qFreeAddr = smemAddr(&qFree[s]);
-            uint32_t const tS = tmemBase + s * kTile, tP = tmemBase + kPColumn + s * kHeadSize, tO = tmemBase + kOColumn + s * kHeadSize;
-            bool ok = true;
-            auto commitAddr = [](uint32_t barAddr) {
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
-            };
-            // A ring stage goes back to the loader when BOTH streams' MMA threads are done with it: each commits once, with
-            // its last tile of the sub-item. A sub-item of a single tile is read by one stream only; the other stream's
-            // thread still takes part in every one of its loads (passThrough below).
-            auto release = [&](uint32_t stage, Walker const& w) {
-                if (w.t >= w.subEnd - 2)
-                    commitAddr(emptyAddr + 8 * stage);
-            };
-            // The loads of a single-tile sub-item of the OTHER stream, in load order: wait until the block has landed, hand
-            // the stage back. A parity wait on an mbarrier is only valid for the barrier's NEXT phase, so a thread that
-            // waits on the `full` barrier of a ring stage has to have seen every earlier fill of that stage - also the
-            // fills whose data it never reads. (Skipping them - the other stream's thread adding the second arrival - let
-            // a thread that came back to a stage two fills later see "complete" at once and multiply blocks that had not
-            // landed: with many long sequences per CTA the attention hung until the waits expired.)
-            auto passThrough = [&](Walker const& w) {
-                ok = ok && passThroughLoads(fullAddr, emptyAddr, w.loadBase, w.loadBase + 2u * static_cast<uint32_t>(w.g.nb), abortFlag);
-            };
-            // scores of key block j of the tile `w` stands on
-            auto issueQk = [&](Walker const& w, int32_t j) {
-                uint32_t const L = w.loadBase + 2u * j;
-                uint32_t const stage = L % kStages;
-                ok = ok && mbarWaitAddr(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull);
-                if (!ok)
-                    return;
-                tcFenceAfter();
-                uint32_t const b = kLo + stage * kStage16;
+        uint32_t const s = static_cast<uint32_t>(warp - 10);
+        // K-major Q / K tiles (128-byte rows, 128-byte swizzle): SBO = 8 rows = 1024 B. V is MN-major (the head
+        // dimension contiguous): one MMA consumes 16 key rows = 2048 B.
+        uint64_t const dQk = makeSmemDesc(0, 16, 1024, kSwizzle128B);
+        uint64_t const dV = makeSmemDesc(0, 1024, 1024, kSwizzle128B);
+        uint32_t const hiQk = static_cast<uint32_t>(dQk >> 32), hiV = static_cast<uint32_t>(dV >> 32);
+        uint32_t const qLo = static_cast<uint32_t>(dQk) + (smemAddr(sQ) >> 4) + s * (kStageBytes >> 4);
+        uint32_t const kLo = static_cast<uint32_t>(dQk) + (smemAddr(sKv) >> 4);
+        uint32_t const vLo = static_cast<uint32_t>(dV) + (smemAddr(sKv) >> 4);
+        constexpr uint32_t kStage16 = kStageBytes >> 4;
+        uint32_t const fullAddr = smemAddr(full), emptyAddr = smemAddr(empty);
+        uint32_t const sFullAddr = smemAddr(&sFull[s]), sFreeAddr = smemAddr(&sFree[s]), pReadyAddr = smemAddr(&pReady[s]);
+        uint32_t const pvDoneAddr = smemAddr(&pvDone[s]), qFullAddr = smemAddr(&qFull[s]), qFreeAddr = smemAddr(&qFree[s]);
+        uint32_t const tS = tmemBase + s * kTile, tP = tmemBase + kPColumn + s * kHeadSize, tO = tmemBase + kOColumn + s * kHeadSize;
+        bool ok = true;
+        auto commitAddr = [](uint32_t barAddr) {
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
+        };
+        // A ring stage goes back to the loader when BOTH streams' MMA threads are done with it: each commits once, with
+        // its last tile of the sub-item. A sub-item of a single tile is read by one stream only; the other stream's
+        // thread still takes part in every one of its loads (passThrough below).
+        auto release = [&](uint32_t stage, Walker const& w) {
+            if (w.t >= w.subEnd - 2)
+                commitAddr(emptyAddr + 8 * stage);
+        };
+        // The loads of a single-tile sub-item of the OTHER stream, in load order: wait until the block has landed, hand
+        // the stage back. A parity wait on an mbarrier is only valid for the barrier's NEXT phase, so a thread that
+        // waits on the `full` barrier of a ring stage has to have seen every earlier fill of that stage - also the
+        // fills whose data it never reads. (Skipping them - the other stream's thread adding the second arrival - let
+        // a thread that came back to a stage two fills later see "complete" at once and multiply blocks that had not
+        // landed: with many long sequences per CTA the attention hung until the waits expired.)
+        auto passThrough = [&](Walker const& w) {
+            ok = ok && passThroughLoads(fullAddr, emptyAddr, w.loadBase, w.loadBase + 2u * static_cast<uint32_t>(w.g.nb), abortFlag);
+        };
+        // scores of key block j of the tile `w` stands on
+        auto issueQk = [&](Walker const& w, int32_t j) {
+            uint32_t const L = w.loadBase + 2u * j;
+            uint32_t const stage = L % kStages;
+            ok = ok && mbarWaitWarp(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull);
+            if (!ok)
+                return;
+            tcFenceAfter();
+            uint32_t const b = kLo + stage * kStage16;
+            if (electOne())
+            {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) // head size 64 = 4 x 16
                     mmaLoHi<false>(tS, qLo + 2 * k, hiQk, b + 2 * k, hiQk, kIdescQk, k != 0);
@@ -510,102 +514,107 @@ __global__ void __maxnreg__(168)
                 release(stage, w);
                 if (j == w.g.nb - 1)
                     commitAddr(qFreeAddr);
-            };
-            auto issuePv = [&](Walker const& w, int32_t j) {
-                uint32_t const L = w.loadBase + 2u * j + 1u;
-                uint32_t const stage = L % kStages;
-                ok = ok && mbarWaitAddr(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull);
-                if (!ok)
-                    return;
-                tcFenceAfter();
-                uint32_t const b = vLo + stage * kStage16;
+            }
+            __syncwarp();
+        };
+        auto issuePv = [&](Walker const& w, int32_t j) {
+            uint32_t const L = w.loadBase + 2u * j + 1u;
+            uint32_t const stage = L % kStages;
+            ok = ok && mbarWaitWarp(fullAddr + 8 * stage, (L / kStages) & 1u, abortFlag, kWaitTmaFull);
+            if (!ok)
+                return;
+            tcFenceAfter();
+            uint32_t const b = vLo + stage * kStage16;
+            if (electOne())
+            {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) // 128 keys = 8 x 16; P: 8 TMEM columns per 16 keys
                     mmaF16TmemA(tO, tP + 8 * k, b + k * 128u, hiV, kIdescPv, (j | k) != 0);
                 commitAddr(pvDoneAddr);
                 release(stage, w);
-            };
+            }
+            __syncwarp();
+        };
 
-            TR_DECL(2 + s);
-            Walker cur(args, geoTable);
-            bool active = cur.begin();
-            if (s == 1 && active)
+        TR_DECL(2 + s);
+        Walker cur(args, geoTable);
+        bool active = cur.begin();
+        if (s == 1 && active)
+        {
+            // tile 0 is stream 0's
+            if (cur.subTiles == 1)
+                passThrough(cur);
+            active = cur.next();
+        }
+        uint32_t qk = 0, pv = 0; // groups of score / context MMAs issued so far
+        if (active && ok)
+        {
+            ok = mbarWaitWarp(qFullAddr, (cur.n >> 1) & 1u, abortFlag, kWaitTmaFull);
+            if (ok)
+                issueQk(cur, 0);
+            qk = 1;
+        }
+        while (active && ok)
+        {
+            // the other stream's tile that follows this one, then this stream's next tile
+            Walker nxt = cur;
+            bool const hasMid = nxt.next();
+            bool const midAlone = hasMid && nxt.subTiles == 1; // a sub-item this thread reads nothing of
+            uint32_t const midFirst = nxt.loadBase, midBlocks = static_cast<uint32_t>(nxt.g.nb);
+            bool const hasNext = hasMid && nxt.next();
+            for (int j = 0; j < cur.g.nb && ok; ++j)
             {
-                // tile 0 is stream 0's
-                if (cur.subTiles == 1)
-                    passThrough(cur);
-                active = cur.next();
-            }
-            uint32_t qk = 0, pv = 0; // groups of score / context MMAs issued so far
-            if (active && ok)
-            {
-                ok = mbarWaitAddr(qFullAddr, (cur.n >> 1) & 1u, abortFlag, kWaitTmaFull);
-                if (ok)
-                    issueQk(cur, 0);
-                qk = 1;
-            }
-            while (active && ok)
-            {
-                // the other stream's tile that follows this one, then this stream's next tile
-                Walker nxt = cur;
-                bool const hasMid = nxt.next();
-                bool const midAlone = hasMid && nxt.subTiles == 1; // a sub-item this thread reads nothing of
-                uint32_t const midFirst = nxt.loadBase, midBlocks = static_cast<uint32_t>(nxt.g.nb);
-                bool const hasNext = hasMid && nxt.next();
-                for (int j = 0; j < cur.g.nb && ok; ++j)
-                {
-                    // Two things to issue per block: the scores that follow block j - block j + 1, or the first block of the
-                    // stream's next tile - and the context product of block j. The scores go first, so that the tensor pipe
-                    // has them done when the softmax threads come for them. Across a tile boundary the wait for their
-                    // operands then holds back the product whose completion frees this tile's last V stage, and the loader
-                    // works in load order: that is safe only while fewer than eleven loads lie between that V block and the
-                    // next tile's first K block (none when the tiles share sub-items; the 2 nb loads of the other stream's
-                    // tile when that is a sub-item of its own). With more, the loader would need the stage of that very V
-                    // block first - a cycle - and the product goes first. (One call site each for the two MMA groups: the
-                    // kernel is sensitive to the size of its code.)
-                    bool const lastBlock = j + 1 == cur.g.nb;
-                    bool qkPending = !lastBlock || hasNext, pvPending = true;
-                    bool const qkFirst = !lastBlock || !midAlone || midBlocks <= 5;
-                    bool midPending = lastBlock && midAlone;
-                    if (qkPending)
-                        ok = mbarWaitAddr(sFreeAddr, (qk - 1) & 1u, abortFlag, kWaitAccFree);
-                    TR_EVT(1);
+                // Two things to issue per block: the scores that follow block j - block j + 1, or the first block of the
+                // stream's next tile - and the context product of block j. The scores go first, so that the tensor pipe
+                // has them done when the softmax threads come for them. Across a tile boundary the wait for their
+                // operands then holds back the product whose completion frees this tile's last V stage, and the loader
+                // works in load order: that is safe only while fewer than eleven loads lie between that V block and the
+                // next tile's first K block (none when the tiles share sub-items; the 2 nb loads of the other stream's
+                // tile when that is a sub-item of its own). With more, the loader would need the stage of that very V
+                // block first - a cycle - and the product goes first. (One call site each for the two MMA groups: the
+                // kernel is sensitive to the size of its code.)
+                bool const lastBlock = j + 1 == cur.g.nb;
+                bool qkPending = !lastBlock || hasNext, pvPending = true;
+                bool const qkFirst = !lastBlock || !midAlone || midBlocks <= 5;
+                bool midPending = lastBlock && midAlone;
+                if (qkPending)
+                    ok = mbarWaitWarp(sFreeAddr, (qk - 1) & 1u, abortFlag, kWaitAccFree);
+                TR_EVT(1);
 #pragma unroll 1
-                    while ((qkPending || pvPending) && ok)
+                while ((qkPending || pvPending) && ok)
+                {
+                    if (qkPending && (qkFirst || !pvPending))
                     {
-                        if (qkPending && (qkFirst || !pvPending))
+                        if (lastBlock)
                         {
-                            if (lastBlock)
-                            {
-                                if (midPending)
-                                    ok = passThroughLoads(fullAddr, emptyAddr, midFirst, midFirst + 2u * midBlocks, abortFlag);
-                                midPending = false;
-                                ok = ok && mbarWaitAddr(qFullAddr, (nxt.n >> 1) & 1u, abortFlag, kWaitTmaFull);
-                            }
-                            if (ok)
-                                issueQk(lastBlock ? nxt : cur, lastBlock ? 0 : j + 1);
-                            TR_EVT(2);
-                            ++qk;
-                            qkPending = false;
+                            if (midPending)
+                                ok = passThroughLoads(fullAddr, emptyAddr, midFirst, midFirst + 2u * midBlocks, abortFlag);
+                            midPending = false;
+                            ok = ok && mbarWaitWarp(qFullAddr, (nxt.n >> 1) & 1u, abortFlag, kWaitTmaFull);
                         }
-                        else
-                        {
-                            ok = mbarWaitAddr(pReadyAddr, pv & 1u, abortFlag, kWaitSoftmax);
-                            TR_EVT(3);
-                            if (ok)
-                                issuePv(cur, j);
-                            TR_EVT(4);
-                            ++pv;
-                            pvPending = false;
-                        }
+                        if (ok)
+                            issueQk(lastBlock ? nxt : cur, lastBlock ? 0 : j + 1);
+                        TR_EVT(2);
+                        ++qk;
+                        qkPending = false;
                     }
-                    // the other stream's last tile, when this stream has none after it
-                    if (midPending && ok)
-                        ok = passThroughLoads(fullAddr, emptyAddr, midFirst, midFirst + 2u * midBlocks, abortFlag);
+                    else
+                    {
+                        ok = mbarWaitWarp(pReadyAddr, pv & 1u, abortFlag, kWaitSoftmax);
+                        TR_EVT(3);
+                        if (ok)
+                            issuePv(cur, j);
+                        TR_EVT(4);
+                        ++pv;
+                        pvPending = false;
+                    }
                 }
-                cur = nxt;
-                active = hasNext;
+                // the other stream's last tile, when this stream has none after it
+                if (midPending && ok)
+                    ok = passThroughLoads(fullAddr, emptyAddr, midFirst, midFirst + 2u * midBlocks, abortFlag);
             }
+            cur = nxt;
+            active = hasNext;
         }
     }
     else

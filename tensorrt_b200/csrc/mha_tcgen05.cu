@@ -294,67 +294,76 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     // running tile count; those that complete once per use of key block j keep one parity bit per block.
     if (warp == 0)
     {
-        if (lane == 0)
+        Item it;
+        uint32_t tiles = 0;       // Q tiles requested so far
+        uint32_t itemsLoaded = 0; // items whose K / V have been requested
+        bool ok = true;
+        for (int item = nextWork(blockIdx.x, it); item < numItems && ok; item = nextWork(item + gridDim.x, it))
         {
-            Item it;
-            uint32_t tiles = 0;       // Q tiles requested so far
-            uint32_t itemsLoaded = 0; // items whose K / V have been requested
-            bool ok = true;
-            for (int item = nextWork(blockIdx.x, it); item < numItems && ok; item = nextWork(item + gridDim.x, it))
+            int32_t const rowK = args.fixedLayout ? 0 : it.rowBase;
+            int32_t const rowKv = rowK; // first key of this item
+            // linear: (channel, which of [N][3], batch, row). interleaved: (channel, row, 32-channel group, which of [3][N])
+            auto load = [&](uint8_t* dst, uint64_t* bar, int which, int32_t row) {
+                if (BNSD) // (channel, position, head, sequence) of the tensor `which` selects
+                    tmaLoad4d(dst, which == 0 ? &mapQkv : (which == 1 ? &mapK : &mapV), bar, 0, row, it.head, it.b);
+                else if (IL)
+                    tmaLoad4d(dst, &mapQkv, bar, 0, row, 0, which * args.N + it.head);
+                else
+                    tmaLoad4d(dst, &mapQkv, bar, 0, it.head * 3 + which, args.fixedLayout ? it.b : 0, row);
+            };
+            for (int t = 0; t < it.nq && ok; ++t)
             {
-                int32_t const rowK = args.fixedLayout ? 0 : it.rowBase;
-                int32_t const rowKv = rowK; // first key of this item
-                // linear: (channel, which of [N][3], batch, row). interleaved: (channel, row, 32-channel group, which of [3][N])
-                auto load = [&](uint8_t* dst, uint64_t* bar, int which, int32_t row) {
-                    if (BNSD) // (channel, position, head, sequence) of the tensor `which` selects
-                        tmaLoad4d(dst, which == 0 ? &mapQkv : (which == 1 ? &mapK : &mapV), bar, 0, row, it.head, it.b);
-                    else if (IL)
-                        tmaLoad4d(dst, &mapQkv, bar, 0, row, 0, which * args.N + it.head);
-                    else
-                        tmaLoad4d(dst, &mapQkv, bar, 0, it.head * 3 + which, args.fixedLayout ? it.b : 0, row);
-                };
-                for (int t = 0; t < it.nq && ok; ++t)
+                // the score MMAs of the previous tile have read Q (and, across items, K)
+                if (tiles > 0)
+                    ok = mbarWaitWarp(qFree, (tiles - 1) & 1, abortFlag, kWaitStageFree);
+                if (!ok)
+                    break;
+                if (electOne())
                 {
-                    // the score MMAs of the previous tile have read Q (and, across items, K)
-                    if (tiles > 0)
-                        ok = mbarWait(qFree, (tiles - 1) & 1, abortFlag, kWaitStageFree);
-                    if (!ok)
-                        break;
                     mbarArriveExpectTx(qFull, L::kTileBytes);
                     load(sQ, qFull, 0, rowK + t * kQTile);
-                    if (t == 0)
+                }
+                __syncwarp();
+                if (t == 0)
+                {
+                    for (int j = 0; j < it.nb; ++j)
                     {
-                        for (int j = 0; j < it.nb; ++j)
+                        if (electOne())
                         {
                             mbarArriveExpectTx(&kFull[j], L::kTileBytes);
                             load(sK + j * L::kTileBytes, &kFull[j], 1, rowKv + j * kKeyBlock);
                         }
-                        // The PV products of the previous item have read V. (Not oFull: this thread may run ahead of
-                        // or behind the per-tile barriers by more than one phase, and a parity wait is only meaningful
-                        // for the very next phase; vFree completes once per item, in step with this loop.)
-                        if (itemsLoaded > 0)
-                            ok = mbarWait(vFree, (itemsLoaded - 1) & 1, abortFlag, kWaitStageFree);
-                        if (!ok)
-                            break;
-                        for (int j = 0; j < it.nb; ++j)
+                        __syncwarp();
+                    }
+                    // The PV products of the previous item have read V. (Not oFull: this thread may run ahead of
+                    // or behind the per-tile barriers by more than one phase, and a parity wait is only meaningful
+                    // for the very next phase; vFree completes once per item, in step with this loop.)
+                    if (itemsLoaded > 0)
+                        ok = mbarWaitWarp(vFree, (itemsLoaded - 1) & 1, abortFlag, kWaitStageFree);
+                    if (!ok)
+                        break;
+                    for (int j = 0; j < it.nb; ++j)
+                    {
+                        if (electOne())
                         {
                             mbarArriveExpectTx(&vFull[j], L::kTileBytes);
                             load(sV + j * L::kTileBytes, &vFull[j], 2, rowKv + j * kKeyBlock);
                         }
+                        __syncwarp();
                     }
-                    ++tiles;
                 }
-                ++itemsLoaded;
+                ++tiles;
             }
+            ++itemsLoaded;
         }
     }
     else if (warp == 1 || warp == kMhaThreads / 32 - 1)
     {
         // ---- MMA issue: scores S_j = Q K_j^T of the tile after the one the softmax warps work on, and
         //      context_t += P_j V_j as they hand over P_j ----
-        // Every tcgen05.mma / tcgen05.commit keeps its issuing thread busy for some 50 cycles (measured), and one
-        // thread issuing both products of a tile was the slowest link of the tile pipeline: the scores are issued by
-        // a second thread in the last warp (+11 % at S = 384). Sequences of a single key block have too few MMAs per
+        // Every tcgen05.mma / tcgen05.commit keeps its issuing warp busy for 30-60 cycles (measured), and one
+        // warp issuing both products of a tile was the slowest link of the tile pipeline: the scores are issued by
+        // a second one, the last warp (+11 % at S = 384). Sequences of a single key block have too few MMAs per
         // tile for that to pay (INT8, S = 128: -7 %) and keep one issuer.
         bool const twoIssuers = !kInt8 || nbMax > 1;
         // Operand descriptors are formed arithmetically: one low word per operand tile (+ bytes >> 4 per key block
@@ -382,19 +391,23 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             uint32_t kBits = 0, vBits = 0, pBits = 0, fBits = 0; // parity per key block: K landed, V landed, P written, S read
             // scores of key block j for the query tile whose Q is in shared memory; nbOf = key blocks of that tile's item
             auto issueScores = [&](int j, int nbOf) {
-#pragma unroll
-                for (int k = 0; k < kQkMmas; ++k)
+                if (electOne())
                 {
-                    uint32_t const off = (IL ? k * kSubTile : k * 32) >> 4; // next 32 bytes of the head dimension
-                    mmaLoHi<kInt8>(tmemBase + j * kKeyBlock, qLo + off, hiQk, kLo + j * kTile16 + off, hiQk, kIdescQk, k != 0);
+#pragma unroll
+                    for (int k = 0; k < kQkMmas; ++k)
+                    {
+                        uint32_t const off = (IL ? k * kSubTile : k * 32) >> 4; // next 32 bytes of the head dimension
+                        mmaLoHi<kInt8>(tmemBase + j * kKeyBlock, qLo + off, hiQk, kLo + j * kTile16 + off, hiQk, kIdescQk, k != 0);
+                    }
+                    tcCommit(&sFull[j]);
+                    if (j == nbOf - 1)
+                        tcCommit(qFree);
                 }
-                tcCommit(&sFull[j]);
-                if (j == nbOf - 1)
-                    tcCommit(qFree);
+                __syncwarp();
             };
             // first use of K_j by an item: wait for it to land
             auto waitK = [&](int j) -> bool {
-                bool const got = mbarWait(&kFull[j], (kBits >> j) & 1u, abortFlag, kWaitTmaFull);
+                bool const got = mbarWaitWarp(&kFull[j], (kBits >> j) & 1u, abortFlag, kWaitTmaFull);
                 kBits ^= 1u << j;
                 return got;
             };
@@ -402,7 +415,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             int item = nextWork(blockIdx.x, cur);
             if (kDoScores && item < numItems)
             {
-                ok = mbarWait(qFull, 0, abortFlag, kWaitTmaFull);
+                ok = mbarWaitWarp(qFull, 0, abortFlag, kWaitTmaFull);
 #pragma unroll 1
                 for (int j = 0; j < kMaxBlocks; ++j)
                 {
@@ -421,7 +434,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             while (item < numItems && ok)
             {
                 // only the scores look one item ahead (its geometry comes from global memory: not in the way of a
-                // thread that only issues context products)
+                // warp that only issues context products)
                 int const nextItem = kDoScores ? nextWork(item + gridDim.x, nxt) : numItems;
                 for (int t = 0; t < cur.nq && ok; ++t)
                 {
@@ -440,10 +453,10 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                             if (kDoScores && j < nbFollow && !oAliasesScores)
                             {
                                 if (j == 0)
-                                    ok = mbarWait(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
+                                    ok = mbarWaitWarp(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
                                 if (ok && lastT)
                                     ok = waitK(j);
-                                ok = ok && mbarWait(&sFree[j], (fBits >> j) & 1u, abortFlag, kWaitSoftmax);
+                                ok = ok && mbarWaitWarp(&sFree[j], (fBits >> j) & 1u, abortFlag, kWaitSoftmax);
                                 if (ok)
                                 {
                                     tcFenceAfter();
@@ -455,33 +468,37 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                             {
                                 if (ok && t == 0)
                                 {
-                                    ok = mbarWait(&vFull[j], (vBits >> j) & 1u, abortFlag, kWaitTmaFull);
+                                    ok = mbarWaitWarp(&vFull[j], (vBits >> j) & 1u, abortFlag, kWaitTmaFull);
                                     vBits ^= 1u << j;
                                 }
                                 if (ok && j == 0 && pvTiles > 0) // the previous tile's context must have been read out
-                                    ok = mbarWait(oFree, (pvTiles - 1) & 1, abortFlag, kWaitAccFree);
-                                ok = ok && mbarWait(&pReady[j], (pBits >> j) & 1u, abortFlag, kWaitSoftmax);
+                                    ok = mbarWaitWarp(oFree, (pvTiles - 1) & 1, abortFlag, kWaitAccFree);
+                                ok = ok && mbarWaitWarp(&pReady[j], (pBits >> j) & 1u, abortFlag, kWaitSoftmax);
                                 pBits ^= 1u << j;
                                 if (ok)
                                 {
                                     tcFenceAfter();
                                     uint32_t const a = pLo + (j & 1) * (L::kPBytes >> 4) + (j >> 1) * pPairStep;
                                     uint32_t const b = vLo + j * kTile16;
+                                    if (electOne())
+                                    {
 #pragma unroll
-                                    for (int k = 0; k < kPvMmas; ++k)
-                                    {
-                                        constexpr uint32_t kVStep = (IL ? 1024u : 2048u) >> 4;
-                                        uint32_t const pOff = (kInt8 ? k * 32 : (k / 4) * (kQTile * 128) + (k % 4) * 32) >> 4;
-                                        mmaLoHi<kInt8>(tmemBase + oCol, a + pOff, hiP, b + k * kVStep, hiV, kIdescPv, (j | k) != 0);
+                                        for (int k = 0; k < kPvMmas; ++k)
+                                        {
+                                            constexpr uint32_t kVStep = (IL ? 1024u : 2048u) >> 4;
+                                            uint32_t const pOff = (kInt8 ? k * 32 : (k / 4) * (kQTile * 128) + (k % 4) * 32) >> 4;
+                                            mmaLoHi<kInt8>(tmemBase + oCol, a + pOff, hiP, b + k * kVStep, hiV, kIdescPv, (j | k) != 0);
+                                        }
+                                        if (oAliasesScores) // otherwise every tile has its own P slots, released with oFull
+                                            tcCommit(&pFree[slotOf(j)]);
+                                        if (j == cur.nb - 1)
+                                        {
+                                            tcCommit(oFull);
+                                            if (lastT)
+                                                tcCommit(vFree);
+                                        }
                                     }
-                                    if (oAliasesScores) // otherwise every tile has its own P slots, released with oFull
-                                        tcCommit(&pFree[slotOf(j)]);
-                                    if (j == cur.nb - 1)
-                                    {
-                                        tcCommit(oFull);
-                                        if (lastT)
-                                            tcCommit(vFree);
-                                    }
+                                    __syncwarp();
                                 }
                             }
                         }
@@ -506,7 +523,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     if (kDoScores && ok && nbFollow > 0 && oAliasesScores)
                     {
                         // the context accumulator occupies score columns: wait until the epilogue has read it
-                        ok = mbarWait(oFree, pvTiles & 1, abortFlag, kWaitAccFree) && mbarWait(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
+                        ok = mbarWaitWarp(oFree, pvTiles & 1, abortFlag, kWaitAccFree) && mbarWaitWarp(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
 #pragma unroll 1
                         for (int j = 0; j < kMaxBlocks; ++j)
                         {
@@ -535,18 +552,15 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     item = nextWork(item + gridDim.x, cur);
             }
         };
-        if (lane == 0)
+        if (!twoIssuers)
         {
-            if (!twoIssuers)
-            {
-                if (warp == 1)
-                    issuer(std::true_type{}, std::true_type{});
-            }
-            else if (warp == 1)
-                issuer(std::false_type{}, std::true_type{});
-            else
-                issuer(std::true_type{}, std::false_type{});
+            if (warp == 1)
+                issuer(std::true_type{}, std::true_type{});
         }
+        else if (warp == 1)
+            issuer(std::false_type{}, std::true_type{});
+        else
+            issuer(std::true_type{}, std::false_type{});
     }
     else if (warp < 2 + kSoftmaxThreads / 32)
     {
