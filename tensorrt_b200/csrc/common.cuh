@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -62,10 +63,39 @@ int32_t smCount();
 bool dependentLaunchEnabled();
 
 #ifdef __CUDACC__
-// `cluster`: CTAs per thread-block cluster (1: none; the grid is a multiple of it).
+// Remembers on which devices a kernel has been allowed its dynamic shared memory (beyond 48 KB it needs an attribute, which
+// costs as much host time as a quarter of a launch). One static object per kernel.
+class SmemOptIn
+{
+public:
+    template <typename K>
+    cudaError_t set(K kernel, size_t bytes, bool again)
+    {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess)
+            return e;
+        uint64_t const bit = dev < 64 ? 1ull << dev : 0ull;
+        if (!again && (mDone.load(std::memory_order_relaxed) & bit) != 0)
+            return cudaSuccess;
+        int max = 0;
+        e = cudaDeviceGetAttribute(&max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess)
+            e = bytes <= static_cast<size_t>(max) ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max) : cudaErrorInvalidValue;
+        if (e == cudaSuccess)
+            mDone.fetch_or(bit, std::memory_order_relaxed);
+        return e;
+    }
+
+private:
+    std::atomic<uint64_t> mDone{0};
+};
+
+// `cluster`: CTAs per thread-block cluster (1: none or the kernel's own; the grid is a multiple of it). `optIn`: null for
+// kernels within 48 KB.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launchDependentCluster(
-    void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args)
+    SmemOptIn* optIn, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -88,13 +118,24 @@ inline cudaError_t launchDependentCluster(
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    cudaError_t e = optIn ? optIn->set(kernel, smem, false) : cudaSuccess;
+    if (e == cudaSuccess)
+        e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    if (e == cudaErrorInvalidValue && optIn)
+    {
+        // the device's context may have been reset since the attribute was set
+        cudaGetLastError();
+        e = optIn->set(kernel, smem, true);
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+    }
+    return e;
 }
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launchDependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args)
 {
-    return launchDependentCluster(kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
+    return launchDependentCluster(nullptr, kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
 }
 #endif
 

@@ -47,6 +47,9 @@ struct bert_b200_encoder
 
 namespace b200
 {
+
+int32_t fcRun(bert_b200_fc_params const& p, cudaStream_t stream, bool weightsReady);
+
 namespace
 {
 
@@ -298,6 +301,8 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         ++launches;                                                                                                    \
     } while (0)
 
+    // The memset also orders the whole forward behind everything ahead of it in the stream: kernels that write weights have
+    // completed before the first kernel below starts, so the FC kernels may fetch weights ahead of their predecessors' end.
     if (cudaMemsetAsync(w.status, 0, sizeof(uint32_t), stream) != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "encoder_forward: clearing the status word failed");
     // FP16: embedding output is the first layer input. INT8: additionally quantised with the first layer's input scale.
@@ -329,7 +334,7 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         fc.alpha = i8 ? l.s_in * l.s_wqkv : 1.f;
         fc.out_scale = i8 ? 1.f / l.s_qkv : 1.f;
         amax(w.x, T * E, li, 0);
-        B200_STEP(BERT_B200_KIND_FC, bert_b200_fc(&fc, stream));
+        B200_STEP(BERT_B200_KIND_FC, fcRun(fc, stream, true));
         amax(w.qkv, T * 3 * E, li, 1);
 
         bert_b200_mha_params mha{};
@@ -360,7 +365,7 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         fc.bias = nullptr;
         fc.alpha = i8 ? l.s_ctx * l.s_wout : 1.f;
         fc.out_scale = i8 ? 1.f / l.s_attn_out : 1.f;
-        B200_STEP(BERT_B200_KIND_FC, bert_b200_fc(&fc, stream));
+        B200_STEP(BERT_B200_KIND_FC, fcRun(fc, stream, true));
         amax(w.ao, T * E, li, 3);
 
         if (i8)
@@ -384,7 +389,7 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         fc.activation = BERT_B200_ACT_GELU_ERF;
         fc.alpha = i8 ? l.s_ln1 * l.s_wffn1 : 1.f;
         fc.out_scale = i8 ? 1.f / l.s_ffn1 : 1.f;
-        B200_STEP(BERT_B200_KIND_FC, bert_b200_fc(&fc, stream));
+        B200_STEP(BERT_B200_KIND_FC, fcRun(fc, stream, true));
         amax(w.f1, T * F, li, 5);
 
         // FFN down projection
@@ -399,7 +404,7 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         fc.activation = BERT_B200_ACT_NONE;
         fc.alpha = i8 ? l.s_ffn1 * l.s_wffn2 : 1.f;
         fc.out_scale = i8 ? 1.f / l.s_ffn2 : 1.f;
-        B200_STEP(BERT_B200_KIND_FC, bert_b200_fc(&fc, stream));
+        B200_STEP(BERT_B200_KIND_FC, fcRun(fc, stream, true));
         amax(w.ao, T * E, li, 6);
 
         bool const last = li + 1 == c.num_layers;

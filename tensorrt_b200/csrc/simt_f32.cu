@@ -538,7 +538,7 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
     B200_REQUIRE(mTiles * nTiles * split < (1ll << 31), "fc (FP32): m=%lld, n=%lld too large", static_cast<long long>(p.m), static_cast<long long>(p.n));
     FcF32Args const args{p.m, p.n, p.k, static_cast<float const*>(p.a), p.lda, static_cast<float const*>(p.wt), static_cast<float*>(p.c), p.ldc,
         p.bias, p.activation, p.alpha, static_cast<int32_t>(nTiles), split};
-    cudaError_t const e = launchDependentCluster(vec ? fcF32Kernel<4> : fcF32Kernel<1>, dim3(static_cast<unsigned>(mTiles * nTiles * split)),
+    cudaError_t const e = launchDependentCluster(nullptr, vec ? fcF32Kernel<4> : fcF32Kernel<1>, dim3(static_cast<unsigned>(mTiles * nTiles * split)),
         dim3(kFcF32Threads), 0, stream, split, args);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "fcF32Kernel: %s", cudaGetErrorString(e));

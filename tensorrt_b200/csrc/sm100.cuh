@@ -222,6 +222,23 @@ __device__ __forceinline__ void tmaLoad2d(void* dst, CUtensorMap const* map, uin
         : "memory");
 }
 
+// The same with shared::cta addresses that the loops of a role keep in registers.
+__device__ __forceinline__ void tmaLoad2dAddr(uint32_t dst, CUtensorMap const* map, uint32_t bar, int32_t c0, int32_t c1)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+
+// Pulls a tile into the L2, where later writes by other SMs land as well: no ordering is needed.
+__device__ __forceinline__ void tmaPrefetch2d(CUtensorMap const* map, int32_t c0, int32_t c1)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tmaLoad4d(
     void* dst, CUtensorMap const* map, uint64_t* bar, int32_t c0, int32_t c1, int32_t c2, int32_t c3)
 {
@@ -290,6 +307,11 @@ __device__ __forceinline__ void tcCommit(uint64_t* bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smemAddr(bar))
                  : "memory");
+}
+
+__device__ __forceinline__ void tcCommitAddr(uint32_t barAddr)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
 }
 
 // D[tmem] (+)= A[smem] * B[smem]; issued by a single thread.

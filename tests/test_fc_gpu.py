@@ -98,6 +98,46 @@ def test_fc_fp32(cuda, m, k, n):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
 
 
+# one row of a tile, one past a row box / a tile, n on both sides of each tile width and of the switch to two CTAs per SM and
+# to pair tiles (148 SMs), K below a ring stage, not a multiple of one, and longer than the ring
+@pytest.mark.parametrize("m,k,n", [(1, 16, 16), (7, 80, 48), (9, 1040, 144), (127, 768, 2368), (128, 4096, 2384), (129, 64, 4736), (130, 3088, 1200),
+                                   (129, 272, 9488), (257, 768, 12624), (300, 96, 12640), (37, 12288, 768)])
+@pytest.mark.parametrize("int8", [False, True])
+def test_fc_tile_edges(cuda, m, k, n, int8):
+    """Every tile width and both kernels against products summed in float64; the tolerance is that of the shapes above."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    bias = 0.5 * torch.randn(n, device=cuda, generator=gen)
+    st = _status(cuda)
+    if int8:
+        a, w = (torch.randint(-127, 128, s, device=cuda, generator=gen, dtype=torch.int32).to(torch.int8) for s in ((m, k), (n, k)))
+        alpha, q = 2.0 / (127 * 127 * k ** 0.5), 50.0
+        ref = (a.double() @ w.double().T).float() * alpha + bias
+        for kind in (torch.int8, torch.float16):
+            out = torch.full((m + 1, n), 77, device=cuda, dtype=kind)
+            T.fc(a, w, bias, alpha=alpha, out_dtype=kind, out_scale=q, status=st, out=out[:m])
+            want = torch.clamp(torch.round(ref * q), -128, 127) if kind == torch.int8 else ref
+            diff = (out[:m].float() - want).abs()
+            if kind == torch.int8:
+                assert float(diff.max()) <= 1 and float((diff > 0).float().mean()) < 1e-2
+            else:
+                assert bool((diff <= 2e-3 * torch.clamp(want.abs(), min=1.0)).all())
+            assert bool((out[m] == 77).all())
+    else:
+        a = torch.randn(m, k, device=cuda, generator=gen).half()
+        w = (torch.randn(n, k, device=cuda, generator=gen) * k ** -0.5).half()
+        ref = (a.double() @ w.double().T).float() + bias
+        out = torch.full((m + 1, n), 77, device=cuda, dtype=torch.float16)
+        T.fc(a, w, bias, status=st, out=out[:m])
+        assert bool(((out[:m].float() - ref).abs() <= 2e-3 * torch.clamp(ref.abs(), min=1.0)).all())
+        assert bool((out[m] == 77).all())
+        # a row does not depend on how many rows are multiplied with it
+        more = T.fc(torch.cat([a, torch.randn(3000, k, device=cuda, generator=gen).half()]), w, bias)
+        assert torch.equal(out[:m], more[:m])
+    assert int(st[0]) == 0
+
+
 # tile and k-block edges of the FP32 kernel: one row, single column past a 64-wide tile, K below and above a k-block, K and
 # strides that are no multiple of four (element copies), shapes that divide K over a cluster (odd shares included)
 @pytest.mark.parametrize("m,k,n", [(1, 4, 1), (65, 20, 67), (64, 7, 64), (33, 1001, 130), (38, 3072, 768), (200, 784, 96), (1024, 768, 768)])
