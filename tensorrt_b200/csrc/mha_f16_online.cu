@@ -6,19 +6,20 @@
 // FusedMHARunnerFP16[v2]::run (plugin/bertQKVToContextPlugin/mhaRunner.cu:835-860, 1127-1265) and its unfused
 // cuBLAS + softmax path (mhaRunner.cu:533-601) for the sequence lengths those kernels do not cover.
 //
-// One persistent CTA per SM keeps TWO 128-query tiles in flight (streams 0 and 1). The tiles of the CTA's work
-// list are dealt alternately to the two streams, across the boundaries of (sequence, head) items, so an odd number
-// of tiles per item (S = 384) leaves no stream idle. 12 warps:
+// One persistent CTA per SM keeps TWO 128-query tiles in flight (streams 0 and 1). The tiles of the CTA's share of the
+// work (mha_share.cuh) are dealt alternately to the two streams, across the boundaries of (sequence, head) pairs, so an
+// odd number of tiles per pair (S = 384) leaves no stream idle. 12 warps:
 //   warps 0-3 / 4-7 : softmax of stream 0 / 1, ONE THREAD PER QUERY ROW (the 32x32b TMEM load hands lane = row):
 //                     no cross-thread reduction, no barrier among softmax threads. Per key block: load the 128
 //                     scores into registers (their TMEM columns are then free for the next block's scores), block
 //                     maximum, lazy rescale (below), p = exp2(x*scale*log2e - m), row sum, P as FP16 pairs into 64
 //                     TMEM columns of its own. The normalising epilogue of a tile is deferred into the first block of
 //                     the stream's next tile, so its wait for the last context product costs nothing.
-//   warp 8          : one lane loads the Q tiles (two slots, one per stream).
-//   warp 9          : one lane loads K / V blocks (128 keys x 64 channels, 16 KB) into a ring of 12 stages. The
-//                     blocks of an item stay resident for all its query tiles when they fit (S <= 768); longer
-//                     sequences stream their blocks once per pair of query tiles.
+//   warp 8          : one lane loads the Q tiles (four slots, two per stream: with one, a tile's Q was requested only
+//                     when the last scores of the tile before were done, which short sequences waited for).
+//   warp 9          : one lane loads K / V blocks (128 keys x 64 channels, 16 KB) into a ring of 10 stages. The
+//                     blocks of a pair stay resident for all its query tiles when they fit (S <= 640); longer
+//                     sequences stream their blocks once per two query tiles.
 //   warps 10 / 11   : the MMA warp of stream 0 / 1 (an elected lane issues). It issues the stream's scores  S = Q K_j^T
 //                     (128 x 128, FP32, TMEM columns 128*stream ..) as soon as the softmax threads hold the previous
 //                     block in registers - the first block of the stream's NEXT tile right behind the last block of
@@ -32,7 +33,11 @@
 // domain (P then stays below 2^8, far inside FP16); when it moves, the softmax threads scale the row sum and the
 // context accumulator in TMEM themselves (after the previous P V product has completed). The final context is
 // O / rowsum. Compared with a softmax over the exact row maximum this changes nothing but the rounding of P.
+// Measured (16 heads of 64; whole pairs dealt round-robin and one Q slot per stream before): 11 sequences of 200 ... 2000
+// tokens 203 -> 122 us, 148 x 128 43.3 us, 148 x 384 167 us, 37 x 1024 271 us; bound by the exponentials (a 128 x 128 block takes 1024
+// cycles of the unit) at half of their rate: the two streams' other work is not hidden behind them completely.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM and reports through the status word.
+#include "mha_share.cuh"
 #include "sm100.cuh"
 
 namespace b200
@@ -52,7 +57,8 @@ namespace
 
 constexpr int kTile = 128;       // query rows per tile = keys per block
 constexpr int kHeadSize = 64;    // channels per tile row (smaller heads are zero-filled by the TMA unit)
-constexpr int kStages = 12;      // K / V ring
+constexpr int kStages = 10;      // K / V ring
+constexpr int kQSlots = 4;       // Q tiles: two per stream, so that a tile's Q is on its way during the whole tile before it
 constexpr int kStageBytes = kTile * kHeadSize * 2; // 16 KB: one Q tile, one K block, one V block
 constexpr int kThreads = 384;    // 8 softmax warps, Q loader, K/V loader, two MMA issuers
 constexpr uint32_t kTmemCols = 512;
@@ -60,29 +66,24 @@ constexpr uint32_t kPColumn = 256; // P blocks (FP16 pairs): 64 columns per stre
 constexpr uint32_t kOColumn = 384; // context accumulators: 64 columns per stream
 constexpr float kRescaleLog2 = 8.f;
 
-struct OnlineArgs
+struct OnlineArgs : ShareArgs
 {
-    int32_t B, S, N, total;
     int32_t d;
-    int32_t fixedLayout;
     void* out;
-    int32_t const* cu;
-    int32_t const* maskIdx;
     float scaleBmm1;
     uint32_t* statusWord;
-    int32_t tilesPerUnit, chunks; // a work unit = (sequence, head, chunk of tilesPerUnit query tiles)
-    int32_t stepChunk, stepHead, stepB; // gridDim.x = stepChunk + chunks * (stepHead + N * stepB)
 };
 
-// [ Q slot 0 ][ Q slot 1 ][ 12 K/V stages ][ barriers ]
+// [ Q slots ][ K/V stages ][ barriers ][ shares ]
 constexpr int kSmemQ = 0;
-constexpr int kSmemKv = 2 * kStageBytes;
+constexpr int kSmemKv = kQSlots * kStageBytes;
 constexpr int kSmemBars = kSmemKv + kStages * kStageBytes;
-// full[12] empty[12] qFull[2] qFree[2] sFull[2] sFree[2] pReady[2] pvDone[2], tmem slot, abort flag
-constexpr int kNumBars = 2 * kStages + 12;
-constexpr int kGeoEntries = 128; // geometry words of the CTA's first work units, read once from global memory
-constexpr int kSmemGeo = kSmemBars + kNumBars * 8 + 16;
-constexpr int kSmemBytes = kSmemGeo + kGeoEntries * 8 + 1024;
+// full[kStages] empty[kStages] qFull[kQSlots] qFree[kQSlots] sFull[2] sFree[2] pReady[2] pvDone[2], tmem slot, abort flag
+constexpr int kNumBars = 2 * kStages + 2 * kQSlots + 8;
+constexpr int kSmemShare = kSmemBars + kNumBars * 8 + 16;
+constexpr int kSmemBytes = kSmemShare + static_cast<int>(sizeof(ShareSmem)) + 1024;
+// a query tile costs its key blocks and about one block more for what is done once per tile
+constexpr uint32_t kTileCost = 1;
 
 __device__ __forceinline__ float ex2Approx(float x)
 {
@@ -135,133 +136,22 @@ __device__ __forceinline__ uint32_t packHalf2(float lo, float hi)
     return *reinterpret_cast<uint32_t const*>(&h);
 }
 
-// Geometry of one work unit; identical in every role (derived from the arguments and two words of global memory).
-struct Unit
+// The CTA's query tiles in processing order. Tile number n (counted per CTA) belongs to stream n & 1.
+// A "sub-item" is the run of tiles that shares one load of the K / V blocks: all tiles of a (sequence, head) in the share
+// when its blocks fit the ring, otherwise pairs of tiles (one per stream). `loadBase` is the number of K / V blocks loaded
+// before it: block j of the sub-item is load number loadBase + 2j (K) and loadBase + 2j + 1 (V); a load number L lives in
+// ring stage L % kStages and is the (L / kStages)-th fill of that stage.
+struct Walker : ShareWalker
 {
-    int32_t b, head, rowBase, rows, len, nb, tBegin, tEnd;
-};
-
-// The CTA's list of query tiles in processing order. Tile number n (counted per CTA) belongs to stream n & 1.
-// A "sub-item" is the run of tiles that shares one load of the K / V blocks: all tiles of a unit when its blocks fit
-// the ring, otherwise pairs of tiles (one per stream). `loadBase` is the number of K / V blocks loaded before it:
-// block j of the sub-item is load number loadBase + 2j (K) and loadBase + 2j + 1 (V); a load number L lives in ring
-// stage L % kStages and is the (L / kStages)-th fill of that stage.
-struct Walker
-{
-    OnlineArgs const* ap;
-    int32_t numUnits;
-    int32_t unit;
-    Unit g;
     int32_t t;        // query tile inside the (sequence, head)
     int32_t subEnd;   // one past the last tile of the sub-item
     int32_t subTiles; // tiles in the sub-item = uses of each of its stages
     uint32_t loadBase;
     uint32_t n;
-    // (row base, end) or mask length of the CTA's k-th unit for k < kGeoEntries, staged in shared memory by the kernel's
-    // prologue: a load from global memory at every change of unit (under streaming traffic often a DRAM access) would
-    // sit on the critical path of every role
-    int2 const* geo;
 
-    __device__ __forceinline__ Walker(OnlineArgs const& args, int2 const* geoTable)
-        : ap(&args)
-        , numUnits(args.B * args.N * args.chunks)
-        , geo(geoTable)
+    __device__ __forceinline__ Walker(OnlineArgs const& args, ShareSmem const* s)
+        : ShareWalker(args, s)
     {
-    }
-
-    __device__ __forceinline__ static void fetch(OnlineArgs const& a, int32_t u, int32_t& wa, int32_t& wb)
-    {
-        int32_t const b = (u / a.chunks) / a.N;
-        wa = 0;
-        wb = 0;
-        if (a.fixedLayout)
-        {
-            if (a.maskIdx)
-                wb = __ldg(a.maskIdx + b);
-        }
-        else
-        {
-            wa = __ldg(a.cu + b);
-            wb = __ldg(a.cu + b + 1);
-        }
-    }
-
-    // The CTA's k-th unit is unit number blockIdx.x + k * gridDim.x = (sequence cb, head ch, chunk cc). Going to the
-    // next one adds the launch's precomputed decomposition of gridDim.x (no division on the way).
-    int32_t k, cb, ch, cc;
-
-    __device__ __forceinline__ void firstUnit()
-    {
-        unit = static_cast<int32_t>(blockIdx.x);
-        k = 0;
-        cc = unit % ap->chunks;
-        int32_t const i = unit / ap->chunks;
-        cb = i / ap->N;
-        ch = i - cb * ap->N;
-    }
-
-    __device__ __forceinline__ void stepUnit()
-    {
-        unit += static_cast<int32_t>(gridDim.x);
-        ++k;
-        cc += ap->stepChunk;
-        if (cc >= ap->chunks)
-        {
-            cc -= ap->chunks;
-            ++ch;
-        }
-        ch += ap->stepHead;
-        if (ch >= ap->N)
-        {
-            ch -= ap->N;
-            ++cb;
-        }
-        cb += ap->stepB;
-    }
-
-    // geometry of the current unit; returns whether it has work for the tensor pipeline (a query row and a valid key)
-    __device__ __forceinline__ bool geometry(Unit& o) const
-    {
-        int32_t wa, wb;
-        if (k < kGeoEntries)
-        {
-            int2 const e = geo[k];
-            wa = e.x;
-            wb = e.y;
-        }
-        else
-            fetch(*ap, unit, wa, wb);
-        o.b = cb;
-        o.head = ch;
-        if (ap->fixedLayout)
-        {
-            o.rowBase = 0;
-            o.rows = ap->S;
-            o.len = ap->maskIdx ? min(max(wb, 0), ap->S) : ap->S;
-        }
-        else
-        {
-            o.rowBase = wa;
-            o.len = min(max(wb - wa, 0), ap->S);
-            o.rows = o.len;
-        }
-        o.nb = (o.len + kTile - 1) / kTile;
-        int32_t const nq = (o.rows + kTile - 1) / kTile;
-        o.tBegin = cc * ap->tilesPerUnit;
-        o.tEnd = min(nq, o.tBegin + ap->tilesPerUnit);
-        return o.len > 0 && o.tBegin < o.tEnd;
-    }
-
-    // settles on the current unit or the first one after it that has work
-    __device__ __forceinline__ bool seek()
-    {
-        while (unit < numUnits && !geometry(g))
-            stepUnit();
-        if (unit >= numUnits)
-            return false;
-        t = g.tBegin;
-        setSub();
-        return true;
     }
 
     __device__ __forceinline__ bool resident() const
@@ -271,7 +161,7 @@ struct Walker
 
     __device__ __forceinline__ void setSub()
     {
-        subTiles = resident() ? g.tEnd - t : min(2, g.tEnd - t);
+        subTiles = resident() ? runEnd - t : min(2, runEnd - t);
         subEnd = t + subTiles;
     }
 
@@ -279,8 +169,11 @@ struct Walker
     {
         n = 0;
         loadBase = 0;
-        firstUnit();
-        return seek();
+        if (!firstRun())
+            return false;
+        t = runBegin;
+        setSub();
+        return true;
     }
 
     __device__ __forceinline__ bool next()
@@ -290,10 +183,11 @@ struct Walker
         if (t == subEnd)
         {
             loadBase += 2u * static_cast<uint32_t>(g.nb);
-            if (t == g.tEnd)
+            if (t == runEnd)
             {
-                stepUnit();
-                return seek();
+                if (!nextRun())
+                    return false;
+                t = runBegin;
             }
             setSub();
         }
@@ -340,17 +234,17 @@ __global__ void __maxnreg__(168)
     uint8_t* sQ = smem + kSmemQ;
     uint8_t* sKv = smem + kSmemKv;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSmemBars);
-    uint64_t* full = bars;                    // [12] K / V block landed
-    uint64_t* empty = bars + kStages;         // [12] every MMA that reads the stage has completed
-    uint64_t* qFull = bars + 2 * kStages;     // [2]  Q tile of the stream landed
-    uint64_t* qFree = qFull + 2;              // [2]  all score MMAs of the stream's tile have completed
-    uint64_t* sFull = qFree + 2;              // [2]  scores of a key block complete               (once per block)
+    uint64_t* full = bars;                    // [kStages] K / V block landed
+    uint64_t* empty = bars + kStages;         // [kStages] every MMA that reads the stage has completed
+    uint64_t* qFull = bars + 2 * kStages;     // [kQSlots] Q tile landed
+    uint64_t* qFree = qFull + kQSlots;        // [kQSlots] all score MMAs of the slot's tile have completed
+    uint64_t* sFull = qFree + kQSlots;        // [2]  scores of a key block complete               (once per block)
     uint64_t* sFree = sFull + 2;              // [2]  scores are in registers, 4 arrivals           (once per block)
     uint64_t* pReady = sFree + 2;             // [2]  P block written, 4 arrivals                   (once per block)
     uint64_t* pvDone = pReady + 2;            // [2]  context product of a block complete           (once per block)
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(pvDone + 2);
     volatile uint32_t* abortFlag = tmemSlot + 1;
-    int2* geoTable = reinterpret_cast<int2*>(smem + kSmemGeo);
+    ShareSmem* share = reinterpret_cast<ShareSmem*>(smem + kSmemShare);
 
     if (threadIdx.x == 0)
     {
@@ -359,10 +253,13 @@ __global__ void __maxnreg__(168)
             mbarInit(&full[i], 1);
             mbarInit(&empty[i], 2); // one arrival per stream (see the MMA threads)
         }
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < kQSlots; ++i)
         {
             mbarInit(&qFull[i], 1);
             mbarInit(&qFree[i], 1);
+        }
+        for (int i = 0; i < 2; ++i)
+        {
             mbarInit(&sFull[i], 1);
             mbarInit(&sFree[i], 4); // one arrival per softmax warp of the stream
             mbarInit(&pReady[i], 4);
@@ -385,42 +282,32 @@ __global__ void __maxnreg__(168)
     uint32_t const tmemBase = *tmemSlot;
     gridDependencyLaunch();
     gridDependencyWait();
-    {
-        int32_t const numUnits = args.B * args.N * args.chunks;
-        int32_t const u = static_cast<int32_t>(blockIdx.x) + static_cast<int32_t>(threadIdx.x) * static_cast<int32_t>(gridDim.x);
-        if (threadIdx.x < kGeoEntries && u < numUnits)
-        {
-            int32_t wa, wb;
-            Walker::fetch(args, u, wa, wb);
-            geoTable[threadIdx.x] = make_int2(wa, wb);
-        }
-        __syncthreads();
-    }
+    bool const anyEmpty = findShare<kThreads, kTileCost>(args, share);
 
     // which: 0 = Q, 1 = K, 2 = V; row = first token of the box inside the (packed or per-sequence) tensor
-    auto load = [&](uint8_t* dst, uint64_t* bar, int which, Unit const& g, int32_t row) {
+    auto load = [&](uint8_t* dst, uint64_t* bar, int which, Walker const& w, int32_t row) {
         if (BNSD) // (channel, position, head, sequence)
-            tmaLoad4d(dst, which == 0 ? &mapQ : (which == 1 ? &mapK : &mapV), bar, 0, row, g.head, g.b);
+            tmaLoad4d(dst, which == 0 ? &mapQ : (which == 1 ? &mapK : &mapV), bar, 0, row, w.head, w.b);
         else // (channel, which of [N][3], batch, row)
-            tmaLoad4d(dst, &mapQ, bar, 0, g.head * 3 + which, args.fixedLayout ? g.b : 0, row);
+            tmaLoad4d(dst, &mapQ, bar, 0, w.head * 3 + which, args.fixedLayout() ? w.b : 0, row);
     };
 
     if (warp == 8)
     {
-        // ---- Q tiles: slot n & 1, refilled when the score MMAs of the stream's previous tile have completed ----
-        Walker w(args, geoTable);
+        // ---- Q tiles: slot n % kQSlots, refilled when the score MMAs of the tile before in it have completed ----
+        Walker w(args, share);
         bool ok = true;
         for (bool more = w.begin(); more && ok; more = w.next())
         {
-            uint32_t const slot = w.n & 1u;
-            if (w.n >= 2)
-                ok = mbarWaitWarp(smemAddr(&qFree[slot]), ((w.n >> 1) - 1) & 1u, abortFlag, kWaitStageFree);
+            uint32_t const slot = w.n % kQSlots;
+            if (w.n >= kQSlots)
+                ok = mbarWaitWarp(smemAddr(&qFree[slot]), (w.n / kQSlots - 1) & 1u, abortFlag, kWaitStageFree);
             if (!ok)
                 break;
             if (electOne())
             {
                 mbarArriveExpectTx(&qFull[slot], kStageBytes);
-                load(sQ + slot * kStageBytes, &qFull[slot], 0, w.g, (args.fixedLayout ? 0 : w.g.rowBase) + w.t * kTile);
+                load(sQ + slot * kStageBytes, &qFull[slot], 0, w, (args.fixedLayout() ? 0 : w.g.rowBase) + w.t * kTile);
             }
             __syncwarp();
         }
@@ -428,13 +315,13 @@ __global__ void __maxnreg__(168)
     else if (warp == 9)
     {
         // ---- K / V blocks of every sub-item, in the order the MMA threads consume them ----
-        Walker w(args, geoTable);
+        Walker w(args, share);
         bool ok = true;
         for (bool more = w.begin(); more && ok; more = w.next())
         {
             if (!w.firstOfSub())
                 continue;
-            int32_t const rowK = args.fixedLayout ? 0 : w.g.rowBase;
+            int32_t const rowK = args.fixedLayout() ? 0 : w.g.rowBase;
             for (int j = 0; j < w.g.nb && ok; ++j)
             {
                 for (int kv = 0; kv < 2 && ok; ++kv)
@@ -449,7 +336,7 @@ __global__ void __maxnreg__(168)
                     if (electOne())
                     {
                         mbarArriveExpectTx(&full[s], kStageBytes);
-                        load(sKv + s * kStageBytes, &full[s], 1 + kv, w.g, rowK + j * kTile);
+                        load(sKv + s * kStageBytes, &full[s], 1 + kv, w, rowK + j * kTile);
                     }
                     __syncwarp();
                 }
@@ -468,13 +355,13 @@ __global__ void __maxnreg__(168)
         uint64_t const dQk = makeSmemDesc(0, 16, 1024, kSwizzle128B);
         uint64_t const dV = makeSmemDesc(0, 1024, 1024, kSwizzle128B);
         uint32_t const hiQk = static_cast<uint32_t>(dQk >> 32), hiV = static_cast<uint32_t>(dV >> 32);
-        uint32_t const qLo = static_cast<uint32_t>(dQk) + (smemAddr(sQ) >> 4) + s * (kStageBytes >> 4);
+        uint32_t const qLo = static_cast<uint32_t>(dQk) + (smemAddr(sQ) >> 4);
         uint32_t const kLo = static_cast<uint32_t>(dQk) + (smemAddr(sKv) >> 4);
         uint32_t const vLo = static_cast<uint32_t>(dV) + (smemAddr(sKv) >> 4);
         constexpr uint32_t kStage16 = kStageBytes >> 4;
         uint32_t const fullAddr = smemAddr(full), emptyAddr = smemAddr(empty);
         uint32_t const sFullAddr = smemAddr(&sFull[s]), sFreeAddr = smemAddr(&sFree[s]), pReadyAddr = smemAddr(&pReady[s]);
-        uint32_t const pvDoneAddr = smemAddr(&pvDone[s]), qFullAddr = smemAddr(&qFull[s]), qFreeAddr = smemAddr(&qFree[s]);
+        uint32_t const pvDoneAddr = smemAddr(&pvDone[s]), qFullAddr = smemAddr(qFull), qFreeAddr = smemAddr(qFree);
         uint32_t const tS = tmemBase + s * kTile, tP = tmemBase + kPColumn + s * kHeadSize, tO = tmemBase + kOColumn + s * kHeadSize;
         bool ok = true;
         auto commitAddr = [](uint32_t barAddr) {
@@ -504,16 +391,16 @@ __global__ void __maxnreg__(168)
             if (!ok)
                 return;
             tcFenceAfter();
-            uint32_t const b = kLo + stage * kStage16;
+            uint32_t const b = kLo + stage * kStage16, slot = w.n % kQSlots, q = qLo + slot * kStage16;
             if (electOne())
             {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) // head size 64 = 4 x 16
-                    mmaLoHi<false>(tS, qLo + 2 * k, hiQk, b + 2 * k, hiQk, kIdescQk, k != 0);
+                    mmaLoHi<false>(tS, q + 2 * k, hiQk, b + 2 * k, hiQk, kIdescQk, k != 0);
                 commitAddr(sFullAddr);
                 release(stage, w);
                 if (j == w.g.nb - 1)
-                    commitAddr(qFreeAddr);
+                    commitAddr(qFreeAddr + 8 * slot);
             }
             __syncwarp();
         };
@@ -537,7 +424,7 @@ __global__ void __maxnreg__(168)
         };
 
         TR_DECL(2 + s);
-        Walker cur(args, geoTable);
+        Walker cur(args, share);
         bool active = cur.begin();
         if (s == 1 && active)
         {
@@ -549,7 +436,7 @@ __global__ void __maxnreg__(168)
         uint32_t qk = 0, pv = 0; // groups of score / context MMAs issued so far
         if (active && ok)
         {
-            ok = mbarWaitWarp(qFullAddr, (cur.n >> 1) & 1u, abortFlag, kWaitTmaFull);
+            ok = mbarWaitWarp(qFullAddr + 8 * (cur.n % kQSlots), (cur.n / kQSlots) & 1u, abortFlag, kWaitTmaFull);
             if (ok)
                 issueQk(cur, 0);
             qk = 1;
@@ -568,14 +455,14 @@ __global__ void __maxnreg__(168)
                 // stream's next tile - and the context product of block j. The scores go first, so that the tensor pipe
                 // has them done when the softmax threads come for them. Across a tile boundary the wait for their
                 // operands then holds back the product whose completion frees this tile's last V stage, and the loader
-                // works in load order: that is safe only while fewer than eleven loads lie between that V block and the
-                // next tile's first K block (none when the tiles share sub-items; the 2 nb loads of the other stream's
+                // works in load order: that is safe only while fewer than kStages - 1 loads lie between that V block and
+                // the next tile's first K block (none when the tiles share sub-items; the 2 nb loads of the other stream's
                 // tile when that is a sub-item of its own). With more, the loader would need the stage of that very V
                 // block first - a cycle - and the product goes first. (One call site each for the two MMA groups: the
                 // kernel is sensitive to the size of its code.)
                 bool const lastBlock = j + 1 == cur.g.nb;
                 bool qkPending = !lastBlock || hasNext, pvPending = true;
-                bool const qkFirst = !lastBlock || !midAlone || midBlocks <= 5;
+                bool const qkFirst = !lastBlock || !midAlone || midBlocks <= (kStages - 2) / 2;
                 bool midPending = lastBlock && midAlone;
                 if (qkPending)
                     ok = mbarWaitWarp(sFreeAddr, (qk - 1) & 1u, abortFlag, kWaitAccFree);
@@ -590,7 +477,7 @@ __global__ void __maxnreg__(168)
                             if (midPending)
                                 ok = passThroughLoads(fullAddr, emptyAddr, midFirst, midFirst + 2u * midBlocks, abortFlag);
                             midPending = false;
-                            ok = ok && mbarWaitWarp(qFullAddr, (nxt.n >> 1) & 1u, abortFlag, kWaitTmaFull);
+                            ok = ok && mbarWaitWarp(qFullAddr + 8 * (nxt.n % kQSlots), (nxt.n / kQSlots) & 1u, abortFlag, kWaitTmaFull);
                         }
                         if (ok)
                             issueQk(lastBlock ? nxt : cur, lastBlock ? 0 : j + 1);
@@ -630,31 +517,28 @@ __global__ void __maxnreg__(168)
         float const thrRaw = kRescaleLog2 / sl2; // the same threshold on the unscaled scores
         bool ok = true;
 
-        if (s == 0 && args.fixedLayout)
+        if (s == 0 && args.fixedLayout() && anyEmpty)
         {
             // sequences without a valid key: every probability is zero and so is the context row
-            Walker z(args, geoTable);
-            Unit g;
             int const chunks16 = args.d / 8;
-            for (z.firstUnit(); z.unit < z.numUnits; z.stepUnit())
+            for (int64_t u = blockIdx.x; u < static_cast<int64_t>(args.B) * args.N; u += gridDim.x)
             {
-                z.geometry(g);
-                if (g.len > 0 || g.tBegin >= g.tEnd)
+                int32_t const b = static_cast<int32_t>(u / args.N), head = static_cast<int32_t>(u % args.N);
+                if (makeSequence(args, fetchGeometry(args, b)).len > 0)
                     continue;
-                int const q0 = g.tBegin * kTile, q1 = min(g.rows, g.tEnd * kTile);
-                for (int i = threadIdx.x; i < (q1 - q0) * chunks16; i += kTile)
+                for (int i = threadIdx.x; i < args.S * chunks16; i += kTile)
                 {
-                    int const q = q0 + i / chunks16, c = i % chunks16;
+                    int const q = i / chunks16, c = i % chunks16;
                     __half* row = BNSD
-                        ? static_cast<__half*>(args.out) + ((static_cast<int64_t>(g.b) * args.N + g.head) * args.S + q) * args.d
-                        : static_cast<__half*>(args.out) + (static_cast<int64_t>(q) * args.B + g.b) * args.N * args.d + g.head * args.d;
+                        ? static_cast<__half*>(args.out) + ((static_cast<int64_t>(b) * args.N + head) * args.S + q) * args.d
+                        : static_cast<__half*>(args.out) + (static_cast<int64_t>(q) * args.B + b) * args.N * args.d + head * args.d;
                     reinterpret_cast<uint4*>(row)[c] = make_uint4(0, 0, 0, 0);
                 }
             }
         }
 
         TR_DECL(lane == 0 && (warp & 3) == 0 ? s : 7);
-        Walker w(args, geoTable);
+        Walker w(args, share);
         bool active = w.begin() && (s == 0 || w.next());
         uint32_t blocks = 0; // key blocks this stream has completed: parity of sFull / pvDone
         // the tile whose context still has to be normalised and stored (null: none, or a row beyond the sequence)
@@ -699,7 +583,7 @@ __global__ void __maxnreg__(168)
         };
         while (active)
         {
-            Unit const g = w.g;
+            Sequence const g = w.g;
             float mRun = -INFINITY, l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
 #pragma unroll 1
             for (int j = 0; j < g.nb; ++j)
@@ -834,11 +718,11 @@ __global__ void __maxnreg__(168)
             if (q < g.rows)
             {
                 if (BNSD)
-                    pendDst = static_cast<__half*>(args.out) + ((static_cast<int64_t>(g.b) * args.N + g.head) * args.S + q) * args.d;
+                    pendDst = static_cast<__half*>(args.out) + ((static_cast<int64_t>(w.b) * args.N + w.head) * args.S + q) * args.d;
                 else
                 {
-                    int64_t const rr = args.fixedLayout ? static_cast<int64_t>(q) * args.B + g.b : static_cast<int64_t>(g.rowBase) + q;
-                    pendDst = static_cast<__half*>(args.out) + rr * args.N * args.d + g.head * args.d;
+                    int64_t const rr = args.fixedLayout() ? static_cast<int64_t>(q) * args.B + w.b : static_cast<int64_t>(g.rowBase) + q;
+                    pendDst = static_cast<__half*>(args.out) + rr * args.N * args.d + w.head * args.d;
                 }
             }
             active = w.next() && w.next();
@@ -867,25 +751,6 @@ __global__ void __maxnreg__(168)
     }
 }
 
-// Query tiles per work unit: all tiles of a (sequence, head) share one load of K / V, so whole items are the
-// cheapest units; they are cut into smaller ones only when that shortens the longest CTA's list.
-int32_t chooseTilesPerUnit(int64_t items, int32_t nqMax, int32_t sms)
-{
-    int32_t best = nqMax;
-    int64_t bestCost = ((items + sms - 1) / sms) * nqMax;
-    for (int32_t tpu = nqMax - 1; tpu >= 1; --tpu)
-    {
-        int64_t const chunks = (nqMax + tpu - 1) / tpu;
-        int64_t const cost = ((items * chunks + sms - 1) / sms) * tpu;
-        if (cost < bestCost)
-        {
-            bestCost = cost;
-            best = tpu;
-        }
-    }
-    return best;
-}
-
 template <bool BNSD>
 int32_t launchOnline(CUtensorMap const (&maps)[3], OnlineArgs args, cudaStream_t stream)
 {
@@ -893,17 +758,7 @@ int32_t launchOnline(CUtensorMap const (&maps)[3], OnlineArgs args, cudaStream_t
     cudaError_t const e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mha: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    int32_t const nqMax = (args.S + kTile - 1) / kTile;
-    int64_t const items = static_cast<int64_t>(args.B) * args.N;
-    args.tilesPerUnit = chooseTilesPerUnit(items, nqMax, smCount());
-    args.chunks = (nqMax + args.tilesPerUnit - 1) / args.tilesPerUnit;
-    int64_t const units = items * args.chunks;
-    if (units > INT32_MAX)
-        B200_FAIL(BERT_B200_NOT_SUPPORTED, "mha: too many work units (%lld)", static_cast<long long>(units));
-    int const grid = static_cast<int>(units < smCount() ? units : smCount());
-    args.stepChunk = grid % args.chunks;
-    args.stepHead = (grid / args.chunks) % args.N;
-    args.stepB = (grid / args.chunks) / args.N;
+    int const grid = shareGrid(args);
     cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, maps[0], maps[1], maps[2], args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaOnlineF16Kernel: %s", cudaGetErrorString(le));
@@ -930,8 +785,7 @@ int32_t mhaOnlineF16(bert_b200_mha_params const& p, cudaStream_t stream)
         return st;
     maps[1] = maps[0];
     maps[2] = maps[0];
-    OnlineArgs const args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx,
-        p.scale_bmm1, p.status_word, 1, 1, 0, 0, 0};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, p.cu_seqlens, p.mask_idx), p.head_size, p.out, p.scale_bmm1, p.status_word};
     return launchOnline<false>(maps, args, stream);
 }
 
@@ -951,7 +805,7 @@ int32_t mhaOnlineF16Bnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t 
         if (st != BERT_B200_OK)
             return st;
     }
-    OnlineArgs const args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.status_word, 1, 1, 0, 0, 0};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, nullptr, p.kv_lengths), p.head_size, p.out, p.scale_bmm1, p.status_word};
     return launchOnline<true>(maps, args, stream);
 }
 

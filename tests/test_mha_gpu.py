@@ -492,3 +492,36 @@ def test_mha_fp16_many_long_ragged_sequences(cuda, seed, N, B, smax):
         ref = (torch.softmax(q @ k.transpose(-1, -2) * d ** -0.5, -1) @ v).transpose(0, 1)
         err = (o[lo:hi] - ref).abs()
         assert bool(((err <= 1e-2) | (err <= 1e-2 * ref.abs())).all()), float(err.max())
+
+
+# Batches around the limits of how the query tiles are divided over the CTAs: one sequence per lane of a warp (32), lengths
+# kept in shared memory (128), one sequence per thread (384 / 608), fewer tiles than SMs; empty sequences at both ends.
+@pytest.mark.parametrize("B,smax", [(2, 512), (32, 150), (33, 300), (128, 140), (129, 260), (700, 130)])
+@pytest.mark.parametrize("packed,int8", [(True, False), (False, False), (True, True), (False, True)])
+def test_mha_division_of_ragged_batches(cuda, B, smax, packed, int8):
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(B + smax)
+    N, d = 2, 32
+    lengths = rng.integers(0, smax + 1, size=B).astype(np.int32)
+    lengths[B // 2] = smax
+    lengths[[0, B - 1]] = 0 if B > 2 else (1, smax)
+    cu = O.cu_seqlens(lengths)
+    shape = (int(cu[-1]), 3 * N * d) if packed else (smax, B, 3 * N * d)
+    x = rng.standard_normal(shape)
+    where = {"cu": cu} if packed else {"lengths": lengths}
+    given = {"cu_seqlens": _t(cu, cuda)} if packed else {"mask_idx": _t(lengths, cuda)}
+    st = _status(cuda)
+    if int8:
+        q8 = np.clip(np.rint(x * (127.0 / 4.0)), -128, 127).astype(np.int8)
+        s1, s2 = float((4.0 / 127) ** 2 / np.sqrt(d)), 2.0 / 127
+        ref = O.mha_int8(q8, B, smax, N, d, s1, 127.0, s2, **where)
+        out = T.mha(_t(q8, cuda), B, smax, N, d, scale_bmm1=s1, scale_softmax=127.0, scale_bmm2=s2, status=st, **given)
+        _assert_int8_attention(out.cpu().numpy(), ref)
+    else:
+        qkv = x.astype(np.float16)
+        ref = O.mha(qkv, B, smax, N, d, **where)
+        out = T.mha(_t(qkv, cuda), B, smax, N, d, status=st, **given)
+        ok, worst, bad = O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-2, 1e-2)
+        assert ok, (worst, bad)
+    assert int(st[0]) == 0
