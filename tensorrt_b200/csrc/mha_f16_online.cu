@@ -34,7 +34,7 @@
 // context accumulator in TMEM themselves (after the previous P V product has completed). The final context is
 // O / rowsum. Compared with a softmax over the exact row maximum this changes nothing but the rounding of P.
 // Measured (16 heads of 64; whole pairs dealt round-robin and one Q slot per stream before): 11 sequences of 200 ... 2000
-// tokens 203 -> 122 us, 148 x 128 43.3 us, 148 x 384 167 us, 37 x 1024 271 us; bound by the exponentials (a 128 x 128 block takes 1024
+// tokens 203 -> 113 us, 148 x 128 43.0 us, 148 x 384 165 us, 37 x 1024 249 us; bound by the exponentials (a 128 x 128 block takes 1024
 // cycles of the unit) at half of their rate: the two streams' other work is not hidden behind them completely.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM and reports through the status word.
 #include "mha_share.cuh"
@@ -584,7 +584,8 @@ __global__ void __maxnreg__(168)
         while (active)
         {
             Sequence const g = w.g;
-            float mRun = -INFINITY, l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+            float mRun = -INFINITY;
+            uint64_t l01 = 0, l23 = 0; // row sums of every fourth key, two to a register pair
 #pragma unroll 1
             for (int j = 0; j < g.nb; ++j)
             {
@@ -643,10 +644,9 @@ __global__ void __maxnreg__(168)
                         float const f = move ? ex2Approx((mRun - mBlk) * sl2) : 1.f;
                         if (move)
                             mRun = mBlk;
-                        l0 *= f;
-                        l1 *= f;
-                        l2 *= f;
-                        l3 *= f;
+                        uint64_t const ff = pack2(f, f);
+                        l01 = mul2(l01, ff);
+                        l23 = mul2(l23, ff);
                         // the context so far, once the previous block's product has completed
                         ok = ok && mbarWait(&pvDone[s], (blocks - 1) & 1u, abortFlag, kWaitAccFull);
                         tcFenceAfter();
@@ -664,20 +664,22 @@ __global__ void __maxnreg__(168)
                     }
                 }
                 float const negM = -mRun * sl2;
+                uint64_t const scale2 = pack2(sl2, sl2), negM2 = pack2(negM, negM);
 
                 // p = exp2(x * scale * log2e - m), row sum, P as FP16 pairs (32 keys -> 16 columns)
                 auto expChunk = [&](uint32_t(&x)[32], uint32_t(&p)[16]) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 4)
                     {
-                        float const e0 = ex2Approx(fmaf(__uint_as_float(x[i]), sl2, negM));
-                        float const e1 = ex2Approx(fmaf(__uint_as_float(x[i + 1]), sl2, negM));
-                        float const e2 = ex2Approx(fmaf(__uint_as_float(x[i + 2]), sl2, negM));
-                        float const e3 = ex2Approx(fmaf(__uint_as_float(x[i + 3]), sl2, negM));
-                        l0 += e0;
-                        l1 += e1;
-                        l2 += e2;
-                        l3 += e3;
+                        float e0, e1, e2, e3;
+                        unpack2(fma2(pack2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), scale2, negM2), e0, e1);
+                        unpack2(fma2(pack2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), scale2, negM2), e2, e3);
+                        e0 = ex2Approx(e0);
+                        e1 = ex2Approx(e1);
+                        e2 = ex2Approx(e2);
+                        e3 = ex2Approx(e3);
+                        l01 = add2(l01, pack2(e0, e1));
+                        l23 = add2(l23, pack2(e2, e3));
                         p[i / 2] = packHalf2(e0, e1);
                         p[i / 2 + 1] = packHalf2(e2, e3);
                     }
@@ -713,6 +715,9 @@ __global__ void __maxnreg__(168)
             }
             int const q = w.t * kTile + r;
             pending = true;
+            float l0, l1, l2, l3;
+            unpack2(l01, l0, l1);
+            unpack2(l23, l2, l3);
             asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(pendInv) : "f"((l0 + l1) + (l2 + l3)));
             pendDst = nullptr;
             if (q < g.rows)

@@ -548,6 +548,36 @@ __device__ __forceinline__ uint64_t makeSmemDesc(uint32_t saddr, uint32_t lboByt
         | (static_cast<uint64_t>((sboBytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (swizzle << 61);
 }
 
+// Two FP32 operations in one issue slot (the pipes' rate is the same).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+
 // Instruction descriptor (32 bit) for kind::f16 / kind::i8, dense, no negate, no saturate.
 //   cFormat: 1 = F32, 2 = S32.  abFormat: kind::f16 -> 0 = F16, 1 = BF16; kind::i8 -> 1 = signed 8 bit.
 //   aMajor / bMajor: 0 = K-major, 1 = MN-major.
