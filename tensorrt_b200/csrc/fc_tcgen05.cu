@@ -6,7 +6,7 @@
 // Two kernels share the epilogue arithmetic:
 //   fcTcgen05PairKernel - persistent, a cluster of two CTAs per 256 x BLOCK_N tile (tcgen05.mma.cta_group::2), for problems with
 //                         enough tiles to keep the SM pairs busy;
-//   fcTcgen05TileKernel - one tile of 128 x BLOCK_N (16 ... 128) per CTA, two CTAs per SM, for few rows: the narrow tiles spread
+//   fcTcgen05TileKernel - one tile of 128 (64) x BLOCK_N (16 ... 128) per CTA, two CTAs per SM, for few rows: the narrow tiles spread
 //                         the weights over all SMs.
 // Warp roles in both: TMA producer (A and Wt tiles of 128-byte rows, 128-byte swizzle, into a shared-memory ring guarded by
 // full / empty mbarriers), MMA issuer (accumulators in TMEM; tcgen05.commit releases ring stages and publishes accumulators),
@@ -258,21 +258,23 @@ FcArgs makeFcArgs(bert_b200_fc_params const& p, int stages, int aRows, bool weig
 }
 
 // ------------------------------------------------------------------------------------------------
-// One 128 x BLOCK_N tile per CTA.
+// One BLOCK_M x BLOCK_N tile per CTA.
 //
 // With few rows a layer is bound by latency and by how fast the weights reach the SMs: one SM takes in about 100 bytes per
-// clock, so the weights of a projection have to be spread over as many SMs as possible - narrow tiles (their MMAs take 40
-// cycles each for any BLOCK_N up to 32). Everything around the main loop is kept short: a single tile per CTA, only BLOCK_N
+// clock, so the weights of a projection have to be spread over as many SMs as possible - narrow tiles. Their MMAs take 40 cycles
+// each for any BLOCK_N up to 32, about as long as 128 rows of A (32 bytes each) take to come from shared memory, and a long K is
+// a chain of them: up to 64 rows the tile has 64 rows. Everything around the main loop is kept short: a single tile per CTA, only BLOCK_N
 // TMEM columns and about 100 KB of shared memory, so that the CTAs of the next launch fit beside the running ones and have
 // their barriers, TMEM and - where the caller says that the weights are not being written by the kernels ahead - their first
 // weight tiles in place when this one ends. The other weight tiles are at least pulled into the L2 while the kernel ahead runs.
 //   warp 0: TMA producer, warp 1: TMEM allocation and MMA issue, then 4 epilogue warps (8 from BLOCK_N = 64 on), one or two
 //   per TMEM lane quadrant. Results go through the drained ring, so that a store instruction of a warp writes whole rows of
 //   its 32 x 32 block instead of 16 bytes of each of 32 rows.
-// Measured (weights from DRAM, back-to-back launches): FP16 37 x 768 x 768 in 3.2 us, 37 x 768 x 3072 in 7.2 us (18.5 us with
-// 128-wide tiles and 18 warps per CTA), 1024 x 768 x 768 in 4.8 us (pair kernel 6.7 us).
+// Measured (weights from DRAM, back-to-back launches): FP16 37 x 768 x 768 in 3.0 us, 37 x 768 x 3072 in 6.3 us (3.5 us and 7.8 us
+// with 128-row tiles; 18.5 us with 128 x 128 tiles and 18 warps per CTA), INT8 64 x 1024 x 4096 in 5.2 us (6.1 us), FP16 1024 x 768
+// x 768 in 4.8 us (pair kernel 6.7 us).
 // ------------------------------------------------------------------------------------------------
-template <int BLOCK_N>
+template <int BLOCK_M, int BLOCK_N>
 struct FcTileSmem
 {
     static constexpr int kEpiWarps = BLOCK_N >= 64 ? 8 : 4;
@@ -285,11 +287,11 @@ struct FcTileSmem
     // [bias][full, empty, accFull][tmem base, abort flag][ring]
     static constexpr int kBarrierOff = BLOCK_N * 4;
     static constexpr int kRingOff = (kBarrierOff + (2 * kMaxStages + 1) * 8 + 16 + 1023) / 1024 * 1024;
-    // The MMA always reads 128 rows of A: past the last A tile lie as many bytes as a full tile has more (what is read there
-    // only reaches accumulator rows beyond M).
+    // The MMA always reads BLOCK_M rows of A: past the last A tile lie as many bytes as a full tile has more (what is read
+    // there only reaches accumulator rows beyond M).
     static constexpr int bytes(int stages, int aRows)
     {
-        return kRingOff + stages * (kBBytes + kSub * aRows * kRowBytes) + (kBlockM - aRows) * kRowBytes + 1024; // 1024: alignment
+        return kRingOff + stages * (kBBytes + kSub * aRows * kRowBytes) + (BLOCK_M - aRows) * kRowBytes + 1024; // 1024: alignment
     }
     // As many stages as `budget` bytes hold or a tile has, at least 2 (which also hold the results of the epilogue warps).
     static int stagesFor(int aRows, int kSteps, int budget)
@@ -301,18 +303,20 @@ struct FcTileSmem
     }
 };
 
-template <typename In, int BLOCK_N, typename Out>
-__global__ void __launch_bounds__(FcTileSmem<BLOCK_N>::kThreads, 2)
+template <typename In, int BLOCK_M, int BLOCK_N, typename Out>
+__global__ void __launch_bounds__(FcTileSmem<BLOCK_M, BLOCK_N>::kThreads, 2)
     fcTcgen05TileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, FcArgs const args)
 {
-    using L = FcTileSmem<BLOCK_N>;
+    using L = FcTileSmem<BLOCK_M, BLOCK_N>;
+    // The accumulator of a 64-row MMA takes 16 lanes of each TMEM quadrant.
+    constexpr int kQuadRows = BLOCK_M / 4;
     constexpr bool kInt8 = sizeof(In) == 1;
     constexpr int kBlockK = kRowBytes / sizeof(In);
     constexpr int kUmmaKBytes = 32; // UMMA K = 16 halves or 32 bytes
     constexpr int kChunk = BLOCK_N < 32 ? BLOCK_N : 32;
     constexpr int kTmem = BLOCK_N < 32 ? 32 : BLOCK_N;
     constexpr uint32_t kIdesc
-        = makeInstrDesc(kInt8 ? 2u : 1u, kInt8 ? 1u : 0u, 0u, 0u, static_cast<uint32_t>(kBlockM), static_cast<uint32_t>(BLOCK_N));
+        = makeInstrDesc(kInt8 ? 2u : 1u, kInt8 ? 1u : 0u, 0u, 0u, static_cast<uint32_t>(BLOCK_M), static_cast<uint32_t>(BLOCK_N));
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(FcTileSmem<BLOCK_N>::kThreads, 2)
     int const stages = args.stages;
     int const tile = static_cast<int>(blockIdx.x);
     int const nBlocks = static_cast<int>((args.N + BLOCK_N - 1) / BLOCK_N);
-    int32_t const m0 = tile / nBlocks * kBlockM;
+    int32_t const m0 = tile / nBlocks * BLOCK_M;
     int32_t const n0 = tile % nBlocks * BLOCK_N;
     constexpr int kSub = L::kSub;
     constexpr int kStepK = kSub * kBlockK; // a step's k-blocks beyond K arrive as zeros
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(FcTileSmem<BLOCK_N>::kThreads, 2)
         asm volatile("bar.sync 1, %0;" ::"n"(L::kEpiWarps * 32) : "memory");
         bool const ok = mbarWaitWarp(accFull, 0, abortFlag, kWaitAccFull);
         tcFenceAfter();
-        int64_t const rowBase = static_cast<int64_t>(m0) + quad * 32;
+        int64_t const rowBase = static_cast<int64_t>(m0) + quad * kQuadRows;
         uint32_t const taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
         Out* const C = static_cast<Out*>(args.C);
         if (ok && rowBase < args.M) // warp-uniform
@@ -513,14 +517,15 @@ __global__ void __launch_bounds__(FcTileSmem<BLOCK_N>::kThreads, 2)
                     constexpr int kRow = kChunk * static_cast<int>(sizeof(Out));
                     constexpr int kPieces = kRow / 16;
                     uint8_t* const block = ring + (warp - 2) * 32 * (kRow + 16);
-                    storeChunk<kChunk>(reinterpret_cast<Out*>(block + lane * (kRow + 16)), v, q, kChunk);
+                    if (kQuadRows == 32 || lane < kQuadRows)
+                        storeChunk<kChunk>(reinterpret_cast<Out*>(block + lane * (kRow + 16)), v, q, kChunk);
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < kPieces; ++i)
                     {
                         int const rr = i * (32 / kPieces) + lane / kPieces;
                         int const piece = lane % kPieces;
-                        if (rowBase + rr < args.M && piece * (16 / static_cast<int>(sizeof(Out))) < validCols)
+                        if ((kQuadRows == 32 || rr < kQuadRows) && rowBase + rr < args.M && piece * (16 / static_cast<int>(sizeof(Out))) < validCols)
                             *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(C + (rowBase + rr) * args.ldc + col) + piece * 16)
                                 = *reinterpret_cast<uint4 const*>(block + rr * (kRow + 16) + piece * 16);
                     }
@@ -550,13 +555,13 @@ __global__ void __launch_bounds__(FcTileSmem<BLOCK_N>::kThreads, 2)
     }
 }
 
-template <typename In, int BLOCK_N, typename Out>
+template <typename In, int BLOCK_M, int BLOCK_N, typename Out>
 int32_t launchFcTile(bert_b200_fc_params const& p, bool weightsReady, cudaStream_t stream)
 {
-    using L = FcTileSmem<BLOCK_N>;
+    using L = FcTileSmem<BLOCK_M, BLOCK_N>;
     constexpr int kBlockK = kRowBytes / sizeof(In);
     CUtensorMapDataType const dt = sizeof(In) == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    int32_t const aRows = p.m < kBlockM ? static_cast<int32_t>((p.m + 7) / 8 * 8) : kBlockM; // no point in zero-filling all 128
+    int32_t const aRows = p.m < BLOCK_M ? static_cast<int32_t>((p.m + 7) / 8 * 8) : BLOCK_M; // no point in zero-filling the rest
     CUtensorMap mapA, mapB;
     {
         uint64_t const dims[2] = {static_cast<uint64_t>(p.k), static_cast<uint64_t>(p.m)};
@@ -574,11 +579,11 @@ int32_t launchFcTile(bert_b200_fc_params const& p, bool weightsReady, cudaStream
         if (st != BERT_B200_OK)
             return st;
     }
-    int64_t const tiles = ((p.m + kBlockM - 1) / kBlockM) * ((p.n + BLOCK_N - 1) / BLOCK_N);
+    int64_t const tiles = ((p.m + BLOCK_M - 1) / BLOCK_M) * ((p.n + BLOCK_N - 1) / BLOCK_N);
     // One CTA per SM may take a longer ring; otherwise two have to fit.
     int const kSteps = static_cast<int>((p.k + L::kSub * kBlockK - 1) / (L::kSub * kBlockK));
     int const stages = L::stagesFor(aRows, kSteps, tiles <= smCount() ? 200 * 1024 : 113 * 1024);
-    auto kernel = fcTcgen05TileKernel<In, BLOCK_N, Out>;
+    auto kernel = fcTcgen05TileKernel<In, BLOCK_M, BLOCK_N, Out>;
     static SmemOptIn optIn;
     FcArgs const args = makeFcArgs(p, stages, aRows, weightsReady);
     cudaError_t const e = launchDependentCluster(
@@ -1035,13 +1040,14 @@ int32_t fcRun(bert_b200_fc_params const& p, cudaStream_t s, bool weightsReady)
     int const outElem = p.out_type_id == BERT_B200_FP16 ? 2 : 1;
     B200_REQUIRE((p.ldc * outElem) % 16 == 0, "fc: row bytes of C must be a multiple of 16");
     FcPlan const plan = planFc(p);
+    bool const shortTile = p.m <= 64; // the narrow tiles also come with 64 rows (see the kernel)
 #define B200_FC_TILE(IN, OUT)                                                                                          \
     switch (plan.blockN)                                                                                               \
     {                                                                                                                  \
-    case 16: return launchFcTile<IN, 16, OUT>(p, weightsReady, s);                                         \
-    case 32: return launchFcTile<IN, 32, OUT>(p, weightsReady, s);                                         \
-    case 64: return launchFcTile<IN, 64, OUT>(p, weightsReady, s);                                         \
-    default: return launchFcTile<IN, 128, OUT>(p, weightsReady, s);                                        \
+    case 16: return shortTile ? launchFcTile<IN, 64, 16, OUT>(p, weightsReady, s) : launchFcTile<IN, 128, 16, OUT>(p, weightsReady, s); \
+    case 32: return shortTile ? launchFcTile<IN, 64, 32, OUT>(p, weightsReady, s) : launchFcTile<IN, 128, 32, OUT>(p, weightsReady, s); \
+    case 64: return launchFcTile<IN, 128, 64, OUT>(p, weightsReady, s);                                                \
+    default: return launchFcTile<IN, 128, 128, OUT>(p, weightsReady, s);                                               \
     }
 #define B200_FC_DISPATCH(IN, OUT)                                                                                      \
     if (plan.pair)                                                                                                     \

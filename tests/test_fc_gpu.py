@@ -138,6 +138,13 @@ def test_fc_tile_edges(cuda, m, k, n, int8):
     assert int(st[0]) == 0
 
 
+# up to 64 rows the narrow tiles have 64: edges of the 16 rows a warp stores, of the tile, and n at the widest such tile
+@pytest.mark.parametrize("m,k,n", [(15, 80, 16), (17, 1040, 144), (48, 3088, 2368), (63, 768, 4736), (64, 4096, 1024), (65, 768, 48)])
+@pytest.mark.parametrize("int8", [False, True])
+def test_fc_64_row_tiles(cuda, m, k, n, int8):
+    test_fc_tile_edges(cuda, m, k, n, int8)
+
+
 # tile and k-block edges of the FP32 kernel: one row, single column past a 64-wide tile, K below and above a k-block, K and
 # strides that are no multiple of four (element copies), shapes that divide K over a cluster (odd shares included)
 @pytest.mark.parametrize("m,k,n", [(1, 4, 1), (65, 20, 67), (64, 7, 64), (33, 1001, 130), (38, 3072, 768), (200, 784, 96), (1024, 768, 768)])
