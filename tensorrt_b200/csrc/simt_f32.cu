@@ -27,14 +27,16 @@ __device__ __forceinline__ float geluErf(float x)
 //
 // Bound by the FP32 FMA pipes (128 per clock and SM). A CTA of two warps computes a 64 x 64 tile, every thread 8 x 8
 // outputs, four CTAs per SM. Both operands are K-contiguous, so they are copied to shared memory as they lie (16-byte
-// cp.async, four stages) and read back as 16-byte pieces along K; rows are padded to 20 floats, which puts the 4 or 8 rows
-// that a warp reads at once into different banks. The sums run on packed fma.rn.f32x2: one half takes the even k, the
+// cp.async, four stages) and read back as 8-byte pieces along K, those of the next two k during the FMAs of these (16-byte
+// pieces left no registers for that: 3 % slower); rows are padded to 20 floats, which puts the 4 or 8 rows that a warp reads
+// at once into different banks. The sums run on packed fma.rn.f32x2: one half takes the even k, the
 // other the odd ones (no operand has to be duplicated), and the two are added at the end; a packed FMA takes half the
-// issue slots, which leaves room for the 16 shared-memory loads that go with 128 of them.
+// issue slots, which leaves room for the loads. These bring 64 bytes per thread and k pair to the registers, at 128 bytes per
+// clock and SM as long as the FMAs take: the loop runs at 0.6 of the FMA rate.
 // A cluster of `split` CTAs divides the K range of a tile where the tiles alone leave SMs idle or fill the last wave badly;
 // its CTAs exchange partial sums through distributed shared memory, each finishing every split-th row.
-// Measured: 1024 x 2304 x 768 in 106 us (34 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x
-// 3072 in 130 us (700 us).
+// Measured: 1024 x 2304 x 768 in 96 us (38 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x
+// 3072 in 141 us (700 us).
 constexpr int kTile = 64;
 constexpr int kTileK = 16;
 constexpr int kPitch = kTileK + 4; // floats
@@ -153,26 +155,28 @@ __global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(Fc
         cpAsyncCommit();
         float const(*const a)[kPitch] = sm[stage][0];
         float const(*const b)[kPitch] = sm[stage][1];
-#pragma unroll
-        for (int k = 0; k < kTileK; k += 4)
-        {
-            ulonglong2 av[8], bv[8];
+        // two k at a time; the next two are on their way from shared memory during the FMAs of these
+        uint64_t av[2][8], bv[2][8];
+        auto fetch = [&](int buf, int k) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                av[i] = *reinterpret_cast<ulonglong2 const*>(&a[row0 + 4 * i][k]);
+                av[buf][i] = *reinterpret_cast<uint64_t const*>(&a[row0 + 4 * i][k]);
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                bv[j] = *reinterpret_cast<ulonglong2 const*>(&b[tx + 8 * j][k]);
+                bv[buf][j] = *reinterpret_cast<uint64_t const*>(&b[tx + 8 * j][k]);
+        };
+        fetch(0, 0);
+#pragma unroll
+        for (int k = 0; k < kTileK; k += 2)
+        {
+            int const cur = (k >> 1) & 1;
+            if (k + 2 < kTileK)
+                fetch(cur ^ 1, k + 2);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    fma2(acc[i][j], av[i].x, bv[j].x);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    fma2(acc[i][j], av[i].y, bv[j].y);
+                    fma2(acc[i][j], av[cur][i], bv[cur][j]);
         }
         stage = stage + 1 == kStages ? 0 : stage + 1;
     }
@@ -504,29 +508,22 @@ __global__ void __launch_bounds__(128) mhaSimtKernel(int32_t const B, int32_t co
 
 } // namespace
 
-// CTAs per tile. A k-block of a tile is 64 x 64 x 16 multiply-adds: 0.5 us on the FMA pipes of half an SM, all that one
-// CTA can use, and twice that once four share an SM. A CTA costs about 1.5 us besides (first loads, result), the exchange
-// of partial sums another 1.5 us.
+// CTAs per tile: the smallest of 1, 2, 4, 8 that gives the SMs nearly all the CTAs that fit at once; with a long K (2048 and more
+// per CTA) twice as many, so that the last ones do not run alone for long. Other cluster sizes leave SMs idle (clusters of three:
+// some SMs none, others four); fewer CTAs leave FMA pipes idle, more exchange partial sums for nothing. Measured with 1 / 2 / 4 / 8
+// per tile: 1024 x 768 x 3072 (192 tiles) 273 / 183 / 141 / 147 us (three: 184), 1024 x 3072 x 768 (768 tiles) 139 / 149 / 151 us,
+// 128 x 768 x 3072 (24 tiles) 182 / 100 / 52 / 44 us, 4096 x 1024 x 4096 (1024 tiles) 890 / 780 us.
 static int pickSplitF32(int64_t tiles, int64_t kBlocks)
 {
-    int64_t const sms = smCount();
-    int64_t const slots = sms * kFcF32CtasPerSm;
-    int best = 1;
-    double bestCost = 0.0;
-    for (int s = 1; s <= 8 && s <= kBlocks; ++s)
+    int split = 1;
+    while (split < 8 && 2 * split <= kBlocks)
     {
-        int64_t const ctas = tiles * s;
-        int64_t const waves = (ctas + slots - 1) / slots;
-        int64_t const perSm = waves > 1 ? kFcF32CtasPerSm : (ctas + sms - 1) / sms;
-        double const block = perSm <= 2 ? 0.53 : 0.265 * static_cast<double>(perSm);
-        double const cost = static_cast<double>(waves) * (static_cast<double>((kBlocks + s - 1) / s) * block + 1.5) + (s > 1 ? 1.5 : 0.0);
-        if (s == 1 || cost < bestCost)
-        {
-            best = s;
-            bestCost = cost;
-        }
+        int64_t const enough = kBlocks / split >= 2048 / kTileK ? 8 * smCount() : 17 * smCount() / 5;
+        if (tiles * split >= enough)
+            break;
+        split *= 2;
     }
-    return best;
+    return split;
 }
 
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
