@@ -10,9 +10,9 @@
 // sum before the first of them can be formed, so the whole score row lives in TMEM (<= 512 keys) and the softmax makes
 // three sweeps over it; that is what keeps the result bit-identical with the reference's INT8 kernels.
 //
-// Persistent CTAs (one per SM) take (sequence, head) work items round-robin. Per item a CTA loops over the 128-query
-// tiles of the sequence, so that K and V are loaded once and the tensor pipe works on the next tile (of this item or
-// the next) while the softmax warps finish the current one. 19 warps:
+// Persistent CTAs (one per SM) take (sequence, head) work items, or parts of them where there are few, round-robin. Per
+// item a CTA loops over its 128-query tiles, so that K and V are loaded once and the tensor pipe works on the next tile
+// (of this item or the next) while the softmax warps finish the current one. 19 warps:
 //   warp 0    : TMA - the K / V blocks (128 keys each) of an item once, the Q tile of each iteration
 //               (swizzled shared-memory tiles, one mbarrier each).
 //   warp 1    : TMEM allocation (512 columns); one lane issues the context products
@@ -67,6 +67,7 @@ struct MhaArgs
     int32_t const* maskIdx;
     float scaleBmm1, scaleSoftmax, scaleBmm2;
     uint32_t* statusWord;
+    int32_t tilesPerItem, chunks; // a work item = (sequence, head, chunk of tilesPerItem query tiles)
 };
 
 template <typename T>
@@ -189,17 +190,20 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     int const warp = threadIdx.x >> 5;
     int const lane = threadIdx.x & 31;
 
-    // ---- work items: one (sequence, head) each, item = b * N + head, dealt round-robin to the persistent CTAs ----
+    // ---- work items: some or all query tiles of a (sequence, head), item = (b * N + head) * chunks + chunk, dealt round-robin
+    //      to the persistent CTAs ----
     struct Item
     {
-        int32_t b, head, rowBase, rows, len, nb, nq;
+        int32_t b, head, rowBase, rows, len, nb, tBegin, tEnd;
     };
-    int const numItems = args.B * args.N;
+    int const numItems = args.B * args.N * args.chunks;
     // Geometry of item i (uniform over the CTA; every role derives the same values). Returns whether the item has
     // work for the tensor pipeline (at least one query row and one valid key).
     auto getItem = [&](int i, Item& it) -> bool {
-        it.b = i / args.N;
-        it.head = i - it.b * args.N;
+        int const pair = i / args.chunks;
+        it.b = pair / args.N;
+        it.head = pair - it.b * args.N;
+        it.tBegin = (i - pair * args.chunks) * args.tilesPerItem;
         if (args.fixedLayout)
         {
             it.rowBase = 0;
@@ -213,8 +217,8 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             it.rows = it.len;
         }
         it.nb = (it.len + kKeyBlock - 1) / kKeyBlock; // key blocks
-        it.nq = (it.rows + kQTile - 1) / kQTile;      // query tiles
-        return it.rows > 0 && it.len > 0;
+        it.tEnd = min((it.rows + kQTile - 1) / kQTile, it.tBegin + args.tilesPerItem);
+        return it.len > 0 && it.tBegin < it.tEnd;
     };
     // first item >= i of this CTA's sequence that has pipeline work; numItems or more if there is none
     auto nextWork = [&](int i, Item& it) -> int {
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 else
                     tmaLoad4d(dst, &mapQkv, bar, 0, it.head * 3 + which, args.fixedLayout ? it.b : 0, row);
             };
-            for (int t = 0; t < it.nq && ok; ++t)
+            for (int t = it.tBegin; t < it.tEnd && ok; ++t)
             {
                 // the score MMAs of the previous tile have read Q (and, across items, K)
                 if (tiles > 0)
@@ -324,7 +328,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     load(sQ, qFull, 0, rowK + t * kQTile);
                 }
                 __syncwarp();
-                if (t == 0)
+                if (t == it.tBegin)
                 {
                     for (int j = 0; j < it.nb; ++j)
                     {
@@ -436,9 +440,9 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 // only the scores look one item ahead (its geometry comes from global memory: not in the way of a
                 // warp that only issues context products)
                 int const nextItem = kDoScores ? nextWork(item + gridDim.x, nxt) : numItems;
-                for (int t = 0; t < cur.nq && ok; ++t)
+                for (int t = cur.tBegin; t < cur.tEnd && ok; ++t)
                 {
-                    bool const lastT = t + 1 == cur.nq;
+                    bool const lastT = t + 1 == cur.tEnd;
                     // the scores issued while this tile's context is formed: the item's next tile, or the first tile
                     // of the CTA's next item (whose K then has to have landed), or none
                     int const nbFollow = !lastT ? cur.nb : (nextItem < numItems ? nxt.nb : 0);
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                             fBits ^= 1u << j; // the softmax warps complete this phase in every tile that uses block j
                             if (kDoContext)
                             {
-                                if (ok && t == 0)
+                                if (ok && t == cur.tBegin)
                                 {
                                     ok = mbarWaitWarp(&vFull[j], (vBits >> j) & 1u, abortFlag, kWaitTmaFull);
                                     vBits ^= 1u << j;
@@ -666,9 +670,10 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             {
                 // no valid key: every probability is zero and so is the context row
                 int const kChunks = args.d * L::kElem / 16;
-                for (int i = threadIdx.x - 64; i < it.rows * kChunks; i += kSoftmaxThreads)
+                int const q0 = it.tBegin * kQTile, q1 = min(it.rows, it.tEnd * kQTile);
+                for (int i = threadIdx.x - 64; i < (q1 - q0) * kChunks; i += kSoftmaxThreads)
                 {
-                    int const q = i / kChunks;
+                    int const q = q0 + i / kChunks;
                     int const c = i % kChunks;
                     if (IL)
                         reinterpret_cast<uint4*>(outPtrIl(q, c / 2))[c % 2] = make_uint4(0, 0, 0, 0);
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             }
             int const nb = it.nb;
             int const len = it.len;
-            for (int t = 0; t < it.nq; ++t)
+            for (int t = it.tBegin; t < it.tEnd; ++t)
             {
                 uint32_t x[32];
 
@@ -898,6 +903,30 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     }
 }
 
+// Query tiles per work item, and the number of CTAs. All tiles of a (sequence, head) share one load of K and V, which an item
+// waits for at about a third of a tile's time; items are cut smaller only when that shortens the longest CTA's list, that is
+// when there are few of them. Measured (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
+// us), 4 x 256 6.5 us (10.2 us), 12 x 384 22.5 us (31.8 us); 8 x 384 whole, 16.7 us.
+int divideItems(MhaArgs& args)
+{
+    int64_t const pairs = static_cast<int64_t>(args.B) * args.N;
+    int32_t const nq = (args.S + kQTile - 1) / kQTile;
+    int64_t best = 0;
+    for (int32_t tiles = nq; tiles >= 1; --tiles)
+    {
+        int32_t const chunks = (nq + tiles - 1) / tiles;
+        int64_t const cost = (pairs * chunks + smCount() - 1) / smCount() * (3 * tiles + 1);
+        if (tiles == nq || (cost < best && pairs * chunks <= INT32_MAX))
+        {
+            best = cost;
+            args.tilesPerItem = tiles;
+            args.chunks = chunks;
+        }
+    }
+    int64_t const items = pairs * args.chunks;
+    return static_cast<int>(items < smCount() ? items : smCount());
+}
+
 template <typename T, bool IL>
 int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
 {
@@ -940,10 +969,9 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mha: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
-        p.scale_softmax, p.scale_bmm2, p.status_word};
+        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1};
     // one persistent CTA per SM (512 TMEM columns and most of the shared memory each), items dealt round-robin
-    int64_t const items = static_cast<int64_t>(p.num_heads) * p.B;
-    int const grid = static_cast<int>(items < smCount() ? items : smCount());
+    int const grid = divideItems(args);
     cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kMhaThreads), smem, stream, map, map, map, args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
@@ -977,9 +1005,8 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "attention_bnsd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
-        p.scale_bmm2, p.status_word};
-    int64_t const items = static_cast<int64_t>(p.num_heads) * p.B;
-    int const grid = static_cast<int>(items < smCount() ? items : smCount());
+        p.scale_bmm2, p.status_word, 1, 1};
+    int const grid = divideItems(args);
     cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kMhaThreads), smem, stream, maps[0], maps[1], maps[2], args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
