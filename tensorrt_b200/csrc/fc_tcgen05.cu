@@ -608,7 +608,7 @@ struct FcPairSmem
     static constexpr int kABytes = kBlockM * kRowBytes;            // this CTA's 128 rows of A
     static constexpr int kBBytes = (BLOCK_N / 2) * kRowBytes;      // this CTA's half of the Wt rows
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kStages = BLOCK_N == 256 ? 6 : 8;
+    static constexpr int kStages = BLOCK_N == 128 ? 8 : (BLOCK_N == 160 ? 7 : 6);
     static constexpr int kOutOff = kStages * kStageBytes;          // epilogue staging: kOutWarpBytes per epilogue warp
     static constexpr int kOutWarpBytes = 2048;                     // one FP16 or two INT8 [32 x 32] chunks
     static constexpr int kBarrierOff = kOutOff + kEpilogueWarps * kOutWarpBytes;
@@ -807,7 +807,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFcThreads, 1)
     {
         int const quad = warp & 3;
         int const part = (warp - 2) >> 2;
-        constexpr int kChunksPerWarp = BLOCK_N / 32 / (kEpilogueWarps / 4);
+        constexpr int kChunks = BLOCK_N / 32;
+        constexpr int kChunksPerWarp = (kChunks + kEpilogueWarps / 4 - 1) / (kEpilogueWarps / 4); // one less in some warps
         constexpr int kChunkBytes = 32 * 32 * static_cast<int>(sizeof(Out));
         constexpr int kBufs = L::kOutWarpBytes / kChunkBytes; // staging tiles of this warp: 2 (INT8) or 1 (FP16)
         uint8_t* const stage0 = smem + L::kOutOff + (warp - 2) * L::kOutWarpBytes;
@@ -826,10 +827,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFcThreads, 1)
             for (int i = 0; i < kChunksPerWarp; ++i) // this warp's 32-column chunks of the tile
             {
                 int const c = part + i * (kEpilogueWarps / 4);
+                if (kChunks % (kEpilogueWarps / 4) != 0 && c >= kChunks)
+                    break;
                 uint32_t r[32];
                 tmemLoad32(taddr + c * 32, r);
                 tmemLoadWait32(r);
-                if (i == kChunksPerWarp - 1)
+                if (c + kEpilogueWarps / 4 >= kChunks)
                 {
                     // The accumulator is in registers: hand the TMEM buffer back before the arithmetic and the store.
                     tcFenceBefore();
@@ -933,19 +936,28 @@ int32_t launchFcPair(bert_b200_fc_params const& p, cudaStream_t stream)
     return checkLaunch("fcTcgen05PairKernel");
 }
 
-// 256 x BLOCK_N pair tiles over the SM pairs: pick the BLOCK_N that wastes less of the last wave.
+// 256 x BLOCK_N pair tiles over the SM pairs: the width that wastes least of the last wave. A launch takes about as long as
+// waves * (BLOCK_N + 110) + BLOCK_N / 2 columns of a 256-row tile: 110 for what does not grow with the width (A, hand-overs,
+// epilogues of the odd widths), the last term for filling and draining the pipeline. Measured with 128 / 160 / 192 / 224 / 256
+// columns: FP16 2600 x 1024 x 4096 28.8 / 33.6 / 24.2 / 26.8 / 29.5 us, 5001 x 1024 x 4096 40.5 / 36.5 / 39.7 / 43.4 / 48.0 us,
+// 5001 x 4096 x 1024 40.0 / 37.6 / 35.2 / 37.3 / 35.4 us, INT8 5001 x 3072 x 1024 21.7 / 22.8 / 21.0 / 19.1 / 19.7 us,
+// 24576 x 1024 x 4096 77 / 78 / 76 / 75 / 71 us.
 int pickBlockNPair(int64_t m, int64_t n)
 {
-    if (n <= 128)
-        return 128;
-    int const pairs = smCount() / 2;
-    auto cost = [&](int bn) {
+    int64_t const pairs = smCount() / 2;
+    int best = 128;
+    int64_t bestCost = 0;
+    for (int bn = 128; bn <= 256 && (bn == 128 || bn - 32 < n); bn += 32)
+    {
         int64_t const tiles = ((m + 2 * kBlockM - 1) / (2 * kBlockM)) * ((n + bn - 1) / bn);
-        int64_t const waves = (tiles + pairs - 1) / pairs;
-        // measured: 256 x 128 pair tiles run at about nine tenths of the rate of 256 x 256 tiles
-        return static_cast<double>(waves) * bn * (bn == 128 ? 1.1 : 1.0);
-    };
-    return cost(128) < cost(256) ? 128 : 256;
+        int64_t const cost = (tiles + pairs - 1) / pairs * (bn + 110) + bn / 2;
+        if (bn == 128 || cost < bestCost)
+        {
+            best = bn;
+            bestCost = cost;
+        }
+    }
+    return best;
 }
 
 struct FcPlan
@@ -955,16 +967,18 @@ struct FcPlan
 };
 
 // Single tiles per CTA as long as they all run at once: the narrowest whose tiles do not outnumber the SMs (more SMs take part
-// in loading the weights, shorter epilogue), 128-wide ones also at two CTAs per SM. Beyond, the persistent pair tiles are ahead:
-// their epilogues overlap the next tile's main loop. Measured at the borders, FP16, K = 768: 192 tiles 9.0 us against 10.5 us
-// in pairs, 288 tiles 8.7 / 9.9 us, 450 tiles 15.4 / 13.8 us; 64-wide at two CTAs per SM (288 tiles) 6.6 us against 6.2 us
-// with 144 128-wide ones.
+// in loading the weights, shorter epilogue), with a short K 128-wide ones also at two CTAs per SM. Beyond, the persistent pair
+// tiles are ahead: their epilogues overlap the next tile's main loop, and they load a third less per product. Measured at the
+// borders, FP16: K = 768, 192 tiles 9.0 us against 10.5 us in pairs, 288 tiles 8.7 / 9.9 us, 450 tiles 15.4 / 13.8 us; 64-wide at
+// two CTAs per SM (288 tiles) 6.6 us against 6.2 us with 144 128-wide ones. 4096 x 1024 (256 tiles), K = 1024 11.9 / 12.2 us, K =
+// 4096 31.6 / 29.1 us; INT8 3100 x 768 (150 tiles), K = 768 7.6 / 7.6 us, K = 3072 14.5 / 12.2 us.
 FcPlan planFc(bert_b200_fc_params const& p)
 {
     int64_t const sms = smCount();
     int64_t const mBlocks = (p.m + kBlockM - 1) / kBlockM;
+    bool const shortK = p.k * (p.type_id == BERT_B200_FP16 ? 2 : 1) < 3072;
     for (int bn = 16; bn <= 128; bn *= 2)
-        if (mBlocks * ((p.n + bn - 1) / bn) <= (bn == 128 ? 2 * sms : sms))
+        if (mBlocks * ((p.n + bn - 1) / bn) <= (bn == 128 && shortK ? 2 * sms : sms))
             return {false, bn};
     if (p.m <= kBlockM) // the second CTA of a pair would have no rows
         return {false, 128};
@@ -1051,7 +1065,14 @@ int32_t fcRun(bert_b200_fc_params const& p, cudaStream_t s, bool weightsReady)
     }
 #define B200_FC_DISPATCH(IN, OUT)                                                                                      \
     if (plan.pair)                                                                                                     \
-        return plan.blockN == 128 ? launchFcPair<IN, 128, OUT>(p, s) : launchFcPair<IN, 256, OUT>(p, s);               \
+        switch (plan.blockN)                                                                                           \
+        {                                                                                                              \
+        case 128: return launchFcPair<IN, 128, OUT>(p, s);                                                             \
+        case 160: return launchFcPair<IN, 160, OUT>(p, s);                                                             \
+        case 192: return launchFcPair<IN, 192, OUT>(p, s);                                                             \
+        case 224: return launchFcPair<IN, 224, OUT>(p, s);                                                             \
+        default: return launchFcPair<IN, 256, OUT>(p, s);                                                              \
+        }                                                                                                              \
     B200_FC_TILE(IN, OUT)
     if (p.type_id == BERT_B200_FP16)
     {

@@ -145,6 +145,14 @@ def test_fc_64_row_tiles(cuda, m, k, n, int8):
     test_fc_tile_edges(cuda, m, k, n, int8)
 
 
+# pair tiles of 160, 192 and 224 columns (an uneven number of column chunks per epilogue warp): last tiles with few columns, an
+# odd number of row blocks, one and several tiles per pair of CTAs
+@pytest.mark.parametrize("m,k,n", [(2600, 3088, 2000), (2600, 3088, 1040), (3100, 3088, 1072), (2305, 208, 3072)])
+@pytest.mark.parametrize("int8", [False, True])
+def test_fc_pair_tile_widths(cuda, m, k, n, int8):
+    test_fc_tile_edges(cuda, m, k, n, int8)
+
+
 # tile and k-block edges of the FP32 kernel: one row, single column past a 64-wide tile, K below and above a k-block, K and
 # strides that are no multiple of four (element copies), shapes that divide K over a cluster (odd shares included)
 @pytest.mark.parametrize("m,k,n", [(1, 4, 1), (65, 20, 67), (64, 7, 64), (33, 1001, 130), (38, 3072, 768), (200, 784, 96), (1024, 768, 768)])
