@@ -154,6 +154,11 @@ __device__ __forceinline__ void gridDependencyWait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+__device__ __forceinline__ void prefetchL2(void const* p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // All threads of the cluster arrive; shared-memory writes made before are visible to every CTA of it afterwards.
 __device__ __forceinline__ void clusterBarrier()
 {
