@@ -525,3 +525,24 @@ def test_mha_division_of_ragged_batches(cuda, B, smax, packed, int8):
         ok, worst, bad = O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-2, 1e-2)
         assert ok, (worst, bad)
     assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("d", [16, 48, 64])
+@pytest.mark.parametrize("lengths", [[37], [1, 16, 17, 32, 33, 0, 64, 65, 96, 97, 127, 128], [5] * 150])
+def test_mha_fp16_single_key_block(cuda, d, lengths):
+    """Launches of sequences up to 128 tokens have a kernel of their own: edges of its 16- and 32-key steps against the oracle,
+    and the same bits as the general kernel, which takes over when longer sequences are announced."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(d + len(lengths))
+    N, lengths = 3, np.array(lengths, np.int32)
+    cu = O.cu_seqlens(lengths)
+    B, S = len(lengths), int(lengths.max())
+    qkv = rng.standard_normal((int(cu[-1]), 3 * N * d)).astype(np.float16)
+    st = _status(cuda)
+    out = T.mha(_t(qkv, cuda), B, S, N, d, cu_seqlens=_t(cu, cuda), status=st)
+    general = T.mha(_t(qkv, cuda), B, 129, N, d, cu_seqlens=_t(cu, cuda), status=st)
+    assert int(st[0]) == 0
+    ok, worst, bad = O.close_abs_or_rel(out.cpu().numpy(), O.mha(qkv, B, S, N, d, cu=cu), 1e-2, 1e-2)
+    assert ok, (worst, bad)
+    assert torch.equal(out, general)
