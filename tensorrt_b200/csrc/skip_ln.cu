@@ -100,9 +100,9 @@ struct Vec<float>
 };
 
 // Asks for the parameters to be brought into the L2, before the kernel ahead in the stream has ended: after a forward's weights
-// they are usually in DRAM, and a launch of few rows waited for them twice (bias, then gamma and beta). One 37-token query through
-// the base encoder, 24 such launches: 428 -> 392 us; 32 sequences of 64 ... 128 tokens: 955 -> 944 us. A prefetch
-// yields no value, so it does not matter who may still be writing them.
+// they are usually in DRAM, and a launch of few rows waited for them twice (bias, then gamma and beta). With the same for the
+// biases of the FC kernels, one 37-token query through the base encoder (24 launches of this kernel): 428 -> 414 us; 32 sequences
+// of 64 ... 128 tokens: 955 -> 949 us. A prefetch yields no value, so it does not matter who may still be writing them.
 template <typename T>
 __device__ __forceinline__ void prefetchParams(int32_t ld, T const* beta, T const* gamma, T const* bias)
 {
