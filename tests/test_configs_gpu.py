@@ -31,7 +31,7 @@ def _enqueue(p, ins, outs, in_descs, out_descs, ws=None):
 
 
 def test_config1_single_layer_through_plugins(cuda):
-    from tensorrt_b200 import plugin_harness as H
+    H = pytest.importorskip("tensorrt_b200.plugin_harness", exc_type=ImportError)  # absent without the TensorRT headers
 
     rng = np.random.default_rng(0)
     B, S, E, N, F = 8, 128, 768, 12, 3072

@@ -21,7 +21,7 @@ def _enqueue(p, ins, outs, in_descs, out_descs, ws=None):
 
 
 def test_skip_ln_legacy_matches_v5(cuda):
-    from tensorrt_b200 import plugin_harness as H
+    H = pytest.importorskip("tensorrt_b200.plugin_harness", exc_type=ImportError)  # absent without the TensorRT headers
 
     rng = np.random.default_rng(0)
     S, B, E = 64, 3, 256
@@ -44,7 +44,7 @@ def test_skip_ln_legacy_matches_v5(cuda):
 
 
 def test_qkv_var_seqlen_legacy_matches_v5(cuda):
-    from tensorrt_b200 import plugin_harness as H
+    H = pytest.importorskip("tensorrt_b200.plugin_harness", exc_type=ImportError)  # absent without the TensorRT headers
 
     rng = np.random.default_rng(1)
     N, dh, S = 4, 64, 160
@@ -74,7 +74,7 @@ def test_qkv_var_seqlen_legacy_matches_v5(cuda):
 
 
 def test_emb_var_seqlen_legacy_matches_v4(cuda):
-    from tensorrt_b200 import plugin_harness as H
+    H = pytest.importorskip("tensorrt_b200.plugin_harness", exc_type=ImportError)  # absent without the TensorRT headers
 
     rng = np.random.default_rng(2)
     E, vocab, S = 128, 300, 64
@@ -110,7 +110,7 @@ def test_emb_var_seqlen_legacy_matches_v4(cuda):
 
 
 def test_fc_v1_matches_v2(cuda):
-    from tensorrt_b200 import plugin_harness as H
+    H = pytest.importorskip("tensorrt_b200.plugin_harness", exc_type=ImportError)  # absent without the TensorRT headers
 
     FC = "CustomFCPluginDynamic"
     rng = np.random.default_rng(3)
