@@ -59,7 +59,8 @@ int32_t smCount();
 
 // Whether kernels are launched with programmatic stream serialisation (on unless BERT_B200_PDL=0): a kernel that
 // follows another one in its stream may then start - set up its barriers, allocate tensor memory, fetch descriptors -
-// while the earlier grid drains; it calls gridDependencyWait() before it touches global memory.
+// while the earlier grid drains; it calls gridDependencyWait() before it touches global memory. Two exceptions: prefetches into the
+// L2, which yield no value, and what the caller says was complete before the kernel ahead began (weightsReady, paramsReady).
 bool dependentLaunchEnabled();
 
 #ifdef __CUDACC__

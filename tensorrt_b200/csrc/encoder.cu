@@ -49,6 +49,8 @@ namespace b200
 {
 
 int32_t fcRun(bert_b200_fc_params const& p, cudaStream_t stream, bool weightsReady);
+int32_t skipLnDqqRun(cudaStream_t s, int32_t ld, int64_t n, int8_t const* input, int8_t const* skip, void const* beta, void const* gamma,
+    int8_t* output, void const* bias, float dq_scale_in, float dq_scale_skip, float q_scale, bool paramsReady);
 
 namespace
 {
@@ -302,7 +304,8 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
     } while (0)
 
     // The memset also orders the whole forward behind everything ahead of it in the stream: kernels that write weights have
-    // completed before the first kernel below starts, so the FC kernels may fetch weights ahead of their predecessors' end.
+    // completed before the first kernel below starts, so the FC and INT8 SkipLayerNorm kernels may fetch weights and parameters
+    // ahead of their predecessors' end.
     if (cudaMemsetAsync(w.status, 0, sizeof(uint32_t), stream) != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "encoder_forward: clearing the status word failed");
     // FP16: embedding output is the first layer input. INT8: additionally quantised with the first layer's input scale.
@@ -369,9 +372,9 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
         amax(w.ao, T * E, li, 3);
 
         if (i8)
-            B200_STEP(BERT_B200_KIND_SKIPLN, bert_b200_skip_layer_norm_dqq(stream, E, T * E, reinterpret_cast<int8_t*>(w.ao),
+            B200_STEP(BERT_B200_KIND_SKIPLN, skipLnDqqRun(stream, E, T * E, reinterpret_cast<int8_t*>(w.ao),
                 reinterpret_cast<int8_t*>(w.x), l.ln1_beta, l.ln1_gamma, reinterpret_cast<int8_t*>(w.h1), l.b_out,
-                l.s_attn_out, l.s_in, 1.f / l.s_ln1));
+                l.s_attn_out, l.s_in, 1.f / l.s_ln1, true));
         else
             B200_STEP(BERT_B200_KIND_SKIPLN, bert_b200_skip_layer_norm(
                 stream, BERT_B200_FP16, E, T * E, w.ao, w.x, l.ln1_beta, l.ln1_gamma, w.h1, l.b_out));
@@ -409,9 +412,9 @@ static int32_t forwardImpl(bert_b200_encoder* enc, cudaStream_t stream, int32_t 
 
         bool const last = li + 1 == c.num_layers;
         if (i8)
-            B200_STEP(BERT_B200_KIND_SKIPLN, bert_b200_skip_layer_norm_dqq(stream, E, T * E, reinterpret_cast<int8_t*>(w.ao),
+            B200_STEP(BERT_B200_KIND_SKIPLN, skipLnDqqRun(stream, E, T * E, reinterpret_cast<int8_t*>(w.ao),
                 reinterpret_cast<int8_t*>(w.h1), l.ln2_beta, l.ln2_gamma, reinterpret_cast<int8_t*>(w.x), l.b_ffn2, l.s_ffn2,
-                l.s_ln1, 1.f / l.s_out));
+                l.s_ln1, 1.f / l.s_out, true));
         else
             B200_STEP(BERT_B200_KIND_SKIPLN, bert_b200_skip_layer_norm(stream, BERT_B200_FP16, E, T * E, w.ao, w.h1, l.ln2_beta, l.ln2_gamma,
                 last ? output : static_cast<void*>(w.x), l.b_ffn2));

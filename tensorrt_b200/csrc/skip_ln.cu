@@ -11,6 +11,10 @@
 
 namespace b200
 {
+
+int32_t skipLnDqqRun(cudaStream_t s, int32_t ld, int64_t n, int8_t const* input, int8_t const* skip, void const* beta, void const* gamma,
+    int8_t* output, void const* bias, float dq_scale_in, float dq_scale_skip, float q_scale, bool paramsReady);
+
 namespace
 {
 
@@ -401,7 +405,7 @@ template <int CPL, int WPR, bool HAS_BIAS, int CB = 16>
 __global__ void __launch_bounds__(kThreads, 3) skipLnDqqPackedKernel(int32_t const ld, int64_t const rows,
     int8_t const* __restrict__ in, int8_t const* __restrict__ skip, __half const* __restrict__ beta,
     __half const* __restrict__ gamma, __half const* __restrict__ bias, int8_t* __restrict__ out, float const dqIn,
-    float const dqSkip, float const qScale, float const eps)
+    float const dqSkip, float const qScale, float const eps, bool const paramsReady)
 {
     constexpr int E = CB;
     constexpr int kWords = CB / 4;     // 32-bit words (four INT8 values each) per chunk
@@ -446,6 +450,15 @@ __global__ void __launch_bounds__(kThreads, 3) skipLnDqqPackedKernel(int32_t con
     __half2* const bqTab = gTab + ld / 2;
     __half2* const biTab = bqTab + ld / 2;
     float sBias = 0.f, sBias2 = 0.f;
+    // The tables are built before the wait only where the caller says that the kernels ahead in the stream do not write the
+    // parameters (the encoder's forward). They are plain loads: one ahead that does, be it a kernel two places ahead that this
+    // one's early start has overtaken, would leave old values in the tables.
+    if (!paramsReady)
+    {
+        gridDependencyLaunch();
+        prefetchParams(ld, beta, gamma, HAS_BIAS ? bias : nullptr);
+        gridDependencyWait();
+    }
     for (int p = threadIdx.x; p < ld / 2; p += kThreads)
     {
         float2 const g = __half22float2(reinterpret_cast<__half2 const*>(gamma)[p]);
@@ -1005,7 +1018,7 @@ int32_t dispatchSkipLn(cudaStream_t stream, int32_t ld, int64_t rows, T const* i
 
 template <int CPL, int WPR>
 int32_t launchDqq(cudaStream_t stream, int32_t ld, int64_t rows, int8_t const* in, int8_t const* skip,
-    __half const* beta, __half const* gamma, __half const* bias, int8_t* out, float dqIn, float dqSkip, float qScale)
+    __half const* beta, __half const* gamma, __half const* bias, int8_t* out, float dqIn, float dqSkip, float qScale, bool paramsReady)
 {
     int const rowsPerCta = kWarpsPerCta / WPR;
     if (CPL <= 2)
@@ -1023,10 +1036,10 @@ int32_t launchDqq(cudaStream_t stream, int32_t ld, int64_t rows, int8_t const* i
         }
         if (bias)
             launchDependent(skipLnDqqPackedKernel<CPL <= 2 ? CPL : 1, WPR, true>, dim3(grid), dim3(kThreads), smem, stream, ld, rows, in,
-                skip, beta, gamma, bias, out, dqIn, dqSkip, qScale, 0.f);
+                skip, beta, gamma, bias, out, dqIn, dqSkip, qScale, 0.f, paramsReady);
         else
             launchDependent(skipLnDqqPackedKernel<CPL <= 2 ? CPL : 1, WPR, false>, dim3(grid), dim3(kThreads), smem, stream, ld, rows, in,
-                skip, beta, gamma, bias, out, dqIn, dqSkip, qScale, 0.f);
+                skip, beta, gamma, bias, out, dqIn, dqSkip, qScale, 0.f, paramsReady);
         return checkLaunch("skipLnDqqPackedKernel");
     }
     int const grid = gridFor((rows + rowsPerCta - 1) / rowsPerCta, 8);
@@ -1042,16 +1055,16 @@ int32_t launchDqq(cudaStream_t stream, int32_t ld, int64_t rows, int8_t const* i
 // One row per warp in 8-byte chunks, CPL of them per lane (see the kernel): rows such as 768 or 256 INT8 values.
 template <int CPL>
 int32_t launchDqq8(cudaStream_t stream, int32_t ld, int64_t rows, int8_t const* in, int8_t const* skip, __half const* beta,
-    __half const* gamma, __half const* bias, int8_t* out, float dqIn, float dqSkip, float qScale)
+    __half const* gamma, __half const* bias, int8_t* out, float dqIn, float dqSkip, float qScale, bool paramsReady)
 {
     int const grid = gridFor((rows + kWarpsPerCta - 1) / kWarpsPerCta, 3);
     size_t const smem = static_cast<size_t>(ld) * 2 * 3;
     if (bias)
         launchDependent(skipLnDqqPackedKernel<CPL, 1, true, 8>, dim3(grid), dim3(kThreads), smem, stream, ld, rows, in, skip, beta,
-            gamma, bias, out, dqIn, dqSkip, qScale, 0.f);
+            gamma, bias, out, dqIn, dqSkip, qScale, 0.f, paramsReady);
     else
         launchDependent(skipLnDqqPackedKernel<CPL, 1, false, 8>, dim3(grid), dim3(kThreads), smem, stream, ld, rows, in, skip, beta,
-            gamma, bias, out, dqIn, dqSkip, qScale, 0.f);
+            gamma, bias, out, dqIn, dqSkip, qScale, 0.f, paramsReady);
     return checkLaunch("skipLnDqqPackedKernel");
 }
 
@@ -1123,9 +1136,10 @@ extern "C" int32_t bert_b200_skip_layer_norm(void* stream, int32_t type_id, int3
     B200_FAIL(BERT_B200_NOT_SUPPORTED, "skip_layer_norm: type_id %d (INT8 uses bert_b200_skip_layer_norm_dqq)", type_id);
 }
 
-extern "C" int32_t bert_b200_skip_layer_norm_dqq(void* stream, int32_t ld, int64_t n, int8_t const* input,
-    int8_t const* skip, void const* beta, void const* gamma, int8_t* output, void const* bias, float dq_scale_in,
-    float dq_scale_skip, float q_scale)
+// `paramsReady`: beta, gamma and bias were complete before the kernel ahead in the stream began, and so before those that it may
+// have overtaken.
+int32_t b200::skipLnDqqRun(cudaStream_t s, int32_t ld, int64_t n, int8_t const* input, int8_t const* skip, void const* beta,
+    void const* gamma, int8_t* output, void const* bias, float dq_scale_in, float dq_scale_skip, float q_scale, bool paramsReady)
 {
     B200_REQUIRE(ld > 0 && n >= 0 && n % ld == 0, "skip_layer_norm_dqq: n=%lld is not a multiple of ld=%d",
         static_cast<long long>(n), ld);
@@ -1139,7 +1153,6 @@ extern "C" int32_t bert_b200_skip_layer_norm_dqq(void* stream, int32_t ld, int64
         "skip_layer_norm_dqq: pointers must be 16-byte aligned");
     if (n == 0)
         return BERT_B200_OK;
-    auto s = static_cast<cudaStream_t>(stream);
     int const chunks = ld / 16;
     int wpr = 1;
     while (chunks > 32 * 4 * wpr)
@@ -1157,13 +1170,13 @@ extern "C" int32_t bert_b200_skip_layer_norm_dqq(void* stream, int32_t ld, int64
     {
         int const cpl8 = ld / 8 / 32;
         if (cpl8 == 1)
-            return launchDqq8<1>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale);
+            return launchDqq8<1>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale, paramsReady);
         if (cpl8 == 3)
-            return launchDqq8<3>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale);
+            return launchDqq8<3>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale, paramsReady);
     }
 #define B200_DQQ_CASE(C, W)                                                                                            \
     if (cpl == C && wpr == W)                                                                                          \
-        return launchDqq<C, W>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale);
+        return launchDqq<C, W>(s, ld, n / ld, input, skip, b, g, bi, output, dq_scale_in, dq_scale_skip, q_scale, paramsReady);
     B200_DQQ_CASE(1, 1)
     B200_DQQ_CASE(2, 1)
     B200_DQQ_CASE(2, 2)
@@ -1173,6 +1186,15 @@ extern "C" int32_t bert_b200_skip_layer_norm_dqq(void* stream, int32_t ld, int64
     B200_DQQ_CASE(4, 8)
 #undef B200_DQQ_CASE
     B200_FAIL(BERT_B200_NOT_SUPPORTED, "skip_layer_norm_dqq: no kernel for ld=%d", ld);
+}
+
+extern "C" int32_t bert_b200_skip_layer_norm_dqq(void* stream, int32_t ld, int64_t n, int8_t const* input,
+    int8_t const* skip, void const* beta, void const* gamma, int8_t* output, void const* bias, float dq_scale_in,
+    float dq_scale_skip, float q_scale)
+{
+    // Nothing is known about who writes the parameters.
+    return skipLnDqqRun(static_cast<cudaStream_t>(stream), ld, n, input, skip, beta, gamma, output, bias, dq_scale_in, dq_scale_skip,
+        q_scale, false);
 }
 
 static int32_t checkInterleaved(char const* name, int32_t ld, int32_t total, void const* a, void const* b,

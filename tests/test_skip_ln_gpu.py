@@ -117,6 +117,39 @@ def test_skip_ln_interleaved(cuda, ld, total):
     assert O.int8_within_lsb(O.from_chw32(out.cpu().numpy()), lin.cpu().numpy())[0]
 
 
+@pytest.mark.parametrize("ld", [256, 768, 1024, 4096])
+@pytest.mark.parametrize("between", [0, 1])
+@pytest.mark.parametrize("which", ["gamma", "beta", "bias"])
+def test_skip_ln_dqq_parameters_written_right_ahead(cuda, ld, between, which):
+    """A parameter that a kernel of this library writes one or two launches ahead, with other values each time: the row
+    of a long projection, which has barely begun when the launches behind it may start."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(ld)
+    x = torch.randint(-127, 128, (40, ld), device=cuda, generator=gen, dtype=torch.int32).to(torch.int8)
+    p = {n: torch.randn(ld, device=cuda, generator=gen).half() for n in ("gamma", "beta", "bias")}
+    a = torch.randn(2, 1, 16384, device=cuda, generator=gen).half()
+    w = (torch.randn(ld, 16384, device=cuda, generator=gen) / 128).half()
+    small, other = torch.ones(16, 16, device=cuda).half(), torch.empty(16, 16, device=cuda, dtype=torch.float16)
+    norm = lambda **q: T.skip_layer_norm_dqq(x, x, q["gamma"], q["beta"], q["bias"], 0.021, 0.017, 30.0)
+    want = []
+    for i in range(2):
+        row = T.fc(a[i], w).view(-1)
+        torch.cuda.synchronize()
+        want.append(norm(**{**p, which: row}))
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    row = torch.empty(1, ld, device=cuda, dtype=torch.float16)
+    got = []
+    for i in range(40):
+        T.fc(a[i % 2], w, out=row)
+        for _ in range(between):
+            T.fc(small, small, out=other)
+        got.append(norm(**{**p, which: row.view(-1)}))
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
+
+
 def test_skip_ln_full_size_properties(cuda):
     """BERT-large S=384 B=64 sizes: LayerNorm output rows have mean beta-mean and unit variance when gamma=1, beta=0."""
     import tensorrt_b200 as T
