@@ -65,7 +65,8 @@ bool dependentLaunchEnabled();
 
 #ifdef __CUDACC__
 // Remembers on which devices a kernel has been allowed its dynamic shared memory (beyond 48 KB it needs an attribute, which
-// costs as much host time as a quarter of a launch). One static object per kernel.
+// costs as much host time as a quarter of a launch). One static object per kernel. The limit belongs to the kernel, not to a call:
+// it is always raised to all that the device has, so that threads whose calls need different amounts don't lower it for each other.
 class SmemOptIn
 {
 public:
@@ -81,8 +82,13 @@ public:
             return cudaSuccess;
         int max = 0;
         e = cudaDeviceGetAttribute(&max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaFuncAttributes attr{};
         if (e == cudaSuccess)
-            e = bytes <= static_cast<size_t>(max) ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max) : cudaErrorInvalidValue;
+            e = cudaFuncGetAttributes(&attr, kernel);
+        if (e != cudaSuccess)
+            return e;
+        max -= static_cast<int>(attr.sharedSizeBytes); // what the kernel declares itself
+        e = bytes <= static_cast<size_t>(max) ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max) : cudaErrorInvalidValue;
         if (e == cudaSuccess)
             mDone.fetch_or(bit, std::memory_order_relaxed);
         return e;

@@ -999,11 +999,9 @@ int32_t launchOnline(CUtensorMap const (&maps)[3], OnlineArgs args, cudaStream_t
         return checkLaunch("mhaShortF16Kernel");
     }
     auto kernel = mhaOnlineF16Kernel<BNSD>;
-    cudaError_t const e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess)
-        B200_FAIL(BERT_B200_CUDA_ERROR, "mha: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    static SmemOptIn optIn;
     int const grid = shareGrid(args);
-    cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, maps[0], maps[1], maps[2], args);
+    cudaError_t const le = launchDependentCluster(&optIn, kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, 1, maps[0], maps[1], maps[2], args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaOnlineF16Kernel: %s", cudaGetErrorString(le));
     return checkLaunch("mhaOnlineF16Kernel");

@@ -965,14 +965,12 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
     int const nbMax = (p.S + kKeyBlock - 1) / kKeyBlock;
     int const smem = L::dynamicBytes(nbMax);
     auto kernel = mhaTcgen05Kernel<T, IL, false>;
-    cudaError_t const e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess)
-        B200_FAIL(BERT_B200_CUDA_ERROR, "mha: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    static SmemOptIn optIn;
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
         p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1};
     // one persistent CTA per SM (512 TMEM columns and most of the shared memory each), items dealt round-robin
     int const grid = divideItems(args);
-    cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kMhaThreads), smem, stream, map, map, map, args);
+    cudaError_t const le = launchDependentCluster(&optIn, kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, map, map, map, args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
     return checkLaunch("mhaTcgen05Kernel");
@@ -1001,13 +999,11 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
     int const nbMax = (p.S + kKeyBlock - 1) / kKeyBlock;
     int const smem = L::dynamicBytes(nbMax);
     auto kernel = mhaTcgen05Kernel<T, false, true>;
-    cudaError_t const e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess)
-        B200_FAIL(BERT_B200_CUDA_ERROR, "attention_bnsd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    static SmemOptIn optIn;
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
         p.scale_bmm2, p.status_word, 1, 1};
     int const grid = divideItems(args);
-    cudaError_t const le = launchDependent(kernel, dim3(grid), dim3(kMhaThreads), smem, stream, maps[0], maps[1], maps[2], args);
+    cudaError_t const le = launchDependentCluster(&optIn, kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
     if (le != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
     return checkLaunch("mhaTcgen05Kernel");

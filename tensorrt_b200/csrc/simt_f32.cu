@@ -548,11 +548,10 @@ namespace
 template <typename T, int D>
 int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 {
-    auto kernel = mhaTiledKernel<T, D>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(AttSmem<D>)));
-    if (e == cudaSuccess)
-        e = launchDependent(kernel, dim3(p.num_heads, p.B, (p.S + kAttRows - 1) / kAttRows), dim3(kAttThreads), sizeof(AttSmem<D>), stream, p.B, p.S,
-            p.num_heads, p.head_size, static_cast<T const*>(p.qkv), static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
+    static SmemOptIn optIn;
+    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D>, dim3(p.num_heads, p.B, (p.S + kAttRows - 1) / kAttRows),
+        dim3(kAttThreads), sizeof(AttSmem<D>), stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
+        static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTiledKernel: %s", cudaGetErrorString(e));
     return checkLaunch("mhaTiledKernel");
@@ -572,7 +571,8 @@ int32_t launchMhaSimt(bert_b200_mha_params const& p, cudaStream_t stream)
     auto kernel = mhaSimtKernel<T>;
     if (smem > 48 * 1024)
     {
-        cudaError_t const e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        static SmemOptIn optIn;
+        cudaError_t const e = optIn.set(kernel, smem, true);
         if (e != cudaSuccess)
             B200_FAIL(BERT_B200_CUDA_ERROR, "mha (SIMT): cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     }
