@@ -381,8 +381,9 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
 #pragma unroll
             for (int x = 1; x < 8; x <<= 1)
                 m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
-            float const next = fmaxf(mx[i], m); // finite: every block has a valid key
-            float const rescale = expf(mx[i] - next);
+            float const next = fmaxf(mx[i], m);
+            float const ref = next == -INFINITY ? 0.f : next; // every score so far has overflowed to -inf: no weight
+            float const rescale = expf(mx[i] - ref);
             mx[i] = next;
             sum[i] *= rescale;
 #pragma unroll
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
 #pragma unroll
             for (int j = 0; j < 8; ++j)
             {
-                float const e = expf(s[j] - next);
+                float const e = expf(s[j] - ref);
                 sum[i] += e;
                 sm.p[row0 + 4 * i][tx + 8 * j] = e;
             }

@@ -384,6 +384,24 @@ def test_mha_simt_tile_edges(cuda, d, half):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, tol, tol)[0]
 
 
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("block", [0, 64])
+def test_mha_fp32_scores_that_overflow(cuda, block, d):
+    """A block of 64 keys whose scores all overflow to -inf has no weight; the rows are those of the other keys."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(d + block)
+    S, B, N = 150, 2, 2
+    qkv = rng.standard_normal((S, B, N, 3, d)).astype(np.float32)
+    qkv[..., 0, 0] = 1e30
+    qkv[..., 1, 0] = 0.0
+    qkv[block:block + 64, :, :, 1, 0] = -1e30
+    qkv = qkv.reshape(S, B, 3 * N * d)
+    out = T.mha(_t(qkv, cuda), B, S, N, d)
+    ok, worst, bad = O.close_abs_or_rel(out.cpu().numpy(), O.mha(qkv, B, S, N, d), 1e-5, 1e-5)
+    assert ok, (worst, bad)
+
+
 def test_mha_full_size_properties(cuda):
     """BERT-large S=384, B=64, N=16: with V = const per head the context equals that constant (rows of the
     softmax sum to one), and attention is invariant to a permutation of the keys."""
