@@ -173,17 +173,17 @@ __device__ __forceinline__ void clusterBarrier()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The float at the same shared-memory location in CTA `rank` of this cluster.
-__device__ __forceinline__ float ldSharedCluster(float const* local, int rank)
+// The four floats at the same shared-memory location in CTA `rank` of this cluster.
+__device__ __forceinline__ float4 ldSharedCluster4(float const* local, int rank)
 {
-    float v;
+    float4 v;
     asm volatile(
         "{\n\t"
         ".reg .b32 a;\n\t"
-        "mapa.shared::cluster.u32 a, %1, %2;\n\t"
-        "ld.shared::cluster.f32 %0, [a];\n\t"
+        "mapa.shared::cluster.u32 a, %4, %5;\n\t"
+        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t"
         "}"
-        : "=f"(v)
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
         : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank)
         : "memory");
     return v;

@@ -31,18 +31,24 @@ __device__ __forceinline__ float geluErf(float x)
 // pieces left no registers for that: 3 % slower); rows are padded to 20 floats, which puts the 4 or 8 rows that a warp reads
 // at once into different banks. The sums run on packed fma.rn.f32x2: one half takes the even k, the
 // other the odd ones (no operand has to be duplicated), and the two are added at the end; a packed FMA takes half the
-// issue slots, which leaves room for the loads. These bring 64 bytes per thread and k pair to the registers, at 128 bytes per
+// issue slots, which leaves room for the loads. These bring 128 bytes per thread and k pair to the registers, at 128 bytes per
 // clock and SM as long as the FMAs take: the loop runs at 0.6 of the FMA rate.
-// A cluster of `split` CTAs divides the K range of a tile where the tiles alone leave SMs idle or fill the last wave badly;
-// its CTAs exchange partial sums through distributed shared memory, each finishing every split-th row.
-// Measured: 1024 x 2304 x 768 in 96 us (38 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x
-// 3072 in 141 us (700 us).
+// K is summed in segments (1, 2, 4 or 8 of about equal length, by K alone), and the segments' sums are added in order: a row of C is the
+// same bits whatever M, although the work is divided by the number of tiles. Where the tiles alone fill the SMs, a CTA takes all segments
+// of its tile and keeps their sum in shared memory (16 KB, four CTAs still fit an SM); otherwise a cluster takes one per CTA, exchanges
+// the sums through distributed shared memory and each CTA finishes its share of every thread's outputs.
+// Measured: 1024 x 2304 x 768 in 97 us (37 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x 3072 in 143 us
+// (700 us). Holding the sums of eight segments costs 3 us of the first (K in one piece: 93 ... 95 us), exchanging them 8 % of 4096 x 1024 x
+// 4096 (843 us; two CTAs per tile 777 us), and few rows gain (37 x 768 x 768 8.7 us, 9.7 us with a scalar exchange).
 constexpr int kTile = 64;
 constexpr int kTileK = 16;
 constexpr int kPitch = kTileK + 4; // floats
 constexpr int kStages = 4;
 constexpr int kFcF32Threads = 64;
 constexpr int kFcF32CtasPerSm = 4;
+constexpr int kFcF32Ring = kStages * 2 * kTile * kPitch; // floats
+constexpr int kFcF32Part = kTile * kTile;                // sums of a segment, as the threads hold them (see partIndex)
+static_assert(kFcF32Ring >= kFcF32Part, "the last segment's sums reuse the ring");
 
 __device__ __forceinline__ void fma2(uint64_t& c, uint64_t a, uint64_t b)
 {
@@ -87,8 +93,8 @@ struct FcF32Args
     float const* bias;
     int32_t act;
     float alpha;
-    int32_t nTiles; // tiles along N
-    int32_t split;  // CTAs per tile = cluster size
+    int32_t nTiles;   // tiles along N
+    int32_t segments; // of K
 };
 
 __device__ __forceinline__ float fcF32Epilogue(FcF32Args const& p, float v, int64_t n)
@@ -97,29 +103,49 @@ __device__ __forceinline__ float fcF32Epilogue(FcF32Args const& p, float v, int6
     return p.act == BERT_B200_ACT_GELU_ERF ? geluErf(v) : v;
 }
 
-// kVec: floats per copy (4, or 1 where K, lda or an address is not a multiple of 16 bytes)
-template <int kVec>
+// Columns n, n + 8, n + 16 and n + 24 of row m.
+__device__ __forceinline__ void storeF32(FcF32Args const& p, float4 v, int64_t m, int64_t n)
+{
+    float const vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (m < p.M && n + 8 * c < p.N)
+            p.C[m * p.ldc + n + 8 * c] = fcF32Epilogue(p, vv[c], n + 8 * c);
+}
+
+// Where the segment's sums of outputs (i, j ... j + 3) of a thread lie: group i * 2 + j / 4, consecutive lanes at consecutive 16
+// bytes (no bank conflicts).
+__device__ __forceinline__ int partIndex(int i, int j, int tid)
+{
+    return ((i * 2 + (j >> 2)) * kFcF32Threads + tid) * 4 + (j & 3);
+}
+
+// kVec: floats per copy (4, or 1 where K, lda or an address is not a multiple of 16 bytes). kAlone: a CTA takes all segments of its
+// tile, otherwise a cluster takes one per CTA.
+template <int kVec, bool kAlone>
 __global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(FcF32Args const p)
 {
-    __shared__ __align__(16) float sm[kStages][2][kTile][kPitch];
-    static_assert(sizeof(sm) >= kTile * kTile * sizeof(float), "partial sums reuse the ring");
+    extern __shared__ __align__(16) float smRaw[]; // the ring, then (kAlone) the sum of the segments so far
+    float(*const sm)[2][kTile][kPitch] = reinterpret_cast<float(*)[2][kTile][kPitch]>(smRaw);
+    float* const held = smRaw + kFcF32Ring;
     int const tid = threadIdx.x;
     int const lane = tid & 31;
     int const ty = lane >> 3;
     int const tx = lane & 7;
     int const row0 = (tid >> 5) * 32 + ty; // rows row0 + 4 i, columns tx + 8 j
-    int const rank = static_cast<int>(blockIdx.x % p.split);
-    int64_t const tile = blockIdx.x / p.split;
+    int const rank = kAlone ? 0 : static_cast<int>(blockIdx.x % p.segments);
+    int64_t const tile = kAlone ? blockIdx.x : blockIdx.x / p.segments;
     int64_t const m0 = tile / p.nTiles * kTile;
     int64_t const n0 = tile % p.nTiles * kTile;
     int64_t const kBlocks = (p.K + kTileK - 1) / kTileK;
-    int const kbFirst = static_cast<int>(kBlocks * rank / p.split);
-    int const kbEnd = static_cast<int>(kBlocks * (rank + 1) / p.split);
+    auto segmentBegin = [&](int s) { return static_cast<int>(kBlocks * s / p.segments); };
+    int const kbFirst = segmentBegin(rank);
+    int const kbEnd = kAlone ? static_cast<int>(kBlocks) : segmentBegin(rank + 1);
 
     gridDependencyLaunch();
     gridDependencyWait();
 
-    uint32_t const smBase = static_cast<uint32_t>(__cvta_generic_to_shared(&sm[0][0][0][0]));
+    uint32_t const smBase = static_cast<uint32_t>(__cvta_generic_to_shared(smRaw));
     auto load = [&](int kb, int stage) {
         constexpr int kPieces = kTileK / kVec; // per row
         constexpr int kRowStep = kFcF32Threads / kPieces;
@@ -145,8 +171,32 @@ __global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(Fc
         cpAsyncCommit();
     }
     int stage = 0;
+    int segment = 0;
+    int segmentEnd = kAlone ? segmentBegin(1) : kbEnd;
+#pragma unroll 1
     for (int kb = kbFirst; kb < kbEnd; ++kb)
     {
+        if (kAlone && kb == segmentEnd)
+        {
+            // the segment's sums to those before it (a thread reads what it has written itself)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; j += 4)
+                {
+                    float4* const h = reinterpret_cast<float4*>(held + partIndex(i, j, tid));
+                    float4 v = make_float4(sumPair(acc[i][j]), sumPair(acc[i][j + 1]), sumPair(acc[i][j + 2]), sumPair(acc[i][j + 3]));
+                    if (segment > 0)
+                    {
+                        float4 const before = *h;
+                        v = make_float4(before.x + v.x, before.y + v.y, before.z + v.z, before.w + v.w);
+                    }
+                    *h = v;
+                    acc[i][j] = acc[i][j + 1] = acc[i][j + 2] = acc[i][j + 3] = 0;
+                }
+            ++segment;
+            segmentEnd = segmentBegin(segment + 1);
+        }
         cpAsyncWait<kStages - 2>();
         __syncthreads(); // this stage has landed; everybody is done with the one that is filled next
         int const ahead = stage == 0 ? kStages - 1 : stage - 1;
@@ -180,40 +230,51 @@ __global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(Fc
         }
         stage = stage + 1 == kStages ? 0 : stage + 1;
     }
-    if (p.split == 1)
+    if constexpr (kAlone)
     {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
         {
             int64_t const m = m0 + row0 + 4 * i;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+            for (int j = 0; j < 8; j += 4)
             {
-                int64_t const n = n0 + tx + 8 * j;
-                if (m < p.M && n < p.N)
-                    p.C[m * p.ldc + n] = fcF32Epilogue(p, sumPair(acc[i][j]), n);
+                float4 v = make_float4(sumPair(acc[i][j]), sumPair(acc[i][j + 1]), sumPair(acc[i][j + 2]), sumPair(acc[i][j + 3]));
+                if (p.segments > 1)
+                {
+                    float4 const before = *reinterpret_cast<float4 const*>(held + partIndex(i, j, tid));
+                    v = make_float4(before.x + v.x, before.y + v.y, before.z + v.z, before.w + v.w);
+                }
+                storeF32(p, v, m, n0 + tx + 8 * j);
             }
         }
         return;
     }
     cpAsyncWait<0>();
     __syncthreads();
-    float* const part = &sm[0][0][0][0];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            part[(row0 + 4 * i) * kTile + tx + 8 * j] = sumPair(acc[i][j]);
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(smRaw + partIndex(i, j, tid))
+                = make_float4(sumPair(acc[i][j]), sumPair(acc[i][j + 1]), sumPair(acc[i][j + 2]), sumPair(acc[i][j + 3]));
     clusterBarrier();
-    int const rows = static_cast<int>(p.M - m0 < kTile ? p.M - m0 : kTile);
-    int64_t const n = n0 + tid; // one column per thread, every split-th row
-    for (int r = rank; r < rows; r += p.split)
+    for (int g = rank; g < 16; g += p.segments)
     {
-        float v = 0.f;
-        for (int q = 0; q < p.split; ++q)
-            v += ldSharedCluster(part + r * kTile + tid, q);
-        if (n < p.N)
-            p.C[(m0 + r) * p.ldc + n] = fcF32Epilogue(p, v, n);
+        int const i = g >> 1, j = (g & 1) * 4;
+        int const at = partIndex(i, j, tid);
+        float4 x[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) // all on their way before the first is added
+            if (s < p.segments)
+                x[s] = ldSharedCluster4(smRaw + at, s);
+        float4 v = x[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s)
+            if (s < p.segments)
+                v = make_float4(v.x + x[s].x, v.y + x[s].y, v.z + x[s].z, v.w + x[s].w);
+        int64_t const m = m0 + row0 + 4 * i;
+        storeF32(p, v, m, n0 + tx + 8 * j);
     }
     clusterBarrier(); // nobody leaves while its partial sums are being read
 }
@@ -509,35 +570,44 @@ __global__ void __launch_bounds__(128) mhaSimtKernel(int32_t const B, int32_t co
 
 } // namespace
 
-// CTAs per tile: the smallest of 1, 2, 4, 8 that gives the SMs nearly all the CTAs that fit at once; with a long K (2048 and more
-// per CTA) twice as many, so that the last ones do not run alone for long. Other cluster sizes leave SMs idle (clusters of three:
-// some SMs none, others four); fewer CTAs leave FMA pipes idle, more exchange partial sums for nothing. Measured with 1 / 2 / 4 / 8
-// per tile: 1024 x 768 x 3072 (192 tiles) 273 / 183 / 141 / 147 us (three: 184), 1024 x 3072 x 768 (768 tiles) 139 / 149 / 151 us,
-// 128 x 768 x 3072 (24 tiles) 182 / 100 / 52 / 44 us, 4096 x 1024 x 4096 (1024 tiles) 890 / 780 us.
-static int pickSplitF32(int64_t tiles, int64_t kBlocks)
+// Segments of K: eight from K = 768 on, else 192 products or more each. More of them are more CTAs for few rows and more sums to hold
+// or exchange for many: with 4 / 8, 37 x 3072 x 768 22.5 / 15.2 us, 37 x 768 x 3072 47 / 26 us, 300 x 768 x 768 25.8 / 15.8 us, and 8192 x
+// 768 x 768 255 / 262 us.
+static int segmentsF32(int64_t kBlocks)
 {
-    int split = 1;
-    while (split < 8 && 2 * split <= kBlocks)
-    {
-        int64_t const enough = kBlocks / split >= 2048 / kTileK ? 8 * smCount() : 17 * smCount() / 5;
-        if (tiles * split >= enough)
-            break;
-        split *= 2;
-    }
-    return split;
+    return kBlocks >= 48 ? 8 : kBlocks >= 24 ? 4 : kBlocks >= 12 ? 2 : 1;
+}
+
+// Whether a CTA takes all segments of its tile: where the tiles alone are nearly all the CTAs that fit at once; with a long K (2048 and
+// more), where a CTA of the last wave runs for long, only when that wave is nearly full. Measured with one CTA per tile / one per
+// segment (waves of 592): 37 x 768 x 768 (12 tiles) 51 / 8.9 us, 300 x 3072 x 768 (240) 90 / 51 us, 2048 x 1024 x 1024 (512) 123 / 124 us,
+// 4096 x 1024 x 1024 (1024) 233 / 237 us, 8192 x 768 x 768 (1536) 262 / 280 us, 3000 x 768 x 3072 (564) 350 / 366 us, 4096 x 1024 x 4096 (1024)
+// 878 / 843 us.
+static bool aloneF32(int64_t tiles, int64_t kBlocks)
+{
+    if (kBlocks < 2048 / kTileK)
+        return tiles >= 17 * smCount() / 5;
+    int64_t const wave = static_cast<int64_t>(kFcF32CtasPerSm) * smCount();
+    return 10 * tiles >= 9 * ((tiles + wave - 1) / wave * wave);
 }
 
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
     int64_t const mTiles = (p.m + kTile - 1) / kTile;
     int64_t const nTiles = (p.n + kTile - 1) / kTile;
+    int64_t const kBlocks = (p.k + kTileK - 1) / kTileK;
     bool const vec = p.k % 4 == 0 && p.lda % 4 == 0 && aligned16(p.a) && aligned16(p.wt);
-    int const split = pickSplitF32(mTiles * nTiles, (p.k + kTileK - 1) / kTileK);
-    B200_REQUIRE(mTiles * nTiles * split < (1ll << 31), "fc (FP32): m=%lld, n=%lld too large", static_cast<long long>(p.m), static_cast<long long>(p.n));
+    int const segments = segmentsF32(kBlocks);
+    bool const alone = segments == 1 || aloneF32(mTiles * nTiles, kBlocks);
+    int const ctas = alone ? 1 : segments; // per tile
+    B200_REQUIRE(mTiles * nTiles * ctas < (1ll << 31), "fc (FP32): m=%lld, n=%lld too large", static_cast<long long>(p.m), static_cast<long long>(p.n));
     FcF32Args const args{p.m, p.n, p.k, static_cast<float const*>(p.a), p.lda, static_cast<float const*>(p.wt), static_cast<float*>(p.c), p.ldc,
-        p.bias, p.activation, p.alpha, static_cast<int32_t>(nTiles), split};
-    cudaError_t const e = launchDependentCluster(nullptr, vec ? fcF32Kernel<4> : fcF32Kernel<1>, dim3(static_cast<unsigned>(mTiles * nTiles * split)),
-        dim3(kFcF32Threads), 0, stream, split, args);
+        p.bias, p.activation, p.alpha, static_cast<int32_t>(nTiles), segments};
+    size_t const smem = sizeof(float) * (kFcF32Ring + (alone && segments > 1 ? kFcF32Part : 0));
+    auto const kernel = alone ? (vec ? fcF32Kernel<4, true> : fcF32Kernel<1, true>) : (vec ? fcF32Kernel<4, false> : fcF32Kernel<1, false>);
+    static SmemOptIn optIn[2];
+    cudaError_t const e = launchDependentCluster(alone ? &optIn[vec] : nullptr, kernel, dim3(static_cast<unsigned>(mTiles * nTiles * ctas)),
+        dim3(kFcF32Threads), smem, stream, ctas, args);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "fcF32Kernel: %s", cudaGetErrorString(e));
     return checkLaunch("fcF32Kernel");

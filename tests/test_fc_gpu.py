@@ -154,7 +154,7 @@ def test_fc_pair_tile_widths(cuda, m, k, n, int8):
 
 
 # tile and k-block edges of the FP32 kernel: one row, single column past a 64-wide tile, K below and above a k-block, K and
-# strides that are no multiple of four (element copies), shapes that divide K over a cluster (odd shares included)
+# strides that are no multiple of four (element copies), shapes that divide K over a cluster (uneven segments included)
 @pytest.mark.parametrize("m,k,n", [(1, 4, 1), (65, 20, 67), (64, 7, 64), (33, 1001, 130), (38, 3072, 768), (200, 784, 96), (1024, 768, 768)])
 @pytest.mark.parametrize("epi", ["none", "bias_gelu"])
 def test_fc_fp32_tile_edges(cuda, m, k, n, epi):
@@ -171,6 +171,24 @@ def test_fc_fp32_tile_edges(cuda, m, k, n, epi):
          T.ACT_GELU_ERF if epi == "bias_gelu" else T.ACT_NONE, out=out[:m])
     assert O.close_abs_or_rel(out[:m].cpu().numpy(), ref, 1e-5, 1e-5)[0]
     assert bool((out[m] == 7.0).all())   # nothing written past the last row
+
+
+# K in one, two, four and eight segments; rows for which a tile's segments go to one CTA each and to one CTA (148 SMs)
+@pytest.mark.parametrize("k,n", [(80, 96), (192, 200), (400, 768), (768, 768), (3072, 768), (1001, 130)])
+def test_fc_fp32_rows_do_not_depend_on_m(cuda, k, n):
+    """The same bits for a row whatever it is multiplied with."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(k + n)
+    one_wave = 64 * (4 * 148 // ((n + 63) // 64)) - 5
+    a = torch.randn(one_wave + 1000, k, device=cuda, generator=gen)
+    w, bias = 0.02 * torch.randn(n, k, device=cuda, generator=gen), 0.02 * torch.randn(n, device=cuda, generator=gen)
+    a[3] = -0.0   # the sign of a zero, too
+    every = T.fc(a, w, None)
+    assert bool(((every.double() - a.double() @ w.double().T).abs() <= 1e-5 * torch.clamp(every.abs(), min=1.0)).all())
+    for m in (1, 37, 130, 520, 1024, 2100, one_wave):
+        assert torch.equal(T.fc(a[:m], w, None).view(torch.int32), every[:m].view(torch.int32)), m
+    assert torch.equal(T.fc(a[:37], w, bias, T.ACT_GELU_ERF), T.fc(a[:one_wave], w, bias, T.ACT_GELU_ERF)[:37])
 
 
 def test_fc_linearity_full_size(cuda):
