@@ -1,0 +1,66 @@
+// How the INT8 attention divides its work into items and deals them to persistent CTAs (plain C++, host and device).
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define B200_HOST_DEVICE __host__ __device__
+#else
+#define B200_HOST_DEVICE
+#endif
+
+namespace b200
+{
+
+constexpr int32_t kItemTile = 128;   // query rows per tile
+constexpr int32_t kItemOrder = 256;  // sequences that a CTA can put in order
+constexpr int32_t kItemRounds = 64;  // items per CTA that it can list
+
+struct ItemPlan
+{
+    int32_t tilesPerItem, chunks; // an item = some (or all) query tiles of a (sequence, head) pair; chunks = items per pair
+    bool longestFirst;            // the sequences are dealt in the order of their lengths, else as they come
+};
+
+// All tiles of a pair share one load of K and V, which an item waits for at about a third of a tile's time; items are cut smaller only
+// when that shortens the longest CTA's list. Measured (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
+// us), 4 x 256 6.5 us (10.2 us), 12 x 384 22.5 us (31.8 us); 8 x 384 whole, 16.7 us.
+// The lengths are on the device; what the host knows is how many tokens the batch has less than B * S (`missing`; INT64_MAX: unknown).
+// With no more pairs than CTAs a cut is never the longer way, whatever they are. With more, pairs are cut only when every sequence is
+// known to have the same number of tiles: whether halves or whole pairs even out better depends on where the long ones lie. Ragged
+// batches keep whole pairs, and every CTA puts the sequences in the order of their lengths first (0.3 us) and takes a long pair, then a
+// short one. Measured, packed, longest first / halves as they come / whole pairs as they come: 14 sequences of 87 ... 338 tokens, 12
+// heads 17.6 / 21.3 / 30.9 us, others of these lengths 17.6 / 20.5 / 17.2 us, 16 of 67 ... 283 17.6 / 20.5 / 24.3 us, 47 of up to 422, 16 heads
+// 95 / 137 / 121 us, 37 interleaved of 100 ... 256 whole either way: 41.0 us in order and as they come.
+inline ItemPlan planItems(int32_t B, int32_t N, int32_t S, int64_t missing, int64_t ctas)
+{
+    int64_t const pairs = static_cast<int64_t>(B) * N;
+    int32_t const nq = (S + kItemTile - 1) / kItemTile;
+    ItemPlan plan{nq, 1, false};
+    if (pairs > ctas && missing >= S - static_cast<int64_t>(nq - 1) * kItemTile) // a sequence may lack a whole tile
+    {
+        plan.longestFirst = B <= kItemOrder && pairs <= kItemRounds * ctas;
+        return plan;
+    }
+    int64_t best = 0;
+    for (int32_t tiles = nq; tiles >= 1; --tiles)
+    {
+        int32_t const chunks = (nq + tiles - 1) / tiles;
+        int64_t const cost = (pairs * chunks + ctas - 1) / ctas * (3 * tiles + 1);
+        if (tiles == nq || (cost < best && pairs * chunks <= INT32_MAX))
+        {
+            best = cost;
+            plan.tilesPerItem = tiles;
+            plan.chunks = chunks;
+        }
+    }
+    return plan;
+}
+
+// The item that CTA `cta` takes in its `round`-th turn, the items being in the order of their lengths: every second round runs
+// backwards, so that who had the longest of a round gets the shortest of the next. May lie beyond the last item in the last round.
+B200_HOST_DEVICE inline int32_t itemOfRound(int32_t round, int32_t cta, int32_t ctas)
+{
+    return round * ctas + ((round & 1) != 0 ? ctas - 1 - cta : cta);
+}
+
+} // namespace b200

@@ -10,8 +10,8 @@
 // sum before the first of them can be formed, so the whole score row lives in TMEM (<= 512 keys) and the softmax makes
 // three sweeps over it; that is what keeps the result bit-identical with the reference's INT8 kernels.
 //
-// Persistent CTAs (one per SM) take (sequence, head) work items, or parts of them where there are few, round-robin. Per
-// item a CTA loops over its 128-query tiles, so that K and V are loaded once and the tensor pipe works on the next tile
+// Persistent CTAs (one per SM) take (sequence, head) work items, or parts of them where there are few, round-robin or, in
+// ragged batches of many, each a long one, then a short one (mha_items.h). Per item a CTA loops over its 128-query tiles, so that K and V are loaded once and the tensor pipe works on the next tile
 // (of this item or the next) while the softmax warps finish the current one. 19 warps:
 //   warp 0    : TMA - the K / V blocks (128 keys each) of an item once, the Q tile of each iteration
 //               (swizzled shared-memory tiles, one mbarrier each).
@@ -33,6 +33,7 @@
 // The kernel template also takes FP16 tensors (exact-maximum two-sweep form, P in shared memory); that instantiation
 // is not built.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM, reports through the status word.
+#include "mha_items.h"
 #include "sm100.cuh"
 
 #include <cstdlib>
@@ -68,6 +69,15 @@ struct MhaArgs
     float scaleBmm1, scaleSoftmax, scaleBmm2;
     uint32_t* statusWord;
     int32_t tilesPerItem, chunks; // a work item = (sequence, head, chunk of tilesPerItem query tiles)
+    int32_t rounds;               // ORDERED: items per CTA
+};
+
+// Sequences by length and the items of a CTA (ORDERED, see the kernel).
+struct alignas(1024) ItemTable
+{
+    int4 ordered[kItemOrder]; // number, first row, length
+    int4 items[kItemRounds];  // sequence (-1: none), head, first row, length
+    int32_t lengths[kItemOrder];
 };
 
 template <typename T>
@@ -169,7 +179,8 @@ __device__ __forceinline__ void tmemStoreWait()
 // [128 tokens][32 B] (32-byte swizzle); the head dimension is covered by one MMA per sub-tile.
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
-template <typename T, bool IL, bool BNSD>
+// ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h).
+template <typename T, bool IL, bool BNSD, bool ORDERED>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
@@ -190,31 +201,55 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     int const warp = threadIdx.x >> 5;
     int const lane = threadIdx.x & 31;
 
+    extern __shared__ uint8_t smemRaw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
+    ItemTable* const table = reinterpret_cast<ItemTable*>(smem);
+    if (ORDERED)
+        smem += sizeof(ItemTable);
+
     // ---- work items: some or all query tiles of a (sequence, head), item = (b * N + head) * chunks + chunk, dealt round-robin
-    //      to the persistent CTAs ----
+    //      to the persistent CTAs; or whole (sequence, head) pairs as the CTA has listed them ----
     struct Item
     {
         int32_t b, head, rowBase, rows, len, nb, tBegin, tEnd;
     };
-    int const numItems = args.B * args.N * args.chunks;
-    // Geometry of item i (uniform over the CTA; every role derives the same values). Returns whether the item has
-    // work for the tensor pipeline (at least one query row and one valid key).
-    auto getItem = [&](int i, Item& it) -> bool {
-        int const pair = i / args.chunks;
-        it.b = pair / args.N;
-        it.head = pair - it.b * args.N;
-        it.tBegin = (i - pair * args.chunks) * args.tilesPerItem;
+    int const numItems = ORDERED ? args.rounds : args.B * args.N * args.chunks;
+    int const firstItem = ORDERED ? 0 : static_cast<int>(blockIdx.x);
+    int const itemStep = ORDERED ? 1 : static_cast<int>(gridDim.x);
+    // first row and valid keys of sequence b
+    auto sequence = [&](int b, int32_t& rowBase, int32_t& len) {
         if (args.fixedLayout)
         {
-            it.rowBase = 0;
-            it.rows = args.S;
-            it.len = args.maskIdx ? min(max(__ldg(args.maskIdx + it.b), 0), args.S) : args.S;
+            rowBase = 0;
+            len = args.maskIdx ? min(max(__ldg(args.maskIdx + b), 0), args.S) : args.S;
         }
         else
         {
-            it.rowBase = __ldg(args.cu + it.b);
-            it.len = min(max(__ldg(args.cu + it.b + 1) - it.rowBase, 0), args.S);
-            it.rows = it.len;
+            rowBase = __ldg(args.cu + b);
+            len = min(max(__ldg(args.cu + b + 1) - rowBase, 0), args.S);
+        }
+    };
+    // Geometry of item i (uniform over the CTA; every role derives the same values). Returns whether the item has
+    // work for the tensor pipeline (at least one query row and one valid key).
+    auto getItem = [&](int i, Item& it) -> bool {
+        if (ORDERED)
+        {
+            int4 const q = table->items[i];
+            it.b = q.x;
+            it.head = q.y;
+            it.rowBase = q.z;
+            it.len = q.w;
+            it.rows = args.fixedLayout && q.x >= 0 ? args.S : it.len;
+            it.tBegin = 0;
+        }
+        else
+        {
+            int const pair = i / args.chunks;
+            it.b = pair / args.N;
+            it.head = pair - it.b * args.N;
+            it.tBegin = (i - pair * args.chunks) * args.tilesPerItem;
+            sequence(it.b, it.rowBase, it.len);
+            it.rows = args.fixedLayout ? args.S : it.len;
         }
         it.nb = (it.len + kKeyBlock - 1) / kKeyBlock; // key blocks
         it.tEnd = min((it.rows + kQTile - 1) / kQTile, it.tBegin + args.tilesPerItem);
@@ -223,7 +258,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     // first item >= i of this CTA's sequence that has pipeline work; numItems or more if there is none
     auto nextWork = [&](int i, Item& it) -> int {
         while (i < numItems && !getItem(i, it))
-            i += gridDim.x;
+            i += itemStep;
         return i;
     };
 
@@ -234,8 +269,6 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     uint32_t const oCol = oAliasesScores ? 0u : kOColumn;
     auto slotOf = [&](int j) { return nbMax <= 3 ? j : (j & 1); };
 
-    extern __shared__ uint8_t smemRaw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* sQ = smem;                          // kTileBytes
     uint8_t* sK = smem + L::kOffset();           // nbMax x kTileBytes
     uint8_t* sV = smem + L::vOffset(nbMax);      // nbMax x kTileBytes
@@ -294,6 +327,45 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     gridDependencyLaunch();
     gridDependencyWait();
 
+    if (ORDERED)
+    {
+        // a sequence's place is the number of longer ones, and of equal ones before it (those beyond the batch count as -1)
+        int const b = static_cast<int>(threadIdx.x);
+        if (b < kItemOrder)
+        {
+            int32_t rowBase = 0, len = -1;
+            if (b < args.B)
+                sequence(b, rowBase, len);
+            table->lengths[b] = len;
+            asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
+            if (b < args.B)
+            {
+                int place = 0;
+                for (int u = 0; u < args.B; u += 4)
+                {
+                    int4 const v = *reinterpret_cast<int4 const*>(table->lengths + u);
+                    place += (v.x > len || (v.x == len && u < b)) + (v.y > len || (v.y == len && u + 1 < b))
+                        + (v.z > len || (v.z == len && u + 2 < b)) + (v.w > len || (v.w == len && u + 3 < b));
+                }
+                table->ordered[place] = make_int4(b, rowBase, len, 0);
+            }
+            asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
+            if (b < args.rounds)
+            {
+                int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+                int const place = item / args.N;
+                int4 q = make_int4(-1, 0, 0, 0);
+                if (place < args.B)
+                {
+                    int4 const o = table->ordered[place];
+                    q = make_int4(o.x, item - place * args.N, o.y, o.z);
+                }
+                table->items[b] = q;
+            }
+        }
+        __syncthreads();
+    }
+
     // Barriers that complete once per tile (qFull, qFree, oFull, oFree) are waited on with the parity of the CTA's
     // running tile count; those that complete once per use of key block j keep one parity bit per block.
     if (warp == 0)
@@ -302,7 +374,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         uint32_t tiles = 0;       // Q tiles requested so far
         uint32_t itemsLoaded = 0; // items whose K / V have been requested
         bool ok = true;
-        for (int item = nextWork(blockIdx.x, it); item < numItems && ok; item = nextWork(item + gridDim.x, it))
+        for (int item = nextWork(firstItem, it); item < numItems && ok; item = nextWork(item + itemStep, it))
         {
             int32_t const rowK = args.fixedLayout ? 0 : it.rowBase;
             int32_t const rowKv = rowK; // first key of this item
@@ -416,7 +488,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 return got;
             };
             Item cur, nxt;
-            int item = nextWork(blockIdx.x, cur);
+            int item = nextWork(firstItem, cur);
             if (kDoScores && item < numItems)
             {
                 ok = mbarWaitWarp(qFull, 0, abortFlag, kWaitTmaFull);
@@ -439,7 +511,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             {
                 // only the scores look one item ahead (its geometry comes from global memory: not in the way of a
                 // warp that only issues context products)
-                int const nextItem = kDoScores ? nextWork(item + gridDim.x, nxt) : numItems;
+                int const nextItem = kDoScores ? nextWork(item + itemStep, nxt) : numItems;
                 for (int t = cur.tBegin; t < cur.tEnd && ok; ++t)
                 {
                     bool const lastT = t + 1 == cur.tEnd;
@@ -553,7 +625,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     item = nextItem;
                 }
                 else
-                    item = nextWork(item + gridDim.x, cur);
+                    item = nextWork(item + itemStep, cur);
             }
         };
         if (!twoIssuers)
@@ -649,7 +721,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         float pendInv = 0.f;
 
         Item it;
-        for (int item = blockIdx.x; item < numItems; item += gridDim.x)
+        for (int item = firstItem; item < numItems; item += itemStep)
         {
             bool const work = getItem(item, it);
             int64_t const outRowStride = static_cast<int64_t>(args.N) * args.d; // elements
@@ -903,40 +975,38 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     }
 }
 
-// Query tiles per work item, and the number of CTAs. All tiles of a (sequence, head) share one load of K and V, which an item
-// waits for at about a third of a tile's time; items are cut smaller only when that shortens the longest CTA's list, that is
-// when there are few of them. Measured (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
-// us), 4 x 256 6.5 us (10.2 us), 12 x 384 22.5 us (31.8 us); 8 x 384 whole, 16.7 us.
-int divideItems(MhaArgs& args)
+// Sets the work items and launches: one persistent CTA per SM (512 TMEM columns and most of the shared memory each).
+template <typename T, bool IL, bool BNSD>
+int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t stream)
 {
-    int64_t const pairs = static_cast<int64_t>(args.B) * args.N;
-    int32_t const nq = (args.S + kQTile - 1) / kQTile;
-    int64_t best = 0;
-    for (int32_t tiles = nq; tiles >= 1; --tiles)
-    {
-        int32_t const chunks = (nq + tiles - 1) / tiles;
-        int64_t const cost = (pairs * chunks + smCount() - 1) / smCount() * (3 * tiles + 1);
-        if (tiles == nq || (cost < best && pairs * chunks <= INT32_MAX))
-        {
-            best = cost;
-            args.tilesPerItem = tiles;
-            args.chunks = chunks;
-        }
-    }
-    int64_t const items = pairs * args.chunks;
-    return static_cast<int>(items < smCount() ? items : smCount());
+    static_assert(kItemTile == kQTile, "tiles of the plan");
+    int64_t const missing = !args.fixedLayout ? static_cast<int64_t>(args.B) * args.S - args.total : (args.maskIdx ? INT64_MAX : 0);
+    ItemPlan const plan = planItems(args.B, args.N, args.S, missing, smCount());
+    args.tilesPerItem = plan.tilesPerItem;
+    args.chunks = plan.chunks;
+    int64_t const items = static_cast<int64_t>(args.B) * args.N * plan.chunks;
+    int const grid = static_cast<int>(items < smCount() ? items : smCount());
+    args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
+    int const smem = MhaSmem<T>::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (plan.longestFirst ? static_cast<int>(sizeof(ItemTable)) : 0);
+    static SmemOptIn optIn[2];
+    auto const kernel = plan.longestFirst ? mhaTcgen05Kernel<T, IL, BNSD, true> : mhaTcgen05Kernel<T, IL, BNSD, false>;
+    cudaError_t const e = launchDependentCluster(
+        &optIn[plan.longestFirst], kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
+    if (e != cudaSuccess)
+        B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(e));
+    return checkLaunch("mhaTcgen05Kernel");
 }
 
 template <typename T, bool IL>
 int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
 {
-    using L = MhaSmem<T>;
     bool const fixedLayout = p.cu_seqlens == nullptr;
     uint64_t const d = static_cast<uint64_t>(p.head_size);
     uint64_t const rowElems = 3ull * static_cast<uint64_t>(p.num_heads) * d;
     // The boxes are always 64 channels wide (two 32-channel groups when interleaved); for a smaller head the channels
     // beyond d lie outside the tensor's channel dimension and arrive as zeros, which change neither Q.K nor P.V.
-    CUtensorMap map;
+    CUtensorMap maps[3];
+    CUtensorMap& map = maps[0];
     if (IL)
     {
         // [3][N][d/32][total][32]: dim0 the 32 channels of a group, dim1 the token, dim2 the group, dim3 which of [3][N]
@@ -962,18 +1032,11 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
         if (st != BERT_B200_OK)
             return st;
     }
-    int const nbMax = (p.S + kKeyBlock - 1) / kKeyBlock;
-    int const smem = L::dynamicBytes(nbMax);
-    auto kernel = mhaTcgen05Kernel<T, IL, false>;
-    static SmemOptIn optIn;
+    maps[1] = map;
+    maps[2] = map;
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
-        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1};
-    // one persistent CTA per SM (512 TMEM columns and most of the shared memory each), items dealt round-robin
-    int const grid = divideItems(args);
-    cudaError_t const le = launchDependentCluster(&optIn, kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, map, map, map, args);
-    if (le != cudaSuccess)
-        B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
-    return checkLaunch("mhaTcgen05Kernel");
+        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1};
+    return launchItems<T, IL, false>(args, maps, stream);
 }
 
 // Separate Q, K, V tensors of shape [B][N][S][d] (the operand layout of TensorRT's attention layer), output
@@ -981,7 +1044,6 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
 template <typename T>
 int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t stream)
 {
-    using L = MhaSmem<T>;
     uint64_t const d = static_cast<uint64_t>(p.head_size), S = static_cast<uint64_t>(p.S), N = static_cast<uint64_t>(p.num_heads);
     CUtensorMap maps[3];
     void const* const base[3] = {p.q, p.k, p.v};
@@ -996,17 +1058,9 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
         if (st != BERT_B200_OK)
             return st;
     }
-    int const nbMax = (p.S + kKeyBlock - 1) / kKeyBlock;
-    int const smem = L::dynamicBytes(nbMax);
-    auto kernel = mhaTcgen05Kernel<T, false, true>;
-    static SmemOptIn optIn;
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
-        p.scale_bmm2, p.status_word, 1, 1};
-    int const grid = divideItems(args);
-    cudaError_t const le = launchDependentCluster(&optIn, kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
-    if (le != cudaSuccess)
-        B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(le));
-    return checkLaunch("mhaTcgen05Kernel");
+        p.scale_bmm2, p.status_word, 1, 1, 1};
+    return launchItems<T, false, true>(args, maps, stream);
 }
 
 } // namespace

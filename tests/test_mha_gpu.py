@@ -545,6 +545,44 @@ def test_mha_division_of_ragged_batches(cuda, B, smax, packed, int8):
     assert int(st[0]) == 0
 
 
+# INT8 pairs dealt longest first: one pair more than SMs, as many sequences as a CTA puts in order and one more (as they come), as
+# many rounds as it lists (64 x 148 pairs) and more; equal lengths among them, empty sequences last
+@pytest.mark.parametrize("B,N,smax", [(149, 1, 140), (75, 2, 300), (256, 3, 130), (257, 3, 130), (256, 37, 6), (256, 38, 6), (8, 30, 512)])
+@pytest.mark.parametrize("layout", ["packed", "interleaved", "fixed", "separate"])
+def test_mha_int8_longest_first(cuda, B, N, smax, layout):
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(B + N)
+    d = 32
+    lengths = rng.integers(0, smax + 1, size=B).astype(np.int32)
+    lengths[rng.integers(0, B, size=B // 4)] = smax // 2
+    lengths[[0, B // 2, B - 1]] = 0, smax, 0
+    cu = O.cu_seqlens(lengths)
+    packed = layout in ("packed", "interleaved")
+    x = rng.integers(-127, 128, size=(int(cu[-1]) if packed else smax * B, 3 * N * d)).astype(np.int8)
+    s1, s2 = float((4.0 / 127) ** 2 / np.sqrt(d)), 2.0 / 127
+    scales = {"scale_bmm1": s1, "scale_softmax": 127.0, "scale_bmm2": s2}
+    st = _status(cuda)
+    if packed:
+        ref = O.mha_int8(x, B, smax, N, d, s1, 127.0, s2, cu=cu)
+    else:
+        x = x.reshape(smax, B, 3 * N * d)
+        ref = O.mha_int8(x, B, smax, N, d, s1, 127.0, s2, lengths=lengths)
+    if layout == "packed":
+        out = T.mha(_t(x, cuda), B, smax, N, d, cu_seqlens=_t(cu, cuda), status=st, **scales).cpu().numpy()
+    elif layout == "fixed":
+        out = T.mha(_t(x, cuda), B, smax, N, d, mask_idx=_t(lengths, cuda), status=st, **scales).cpu().numpy()
+    elif layout == "separate":
+        q, k, v = (_t(a, cuda) for a in x.reshape(smax, B, N, 3, d).transpose(3, 1, 2, 0, 4))
+        out = T.attention_bnsd(q, k, v, kv_lengths=_t(lengths, cuda), status=st, **scales)
+        out = out.cpu().numpy().transpose(2, 0, 1, 3).reshape(smax, B, N * d)
+    else:
+        il = x.reshape(-1, N, 3, d).transpose(0, 2, 1, 3).reshape(-1, 3 * N * d)   # [3][N][d / 32][total][32]
+        out = O.from_chw32(T.mha(_t(O.to_chw32(il), cuda), B, smax, N, d, cu_seqlens=_t(cu, cuda), interleaved=True, status=st, **scales).cpu().numpy())
+    assert int(st[0]) == 0
+    _assert_int8_attention(out, ref)
+
+
 @pytest.mark.parametrize("d", [16, 48, 64])
 @pytest.mark.parametrize("lengths", [[37], [1, 16, 17, 32, 33, 0, 64, 65, 96, 97, 127, 128], [5] * 150])
 def test_mha_fp16_single_key_block(cuda, d, lengths):
