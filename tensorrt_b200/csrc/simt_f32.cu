@@ -619,8 +619,10 @@ namespace
 template <typename T, int D>
 int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 {
+    int32_t const rowBlocks = (p.S - 1) / kAttRows + 1;
+    B200_REQUIRE(rowBlocks <= 65535, "mha (SIMT): S=%d too large", p.S); // the grid's third dimension
     static SmemOptIn optIn;
-    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D>, dim3(p.num_heads, p.B, (p.S + kAttRows - 1) / kAttRows),
+    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D>, dim3(p.num_heads, p.B, rowBlocks),
         dim3(kAttThreads), sizeof(AttSmem<D>), stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
         static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
     if (e != cudaSuccess)

@@ -53,6 +53,19 @@ def test_fc_and_mha_validation():
     assert _lib.lib.bert_b200_mha(C.byref(m), None) == 3
 
 
+@pytest.mark.parametrize("head_size,limit", [(4, 65535 * 64), (64, 65535 * 64), (128, 65535 * 64), (6, 12794), (132, 12668)])
+def test_longest_fp32_attention(head_size, limit):
+    """Sequences that the kernel's grid or shared memory cannot take are refused before anything is launched."""
+    from tensorrt_b200 import _lib
+
+    m = _lib.MhaParams()
+    m.type_id, m.B, m.num_heads, m.head_size, m.scale_bmm1 = 0, 1, 1, head_size, 1.0
+    m.qkv = m.out = C.c_void_p(0x1000)
+    for m.S in (limit + 1, 2 ** 31 - 1):
+        assert _lib.lib.bert_b200_mha(C.byref(m), None) == 2   # BERT_B200_BAD_PARAM
+        assert b"S=" in _lib.lib.bert_b200_last_error()
+
+
 def test_attention_workspace_and_separate_tensor_entry_validation():
     from tensorrt_b200 import _lib
 
