@@ -117,6 +117,52 @@ def test_forward_host_async_matches_forward_host(cuda):
 
 
 @pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("writer", ["copy", "fc"])
+def test_forward_reads_weights_written_right_ahead(cuda, int8, writer):
+    """Weights and parameters overwritten on the stream between forwards, nothing synchronised: the kernels of a forward fetch
+    them ahead of their predecessors' end, but never ahead of what was enqueued before the forward. `fc`: the last matrix of a
+    layer is written by this library's own product with the unit matrix, which lets the kernels behind it start early."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(17)
+    p = _small(rng, hidden=256, heads=4, ffn=1024)
+    lengths = np.array([20, 1, 16], dtype=np.int32)
+    cu = O.cu_seqlens(lengths)
+    total, S = int(cu[-1]), int(lengths.max())
+    ids, seg = rng.integers(0, 1000, size=total).astype(np.int32), rng.integers(0, 2, size=total).astype(np.int32)
+    if int8:
+        O.calibrate_int8(p, ids, seg, cu, S)
+    enc = T.BertEncoder(p, T.INT8 if int8 else T.FP16, cuda)
+    args = (_t(ids, cuda), _t(seg, cuda), _t(cu, cuda), S)
+    sets = [[t.clone() for t in enc._keep], [torch.roll(t, 1, 0) for t in enc._keep]]
+    unit = torch.eye(1024, device=cuda, dtype=enc._keep[3].dtype)   # the feed-forward down projection: [256, 1024]
+    assert tuple(enc._keep[3].shape) == (256, 1024)
+
+    def write(i):
+        for n, (t, src) in enumerate(zip(enc._keep, sets[i])):
+            if writer == "copy" or n != 3:
+                t.copy_(src)
+        if writer == "fc":
+            T.fc(sets[i][3], unit, out_dtype=unit.dtype, out=enc._keep[3])
+
+    want = []
+    for i in range(2):
+        write(i)
+        torch.cuda.synchronize()
+        want.append(enc.forward(*args).clone())
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    got = []
+    for i in range(30):
+        write(i % 2)
+        got.append(enc.forward(*args))
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
+    assert enc.status_word() == 0
+    enc.close()
+
+
+@pytest.mark.parametrize("int8", [False, True])
 def test_forward_is_graph_capturable(cuda, int8):
     """TensorRT replays engines as CUDA graphs: a forward captured into a graph (kernels launched with programmatic
     stream serialisation included) must replay to the same bits as the eager call."""
