@@ -111,41 +111,32 @@ __device__ __forceinline__ uint32_t quantChar4(float a, float b, float c, float 
     return q.useConvert ? (q.unitScale ? packChar4Cvt(a, b, c, d) : packChar4Cvt(a, b, c, d, q.s)) : packChar4Scaled(a, b, c, d, q.s, q.lo, q.hi);
 }
 
+// W values of one row to shared memory, in 16-byte pieces.
 template <int W>
-__device__ __forceinline__ void storeChunk(__half* dst, float const (&v)[W], QuantStep const&, int validCols)
+__device__ __forceinline__ void storeChunk(__half* dst, float const (&v)[W], QuantStep const&)
 {
 #pragma unroll
     for (int g = 0; g < W / 8; ++g)
     {
-        if (g * 8 < validCols)
-        {
-            float f[8];
+        float f[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                f[j] = v[g * 8 + j];
-            *reinterpret_cast<uint4*>(dst + g * 8) = packHalf8(f);
-        }
+        for (int j = 0; j < 8; ++j)
+            f[j] = v[g * 8 + j];
+        *reinterpret_cast<uint4*>(dst + g * 8) = packHalf8(f);
     }
 }
 
 template <int W>
-__device__ __forceinline__ void storeChunk(int8_t* dst, float const (&v)[W], QuantStep const& q, int validCols)
+__device__ __forceinline__ void storeChunk(int8_t* dst, float const (&v)[W], QuantStep const& q)
 {
-    constexpr int kPiece = W < 16 ? W : 16;
 #pragma unroll
-    for (int g = 0; g < W / kPiece; ++g)
+    for (int g = 0; g < W / 16; ++g)
     {
-        if (g * 16 < validCols)
-        {
-            uint32_t w[kPiece / 4];
+        uint32_t w[4];
 #pragma unroll
-            for (int j = 0; j < kPiece / 4; ++j)
-                w[j] = quantChar4(v[g * 16 + 4 * j], v[g * 16 + 4 * j + 1], v[g * 16 + 4 * j + 2], v[g * 16 + 4 * j + 3], q);
-            if constexpr (kPiece == 16)
-                *reinterpret_cast<uint4*>(dst + g * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-            else
-                *reinterpret_cast<uint2*>(dst + g * 16) = make_uint2(w[0], w[1]);
-        }
+        for (int j = 0; j < 4; ++j)
+            w[j] = quantChar4(v[g * 16 + 4 * j], v[g * 16 + 4 * j + 1], v[g * 16 + 4 * j + 2], v[g * 16 + 4 * j + 3], q);
+        *reinterpret_cast<uint4*>(dst + g * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -208,8 +199,8 @@ __device__ __forceinline__ QuantStep fcEpilogueMath(uint32_t const (&r)[W], floa
     return QuantStep{args.outScale, args.qLo, args.qHi, true, false};
 }
 
-// ... then 128-bit stores straight from the registers of the row's thread (tile kernel).
-// ... or into a [32 rows x 32 columns] staging tile in shared memory, laid out the way a TMA store with the 32-byte
+// ... then, in the tile kernel, storeChunk into a block of the drained ring, from which whole rows are stored;
+// ... in the pair kernel into a [32 rows x 32 columns] staging tile in shared memory, laid out the way a TMA store with the 32-byte
 // (INT8) or 64-byte (FP16) swizzle expects it: row `lane`, 16-byte piece c at (c ^ f(lane)) - which also spreads the
 // 32 lanes' 128-bit stores over all banks.
 template <typename Out>
@@ -263,9 +254,10 @@ FcArgs makeFcArgs(bert_b200_fc_params const& p, int stages, int aRows, bool weig
 // With few rows a layer is bound by latency and by how fast the weights reach the SMs: one SM takes in about 100 bytes per
 // clock, so the weights of a projection have to be spread over as many SMs as possible - narrow tiles. Their MMAs take 40 cycles
 // each for any BLOCK_N up to 32, about as long as 128 rows of A (32 bytes each) take to come from shared memory, and a long K is
-// a chain of them: up to 64 rows the tile has 64 rows. Everything around the main loop is kept short: a single tile per CTA, only BLOCK_N
-// TMEM columns and about 100 KB of shared memory, so that the CTAs of the next launch fit beside the running ones and have
-// their barriers, TMEM and - where the caller says that the weights are not being written by the kernels ahead - their first
+// a chain of them: up to 64 rows the tile has 64 rows. Everything around the main loop is kept short: a single tile per CTA and only
+// BLOCK_N TMEM columns. Shared memory: about 100 KB where two CTAs share an SM, up to 200 KB where the tiles do not outnumber the SMs
+// (37 rows: 86 KB at K = 768, 173 KB at K = 3072). Where the CTAs of the next launch fit beside the running ones, they have their
+// barriers, TMEM and - where the caller says that the weights are not being written by the kernels ahead - their first
 // weight tiles in place when this one ends. The other weight tiles are at least pulled into the L2 while the kernel ahead runs.
 //   warp 0: TMA producer, warp 1: TMEM allocation and MMA issue, then 4 epilogue warps (8 from BLOCK_N = 64 on), one or two
 //   per TMEM lane quadrant. Results go through the drained ring, so that a store instruction of a warp writes whole rows of
@@ -522,7 +514,7 @@ __global__ void __launch_bounds__(FcTileSmem<BLOCK_M, BLOCK_N>::kThreads, 2)
                     constexpr int kPieces = kRow / 16;
                     uint8_t* const block = ring + (warp - 2) * 32 * (kRow + 16);
                     if (kQuadRows == 32 || lane < kQuadRows)
-                        storeChunk<kChunk>(reinterpret_cast<Out*>(block + lane * (kRow + 16)), v, q, kChunk);
+                        storeChunk<kChunk>(reinterpret_cast<Out*>(block + lane * (kRow + 16)), v, q);
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < kPieces; ++i)

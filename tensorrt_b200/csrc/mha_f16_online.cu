@@ -15,9 +15,9 @@
 //                     maximum, lazy rescale (below), p = exp2(x*scale*log2e - m), row sum, P as FP16 pairs into 64
 //                     TMEM columns of its own. The normalising epilogue of a tile is deferred into the first block of
 //                     the stream's next tile, so its wait for the last context product costs nothing.
-//   warp 8          : one lane loads the Q tiles (four slots, two per stream: with one, a tile's Q was requested only
+//   warp 8          : loads the Q tiles (four slots, two per stream: with one, a tile's Q was requested only
 //                     when the last scores of the tile before were done, which short sequences waited for).
-//   warp 9          : one lane loads K / V blocks (128 keys x 64 channels, 16 KB) into a ring of 10 stages. The
+//   warp 9          : loads K / V blocks (128 keys x 64 channels, 16 KB) into a ring of 10 stages. The
 //                     blocks of a pair stay resident for all its query tiles when they fit (S <= 640); longer
 //                     sequences stream their blocks once per two query tiles.
 //   warps 10 / 11   : the MMA warp of stream 0 / 1 (an elected lane issues). It issues the stream's scores  S = Q K_j^T
@@ -34,7 +34,7 @@
 // context accumulator in TMEM themselves (after the previous P V product has completed). The final context is
 // O / rowsum. Compared with a softmax over the exact row maximum this changes nothing but the rounding of P.
 // Measured (16 heads of 64; whole pairs dealt round-robin and one Q slot per stream before): 11 sequences of 200 ... 2000
-// tokens 203 -> 113 us, 148 x 128 43.0 us, 148 x 384 165 us, 37 x 1024 249 us; bound by the exponentials (a 128 x 128 block takes 1024
+// tokens 203 -> 113 us, 148 x 384 165 us, 37 x 1024 249 us; bound by the exponentials (a 128 x 128 block takes 1024
 // cycles of the unit) at half of their rate: the two streams' other work is not hidden behind them completely.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM and reports through the status word.
 #include "mha_share.cuh"
@@ -47,7 +47,7 @@ namespace
 {
 
 #ifdef MHA_TRACE
-// timeline of CTA 0: (role, event code, cycle) triples, 512 events per role, roles 0/1 softmax, 2/3 MMA threads
+// timeline of CTA 0: (role, event code, cycle) triples, 512 events per role, roles 0/1 softmax, 2/3 MMA warps
 #define TR_DECL(role) uint32_t trN = 0; uint32_t* const trBuf = (blockIdx.x == 0 && args.statusWord) ? args.statusWord + 16 + (role) * 1024 : nullptr
 #define TR_EVT(code) do { if (trBuf && trN < 512) { trBuf[2 * trN] = (code); trBuf[2 * trN + 1] = static_cast<uint32_t>(clock64()); ++trN; } } while (0)
 #else
@@ -251,7 +251,7 @@ __global__ void __maxnreg__(168)
         for (int i = 0; i < kStages; ++i)
         {
             mbarInit(&full[i], 1);
-            mbarInit(&empty[i], 2); // one arrival per stream (see the MMA threads)
+            mbarInit(&empty[i], 2); // one arrival per stream (see the MMA warps)
         }
         for (int i = 0; i < kQSlots; ++i)
         {
@@ -314,7 +314,7 @@ __global__ void __maxnreg__(168)
     }
     else if (warp == 9)
     {
-        // ---- K / V blocks of every sub-item, in the order the MMA threads consume them ----
+        // ---- K / V blocks of every sub-item, in the order the MMA warps consume them ----
         Walker w(args, share);
         bool ok = true;
         for (bool more = w.begin(); more && ok; more = w.next())
@@ -367,7 +367,7 @@ __global__ void __maxnreg__(168)
         auto commitAddr = [](uint32_t barAddr) {
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
         };
-        // A ring stage goes back to the loader when BOTH streams' MMA threads are done with it: each commits once, with
+        // A ring stage goes back to the loader when BOTH streams' MMA warps are done with it: each commits once, with
         // its last tile of the sub-item. A sub-item of a single tile is read by one stream only; the other stream's
         // thread still takes part in every one of its loads (passThrough below).
         auto release = [&](uint32_t stage, Walker const& w) {

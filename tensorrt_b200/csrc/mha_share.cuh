@@ -5,8 +5,8 @@
 // costs its key blocks (128 keys) and a fixed amount for what is done once per tile. Neighbours of the list share keys and
 // values, so a CTA still loads most of them once; cutting by cost instead of dealing whole pairs round-robin keeps all SMs busy
 // to the end when the sequences differ in length, and lets several SMs work on a pair when there are few pairs. Measured in
-// mha_f16_online.cu. (The INT8 kernel keeps whole pairs: it works on one tile at a time and waits for the keys of every pair it
-// starts, so cut pairs cost more there than the uneven lengths: 37 interleaved sequences of 100 ... 256 tokens 45 us, 41 us whole.)
+// mha_f16_online.cu. (The INT8 kernel divides its work in its own way, mha_items.h: it works on one tile at a time and waits for the keys of every pair
+// it starts, so pairs cut at equal costs take longer there: 37 interleaved sequences of 100 ... 256 tokens 45 us, 41 us whole.)
 #pragma once
 #include "common.cuh"
 
@@ -85,8 +85,8 @@ __device__ __forceinline__ uint64_t divideCost(uint64_t x, uint32_t y)
 // Finds the CTA's share; called by all threads. Returns whether there may be a sequence without a valid key.
 // Fewer tiles than SMs: the CTA's number says which tile is its own. Few sequences: one per lane of warp 0. In general every
 // thread sums the costs of a run of sequences, a scan over the block places the runs, and the threads in whose runs the share's
-// two ends fall write them down. That takes 1.2 us (code fetched for a single use, three barriers), which the small launches
-// would feel: one sequence of 37 tokens takes 5 us in all. Few sequences: 0.3 us.
+// two ends fall write them down. That takes 1.2 us (code fetched for a single use, three barriers), which small launches would feel:
+// a sequence of two key blocks takes some 6 us in all. Few sequences: 0.3 us.
 template <int kThreads, uint32_t kTileCost>
 __device__ __forceinline__ bool findShare(ShareArgs const& a, ShareSmem* sm)
 {

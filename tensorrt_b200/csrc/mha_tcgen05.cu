@@ -11,14 +11,15 @@
 // three sweeps over it; that is what keeps the result bit-identical with the reference's INT8 kernels.
 //
 // Persistent CTAs (one per SM) take (sequence, head) work items, or parts of them where there are few, round-robin or, in
-// ragged batches of many, each a long one, then a short one (mha_items.h). Per item a CTA loops over its 128-query tiles, so that K and V are loaded once and the tensor pipe works on the next tile
-// (of this item or the next) while the softmax warps finish the current one. 19 warps:
+// ragged batches of many, each a long one, then a short one (mha_items.h). Per item a CTA loops over its 128-query tiles,
+// so that K and V are loaded once and the tensor pipe works on the next tile (of this item or the next) while the
+// softmax warps finish the current one. 19 warps:
 //   warp 0    : TMA - the K / V blocks (128 keys each) of an item once, the Q tile of each iteration
 //               (swizzled shared-memory tiles, one mbarrier each).
-//   warp 1    : TMEM allocation (512 columns); one lane issues the context products
+//   warp 1    : TMEM allocation (512 columns); issues the context products (an elected lane does)
 //                 O  += P_j V_j           (128 x 64, accumulator in TMEM columns 384..447; for S > 384 it re-uses
 //                                          the columns of S_0, which serialises consecutive tiles)
-//   warp 18   : one lane issues the scores of the following tile, per key block as soon as the softmax warps hold
+//   warp 18   : issues the scores of the following tile, per key block as soon as the softmax warps hold
 //               the current S_j in registers:
 //                 S_j = Q K_j^T           (128 x 128 per key block, accumulators in TMEM columns 128j..)
 //               (with a single key block per sequence warp 1 issues both and this warp idles).
@@ -146,7 +147,7 @@ __device__ __forceinline__ uint32_t packProb4(float a, float b, float c, float d
 
 // The row reductions only join the four warps that own the columns of the same 32 query rows (one TMEM lane
 // quadrant). FP16: one named barrier per quadrant, so that the quadrants drift apart instead of waiting for the
-// slowest (+6 % at S = 384). INT8: all sixteen warps in step - its per-key-block hand-overs to the MMA threads need
+// slowest (+6 % at S = 384). INT8: all sixteen warps in step - its per-key-block hand-overs to the MMA warps need
 // every warp's arrival anyway, and drifting quadrants delay them (per-quadrant barriers: -4 %).
 template <bool kPerQuadrant>
 __device__ __forceinline__ void softmaxBarrier(int quad)

@@ -2,9 +2,9 @@
 // full precision (TF32 would break the 1e-5 tolerance the reference configuration states for FP32,
 // plugin/bertQKVToContextPlugin/CustomQKVToContextPluginDynamic_PluginConfig.yaml:72-76), so these
 // are SIMT kernels; the FP16 / INT8 paths live in fc_tcgen05.cu and mha_tcgen05.cu.
-// The attention kernel also serves FP16 tensors (FP32 arithmetic) for the shapes the tensor-core kernel does not
-// take - heads wider than 64 or not a multiple of 16, sequences longer than 512 - the shapes the reference sends
-// to its unfused runner as well.
+// The attention kernels also serve FP16 tensors (FP32 arithmetic) for the shapes the tensor-core kernels do not
+// take - heads wider than 64 or not a multiple of 16, a scale that is not positive - which the reference sends to its unfused
+// runner as well.
 //
 // Replaces cublas{S,H}gemmStridedBatched + softmax kernels of UnfusedMHARunner::run
 // (plugin/bertQKVToContextPlugin/mhaRunner.cu:533-601) and the FP32 cublasLtMatmul of the FC plugin
@@ -50,14 +50,11 @@ constexpr int kFcF32Ring = kStages * 2 * kTile * kPitch; // floats
 constexpr int kFcF32Part = kTile * kTile;                // sums of a segment, as the threads hold them (see partIndex)
 static_assert(kFcF32Ring >= kFcF32Part, "the last segment's sums reuse the ring");
 
-__device__ __forceinline__ void fma2(uint64_t& c, uint64_t a, uint64_t b)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-
 __device__ __forceinline__ float sumPair(uint64_t v)
 {
-    return __uint_as_float(static_cast<uint32_t>(v)) + __uint_as_float(static_cast<uint32_t>(v >> 32));
+    float lo, hi;
+    unpack2(v, lo, hi);
+    return lo + hi;
 }
 
 // kBytes (16 or 4) from global to shared memory, zeros when `valid` is false.
@@ -226,7 +223,7 @@ __global__ void __launch_bounds__(kFcF32Threads, kFcF32CtasPerSm) fcF32Kernel(Fc
             for (int i = 0; i < 8; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    fma2(acc[i][j], av[cur][i], bv[cur][j]);
+                    acc[i][j] = fma2(av[cur][i], bv[cur][j], acc[i][j]);
         }
         stage = stage + 1 == kStages ? 0 : stage + 1;
     }
@@ -423,8 +420,8 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                 {
-                    fma2(acc[i][j], a[i].x, b.x);
-                    fma2(acc[i][j], a[i].y, b.y);
+                    acc[i][j] = fma2(a[i].x, b.x, acc[i][j]);
+                    acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
                 }
             }
         }

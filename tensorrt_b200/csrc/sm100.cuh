@@ -90,24 +90,6 @@ __device__ __forceinline__ bool mbarTryWaitAddr(uint32_t barAddr, uint32_t parit
     return ok != 0;
 }
 
-// Non-blocking form: mbarrier.try_wait may suspend the thread for a system-dependent time before it reports an
-// incomplete phase; a thread that polls several barriers in turn (and must not sleep on one while another completes)
-// uses test_wait, which returns at once.
-__device__ __forceinline__ bool mbarTestWaitAddr(uint32_t barAddr, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(ok)
-        : "r"(barAddr), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
 // Every spin in these kernels is bounded: after kWaitLimitNs without progress the waiter records
 // `code` in *abortFlag (shared memory; every later wait in the CTA returns immediately) and
 // returns false. The kernel then drains, frees its TMEM and exits; the host sees the status word.
@@ -213,16 +195,8 @@ __device__ __forceinline__ void prefetchTensorMap(CUtensorMap const* map)
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// Tiled loads into this CTA's shared memory, completion on an mbarrier of this CTA. No multicast.
-__device__ __forceinline__ void tmaLoad2d(void* dst, CUtensorMap const* map, uint64_t* bar, int32_t c0, int32_t c1)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smemAddr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(c0), "r"(c1)
-        : "memory");
-}
-
-// The same with shared::cta addresses that the loops of a role keep in registers.
+// Tiled loads into this CTA's shared memory, completion on an mbarrier of this CTA. No multicast. Here with shared::cta addresses
+// that the loops of a role keep in registers.
 __device__ __forceinline__ void tmaLoad2dAddr(uint32_t dst, CUtensorMap const* map, uint32_t bar, int32_t c0, int32_t c1)
 {
     asm volatile(
@@ -314,32 +288,7 @@ __device__ __forceinline__ void tcCommitAddr(uint32_t barAddr)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by a single thread.
-__device__ __forceinline__ void mmaF16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t iDesc, bool accumulate)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}" ::"r"(dTmem),
-        "l"(aDesc), "l"(bDesc), "r"(iDesc), "r"(static_cast<uint32_t>(accumulate))
-        : "memory");
-}
-
-__device__ __forceinline__ void mmaI8(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t iDesc, bool accumulate)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
-        "}" ::"r"(dTmem),
-        "l"(aDesc), "l"(bDesc), "r"(iDesc), "r"(static_cast<uint32_t>(accumulate))
-        : "memory");
-}
-
-// The same with the 64-bit descriptors assembled inside the asm block from their 32-bit halves: a thread that issues
+// D[tmem] (+)= A[smem] * B[smem]; issued by a single thread. The 64-bit descriptors are assembled inside the asm block from their 32-bit halves: a thread that issues
 // many small MMAs keeps one low word per operand tile (start address in bits 0-13; + bytes >> 4 moves it) and one
 // constant high word per operand kind in registers instead of rebuilding or holding dozens of 64-bit descriptors.
 template <bool kInt8>
@@ -546,36 +495,6 @@ __device__ __forceinline__ uint64_t makeSmemDesc(uint32_t saddr, uint32_t lboByt
 {
     return static_cast<uint64_t>((saddr >> 4) & 0x3fffu) | (static_cast<uint64_t>((lboBytes >> 4) & 0x3fffu) << 16)
         | (static_cast<uint64_t>((sboBytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (swizzle << 61);
-}
-
-// Two FP32 operations in one issue slot (the pipes' rate is the same).
-__device__ __forceinline__ uint64_t pack2(float lo, float hi)
-{
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t v;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-    return v;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
-{
-    uint64_t v;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-    uint64_t v;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
 }
 
 // Instruction descriptor (32 bit) for kind::f16 / kind::i8, dense, no negate, no saturate.
