@@ -200,6 +200,7 @@ enum
  * and the host layer transposes it once at plugin construction.
  * lda/ldc are row strides in elements. FP16/INT8 require k % 16 == 0 (bytes of a row multiple
  * of 16) and 16-byte aligned A/Wt/C.
+ * A row of C has the same bits whatever m.
  * `status_word` (may be NULL) is a device uint32 that receives a non-zero code if a bounded
  * device wait expired.
  * ref: plugin/fcPlugin/fcPlugin.cpp:551-610 (FCPluginDynamic::enqueue -> cublasLtMatmul);
