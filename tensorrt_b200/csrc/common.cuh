@@ -219,6 +219,28 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
     return v;
 }
 
+// The word at the same shared-memory location in CTA `rank` of this cluster.
+__device__ __forceinline__ uint32_t ldSharedCluster(uint32_t const* local, int rank)
+{
+    uint32_t v;
+    asm volatile(
+        "{\n\t"
+        ".reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %1, %2;\n\t"
+        "ld.shared::cluster.u32 %0, [a];\n\t"
+        "}"
+        : "=r"(v)
+        : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank)
+        : "memory");
+    return v;
+}
+
+// x/2 (1 + erf(x / sqrt 2)) at full FP32 precision.
+__device__ __forceinline__ float geluErfF32(float x)
+{
+    return 0.5f * x * (1.f + erff(x * 0.70710678118654752440f));
+}
+
 __device__ __forceinline__ float warpSum(float v)
 {
 #pragma unroll

@@ -1,0 +1,559 @@
+// FP32 (type_id 0) fully connected layer on the sm_100a tensor cores: C = act(alpha * A * Wt^T + bias) at full FP32 precision.
+//
+// Replaces the FP32 cublasLtMatmul of the FC plugin (plugin/fcPlugin/fcPlugin.cpp:551-610). TF32 would break the 1e-5 tolerance
+// that the reference configuration states for FP32 (plugin/bertQKVToContextPlugin/CustomQKVToContextPluginDynamic_PluginConfig.yaml:72-76),
+// so every operand is cut into three BF16 numbers by truncation, x = h + m + l, which is exact (8 + 8 + 8 bits of the mantissa), and
+// the six products of at least 2^-16 of the largest are formed: h h + (h m + m h) + (h l + m m + l h). The three that are left
+// out are below 2^-24 of a product in sum, less than the rounding of one FP32 addition.
+//
+// The tensor core adds into its FP32 accumulator by truncation, so nothing is summed there for long: a chunk of 64 products per
+// output starts from zero, its five small products first and h h last (four additions at the chunk's own magnitude), and
+// the chunks are added in registers, rounded to nearest. Error against 64 bits: see fcF32.
+#include "sm100.cuh"
+
+namespace b200
+{
+
+int32_t fcF32Simt(bert_b200_fc_params const& p, cudaStream_t stream);
+
+namespace
+{
+
+constexpr int kTileM = 128;
+constexpr int kChunk = 64;      // of K: one 128-byte row of a BF16 operand tile, two of the FP32 tiles
+constexpr int kWorkers = 16;    // warps, in two groups of eight
+constexpr int kThreadsF32 = 64 + kWorkers * 32;
+constexpr int kMaxSegments = 8; // portable cluster size
+constexpr int kParts = 2;       // chunks whose parts are in place
+
+struct FcF32TcArgs
+{
+    int64_t M, N, K, lda, ldc;
+    float const* A;
+    float const* Wt;
+    float* C;
+    float const* bias;
+    int32_t act;
+    float alpha;
+    int32_t nTiles;   // tiles along N
+    int32_t segments; // of K
+    int32_t ctas;     // per tile: 1 or `segments`
+    int32_t wide;     // rows of C may be stored in 16-byte pieces
+    uint32_t* statusWord;
+};
+
+template <int BN>
+struct FcF32Smem
+{
+    static constexpr int kStages = BN >= 96 ? 2 : 3; // FP32 tiles
+    static constexpr int kABytes = kTileM * kChunk * 4;
+    static constexpr int kWBytes = BN * kChunk * 4;
+    static constexpr int kStageBytes = kABytes + kWBytes;
+    static constexpr int kPlaneBytes = BN * kChunk * 2; // one BF16 part of the Wt tile
+    static constexpr int kPlanesOff = kStages * kStageBytes;
+    static constexpr int kBarrierOff = kPlanesOff + kParts * 3 * kPlaneBytes;
+    // stFull[stages] stFree[stages] ready[parts] done[parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt, whether any is set
+    static constexpr int kFlagsOff = kBarrierOff + (2 * kStages + 2 * kParts + 2) * 8 + 16;
+    static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
+    static constexpr int kDynamic = kTotal + 1024;
+    static constexpr int kPitch = BN + 4; // floats: sums of a tile over the drained FP32 tiles
+    static constexpr int kTmem = 2 * BN + kParts * 96 <= 256 ? 256 : 512;
+    static_assert(kDynamic <= 232448, "shared memory of one CTA");
+    static_assert(kTileM * kPitch * 4 <= kPlanesOff, "the sums fit the ring");
+    static_assert(2 * BN + kParts * 96 <= kTmem, "tensor memory");
+};
+
+// Two floats into packed BF16 parts; `range` becomes the largest magnitude so far (NaN once there is one).
+__device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, float& range)
+{
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(range) : "f"(a), "f"(b));
+    uint32_t const ua = __float_as_uint(a), ub = __float_as_uint(b);
+    h = __byte_perm(ua, ub, 0x7632);
+    float ra, rb;
+    unpack2(add2(pack2(a, b), pack2(__uint_as_float((ua & 0xffff0000u) ^ 0x80000000u), __uint_as_float((ub & 0xffff0000u) ^ 0x80000000u))), ra, rb);
+    uint32_t const va = __float_as_uint(ra), vb = __float_as_uint(rb);
+    m = __byte_perm(va, vb, 0x7632);
+    float la, lb;
+    unpack2(add2(pack2(ra, rb), pack2(__uint_as_float((va & 0xffff0000u) ^ 0x80000000u), __uint_as_float((vb & 0xffff0000u) ^ 0x80000000u))), la, lb);
+    l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+}
+
+// Whether numbers up to `range` in magnitude have parts that are good enough: infinities and NaN have none, and the last parts of
+// the largest must be normal BF16 numbers (from 2^-102 on) for the sum to keep FP32 precision. Zeros are fine.
+__device__ __forceinline__ bool splitIsInexact(float range)
+{
+    return !(range < INFINITY) || (range > 0.f && range < 1.9721522630525295e-31f);
+}
+
+__device__ __forceinline__ void tmemStore8(uint32_t taddr, uint32_t const (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+// 32, 24, 16 or 8 columns, waited for.
+__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[32])
+{
+    tmemLoad32(taddr, r);
+    tmemLoadWait32(r);
+}
+__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[16])
+{
+    tmemLoad16(taddr, r);
+    tmemLoadWait16(r);
+}
+__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[24])
+{
+    tmemLoadCols(taddr, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
+    tmemLoadCols(taddr + 16, *reinterpret_cast<uint32_t(*)[8]>(&r[16]));
+}
+
+// Bound by the ALU work of cutting the operands (next to it: the tensor cores at six products, 1830 cycles per chunk of a 128 x 128
+// tile). One 128 x BN tile per CTA, or one segment of its K:
+//   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
+//   warp 1    : TMEM allocation, MMA issue. The parts of A are operands in TMEM - from shared memory both operands of a
+//               128 x 128 tile would take its whole bandwidth -, those of Wt in shared memory.
+//   warps 2-17: the parts of a chunk, the two groups of eight warps taking chunks in turn: 32 numbers of a row of A per thread, to
+//               TMEM, and whole 16-byte pieces of the parts of Wt, to shared memory. And all of them, for every chunk, its
+//               sums (32 rows, a quarter of the columns per warp) from TMEM into registers. TMEM accumulators and parts are
+//               double-buffered.
+// K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
+// all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
+// An output whose row of A or Wt holds numbers without exact parts (splitIsInexact) is computed again by plain FP32 multiply-adds.
+template <int BN, bool kHold>
+__global__ void __launch_bounds__(kThreadsF32, 1)
+    fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, FcF32TcArgs const p)
+{
+    using L = FcF32Smem<BN>;
+    constexpr uint32_t kIdesc = makeInstrDesc(1u, 1u, 0u, 0u, 128u, static_cast<uint32_t>(BN));
+    constexpr int kCols = BN / 4; // accumulator columns per worker thread
+    constexpr uint32_t kPartsCol = 2 * BN;
+
+    extern __shared__ uint8_t smemRaw[];
+    uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t* const stFull = reinterpret_cast<uint64_t*>(smem + L::kBarrierOff);
+    uint64_t* const stFree = stFull + L::kStages;
+    uint64_t* const ready = stFree + L::kStages; // parts of a chunk in place
+    uint64_t* const done = ready + kParts;       // their products complete
+    uint64_t* const accFree = done + kParts;     // an accumulator has been read
+    uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(accFree + 2);
+    volatile uint32_t* const abortFlag = tmemSlot + 1;
+    uint32_t* const flagA = reinterpret_cast<uint32_t*>(smem + L::kFlagsOff);
+    uint32_t* const flagW = flagA + kTileM;
+    uint32_t* const flagAny = flagW + BN;
+    float* const sums = reinterpret_cast<float*>(smem);
+
+    int const warp = threadIdx.x >> 5;
+    int const lane = threadIdx.x & 31;
+    int const rank = p.ctas > 1 ? static_cast<int>(blockIdx.x % p.ctas) : 0;
+    int64_t const tile = blockIdx.x / p.ctas;
+    int64_t const m0 = tile / p.nTiles * kTileM;
+    int64_t const n0 = tile % p.nTiles * BN;
+    int const kChunks = static_cast<int>((p.K + kChunk - 1) / kChunk);
+    auto segmentBegin = [&](int s) { return static_cast<int>(static_cast<int64_t>(kChunks) * s / p.segments); };
+    int const first = p.ctas > 1 ? segmentBegin(rank) : 0;
+    int const count = (p.ctas > 1 ? segmentBegin(rank + 1) : kChunks) - first;
+
+    if (threadIdx.x == 0)
+    {
+        for (int i = 0; i < L::kStages; ++i)
+        {
+            mbarInit(&stFull[i], 1);
+            mbarInit(&stFree[i], kWorkers / 2);
+        }
+        for (int i = 0; i < kParts; ++i)
+        {
+            mbarInit(&ready[i], kWorkers / 2);
+            mbarInit(&done[i], 1);
+        }
+        for (int i = 0; i < 2; ++i)
+            mbarInit(&accFree[i], kWorkers);
+        *abortFlag = 0;
+        fenceBarrierInit();
+        prefetchTensorMap(&mapA);
+        prefetchTensorMap(&mapW);
+    }
+    for (int i = threadIdx.x; i < kTileM + BN + 1; i += kThreadsF32)
+        flagA[i] = 0;
+    if (warp == 1)
+        tmemAlloc(tmemSlot, L::kTmem);
+    tcFenceBefore();
+    __syncthreads();
+    tcFenceAfter();
+    uint32_t const tmemBase = *tmemSlot;
+    gridDependencyLaunch();
+    gridDependencyWait();
+
+    uint64_t acc[kCols / 2] = {}; // sums over the chunks, column pairs
+    if (warp == 0)
+    {
+        bool ok = true;
+        int stage = 0;
+        uint32_t phase = 1;
+        for (int c = 0; c < count && ok; ++c)
+        {
+            ok = mbarWaitWarp(&stFree[stage], phase, abortFlag, kWaitStageFree);
+            if (ok && electOne())
+            {
+                uint32_t const bar = smemAddr(&stFull[stage]);
+                uint32_t const a = smemAddr(smem) + stage * L::kStageBytes;
+                int32_t const k = (first + c) * kChunk;
+                mbarArriveExpectTxAddr(bar, L::kStageBytes);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    tmaLoad2dAddr(a + h * (L::kABytes / 2), &mapA, bar, k + h * 32, static_cast<int32_t>(m0));
+                    tmaLoad2dAddr(a + L::kABytes + h * (L::kWBytes / 2), &mapW, bar, k + h * 32, static_cast<int32_t>(n0));
+                }
+            }
+            __syncwarp();
+            if (++stage == L::kStages)
+            {
+                stage = 0;
+                phase ^= 1u;
+            }
+        }
+    }
+    else if (warp == 1)
+    {
+        uint64_t const descZero = makeSmemDesc(0, 16, 1024, kSwizzle128B);
+        uint32_t const descHi = static_cast<uint32_t>(descZero >> 32);
+        uint32_t const wLo = static_cast<uint32_t>(descZero) + (smemAddr(smem + L::kPlanesOff) >> 4);
+        bool ok = true;
+        for (int c = 0; c < count && ok; ++c)
+        {
+            uint32_t const s = c & 1, round = c >> 1;
+            ok = (c < 2 || mbarWaitWarp(&accFree[s], (round - 1) & 1u, abortFlag, kWaitAccFree))
+                && mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
+            tcFenceAfter();
+            if (ok && electOne())
+            {
+                // parts (A, Wt), the smallest products first
+                constexpr int kOrder[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+                uint32_t const a = tmemBase + kPartsCol + s * 96;
+                uint32_t const w = wLo + s * (3 * L::kPlaneBytes >> 4);
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mmaF16TmemA(tmemBase + s * BN, a + kOrder[i][0] * 32 + k * 8, w + kOrder[i][1] * (L::kPlaneBytes >> 4) + k * 2, descHi,
+                            kIdesc, i != 0 || k != 0);
+                tcCommit(&done[s]);
+            }
+            __syncwarp();
+        }
+    }
+    else
+    {
+        int const quad = warp & 3;
+        int const group = (warp - 2) >> 3; // takes every second chunk
+        int const w = (warp - 2) & 7;
+        int const half = w >> 2;           // which 32 of a chunk's K of A
+        int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns
+        bool const hasRows = m0 + quad * 32 < p.M; // warp-uniform; products of the other rows are never read
+        uint32_t const tRow = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
+        // Sums of the segments before: touched once per segment and kept out of the registers on purpose, which are all taken in the
+        // loop (spilled by the compiler they cost 14 us of 1024 x 2304 x 768: beside so much shared memory the L1 holds little).
+        volatile uint64_t tot[kHold ? kCols / 2 : 1];
+        int segment = 0;
+        int segmentEnd = segmentBegin(1);
+        bool ok = true;
+        // the sums of chunk c
+        auto promote = [&](int c) {
+            ok = ok && mbarWaitWarp(&done[c & 1], (c >> 1) & 1u, abortFlag, kWaitAccFull);
+            tcFenceAfter();
+            if (hasRows)
+            {
+                uint32_t x[kCols];
+                tmemLoadCols(tRow + (c & 1) * BN + cols * kCols, x);
+#pragma unroll
+                for (int i = 0; i < kCols / 2; ++i)
+                    acc[i] = add2(acc[i], pack2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])));
+            }
+            tcFenceBefore();
+            __syncwarp();
+            if (lane == 0)
+                mbarArrive(&accFree[c & 1]);
+            if constexpr (kHold)
+                if (c + 1 == segmentEnd)
+                {
+                    ++segment;
+                    segmentEnd = segmentBegin(segment + 1);
+#pragma unroll
+                    for (int i = 0; i < kCols / 2; ++i)
+                    {
+                        if (segment > 1)
+                            acc[i] = add2(tot[i], acc[i]);
+                        if (segment < p.segments)
+                        {
+                            tot[i] = acc[i];
+                            acc[i] = 0;
+                        }
+                    }
+                }
+        };
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int c = 0; c < count; ++c)
+        {
+            uint32_t const s = c & 1;
+            if (c >= 2)
+                promote(c - 2); // its products are complete: so is what they read where this chunk's parts go
+            if (static_cast<int>(s) == group)
+            {
+                ok = ok && mbarWaitWarp(&stFull[stage], phase, abortFlag, kWaitTmaFull);
+                uint8_t const* const fp = smem + stage * L::kStageBytes;
+                if (hasRows)
+                {
+                    int const row = quad * 32 + lane;
+                    float4 const* const src = reinterpret_cast<float4 const*>(fp + half * (L::kABytes / 2) + row * 128);
+                    uint32_t const t = tRow + kPartsCol + s * 96 + half * 16;
+                    float range = 0.f;
+#pragma unroll
+                    for (int g = 0; g < 2; ++g)
+                    {
+                        float4 v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            v[i] = src[(4 * g + i) ^ (row & 7)];
+                        uint32_t h[8], m[8], l[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                        {
+                            splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], range);
+                            splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], range);
+                        }
+                        tmemStore8(t + g * 8, h);
+                        tmemStore8(t + g * 8 + 32, m);
+                        tmemStore8(t + g * 8 + 64, l);
+                    }
+                    if (splitIsInexact(range))
+                        flagA[row] = *flagAny = 1;
+                }
+                // eight numbers of a row of Wt: 16 bytes of each part
+                uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
+                constexpr int kAhead = BN == 32 ? 1 : BN == 96 ? 3 : 2; // rows on their way before the first is cut
+#pragma unroll
+                for (int r0 = 0; r0 < BN / 32; r0 += kAhead)
+                {
+                    float4 v[kAhead][2];
+#pragma unroll
+                    for (int i = 0; i < kAhead; ++i)
+                    {
+                        int const row = (r0 + i) * 32 + lane;
+                        float4 const* const src = reinterpret_cast<float4 const*>(fp + L::kABytes + (w >> 2) * (L::kWBytes / 2) + row * 128);
+                        v[i][0] = src[(2 * (w & 3)) ^ (row & 7)];
+                        v[i][1] = src[(2 * (w & 3) + 1) ^ (row & 7)];
+                    }
+#pragma unroll
+                    for (int i = 0; i < kAhead; ++i)
+                    {
+                        int const row = (r0 + i) * 32 + lane;
+                        uint4 h, m, l;
+                        float range = 0.f;
+                        splitPair(v[i][0].x, v[i][0].y, h.x, m.x, l.x, range);
+                        splitPair(v[i][0].z, v[i][0].w, h.y, m.y, l.y, range);
+                        splitPair(v[i][1].x, v[i][1].y, h.z, m.z, l.z, range);
+                        splitPair(v[i][1].z, v[i][1].w, h.w, m.w, l.w, range);
+                        uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
+                        *reinterpret_cast<uint4*>(dst) = h;
+                        *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
+                        *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
+                        if (splitIsInexact(range))
+                            flagW[row] = *flagAny = 1;
+                    }
+                }
+                fenceProxyAsync();
+                tmemStoreWait();
+                tcFenceBefore();
+                __syncwarp();
+                if (lane == 0)
+                {
+                    mbarArrive(&ready[s]);
+                    mbarArrive(&stFree[stage]);
+                }
+            }
+            if (++stage == L::kStages)
+            {
+                stage = 0;
+                phase ^= 1u;
+            }
+        }
+        for (int c = count < 2 ? 0 : count - 2; c < count; ++c)
+            promote(c);
+    }
+
+    __syncthreads(); // the ring is drained
+    bool const aborted = *abortFlag != 0;
+    if (aborted)
+    {
+        uint64_t const t0 = globalTimerNs();
+        while (globalTimerNs() - t0 < 1000000ull)
+            __nanosleep(1000);
+        if (threadIdx.x == 0 && p.statusWord)
+            atomicMax(p.statusWord, *abortFlag);
+        __syncthreads();
+    }
+    if (warp == 1)
+    {
+        tcFenceAfter();
+        tmemFree(tmemBase, L::kTmem);
+    }
+    if (warp >= 2)
+    {
+        float* const dst = sums + ((warp & 3) * 32 + lane) * L::kPitch + ((warp - 2) >> 2) * kCols;
+#pragma unroll
+        for (int i = 0; i < kCols / 4; ++i)
+        {
+            float4 v;
+            unpack2(acc[2 * i], v.x, v.y);
+            unpack2(acc[2 * i + 1], v.z, v.w);
+            *reinterpret_cast<float4*>(dst + 4 * i) = v;
+        }
+    }
+    bool exact = true;
+    if (p.ctas > 1)
+    {
+        clusterBarrier();
+        for (int s = 0; s < p.ctas; ++s)
+            exact = exact && ldSharedCluster(flagAny, s) == 0;
+    }
+    else
+    {
+        __syncthreads();
+        exact = *flagAny == 0;
+    }
+    constexpr int kPieces = BN / 4;
+    for (int i = rank * kThreadsF32 + threadIdx.x; i < kTileM * kPieces && !aborted; i += p.ctas * kThreadsF32)
+    {
+        int const r = i / kPieces, c = i % kPieces * 4;
+        int64_t const m = m0 + r, n = n0 + c;
+        if (m >= p.M || n >= p.N)
+            continue;
+        float const* const at = sums + r * L::kPitch + c;
+        float4 v;
+        if (p.ctas > 1)
+        {
+            float4 x[kMaxSegments];
+#pragma unroll
+            for (int s = 0; s < kMaxSegments; ++s) // all on their way before the first is added
+                if (s < p.ctas)
+                    x[s] = ldSharedCluster4(at, s);
+            v = x[0];
+#pragma unroll
+            for (int s = 1; s < kMaxSegments; ++s)
+                if (s < p.ctas)
+                    v = make_float4(v.x + x[s].x, v.y + x[s].y, v.z + x[s].z, v.w + x[s].w);
+        }
+        else
+            v = *reinterpret_cast<float4 const*>(at);
+        float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            if (n + j >= p.N)
+                break;
+            if (!exact)
+            {
+                bool again = false;
+                for (int s = 0; s < p.ctas; ++s)
+                    again = again || (p.ctas > 1 ? (ldSharedCluster(flagA + r, s) | ldSharedCluster(flagW + c + j, s)) : (flagA[r] | flagW[c + j])) != 0;
+                if (again)
+                {
+                    o[j] = 0.f;
+                    for (int64_t k = 0; k < p.K; ++k)
+                        o[j] = fmaf(p.A[m * p.lda + k], p.Wt[(n + j) * p.K + k], o[j]);
+                }
+            }
+            o[j] = o[j] * p.alpha + (p.bias ? __ldg(p.bias + n + j) : 0.f);
+            if (p.act == BERT_B200_ACT_GELU_ERF)
+                o[j] = geluErfF32(o[j]);
+        }
+        float* const dst = p.C + m * p.ldc + n;
+        if (p.wide && n + 3 < p.N)
+            *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+        else
+            for (int j = 0; j < 4 && n + j < p.N; ++j)
+                dst[j] = o[j];
+    }
+    if (p.ctas > 1)
+        clusterBarrier(); // nobody leaves while its sums are being read
+}
+
+template <int BN, bool kHold>
+int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaStream_t stream)
+{
+    CUtensorMap mapA, mapW;
+    uint64_t const dimsA[2] = {static_cast<uint64_t>(p.k), static_cast<uint64_t>(p.m)}, stridesA[1] = {static_cast<uint64_t>(p.lda) * 4};
+    uint64_t const dimsW[2] = {static_cast<uint64_t>(p.k), static_cast<uint64_t>(p.n)}, stridesW[1] = {static_cast<uint64_t>(p.k) * 4};
+    uint32_t const boxA[2] = {32, kTileM}, boxW[2] = {32, BN};
+    int32_t st = makeTensorMap(&mapA, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.a, dimsA, stridesA, boxA, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (st == BERT_B200_OK)
+        st = makeTensorMap(&mapW, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.wt, dimsW, stridesW, boxW, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (st != BERT_B200_OK)
+        return st;
+    int64_t const mTiles = (p.m + kTileM - 1) / kTileM, nTiles = (p.n + BN - 1) / BN;
+    FcF32TcArgs const args{p.m, p.n, p.k, p.lda, p.ldc, static_cast<float const*>(p.a), static_cast<float const*>(p.wt), static_cast<float*>(p.c),
+        p.bias, p.activation, p.alpha, static_cast<int32_t>(nTiles), segments, ctas, p.ldc % 4 == 0 && aligned16(p.c) ? 1 : 0, p.status_word};
+    static SmemOptIn optIn;
+    cudaError_t const e = launchDependentCluster(&optIn, fcF32TcKernel<BN, kHold>, dim3(static_cast<unsigned>(mTiles * nTiles * ctas)),
+        dim3(kThreadsF32), FcF32Smem<BN>::kDynamic, stream, ctas, mapA, mapW, args);
+    if (e != cudaSuccess)
+        B200_FAIL(BERT_B200_CUDA_ERROR, "fcF32TcKernel: %s", cudaGetErrorString(e));
+    return checkLaunch("fcF32TcKernel");
+}
+
+} // namespace
+
+// From K = 384 on. Error against 64 bits (2-norm, normal inputs) here / of the FP32 multiply-adds of fcF32Simt: K = 384 1.31e-7 / 1.34e-7,
+// 768 1.34e-7 / 1.40e-7, 1024 1.36e-7 / 1.57e-7, 3072 1.44e-7 / 2.56e-7, 4096 1.47e-7 / 2.94e-7; below, the truncation of the tensor core
+// shows (K = 36 1.12e-7 / 0.81e-7) and the multiply-adds stay. They also take what the TMA unit does not: rows that are no
+// multiple of 16 bytes apart, sizes beyond its coordinates. Time, same order: 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 10.9 / 14.9 us, 128 x 768 x
+// 3072 13.8 / 44.6 us, 1024 x 2304 x 768 31.5 / 95.7 us, 4096 x 1024 x 4096 217 / 843 us.
+int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
+{
+    constexpr int64_t kMax = 1ll << 31;
+    bool const tma = p.k % 4 == 0 && p.lda % 4 == 0 && aligned16(p.a) && aligned16(p.wt) && p.m < kMax && p.n < kMax && p.k < kMax && p.lda < (1ll << 37);
+    int64_t const mTiles = (p.m + kTileM - 1) / kTileM;
+    if (!tma || p.k < 384 || mTiles * ((p.n + 31) / 32) * kMaxSegments >= kMax)
+        return fcF32Simt(p, stream);
+    // Segments: few rows are spread over more SMs by them, and each costs a CTA that takes them in turn another pass over its sums.
+    int64_t const kChunks = (p.k + kChunk - 1) / kChunk;
+    int const segments = kChunks >= 24 ? 8 : kChunks >= 12 ? 4 : 2;
+    // Width of the tiles, and whether a CTA takes all segments: what the measured cycles per chunk and per CTA, times the waves of CTAs,
+    // make shortest. Clusters find fewer places than there are SMs.
+    int bestN = 128, bestCtas = 1;
+    int64_t best = 0;
+    for (int bn = 128; bn >= 32; bn -= 32)
+        for (int ctas = 1; ctas <= segments; ctas += segments - 1)
+        {
+            int64_t const slots = smCount() * (ctas == 1 ? 148 : ctas == 2 ? 140 : ctas == 4 ? 128 : 112) / 148;
+            int64_t const waves = (mTiles * ((p.n + bn - 1) / bn) * ctas + slots - 1) / slots;
+            int64_t const fixed = ctas == 1 ? 9000 + (bn == 128 ? 3000 : 1000) * (segments - 1) : 10000 + 700 * ctas;
+            int64_t const cost = waves * ((kChunks + ctas - 1) / ctas * (bn == 128 ? 2880 : bn == 96 ? 2330 : bn == 64 ? 1880 : 1400) + fixed);
+            if (best == 0 || cost < best)
+            {
+                best = cost;
+                bestN = bn;
+                bestCtas = ctas;
+            }
+        }
+    using Launch = int32_t (*)(bert_b200_fc_params const&, int, int, cudaStream_t);
+    static constexpr Launch kLaunch[2][4] = {{launchF32Tc<32, false>, launchF32Tc<64, false>, launchF32Tc<96, false>, launchF32Tc<128, false>},
+        {launchF32Tc<32, true>, launchF32Tc<64, true>, launchF32Tc<96, true>, launchF32Tc<128, true>}};
+    return kLaunch[segments > bestCtas][bestN / 32 - 1](p, segments, bestCtas, stream);
+}
+
+} // namespace b200

@@ -171,11 +171,6 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
         : "memory");
 }
 
-__device__ __forceinline__ void tmemStoreWait()
-{
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 // IL (INT8 only): CHW32-interleaved tensors. Q, K and V tiles then arrive as two 32-channel sub-tiles of
 // [128 tokens][32 B] (32-byte swizzle); the head dimension is covered by one MMA per sub-tile.
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];

@@ -1,7 +1,5 @@
-// FP32 (type_id 0) fully-connected and attention kernels. FP32 has no tensor-core path that keeps
-// full precision (TF32 would break the 1e-5 tolerance the reference configuration states for FP32,
-// plugin/bertQKVToContextPlugin/CustomQKVToContextPluginDynamic_PluginConfig.yaml:72-76), so these
-// are SIMT kernels; the FP16 / INT8 paths live in fc_tcgen05.cu and mha_tcgen05.cu.
+// FP32 (type_id 0) attention, and the fully-connected layers that the tensor-core kernel of fc_f32_tcgen05.cu does not take (a short K,
+// rows that are not 16-byte aligned): SIMT kernels at full FP32 precision.
 // The attention kernels also serve FP16 tensors (FP32 arithmetic) for the shapes the tensor-core kernels do not
 // take - heads wider than 64 or not a multiple of 16, a scale that is not positive - which the reference sends to its unfused
 // runner as well.
@@ -16,11 +14,6 @@ namespace b200
 
 namespace
 {
-
-__device__ __forceinline__ float geluErf(float x)
-{
-    return 0.5f * x * (1.f + erff(x * 0.70710678118654752440f));
-}
 
 // ---- fully connected ------------------------------------------------------------------------------------------------
 // C[m,n] = act(alpha * sum_k A[m,k] * Wt[n,k] + bias[n]).
@@ -97,7 +90,7 @@ struct FcF32Args
 __device__ __forceinline__ float fcF32Epilogue(FcF32Args const& p, float v, int64_t n)
 {
     v = v * p.alpha + (p.bias ? p.bias[n] : 0.f);
-    return p.act == BERT_B200_ACT_GELU_ERF ? geluErf(v) : v;
+    return p.act == BERT_B200_ACT_GELU_ERF ? geluErfF32(v) : v;
 }
 
 // Columns n, n + 8, n + 16 and n + 24 of row m.
@@ -588,7 +581,7 @@ static bool aloneF32(int64_t tiles, int64_t kBlocks)
     return 10 * tiles >= 9 * ((tiles + wave - 1) / wave * wave);
 }
 
-int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
+int32_t fcF32Simt(bert_b200_fc_params const& p, cudaStream_t stream)
 {
     int64_t const mTiles = (p.m + kTile - 1) / kTile;
     int64_t const nTiles = (p.n + kTile - 1) / kTile;

@@ -370,6 +370,37 @@ __device__ __forceinline__ void tmemLoadWait16(uint32_t (&r)[16])
                  : "memory");
 }
 
+// D[tmem] (+)= A[tmem] * B[smem]: the A operand (FP16 or BF16, two along K per 32-bit column, lane = row) is read from
+// tensor memory. The 64-bit B descriptor is assembled from its halves inside the asm block.
+__device__ __forceinline__ void mmaF16TmemA(uint32_t dTmem, uint32_t aTmem, uint32_t bLo, uint32_t bHi, uint32_t iDesc, bool accumulate)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 db;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
+        "}" ::"r"(dTmem),
+        "r"(aTmem), "r"(bLo), "r"(bHi), "r"(iDesc), "r"(static_cast<uint32_t>(accumulate))
+        : "memory");
+}
+
+__device__ __forceinline__ void tmemStore16(uint32_t taddr, uint32_t const (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
+__device__ __forceinline__ void tmemStoreWait()
+{
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // ---- two-CTA (cta_group::2) variants ---------------------------------------------------------
 // A cluster of two CTAs on neighbouring SMs issues one MMA of M = 256: each CTA supplies its own 128 rows of A and its
 // own half of the B rows from its own shared memory and keeps its own 128 accumulator rows in its own TMEM. Only

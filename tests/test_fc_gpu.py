@@ -1,4 +1,4 @@
-"""Parity of the fully connected kernels (tcgen05 FP16 / INT8, SIMT FP32) with the CPU oracle."""
+"""Parity of the fully connected kernels (tcgen05 FP16 / INT8 / FP32, SIMT FP32) with the CPU oracle."""
 import numpy as np
 import pytest
 import torch
@@ -189,6 +189,38 @@ def test_fc_fp32_rows_do_not_depend_on_m(cuda, k, n):
     for m in (1, 37, 130, 520, 1024, 2100, one_wave):
         assert torch.equal(T.fc(a[:m], w, None).view(torch.int32), every[:m].view(torch.int32)), m
     assert torch.equal(T.fc(a[:37], w, bias, T.ACT_GELU_ERF), T.fc(a[:one_wave], w, bias, T.ACT_GELU_ERF)[:37])
+
+
+# K on either side of where the FP32 product goes to the tensor cores; one row and column, edges of their tiles, a tail of K
+@pytest.mark.parametrize("m,k,n", [(1, 384, 1), (70, 380, 130), (129, 388, 97), (70, 1000, 130), (300, 768, 96), (129, 4096, 257)])
+def test_fc_fp32_values_without_exact_parts(cuda, m, k, n):
+    """Infinities, NaN and numbers below 2^-102 have no three exact BF16 parts: the outputs that they meet come out as FP32 multiply-adds
+    give them (infinities and NaN where float64 has them, others within k 2^-24 of the sum of the products' magnitudes)."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    plain = T.fc(a, w)
+    bound = k * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((plain.double() - a.double() @ w.double().T).abs() <= bound).all())
+    a[0, 3] = float("inf")
+    w[n - 1, 5] = float("nan")
+    if m > 2:
+        a[2] *= 1e-36
+        a[m - 1, k - 1] = -float("inf")
+        a[1] = 0
+        w[1] *= 1e-34
+        w[2] = 0
+    ref, out = a.double() @ w.double().T, T.fc(a, w)
+    finite = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(ref), torch.isnan(out))
+    assert torch.equal(ref[torch.isinf(ref)].float(), out[torch.isinf(ref)])
+    size = torch.nan_to_num(a.double().abs(), 0, 0, 0) @ torch.nan_to_num(w.double().abs(), 0, 0, 0).T
+    assert bool(((out.double() - ref).abs() <= k * 2.0 ** -24 * size + 1e-42)[finite].all())
+    # rows and columns that meet none of these are untouched by them
+    rows = [i for i in range(m) if i not in (0, 1, 2, m - 1)]
+    if rows:
+        assert torch.equal(out[rows][:, 3:n - 1], plain[rows][:, 3:n - 1])
 
 
 def test_fc_linearity_full_size(cuda):
