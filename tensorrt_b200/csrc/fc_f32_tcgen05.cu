@@ -57,7 +57,9 @@ struct FcF32Smem
     static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
     static constexpr int kDynamic = kTotal + 1024;
     static constexpr int kPitch = BN + 4; // floats: sums of a tile over the drained FP32 tiles
-    static constexpr int kTmem = 2 * BN + kParts * 96 <= 256 ? 256 : 512;
+    static constexpr int kTmem = 512;
+    // Columns that a worker's sums of the segments before take in tensor memory: all of them but for the 128-wide tile (half).
+    static constexpr int kHeldCols = BN / 4 < (kTmem - 2 * BN - kParts * 96) / 4 ? BN / 4 : (kTmem - 2 * BN - kParts * 96) / 4;
     static_assert(kDynamic <= 232448, "shared memory of one CTA");
     static_assert(kTileM * kPitch * 4 <= kPlanesOff, "the sums fit the ring");
     static_assert(2 * BN + kParts * 96 <= kTmem, "tensor memory");
@@ -264,9 +266,11 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns
         bool const hasRows = m0 + quad * 32 < p.M; // warp-uniform; products of the other rows are never read
         uint32_t const tRow = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
-        // Sums of the segments before: touched once per segment and kept out of the registers on purpose, which are all taken in the
-        // loop (spilled by the compiler they cost 14 us of 1024 x 2304 x 768: beside so much shared memory the L1 holds little).
-        volatile uint64_t tot[kHold ? kCols / 2 : 1];
+        // Sums of the segments before: touched once per segment and kept out of the registers, which are all taken in the loop
+        // (spilled by the compiler they cost 14 us of 1024 x 2304 x 768: beside so much shared memory the L1 holds little). What does
+        // not fit tensor memory is in local memory on purpose. (All of them there: 31.5 us instead of 28.9 us.)
+        uint32_t const tHeld = tRow + kPartsCol + kParts * 96 + cols * L::kHeldCols;
+        volatile uint64_t rest[kHold && kCols > L::kHeldCols ? (kCols - L::kHeldCols) / 2 : 1];
         int segment = 0;
         int segmentEnd = segmentBegin(1);
         bool ok = true;
@@ -291,16 +295,49 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                 {
                     ++segment;
                     segmentEnd = segmentBegin(segment + 1);
-#pragma unroll
-                    for (int i = 0; i < kCols / 2; ++i)
+                    constexpr int kHeldPairs = L::kHeldCols / 2, kRest = kCols / 2 - kHeldPairs;
+                    if (segment > 1)
                     {
-                        if (segment > 1)
-                            acc[i] = add2(tot[i], acc[i]);
-                        if (segment < p.segments)
+#pragma unroll
+                        for (int g = 0; g < L::kHeldCols / 8; ++g)
                         {
-                            tot[i] = acc[i];
-                            acc[i] = 0;
+                            uint32_t x[8];
+                            tmemLoadCols(tHeld + g * 8, x);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                acc[g * 4 + i] = add2(pack2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), acc[g * 4 + i]);
                         }
+                        uint64_t x[kRest > 0 ? kRest : 1];
+#pragma unroll
+                        for (int i = 0; i < kRest; ++i)
+                            x[i] = rest[i];
+#pragma unroll
+                        for (int i = 0; i < kRest; ++i)
+                            acc[kHeldPairs + i] = add2(x[i], acc[kHeldPairs + i]);
+                    }
+                    if (segment < p.segments)
+                    {
+#pragma unroll
+                        for (int g = 0; g < L::kHeldCols / 8; ++g)
+                        {
+                            uint32_t x[8];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                            {
+                                float lo, hi;
+                                unpack2(acc[g * 4 + i], lo, hi);
+                                x[2 * i] = __float_as_uint(lo);
+                                x[2 * i + 1] = __float_as_uint(hi);
+                            }
+                            tmemStore8(tHeld + g * 8, x);
+                        }
+#pragma unroll
+                        for (int i = 0; i < kRest; ++i)
+                            rest[i] = acc[kHeldPairs + i];
+                        tmemStoreWait();
+#pragma unroll
+                        for (int i = 0; i < kCols / 2; ++i)
+                            acc[i] = 0;
                     }
                 }
         };
@@ -521,7 +558,7 @@ int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaSt
 // 768 1.34e-7 / 1.40e-7, 1024 1.36e-7 / 1.57e-7, 3072 1.44e-7 / 2.56e-7, 4096 1.47e-7 / 2.94e-7; below, the truncation of the tensor core
 // shows (K = 36 1.12e-7 / 0.81e-7) and the multiply-adds stay. They also take what the TMA unit does not: rows that are no
 // multiple of 16 bytes apart, sizes beyond its coordinates. Time, same order: 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 10.9 / 14.9 us, 128 x 768 x
-// 3072 13.8 / 44.6 us, 1024 x 2304 x 768 31.5 / 95.7 us, 4096 x 1024 x 4096 217 / 843 us.
+// 3072 13.9 / 44.6 us, 1024 x 2304 x 768 28.9 / 95.7 us, 4096 x 1024 x 4096 205 / 843 us.
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
     constexpr int64_t kMax = 1ll << 31;
@@ -533,7 +570,9 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
     int64_t const kChunks = (p.k + kChunk - 1) / kChunk;
     int const segments = kChunks >= 24 ? 8 : kChunks >= 12 ? 4 : 2;
     // Width of the tiles, and whether a CTA takes all segments: what the measured cycles per chunk and per CTA, times the waves of CTAs,
-    // make shortest. Clusters find fewer places than there are SMs.
+    // make shortest. Clusters find fewer places than there are SMs. Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768
+    // 29.1 / 42.5 / 36.0 / 55.0 us, 1024 x 3072 x 768 55.1 / 42.9 / 52.2 / 80.4 us, 1024 x 768 x 768 27.6 / 21.2 / 17.6 / 27.0 us; one segment per
+    // CTA, 128 / 64 columns: 1024 x 768 x 3072 73.4 / 94.5 us (64 columns in one CTA 51.9 us), 128 x 768 x 3072 17.9 / 13.8 us (50.1 us).
     int bestN = 128, bestCtas = 1;
     int64_t best = 0;
     for (int bn = 128; bn >= 32; bn -= 32)
@@ -541,7 +580,7 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
         {
             int64_t const slots = smCount() * (ctas == 1 ? 148 : ctas == 2 ? 140 : ctas == 4 ? 128 : 112) / 148;
             int64_t const waves = (mTiles * ((p.n + bn - 1) / bn) * ctas + slots - 1) / slots;
-            int64_t const fixed = ctas == 1 ? 9000 + (bn == 128 ? 3000 : 1000) * (segments - 1) : 10000 + 700 * ctas;
+            int64_t const fixed = ctas == 1 ? 9000 + 700 * (segments - 1) : 10000 + 700 * ctas;
             int64_t const cost = waves * ((kChunks + ctas - 1) / ctas * (bn == 128 ? 2880 : bn == 96 ? 2330 : bn == 64 ? 1880 : 1400) + fixed);
             if (best == 0 || cost < best)
             {
