@@ -10,6 +10,7 @@
 // sum before the first of them can be formed, so the whole score row lives in TMEM (<= 512 keys) and the softmax makes
 // three sweeps over it; that is what keeps the result bit-identical with the reference's INT8 kernels.
 //
+// Sequences of one key block go through mhaShortInt8Kernel (see there), longer ones through the persistent kernel:
 // Persistent CTAs (one per SM) take (sequence, head) work items, or parts of them where there are few, round-robin or, in
 // ragged batches of many, each a long one, then a short one (mha_items.h). Per item a CTA loops over its 128-query tiles,
 // so that K and V are loaded once and the tensor pipe works on the next tile (of this item or the next) while the
@@ -22,7 +23,6 @@
 //   warp 18   : issues the scores of the following tile, per key block as soon as the softmax warps hold
 //               the current S_j in registers:
 //                 S_j = Q K_j^T           (128 x 128 per key block, accumulators in TMEM columns 128j..)
-//               (with a single key block per sequence warp 1 issues both and this warp idles).
 //   warps 2-17: softmax, four threads per query row (each owns 32 of every 128 key columns):
 //                 pass A  row maximum over all key blocks straight from TMEM (integer maximum, no conversions),
 //                 pass B  p = exp2((x - max) * scale * log2e), row sum; the exponentials go back to TMEM,
@@ -435,9 +435,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         //      context_t += P_j V_j as they hand over P_j ----
         // Every tcgen05.mma / tcgen05.commit keeps its issuing warp busy for 30-60 cycles (measured), and one
         // warp issuing both products of a tile was the slowest link of the tile pipeline: the scores are issued by
-        // a second one, the last warp (+11 % at S = 384). Sequences of a single key block have too few MMAs per
-        // tile for that to pay (INT8, S = 128: -7 %) and keep one issuer.
-        bool const twoIssuers = !kInt8 || nbMax > 1;
+        // a second one, the last warp (+11 % at S = 384).
         // Operand descriptors are formed arithmetically: one low word per operand tile (+ bytes >> 4 per key block
         // and MMA step, compile-time constants of the unrolled loops) and one high word per operand kind (mmaLoHi).
         auto issuer = [&](auto doScoresTag, auto doContextTag) {
@@ -624,12 +622,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     item = nextWork(item + itemStep, cur);
             }
         };
-        if (!twoIssuers)
-        {
-            if (warp == 1)
-                issuer(std::true_type{}, std::true_type{});
-        }
-        else if (warp == 1)
+        if (warp == 1)
             issuer(std::false_type{}, std::true_type{});
         else
             issuer(std::true_type{}, std::false_type{});
@@ -971,11 +964,330 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     }
 }
 
+// Sequences of at most one key block: one CTA per (sequence, head), four warps that do everything in turn, a thread per query row.
+//
+// Bound by the exponentials' unit (1024 cycles per pair) where there are many pairs, by a pair's chain of latencies (lengths, loads,
+// scores, softmax, product, store) where there are few. The persistent kernel works on one tile at a time: its sixteen warps
+// pass through the same phase together, so the exponentials' unit waits for the maximum and the quantisation and the other way
+// round, and two barriers per tile keep them in step. Here four CTAs share an SM (128 columns of tensor memory each, the context
+// in the first ones once the exponentials there have been read), each in a phase of its own, no row is shared between threads, and the
+// code is small: loops over pieces of 32 columns. The arithmetic is that of the persistent kernel, to the bit, the row sum's order included.
+// Measured (persistent kernel in brackets): 1 x 37 tokens, 12 heads 4.2 us (5.2 us), 32 x 64 ... 128, 12 heads 9.0 us (11.0 us), 64 x 128, 16
+// heads 13.8 us (21.8 us), 128 x 16, 16 heads 16.7 us (40.8 us). Two threads per row: 4.4, 9.0, 14.7 and 20.1 us. The same for two key
+// blocks (256 columns, two CTAs per SM) is no clear gain: 9 x 256, 16 heads 8.3 us (10.0 us), 64 x 256 49.5 us (53.4 us), but 2 x 256 7.1
+// us (6.3 us), 37 interleaved sequences of 100 ... 256 28.4 us (26.5 us).
+constexpr int kShortThreads = 128;
+constexpr int kShortTile = kQTile * kHeadSize;  // bytes of the Q, K or V tile
+constexpr int kShortP = 3 * kShortTile;         // after Q, K and V
+constexpr int kShortBars = kShortP + kQTile * kKeyBlock;
+constexpr int kShortSmemBytes = kShortBars + 64 + 1024;
+constexpr uint32_t kShortTmemCols = kKeyBlock;
+
+template <bool IL, bool BNSD>
+__global__ void __launch_bounds__(kShortThreads, 4) mhaShortInt8Kernel(const __grid_constant__ CUtensorMap mapQkv,
+    const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
+{
+    constexpr uint64_t kSwz = IL ? kSwizzle32B : kSwizzle64B;
+    constexpr uint32_t kAtomBytes = IL ? 256u : 512u;
+    constexpr uint32_t kSubTile = kShortTile / 2; // interleaved: bytes of one 32-channel sub-tile
+    constexpr uint32_t kIdescQk = makeInstrDesc(2u, 1u, 0u, 0u, 128u, 128u);
+    constexpr uint32_t kIdescPv = makeInstrDesc(2u, 1u, 0u, 1u, 128u, 64u);
+    int const warp = threadIdx.x >> 5;
+
+    extern __shared__ uint8_t smemRaw[];
+    uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint8_t* const sK = smem + kShortTile;
+    uint8_t* const sV = smem + 2 * kShortTile;
+    uint8_t* const sP = smem + kShortP;
+    uint64_t* const qkFull = reinterpret_cast<uint64_t*>(smem + kShortBars);
+    uint64_t* const vFull = qkFull + 1;
+    uint64_t* const sFull = qkFull + 2;
+    uint64_t* const oFull = qkFull + 3;
+    uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(qkFull + 4);
+    volatile uint32_t* const abortFlag = tmemSlot + 1;
+    if (threadIdx.x == 0)
+    {
+        for (int i = 0; i < 4; ++i)
+            mbarInit(&qkFull[i], 1);
+        *abortFlag = 0;
+        fenceBarrierInit();
+        prefetchTensorMap(&mapQkv);
+        if (BNSD)
+        {
+            prefetchTensorMap(&mapK);
+            prefetchTensorMap(&mapV);
+        }
+    }
+    __syncwarp();
+    if (warp == 0)
+        tmemAlloc(tmemSlot, kShortTmemCols);
+    tcFenceBefore();
+    __syncthreads();
+    tcFenceAfter();
+    uint32_t const tmemBase = *tmemSlot;
+    gridDependencyLaunch();
+    gridDependencyWait();
+
+    int32_t const b = static_cast<int32_t>(blockIdx.x) / args.N, head = static_cast<int32_t>(blockIdx.x) - b * args.N;
+    int32_t rowBase, len;
+    if (args.fixedLayout)
+    {
+        rowBase = 0;
+        len = args.maskIdx ? min(max(__ldg(args.maskIdx + b), 0), args.S) : args.S;
+    }
+    else
+    {
+        rowBase = __ldg(args.cu + b);
+        len = min(max(__ldg(args.cu + b + 1) - rowBase, 0), args.S);
+    }
+    int32_t const rows = args.fixedLayout ? args.S : len;
+    int const q = static_cast<int>(threadIdx.x); // query row = TMEM lane
+    // the 16 context channels from c on of this thread's row
+    auto outPtr = [&](int c) -> uint4* {
+        int8_t* const out = static_cast<int8_t*>(args.out);
+        if (BNSD)
+            return reinterpret_cast<uint4*>(out + ((static_cast<int64_t>(b) * args.N + head) * args.S + q) * args.d + c);
+        if (IL)
+            return reinterpret_cast<uint4*>(
+                out + ((static_cast<int64_t>(head) * (args.d / 32) + c / 32) * args.total + rowBase + q) * 32 + c % 32);
+        int64_t const row = args.fixedLayout ? static_cast<int64_t>(q) * args.B + b : static_cast<int64_t>(rowBase) + q;
+        return reinterpret_cast<uint4*>(out + (row * args.N + head) * args.d + c);
+    };
+    if (len > 0) // the same for all threads
+    {
+        // linear: (channel, which of [N][3], batch, row). interleaved: (channel, row, 32-channel group, which of [3][N])
+        auto load = [&](uint8_t* dst, uint64_t* bar, int which) {
+            if (BNSD) // (channel, position, head, sequence) of the tensor `which` selects
+                tmaLoad4d(dst, which == 0 ? &mapQkv : (which == 1 ? &mapK : &mapV), bar, 0, 0, head, b);
+            else if (IL)
+                tmaLoad4d(dst, &mapQkv, bar, 0, rowBase, 0, which * args.N + head);
+            else
+                tmaLoad4d(dst, &mapQkv, bar, 0, head * 3 + which, args.fixedLayout ? b : 0, rowBase);
+        };
+        bool ok = true;
+        if (warp == 0)
+        {
+            if (electOne())
+            {
+                mbarArriveExpectTx(qkFull, 2 * kShortTile);
+                load(smem, qkFull, 0);
+                load(sK, qkFull, 1);
+                mbarArriveExpectTx(vFull, kShortTile);
+                load(sV, vFull, 2);
+            }
+            __syncwarp();
+            ok = mbarWaitWarp(smemAddr(qkFull), 0, abortFlag, kWaitTmaFull);
+            tcFenceAfter();
+            if (electOne() && ok)
+            {
+                uint64_t const dQk = makeSmemDesc(0, 16, kAtomBytes, kSwz);
+                uint32_t const lo = static_cast<uint32_t>(dQk), hi = static_cast<uint32_t>(dQk >> 32);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) // head size 64 = 2 x 32
+                {
+                    uint32_t const off = (IL ? k * kSubTile : k * 32) >> 4;
+                    mmaLoHi<true>(tmemBase, lo + (smemAddr(smem) >> 4) + off, hi, lo + (smemAddr(sK) >> 4) + off, hi, kIdescQk, k != 0);
+                }
+                tcCommit(sFull);
+            }
+            __syncwarp();
+        }
+        uint32_t const tRow = tmemBase + (static_cast<uint32_t>(warp * 32) << 16);
+        float const sl2 = args.scaleBmm1 * 1.4426950408889634f;
+        constexpr float kMagic = 12582912.f; // 1.5 * 2^23: as_float(0x4B400000 + v) == kMagic + v for |v| < 2^22
+        constexpr uint32_t kMagicBits = 0x4B400000u;
+        ok = ok && mbarWait(sFull, 0, abortFlag, kWaitSoftmax);
+        __syncwarp();
+        tcFenceAfter();
+
+        // row maximum (integers, no conversions); pieces of keys beyond the sequence are left out of all passes
+        int const pieces = (len + 31) / 32;
+        int32_t m0 = INT32_MIN, m1 = INT32_MIN, m2 = INT32_MIN, m3 = INT32_MIN;
+#pragma unroll 1
+        for (int p = 0; p < pieces; ++p)
+        {
+            uint32_t x[32];
+            tmemLoad32(tRow + p * 32, x);
+            tmemLoadWait32(x);
+            int const limit = len - p * 32;
+            if (limit < 32)
+            {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    x[i] = i < limit ? x[i] : 0x80000000u;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+            {
+                m0 = max(max(m0, static_cast<int32_t>(x[i])), static_cast<int32_t>(x[i + 1]));
+                m1 = max(max(m1, static_cast<int32_t>(x[i + 2])), static_cast<int32_t>(x[i + 3]));
+                m2 = max(max(m2, static_cast<int32_t>(x[i + 4])), static_cast<int32_t>(x[i + 5]));
+                m3 = max(max(m3, static_cast<int32_t>(x[i + 6])), static_cast<int32_t>(x[i + 7]));
+            }
+        }
+        float const mxMagic = kMagic + static_cast<float>(max(max(m0, m1), max(m2, m3))); // exact: both are integers below 2^24
+
+        // exponentials, back to where the scores were, and the row sum: (p0 + p1) + (p2 + p3) of the pieces' sums
+        float total = 0.f, before = 0.f;
+#pragma unroll 1
+        for (int p = 0; p < pieces; ++p)
+        {
+            uint32_t x[32];
+            tmemLoad32(tRow + p * 32, x);
+            tmemLoadWait32(x);
+            int const limit = len - p * 32;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                x[i] = __float_as_uint(ex2Approx((__uint_as_float(x[i] + kMagicBits) - mxMagic) * sl2));
+            if (limit < 32)
+            {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    x[i] = i < limit ? x[i] : 0u;
+            }
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                sum += __uint_as_float(x[i]);
+            tmemStore32(tRow + p * 32, x);
+            if ((p & 1) == 0)
+                before = sum;
+            else
+                total += before + sum;
+        }
+        if ((pieces & 1) != 0)
+            total += before;
+        tmemStoreWait();
+        float const inv = 1.f / total;
+        float const pq = inv * args.scaleSoftmax;
+
+        // P_q = rni(p / sum * scale_softmax); see the persistent kernel for the clamp
+        bool const noClamp = args.scaleSoftmax <= 127.f;
+#pragma unroll 1
+        for (int p = 0; p < 4; ++p)
+        {
+            uint4 w[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+            if (p < pieces)
+            {
+                uint32_t x[32];
+                tmemLoad32(tRow + p * 32, x);
+                tmemLoadWait32(x);
+                uint32_t* const o = reinterpret_cast<uint32_t*>(w);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                {
+                    float f[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        f[j] = __uint_as_float(x[4 * i + j]) * pq;
+                    if (!noClamp)
+                    {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            f[j] = fminf(f[j], 127.f);
+                    }
+                    o[i] = packProb4<false>(f[0], f[1], f[2], f[3]);
+                }
+            }
+            uint8_t* const pRow = sP + q * 128; // P: [128 rows][128 keys]
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+                *reinterpret_cast<uint4*>(pRow + (((p * 2 + g) ^ (q & 7)) << 4)) = w[g];
+        }
+        fenceProxyAsync();
+        tcFenceBefore();
+        __syncthreads();
+        if (warp == 0)
+        {
+            ok = ok && mbarWaitWarp(smemAddr(vFull), 0, abortFlag, kWaitTmaFull);
+            tcFenceAfter();
+            if (electOne() && ok)
+            {
+                uint64_t const dP = makeSmemDesc(0, 16, 1024, kSwizzle128B);
+                uint64_t const dV = IL ? makeSmemDesc(0, kSubTile, kAtomBytes, kSwz) : makeSmemDesc(0, kAtomBytes, kAtomBytes, kSwz);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) // 128 keys = 4 x 32
+                    mmaLoHi<true>(tmemBase, static_cast<uint32_t>(dP) + (smemAddr(sP) >> 4) + k * 2, static_cast<uint32_t>(dP >> 32),
+                        static_cast<uint32_t>(dV) + (smemAddr(sV) >> 4) + k * ((IL ? 1024u : 2048u) >> 4), static_cast<uint32_t>(dV >> 32), kIdescPv, k != 0);
+                tcCommit(oFull);
+            }
+            __syncwarp();
+        }
+        ok = ok && mbarWait(oFull, 0, abortFlag, kWaitAccFull);
+        __syncwarp();
+        tcFenceAfter();
+        float const s2 = args.scaleBmm2;
+#pragma unroll 1
+        for (int c = 0; c < args.d; c += 16)
+        {
+            uint32_t x[16];
+            tmemLoad16(tRow + c, x);
+            tmemLoadWait16(x);
+            float v[16];
+            if (noClamp) // |context| <= (127 + 256 / 2) * 128 < 2^22: the integer becomes a number without the conversion unit
+            {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    v[i] = __uint_as_float(x[i] + kMagicBits) - kMagic;
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    v[i] = static_cast<float>(static_cast<int32_t>(x[i]));
+            }
+            if (q < rows && ok)
+            {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    w[i] = packChar4(v[4 * i] * s2, v[4 * i + 1] * s2, v[4 * i + 2] * s2, v[4 * i + 3] * s2);
+                *outPtr(c) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            __syncwarp();
+        }
+        tcFenceBefore();
+    }
+    else if (q < rows) // no valid key: every probability is zero and so is the context row
+    {
+        for (int c = 0; c < args.d; c += 16)
+            *outPtr(c) = make_uint4(0, 0, 0, 0);
+    }
+
+    __syncthreads();
+    uint32_t const aborted = *abortFlag;
+    if (aborted != 0)
+    {
+        uint64_t const t0 = globalTimerNs();
+        while (globalTimerNs() - t0 < 1000000ull)
+            __nanosleep(1000);
+        if (threadIdx.x == 0 && args.statusWord)
+            atomicMax(args.statusWord, aborted);
+        __syncthreads();
+    }
+    if (warp == 0)
+    {
+        __syncwarp();
+        tcFenceAfter();
+        tmemFree(tmemBase, kShortTmemCols);
+    }
+}
+
 // Sets the work items and launches: one persistent CTA per SM (512 TMEM columns and most of the shared memory each).
 template <typename T, bool IL, bool BNSD>
 int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t stream)
 {
     static_assert(kItemTile == kQTile, "tiles of the plan");
+    int64_t const pairs = static_cast<int64_t>(args.B) * args.N;
+    if (args.S <= kKeyBlock && pairs <= INT32_MAX) // one key block: the short kernel is ahead from one pair to thousands (see there)
+    {
+        static SmemOptIn optIn;
+        cudaError_t const e = launchDependentCluster(&optIn, mhaShortInt8Kernel<IL, BNSD>, dim3(static_cast<unsigned>(pairs)), dim3(kShortThreads),
+            kShortSmemBytes, stream, 1, maps[0], maps[1], maps[2], args);
+        if (e != cudaSuccess)
+            B200_FAIL(BERT_B200_CUDA_ERROR, "mhaShortInt8Kernel: %s", cudaGetErrorString(e));
+        return checkLaunch("mhaShortInt8Kernel");
+    }
     int64_t const missing = !args.fixedLayout ? static_cast<int64_t>(args.B) * args.S - args.total : (args.maskIdx ? INT64_MAX : 0);
     ItemPlan const plan = planItems(args.B, args.N, args.S, missing, smCount());
     args.tilesPerItem = plan.tilesPerItem;

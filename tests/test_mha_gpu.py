@@ -92,6 +92,50 @@ def test_mha_packed_int8(cuda, lengths, N):
     _assert_int8_attention(out.cpu().numpy(), ref)
 
 
+# pieces of 32 keys and their edges, no key, one key, a full block; probabilities that saturate; many pairs per SM
+@pytest.mark.parametrize("lengths,N,scale_softmax", [([128, 1, 31, 0, 32, 33, 64, 65, 95, 96, 97, 127], 5, 127.0),
+                                                     ([3, 1, 100, 2, 40], 3, 200.0), ([int(7 * i) % 129 for i in range(150)], 16, 127.0)])
+@pytest.mark.parametrize("d,interleaved", [(64, False), (64, True), (32, True), (48, False), (16, False)])
+def test_mha_int8_one_key_block_is_the_persistent_kernel_to_the_bit(cuda, lengths, N, scale_softmax, d, interleaved):
+    """Sequences of at most 128 tokens have a kernel of their own; with a larger S (an upper bound only, in the packed layouts) the
+    same sequences go through the persistent one, which the other tests compare with the oracle. Same bytes."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(len(lengths) + d)
+    cu = _t(O.cu_seqlens(np.array(lengths, dtype=np.int32)), cuda)
+    total, B = sum(lengths), len(lengths)
+    shape = (3 * N * d // 32, total, 32) if interleaved else (total, 3 * N * d)
+    q8 = torch.clamp(torch.round(40 * torch.randn(shape, device=cuda, generator=gen)), -128, 127).to(torch.int8)
+    st = _status(cuda)
+    for s1 in (2e-4, -1e-5):   # nothing keeps a caller from a scale below zero
+        out = [T.mha(q8, B, S, N, d, cu_seqlens=cu, scale_bmm1=s1, scale_softmax=scale_softmax, scale_bmm2=0.02, status=st,
+                     interleaved=interleaved) for S in (128, 129)]
+        assert int(st[0]) == 0 and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("S", [1, 37, 128])
+def test_mha_int8_one_key_block_fixed_and_separate(cuda, S):
+    """The layouts whose rows S itself places: queries beyond a sequence's keys, a sequence without keys."""
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(S + 5)
+    B, N, d = 4, 3, 64
+    q8, s_qkv = _int8_case(rng, S * B, N, d)
+    q8 = q8.reshape(S, B, -1)
+    lengths = np.array([S, 0, (S + 1) // 2, 1], dtype=np.int32)
+    s1 = float(np.float32(s_qkv) * np.float32(s_qkv) * np.float32(0.125))
+    s2 = 2.0 / 127.0
+    ref = O.mha_int8(q8, B, S, N, d, s1, 127.0, s2, lengths=lengths)
+    st = _status(cuda)
+    scales = dict(scale_bmm1=s1, scale_softmax=127.0, scale_bmm2=s2, status=st)
+    out = T.mha(_t(q8, cuda), B, S, N, mask_idx=_t(lengths, cuda), **scales)
+    _assert_int8_attention(out.cpu().numpy(), ref)
+    q, k, v = _split_bnsd(q8, S, B, N, d)
+    out = T.attention_bnsd(_t(q, cuda), _t(k, cuda), _t(v, cuda), kv_lengths=_t(lengths, cuda), **scales)
+    _assert_int8_attention(out.cpu().numpy(), ref.reshape(S, B, N, d).transpose(1, 2, 0, 3))
+    assert int(st[0]) == 0
+
+
 def test_mha_int8_saturating_probabilities(cuda):
     """scale_softmax > 127: probabilities near 1 saturate at 127 like the reference's conversion (the kernel leaves the
     clamp out when scale_softmax <= 127)."""
