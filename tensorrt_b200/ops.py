@@ -26,13 +26,16 @@ def _ptr(t: torch.Tensor | None):
         raise ValueError("tensorrt_b200 kernels need CUDA tensors; there is no CPU path")
     if not t.is_contiguous():
         raise ValueError("tensor must be contiguous")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()  # ctypes takes the number; an object around every pointer was a quarter of a call's host time
 
 
 def _stream():
+    # A call on a few rows takes the GPU less time than the host: is_available() and a Stream object only before the first use.
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     if not torch.cuda.is_available():
         raise ValueError("tensorrt_b200 kernels need a CUDA device; there is no CPU path")
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch.cuda.current_stream().cuda_stream
 
 
 def skip_layer_norm(x, skip, gamma, beta, bias=None, out=None):
@@ -195,10 +198,7 @@ def mha(qkv, B, S, num_heads, head_size=64, cu_seqlens=None, mask_idx=None, scal
         scale_bmm1 = head_size ** -0.5
     p = _lib.MhaParams(_TYPE_ID[qkv.dtype], B, S, num_heads, head_size, total, _ptr(qkv), _ptr(out), _ptr(cu_seqlens),
                        _ptr(mask_idx), 1 if interleaved else 0, scale_bmm1, scale_softmax, scale_bmm2, _ptr(status))
-    if workspace is None and use_workspace:
-        need = int(lib.bert_b200_mha_workspace_size(C.byref(p)))
-        workspace = torch.empty(need, dtype=torch.uint8, device=qkv.device) if need > 0 else None
-    if workspace is not None:
+    if workspace is not None:  # no kernel needs one (bert_b200_mha_workspace_size is 0): nothing is asked for or allocated
         p.workspace, p.workspace_bytes = _ptr(workspace), workspace.numel() * workspace.element_size()
     check(lib.bert_b200_mha(C.byref(p), _stream()), "mha")
     return out
