@@ -30,9 +30,8 @@ namespace
 // same bits whatever M, although the work is divided by the number of tiles. Where the tiles alone fill the SMs, a CTA takes all segments
 // of its tile and keeps their sum in shared memory (16 KB, four CTAs still fit an SM); otherwise a cluster takes one per CTA, exchanges
 // the sums through distributed shared memory and each CTA finishes its share of every thread's outputs.
-// Measured: 1024 x 2304 x 768 in 97 us (37 TFLOP/s; a 4 x 4-per-thread kernel with scalar copies took 195 us), 1024 x 768 x 3072 in 143 us
-// (700 us). Holding the sums of eight segments costs 3 us of the first (K in one piece: 93 ... 95 us), exchanging them 8 % of 4096 x 1024 x
-// 4096 (843 us; two CTAs per tile 777 us), and few rows gain (37 x 768 x 768 8.7 us, 9.7 us with a scalar exchange).
+// It takes a K below 384 and what the tensor-core kernel cannot load (see fcF32). Measured: 512 x 768 x 384 in 15.6 us; holding the sums of the
+// segments costs 3 % where they are eight, exchanging them 8 %, and few rows gain (37 x 768 x 768 8.7 us, 9.7 us with a scalar exchange).
 constexpr int kTile = 64;
 constexpr int kTileK = 16;
 constexpr int kPitch = kTileK + 4; // floats
