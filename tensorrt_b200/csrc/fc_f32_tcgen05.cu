@@ -65,10 +65,10 @@ struct FcF32Smem
     static_assert(2 * BN + kParts * 96 <= kTmem, "tensor memory");
 };
 
-// Two floats into packed BF16 parts; `range` becomes the largest magnitude so far (NaN once there is one).
-__device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, float& range)
+// Two floats into packed BF16 parts. What is left when the last part is cut goes into the lower halves of `lost`: numbers below 2^-110 have bits
+// that BF16 does not (its smallest is 2^-133), infinities and NaN leave a NaN.
+__device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, uint32_t& lost)
 {
-    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(range) : "f"(a), "f"(b));
     uint32_t const ua = __float_as_uint(a), ub = __float_as_uint(b);
     h = __byte_perm(ua, ub, 0x7632);
     float ra, rb;
@@ -78,13 +78,7 @@ __device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_
     float la, lb;
     unpack2(add2(pack2(ra, rb), pack2(__uint_as_float((va & 0xffff0000u) ^ 0x80000000u), __uint_as_float((vb & 0xffff0000u) ^ 0x80000000u))), la, lb);
     l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
-}
-
-// Whether numbers up to `range` in magnitude have parts that are good enough: infinities and NaN have none, and the last parts of
-// the largest must be normal BF16 numbers (from 2^-102 on) for the sum to keep FP32 precision. Zeros are fine.
-__device__ __forceinline__ bool splitIsInexact(float range)
-{
-    return !(range < INFINITY) || (range > 0.f && range < 1.9721522630525295e-31f);
+    lost |= __float_as_uint(la) | __float_as_uint(lb);
 }
 
 __device__ __forceinline__ void tmemStore8(uint32_t taddr, uint32_t const (&r)[8])
@@ -134,7 +128,7 @@ __device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[24])
 //               double-buffered.
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
-// An output whose row of A or Wt holds numbers without exact parts (splitIsInexact) is computed again by plain FP32 multiply-adds.
+// An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by plain FP32 multiply-adds.
 template <int BN, bool kHold>
 __global__ void __launch_bounds__(kThreadsF32, 1)
     fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, FcF32TcArgs const p)
@@ -358,7 +352,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     int const row = quad * 32 + lane;
                     float4 const* const src = reinterpret_cast<float4 const*>(fp + half * (L::kABytes / 2) + row * 128);
                     uint32_t const t = tRow + kPartsCol + s * 96 + half * 16;
-                    float range = 0.f;
+                    uint32_t lost = 0;
 #pragma unroll
                     for (int g = 0; g < 2; ++g)
                     {
@@ -370,14 +364,14 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                         {
-                            splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], range);
-                            splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], range);
+                            splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], lost);
+                            splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], lost);
                         }
                         tmemStore8(t + g * 8, h);
                         tmemStore8(t + g * 8 + 32, m);
                         tmemStore8(t + g * 8 + 64, l);
                     }
-                    if (splitIsInexact(range))
+                    if ((lost & 0xffffu) != 0)
                         flagA[row] = *flagAny = 1;
                 }
                 // eight numbers of a row of Wt: 16 bytes of each part
@@ -400,16 +394,16 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     {
                         int const row = (r0 + i) * 32 + lane;
                         uint4 h, m, l;
-                        float range = 0.f;
-                        splitPair(v[i][0].x, v[i][0].y, h.x, m.x, l.x, range);
-                        splitPair(v[i][0].z, v[i][0].w, h.y, m.y, l.y, range);
-                        splitPair(v[i][1].x, v[i][1].y, h.z, m.z, l.z, range);
-                        splitPair(v[i][1].z, v[i][1].w, h.w, m.w, l.w, range);
+                        uint32_t lost = 0;
+                        splitPair(v[i][0].x, v[i][0].y, h.x, m.x, l.x, lost);
+                        splitPair(v[i][0].z, v[i][0].w, h.y, m.y, l.y, lost);
+                        splitPair(v[i][1].x, v[i][1].y, h.z, m.z, l.z, lost);
+                        splitPair(v[i][1].z, v[i][1].w, h.w, m.w, l.w, lost);
                         uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
                         *reinterpret_cast<uint4*>(dst) = h;
                         *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
                         *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
-                        if (splitIsInexact(range))
+                        if ((lost & 0xffffu) != 0)
                             flagW[row] = *flagAny = 1;
                     }
                 }

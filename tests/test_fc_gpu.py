@@ -194,7 +194,7 @@ def test_fc_fp32_rows_do_not_depend_on_m(cuda, k, n):
 # K on either side of where the FP32 product goes to the tensor cores; one row and column, edges of their tiles, a tail of K
 @pytest.mark.parametrize("m,k,n", [(1, 384, 1), (70, 380, 130), (129, 388, 97), (70, 1000, 130), (300, 768, 96), (129, 4096, 257)])
 def test_fc_fp32_values_without_exact_parts(cuda, m, k, n):
-    """Infinities, NaN and numbers below 2^-102 have no three exact BF16 parts: the outputs that they meet come out as FP32 multiply-adds
+    """Infinities, NaN and numbers with bits below 2^-133 have no three exact BF16 parts: the outputs that they meet come out as FP32 multiply-adds
     give them (infinities and NaN where float64 has them, others within k 2^-24 of the sum of the products' magnitudes)."""
     import tensorrt_b200 as T
 
@@ -221,6 +221,26 @@ def test_fc_fp32_values_without_exact_parts(cuda, m, k, n):
     rows = [i for i in range(m) if i not in (0, 1, 2, m - 1)]
     if rows:
         assert torch.equal(out[rows][:, 3:n - 1], plain[rows][:, 3:n - 1])
+
+
+# a group that is cut together (32 numbers of a row of A, 8 of a row of Wt) and its edges; a small number on either side of the limit
+@pytest.mark.parametrize("m,k,n", [(130, 384, 140), (3, 772, 33), (200, 4096, 70)])
+@pytest.mark.parametrize("size", [1e-41, 1e-38, 2.0 ** -109, 2.0 ** -103, 1e-30])
+@pytest.mark.parametrize("small_wt", [False, True])
+def test_fc_fp32_small_numbers_beside_large_ones(cuda, m, k, n, size, small_wt):
+    """Numbers too small for three BF16 parts, or nearly so, that share a row with ordinary ones, which meet zeros: the outputs consist of the small ones alone.
+    k roundings to 2^-24 in a row, as a random walk."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    small, large = (w, a) if small_wt else (a, w)
+    small *= size
+    large *= 1e35
+    small[:, ::8] = 1.0
+    large[:, ::8] = 0.0
+    ref = a.double() @ w.double().T
+    assert float((T.fc(a, w).double() - ref).norm() / ref.norm()) <= k ** 0.5 * 2.0 ** -24
 
 
 def test_fc_linearity_full_size(cuda):
