@@ -52,7 +52,8 @@ struct FcF32Smem
     static constexpr int kPlaneBytes = BN * kChunk * 2; // one BF16 part of the Wt tile
     static constexpr int kPlanesOff = kStages * kStageBytes;
     static constexpr int kBarrierOff = kPlanesOff + kParts * 3 * kPlaneBytes;
-    // stFull[stages] stFree[stages] ready[parts] done[parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt, whether any is set
+    // stFull[stages] stFree[stages] ready[parts] done[parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
+    // whether any is 1
     static constexpr int kFlagsOff = kBarrierOff + (2 * kStages + 2 * kParts + 2) * 8 + 16;
     static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
     static constexpr int kDynamic = kTotal + 1024;
@@ -61,7 +62,7 @@ struct FcF32Smem
     // Columns that a worker's sums of the segments before take in tensor memory: all of them but for the 128-wide tile (half).
     static constexpr int kHeldCols = BN / 4 < (kTmem - 2 * BN - kParts * 96) / 4 ? BN / 4 : (kTmem - 2 * BN - kParts * 96) / 4;
     static_assert(kDynamic <= 232448, "shared memory of one CTA");
-    static_assert(kTileM * kPitch * 4 <= kPlanesOff, "the sums fit the ring");
+    static_assert(kTileM * kPitch * 4 + kTileM * BN / 8 + kTileM * BN / 4 + 4 <= kPlanesOff, "the sums, and what is computed again, fit the ring");
     static_assert(2 * BN + kParts * 96 <= kTmem, "tensor memory");
 };
 
@@ -79,6 +80,11 @@ __device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_
     unpack2(add2(pack2(ra, rb), pack2(__uint_as_float((va & 0xffff0000u) ^ 0x80000000u), __uint_as_float((vb & 0xffff0000u) ^ 0x80000000u))), la, lb);
     l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
     lost |= __float_as_uint(la) | __float_as_uint(lb);
+}
+
+__device__ __forceinline__ bool hasNan(float4 v)
+{
+    return isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
 }
 
 __device__ __forceinline__ void tmemStore8(uint32_t taddr, uint32_t const (&r)[8])
@@ -116,6 +122,97 @@ __device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[24])
     tmemLoadCols(taddr + 16, *reinterpret_cast<uint32_t(*)[8]>(&r[16]));
 }
 
+__device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, int64_t n)
+{
+    v = v * p.alpha + (p.bias ? __ldg(p.bias + n) : 0.f);
+    return p.act == BERT_B200_ACT_GELU_ERF ? geluErfF32(v) : v;
+}
+
+// The outputs of a tile whose bit in `again` (BN bits per row) is set, by FP32 multiply-adds: a warp takes 4 x 4 outputs, its lanes every 32nd four
+// of K, even and odd ones apart, and their sums are added as a tree, so an output has the same bits wherever its tile lies. The chains are a
+// quarter or less as long as those of fcF32Simt (error on normal values K = 768 0.9e-7 / 1.4e-7, 4096 1.6e-7 / 2.9e-7). Bound by the loads' latency for a
+// few outputs, by what the L2 brings for all (4 x 4 outputs are read by 8 rows). 1024 x 2304 x 768, nothing to compute again / an infinity in A / a number
+// below 2^-110 in Wt / A full of them: 29.6 / 39.6 / 39.5 / 285 us; a thread per output and all of K in one chain 29.6 / 140 / 169 / 10 100 us;
+// fcF32Simt 97 us.
+template <int BN>
+__device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* again, uint32_t* list, int64_t m0, int64_t n0)
+{
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kAcross = BN / 4;
+    auto const maskOf = [&](int i) {
+        int const r = i / kAcross * 4, c = i % kAcross * 4;
+        uint32_t mask = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            mask |= (again[(r + j) * (BN / 32) + c / 32] >> (c % 32) & 15u) << (4 * j);
+        return mask;
+    };
+    for (int i = threadIdx.x; i < kTileM / 4 * kAcross; i += kThreadsF32)
+        if (maskOf(i) != 0)
+            list[1 + atomicAdd(list, 1u)] = i;
+    __syncthreads();
+    int const blocks = static_cast<int>(list[0]);
+#pragma unroll 1
+    for (int i = warp; i < blocks; i += kThreadsF32 / 32)
+    {
+        int const block = static_cast<int>(list[1 + i]);
+        uint32_t const mask = maskOf(block);
+        int const r = block / kAcross * 4, c = block % kAcross * 4;
+        float const *a[4], *w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            a[j] = p.A + min(m0 + r + j, p.M - 1) * p.lda;
+            w[j] = p.Wt + min(n0 + c + j, p.N - 1) * p.K;
+        }
+        uint64_t acc[16] = {};
+#pragma unroll 1
+        for (int64_t k = lane * 4; k < p.K; k += 128)
+        {
+            float4 av[4], wv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+            {
+                av[j] = __ldg(reinterpret_cast<float4 const*>(a[j] + k));
+                wv[j] = __ldg(reinterpret_cast<float4 const*>(w[j] + k));
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+            {
+                acc[j] = fma2(pack2(av[j >> 2].x, av[j >> 2].y), pack2(wv[j & 3].x, wv[j & 3].y), acc[j]);
+                acc[j] = fma2(pack2(av[j >> 2].z, av[j >> 2].w), pack2(wv[j & 3].z, wv[j & 3].w), acc[j]);
+            }
+        }
+        // lane 2 j gets the sum of output j: each step halves the outputs that a lane holds
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+        {
+            float lo, hi;
+            unpack2(acc[j], lo, hi);
+            v[j] = lo + hi;
+        }
+#pragma unroll
+        for (int half = 8; half >= 1; half >>= 1)
+        {
+            bool const upper = (lane & (2 * half)) != 0;
+#pragma unroll
+            for (int j = 0; j < half; ++j)
+            {
+                float const other = __shfl_xor_sync(0xffffffffu, upper ? v[j] : v[j + half], 2 * half);
+                v[j] = (upper ? v[j + half] : v[j]) + other;
+            }
+        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+        int const j = lane >> 1;
+        if ((lane & 1) == 0 && (mask >> j & 1u) != 0)
+        {
+            int64_t const n = n0 + c + (j & 3);
+            p.C[(m0 + r + (j >> 2)) * p.ldc + n] = finishF32(p, v[0], n);
+        }
+    }
+}
+
 // Bound by the chain of a chunk - its place free, operands cut, products, sums read -, 2880 cycles for a 128 x 128 tile, of which the
 // tensor cores are busy 1490; no unit is full (ALU 46 %, issue slots 45 %, the shared-memory pipe 21 %). Half the code, or scalar instead of
 // packed subtractions, changes nothing. One 128 x BN tile per CTA, or one segment of its K:
@@ -128,10 +225,11 @@ __device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[24])
 //               double-buffered.
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
-// An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by plain FP32 multiply-adds.
+// An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by FP32 multiply-adds (computeAgain), unless one
+// of them is NaN: then it comes out as that.
 template <int BN, bool kHold>
 __global__ void __launch_bounds__(kThreadsF32, 1)
-    fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, FcF32TcArgs const p)
+    fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ FcF32TcArgs p)
 {
     using L = FcF32Smem<BN>;
     constexpr uint32_t kIdesc = makeInstrDesc(1u, 1u, 0u, 0u, 128u, static_cast<uint32_t>(BN));
@@ -151,6 +249,8 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     uint32_t* const flagW = flagA + kTileM;
     uint32_t* const flagAny = flagW + BN;
     float* const sums = reinterpret_cast<float*>(smem);
+    uint32_t* const again = reinterpret_cast<uint32_t*>(sums + kTileM * L::kPitch); // a bit per output that is computed again
+    uint32_t* const list = again + kTileM * BN / 32;                               // see computeAgain
 
     int const warp = threadIdx.x >> 5;
     int const lane = threadIdx.x & 31;
@@ -336,6 +436,11 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     }
                 }
         };
+        auto flag = [&](uint32_t* at, bool nan) {
+            atomicOr(at, nan ? 2u : 1u);
+            if (!nan)
+                *flagAny = 1;
+        };
         int stage = 0;
         uint32_t phase = 0;
         for (int c = 0; c < count; ++c)
@@ -372,7 +477,13 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                         tmemStore8(t + g * 8 + 64, l);
                     }
                     if ((lost & 0xffffu) != 0)
-                        flagA[row] = *flagAny = 1;
+                    {
+                        bool nan = false;
+#pragma unroll 1
+                        for (int i = 0; i < 8; ++i)
+                            nan = nan || hasNan(src[i]);
+                        flag(flagA + row, nan);
+                    }
                 }
                 // eight numbers of a row of Wt: 16 bytes of each part
                 uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
@@ -404,7 +515,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                         *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
                         *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
                         if ((lost & 0xffffu) != 0)
-                            flagW[row] = *flagAny = 1;
+                            flag(flagW + row, hasNan(v[i][0]) || hasNan(v[i][1]));
                     }
                 }
                 fenceProxyAsync();
@@ -455,12 +566,25 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             *reinterpret_cast<float4*>(dst + 4 * i) = v;
         }
     }
-    bool exact = true;
+    for (int i = threadIdx.x; i <= kTileM * BN / 32; i += kThreadsF32)
+        again[i] = 0; // and the list's length
+    bool exact = true; // the same for all threads of the cluster
     if (p.ctas > 1)
     {
         clusterBarrier();
         for (int s = 0; s < p.ctas; ++s)
             exact = exact && ldSharedCluster(flagAny, s) == 0;
+        if (!exact)
+        {
+            uint32_t merged = 0; // flags of a row over all of K
+            if (threadIdx.x < kTileM + BN)
+                for (int s = 0; s < p.ctas; ++s)
+                    merged |= ldSharedCluster(flagA + threadIdx.x, s);
+            clusterBarrier();
+            if (threadIdx.x < kTileM + BN)
+                flagA[threadIdx.x] = merged;
+            __syncthreads();
+        }
     }
     else
     {
@@ -492,33 +616,30 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         else
             v = *reinterpret_cast<float4 const*>(at);
         float o[4] = {v.x, v.y, v.z, v.w};
+        int const inside = p.N - n < 4 ? static_cast<int>(p.N - n) : 4;
+        if (!exact)
+        {
+            uint32_t bits = 0;
+            for (int j = 0; j < inside; ++j)
+                bits |= (flagA[r] | flagW[c + j]) == 1 ? 1u << j : 0u;
+            if (bits != 0)
+                atomicOr(again + r * (BN / 32) + c / 32, bits << (c % 32));
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-        {
-            if (n + j >= p.N)
-                break;
-            if (!exact)
-            {
-                bool again = false;
-                for (int s = 0; s < p.ctas; ++s)
-                    again = again || (p.ctas > 1 ? (ldSharedCluster(flagA + r, s) | ldSharedCluster(flagW + c + j, s)) : (flagA[r] | flagW[c + j])) != 0;
-                if (again)
-                {
-                    o[j] = 0.f;
-                    for (int64_t k = 0; k < p.K; ++k)
-                        o[j] = fmaf(p.A[m * p.lda + k], p.Wt[(n + j) * p.K + k], o[j]);
-                }
-            }
-            o[j] = o[j] * p.alpha + (p.bias ? __ldg(p.bias + n + j) : 0.f);
-            if (p.act == BERT_B200_ACT_GELU_ERF)
-                o[j] = geluErfF32(o[j]);
-        }
+            if (j < inside)
+                o[j] = finishF32(p, o[j], n + j);
         float* const dst = p.C + m * p.ldc + n;
-        if (p.wide && n + 3 < p.N)
+        if (p.wide && inside == 4)
             *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
         else
-            for (int j = 0; j < 4 && n + j < p.N; ++j)
+            for (int j = 0; j < inside; ++j)
                 dst[j] = o[j];
+    }
+    if (!exact && !aborted) // the same for all threads of the CTA
+    {
+        __syncthreads();
+        computeAgain<BN>(p, again, list, m0, n0);
     }
     if (p.ctas > 1)
         clusterBarrier(); // nobody leaves while its sums are being read

@@ -243,6 +243,35 @@ def test_fc_fp32_small_numbers_beside_large_ones(cuda, m, k, n, size, small_wt):
     assert float((T.fc(a, w).double() - ref).norm() / ref.norm()) <= k ** 0.5 * 2.0 ** -24
 
 
+def _off_by_four_bytes(x):
+    """The same numbers where the TMA unit cannot read them: the product is then formed by the FP32 multiply-add kernel."""
+    moved = torch.empty(x.numel() + 1, device=x.device)[1:].view(x.shape)
+    return moved.copy_(x)
+
+
+# one CTA per segment of K and one for all; a row's, a column's and a whole tile's outputs; edges of the 4 x 4 outputs that a warp computes
+@pytest.mark.parametrize("m,k,n", [(130, 384, 142), (129, 772, 97), (70, 4096, 130), (1030, 768, 770), (1030, 3072, 770)])
+def test_fc_fp32_outputs_computed_again(cuda, m, k, n):
+    """Outputs that meet numbers without exact parts: no further from float64 than the multiply-add kernel on the same numbers, and
+    the same bits whatever they are multiplied with."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    a[2] *= 2.0 ** -120
+    a[m - 1] *= 2.0 ** -115
+    w[1] *= 2.0 ** -112
+    every = T.fc(a, w)
+    for rows, cols in ((slice(2, 3), slice(2, n)), (slice(m - 1, m), slice(2, n)), (slice(3, m - 1), slice(1, 2))):
+        ref = a[rows].double() @ w[cols].double().T
+        plain = T.fc(_off_by_four_bytes(a[rows]), w[cols].contiguous())
+        assert float((every[rows, cols].double() - ref).norm()) <= float((plain.double() - ref).norm())
+    assert torch.equal(T.fc(a[:33], w).view(torch.int32), every[:33].view(torch.int32))
+    a = torch.randn(m, k, device=cuda, generator=gen) * 2.0 ** -112
+    ref = a.double() @ w.double().T
+    assert float((T.fc(a, w).double() - ref).norm()) <= float((T.fc(_off_by_four_bytes(a), w).double() - ref).norm())
+
+
 def test_fc_linearity_full_size(cuda):
     """BERT-large sizes (24576 x 1024 -> 4096): fc(a1 + a2) == fc(a1) + fc(a2) within FP16 rounding, and a
     checksum of the INT8 product equals the checksum computed from row/column sums."""
