@@ -128,6 +128,13 @@ __device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, int64_
     return p.act == BERT_B200_ACT_GELU_ERF ? geluErfF32(v) : v;
 }
 
+// Whether a sum may not be what FP32 multiply-adds give although its numbers have exact parts: the tensor core cuts off below 2^-149 with every addition
+// (error on products of 2^-126 2.3e-7 instead of 1.4e-7, of 2^-132 9e-6 instead of 2.2e-6), which a sum of 2^-100 and more does not notice.
+__device__ __forceinline__ bool sumIsInexact(float v)
+{
+    return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x0d800000u - 1u; // 0 < |v| < 2^-100
+}
+
 // The outputs of a tile whose bit in `again` (BN bits per row) is set, by FP32 multiply-adds: a warp takes 4 x 4 outputs, its lanes every 32nd four
 // of K, even and odd ones apart, and their sums are added as a tree, so an output has the same bits wherever its tile lies. The chains are a
 // quarter or less as long as those of fcF32Simt (error on normal values K = 768 0.9e-7 / 1.4e-7, 4096 1.6e-7 / 2.9e-7). Bound by the loads' latency for a
@@ -226,7 +233,7 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
 // An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by FP32 multiply-adds (computeAgain), unless one
-// of them is NaN: then it comes out as that.
+// of them is NaN: then it comes out as that. So is a sum near the smallest numbers (sumIsInexact).
 template <int BN, bool kHold>
 __global__ void __launch_bounds__(kThreadsF32, 1)
     fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ FcF32TcArgs p)
@@ -592,6 +599,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         exact = *flagAny == 0;
     }
     constexpr int kPieces = BN / 4;
+    bool any = false;
     for (int i = rank * kThreadsF32 + threadIdx.x; i < kTileM * kPieces && !aborted; i += p.ctas * kThreadsF32)
     {
         int const r = i / kPieces, c = i % kPieces * 4;
@@ -617,13 +625,19 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             v = *reinterpret_cast<float4 const*>(at);
         float o[4] = {v.x, v.y, v.z, v.w};
         int const inside = p.N - n < 4 ? static_cast<int>(p.N - n) : 4;
+        uint32_t bits = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            bits |= sumIsInexact(o[j]) ? 1u << j : 0u;
         if (!exact)
-        {
-            uint32_t bits = 0;
-            for (int j = 0; j < inside; ++j)
+            for (int j = 0; j < 4; ++j)
                 bits |= (flagA[r] | flagW[c + j]) == 1 ? 1u << j : 0u;
-            if (bits != 0)
-                atomicOr(again + r * (BN / 32) + c / 32, bits << (c % 32));
+        if (inside < 4)
+            bits &= (1u << inside) - 1u;
+        if (bits != 0)
+        {
+            atomicOr(again + r * (BN / 32) + c / 32, bits << (c % 32));
+            any = true;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -636,11 +650,8 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             for (int j = 0; j < inside; ++j)
                 dst[j] = o[j];
     }
-    if (!exact && !aborted) // the same for all threads of the CTA
-    {
-        __syncthreads();
+    if (__syncthreads_or(any))
         computeAgain<BN>(p, again, list, m0, n0);
-    }
     if (p.ctas > 1)
         clusterBarrier(); // nobody leaves while its sums are being read
 }

@@ -272,6 +272,23 @@ def test_fc_fp32_outputs_computed_again(cuda, m, k, n):
     assert float((T.fc(a, w).double() - ref).norm()) <= float((T.fc(_off_by_four_bytes(a), w).double() - ref).norm())
 
 
+# products around the smallest normal number, a row of zeros among them
+@pytest.mark.parametrize("exponent", [-50, -56, -63, -66, -70])
+@pytest.mark.parametrize("m,k,n", [(130, 384, 142), (1030, 768, 770), (70, 4096, 130)])
+def test_fc_fp32_sums_near_the_smallest_numbers(cuda, exponent, m, k, n):
+    """No further from float64 than the multiply-add kernel (which rounds to 2^-149 there, where the tensor core cuts off). At the smallest
+    exponents both round every product to 2^-149: errors of one size, whose norm over m n outputs scatters by (2 m n)^-0.5 on each side."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w = (torch.randn(s, k, device=cuda, generator=gen) * 2.0 ** exponent for s in (m, n))
+    a[5] = 0.0
+    ref, out, plain = a.double() @ w.double().T, T.fc(a, w), T.fc(_off_by_four_bytes(a), w)
+    assert float((out.double() - ref).norm()) <= (1 + 4 / (m * n) ** 0.5) * float((plain.double() - ref).norm())
+    assert bool((out[5] == 0.0).all())
+    assert torch.equal(T.fc(a[:33], w), out[:33])
+
+
 def test_fc_linearity_full_size(cuda):
     """BERT-large sizes (24576 x 1024 -> 4096): fc(a1 + a2) == fc(a1) + fc(a2) within FP16 rounding, and a
     checksum of the INT8 product equals the checksum computed from row/column sums."""
