@@ -2,13 +2,15 @@
 //
 // Replaces the FP32 cublasLtMatmul of the FC plugin (plugin/fcPlugin/fcPlugin.cpp:551-610). TF32 would break the 1e-5 tolerance
 // that the reference configuration states for FP32 (plugin/bertQKVToContextPlugin/CustomQKVToContextPluginDynamic_PluginConfig.yaml:72-76),
-// so every operand is cut into three BF16 numbers by truncation, x = h + m + l, which is exact (8 + 8 + 8 bits of the mantissa), and
-// the six products of at least 2^-16 of the largest are formed: h h + (h m + m h) + (h l + m m + l h). The three that are left
-// out are below 2^-24 of a product in sum, less than the rounding of one FP32 addition.
+// so every operand is cut into three BF16 numbers, x = h + m + l (the split of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial
+// intelligence datatype for higher-precision computations", 2019). h and m are rounded to nearest, which is exact: |m| <= 2^-8, |l| <= 2^-17 of the
+// largest number of x's exponent. Six products are formed: h h + (h m + m h) + (h l + m m + l h). The three that are left out are below
+// 2^-24 of a product in sum and have either sign.
 //
-// The tensor core adds into its FP32 accumulator by truncation, so nothing is summed there for long: a chunk of 64 products per
-// output starts from zero, its five small products first and h h last (four additions at the chunk's own magnitude), and
-// the chunks are added in registers, rounded to nearest. Error against 64 bits: see fcF32.
+// The tensor core cuts off what does not fit its FP32 accumulator, always towards zero, so nothing is summed there for long, and what is lost on
+// the way up is lost again on the way down: of a chunk of 64 products per output, the first half of h h goes into one accumulator, P; the other gets
+// the five small products (from zero, so that their additions lose little), minus that first half and plus the second one, Q. The sum is 2 P + Q,
+// and on products of one sign Q ends near zero. Chunks are added in registers, rounded to nearest. Error against 64 bits: see fcF32.
 #include "sm100.cuh"
 
 namespace b200
@@ -53,38 +55,38 @@ struct FcF32Smem
     static constexpr int kPlanesOff = kStages * kStageBytes;
     static constexpr int kBarrierOff = kPlanesOff + kParts * 3 * kPlaneBytes;
     // stFull[stages] stFree[stages] ready[parts] done[parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
-    // whether any is 1
+    // whether any is set
     static constexpr int kFlagsOff = kBarrierOff + (2 * kStages + 2 * kParts + 2) * 8 + 16;
     static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
     static constexpr int kDynamic = kTotal + 1024;
     static constexpr int kPitch = BN + 4; // floats: sums of a tile over the drained FP32 tiles
     static constexpr int kTmem = 512;
+    static constexpr int kAccs = BN <= 64 ? 2 : 1; // chunks whose sums are in tensor memory, two accumulators each
+    static constexpr int kAccCols = kAccs * 2 * BN;
     // Columns that a worker's sums of the segments before take in tensor memory: all of them but for the 128-wide tile (half).
-    static constexpr int kHeldCols = BN / 4 < (kTmem - 2 * BN - kParts * 96) / 4 ? BN / 4 : (kTmem - 2 * BN - kParts * 96) / 4;
+    static constexpr int kHeldCols = BN / 4 < (kTmem - kAccCols - kParts * 96) / 4 ? BN / 4 : (kTmem - kAccCols - kParts * 96) / 4;
     static_assert(kDynamic <= 232448, "shared memory of one CTA");
     static_assert(kTileM * kPitch * 4 + kTileM * BN / 8 + kTileM * BN / 4 + 4 <= kPlanesOff, "the sums, and what is computed again, fit the ring");
-    static_assert(2 * BN + kParts * 96 <= kTmem, "tensor memory");
+    static_assert(kAccCols + kParts * 96 + 4 * kHeldCols <= kTmem, "tensor memory");
 };
 
-// Two floats into packed BF16 parts. What is left when the last part is cut goes into the lower halves of `lost`: numbers below 2^-110 have bits
-// that BF16 does not (its smallest is 2^-133), infinities and NaN leave a NaN.
-__device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, uint32_t& lost)
+// Two floats to BF16 (the first in the lower half), rounded to nearest, and what that leaves of them.
+__device__ __forceinline__ uint64_t cutPair(uint64_t x, uint32_t& part)
 {
-    uint32_t const ua = __float_as_uint(a), ub = __float_as_uint(b);
-    h = __byte_perm(ua, ub, 0x7632);
-    float ra, rb;
-    unpack2(add2(pack2(a, b), pack2(__uint_as_float((ua & 0xffff0000u) ^ 0x80000000u), __uint_as_float((ub & 0xffff0000u) ^ 0x80000000u))), ra, rb);
-    uint32_t const va = __float_as_uint(ra), vb = __float_as_uint(rb);
-    m = __byte_perm(va, vb, 0x7632);
-    float la, lb;
-    unpack2(add2(pack2(ra, rb), pack2(__uint_as_float((va & 0xffff0000u) ^ 0x80000000u), __uint_as_float((vb & 0xffff0000u) ^ 0x80000000u))), la, lb);
-    l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
-    lost |= __float_as_uint(la) | __float_as_uint(lb);
+    float a, b;
+    unpack2(x, a, b);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(part) : "f"(b), "f"(a));
+    return fma2(pack2(__uint_as_float(part << 16), __uint_as_float(part & 0xffff0000u)), pack2(-1.f, -1.f), x);
 }
 
-__device__ __forceinline__ bool hasNan(float4 v)
+// Two floats into packed BF16 parts. What is left when the last part is cut goes into the lower halves of `lost`: numbers below 2^-110 have bits
+// that BF16 does not (its smallest is 2^-133); infinities, NaN and what rounds to infinity leave a NaN.
+__device__ __forceinline__ void splitPair(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, uint32_t& lost)
 {
-    return isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
+    float la, lb;
+    unpack2(cutPair(cutPair(pack2(a, b), h), m), la, lb);
+    l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+    lost |= __float_as_uint(la) | __float_as_uint(lb);
 }
 
 __device__ __forceinline__ void tmemStore8(uint32_t taddr, uint32_t const (&r)[8])
@@ -94,32 +96,48 @@ __device__ __forceinline__ void tmemStore8(uint32_t taddr, uint32_t const (&r)[8
                  : "memory");
 }
 
-// 32, 24, 16 or 8 columns, waited for.
-__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[32])
-{
-    tmemLoad32(taddr, r);
-    tmemLoadWait32(r);
-}
-__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[16])
-{
-    tmemLoad16(taddr, r);
-    tmemLoadWait16(r);
-}
-__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[8])
+__device__ __forceinline__ void tmemLoad8(uint32_t taddr, uint32_t (&r)[8])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
+}
+__device__ __forceinline__ void tmemLoadWait8(uint32_t (&r)[8])
+{
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                  :
                  : "memory");
 }
-__device__ __forceinline__ void tmemLoadCols(uint32_t taddr, uint32_t (&r)[24])
+
+// 16 or 8 columns at two places, waited for.
+__device__ __forceinline__ void tmemLoadTwo(uint32_t ta, uint32_t (&a)[16], uint32_t tb, uint32_t (&b)[16])
 {
-    tmemLoadCols(taddr, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
-    tmemLoadCols(taddr + 16, *reinterpret_cast<uint32_t(*)[8]>(&r[16]));
+    tmemLoad16(ta, a);
+    tmemLoad16(tb, b);
+    tmemLoadWait16(a);
+    tmemLoadWait16(b);
+}
+__device__ __forceinline__ void tmemLoadTwo(uint32_t ta, uint32_t (&a)[8], uint32_t tb, uint32_t (&b)[8])
+{
+    tmemLoad8(ta, a);
+    tmemLoad8(tb, b);
+    tmemLoadWait8(a);
+    tmemLoadWait8(b);
+}
+
+// sums[i] += 2 * P + Q for N columns.
+template <int N>
+__device__ __forceinline__ void addSums(uint32_t tP, uint32_t tQ, uint64_t* sums)
+{
+    uint32_t x[N], y[N];
+    tmemLoadTwo(tP, x, tQ, y);
+    uint64_t const two = pack2(2.f, 2.f);
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i)
+        sums[i] = add2(sums[i], fma2(pack2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), two,
+                                    pack2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1]))));
 }
 
 __device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, int64_t n)
@@ -128,11 +146,27 @@ __device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, int64_
     return p.act == BERT_B200_ACT_GELU_ERF ? geluErfF32(v) : v;
 }
 
-// Whether a sum may not be what FP32 multiply-adds give although its numbers have exact parts: the tensor core cuts off below 2^-149 with every addition
-// (error on products of 2^-126 2.3e-7 instead of 1.4e-7, of 2^-132 9e-6 instead of 2.2e-6), which a sum of 2^-100 and more does not notice.
+// Whether a sum may not be what FP32 multiply-adds give although its numbers have exact parts. The tensor core cuts off below 2^-149 with every
+// addition (error on products of 2^-126 2.3e-7 instead of 1.4e-7, of 2^-132 9e-6 instead of 2.2e-6), which a sum of 2^-100 and more does
+// not notice. And sums on the way may be twice as large as the result.
 __device__ __forceinline__ bool sumIsInexact(float v)
 {
-    return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x0d800000u - 1u; // 0 < |v| < 2^-100
+    constexpr uint32_t kLeast = 0x0d800000u, kInf = 0x7f800000u; // 2^-100
+    uint32_t const u = __float_as_uint(v) & 0x7fffffffu;
+    return u != 0 && u - kLeast >= kInf - kLeast;
+}
+
+// Whether a NaN is among the k numbers (a multiple of four, 16-byte aligned), for a warp.
+__device__ __forceinline__ bool hasNan(float const* row, int64_t k)
+{
+    bool nan = false;
+#pragma unroll 4
+    for (int64_t i = (threadIdx.x & 31) * 4; i < k; i += 128)
+    {
+        float4 const v = __ldg(reinterpret_cast<float4 const*>(row + i));
+        nan |= isnan(v.x) | isnan(v.y) | isnan(v.z) | isnan(v.w);
+    }
+    return __any_sync(0xffffffffu, nan);
 }
 
 // The outputs of a tile whose bit in `again` (BN bits per row) is set, by FP32 multiply-adds: a warp takes 4 x 4 outputs, its lanes every 32nd four
@@ -220,20 +254,22 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
     }
 }
 
-// Bound by the chain of a chunk - its place free, operands cut, products, sums read -, 2880 cycles for a 128 x 128 tile, of which the
-// tensor cores are busy 1490; no unit is full (ALU 46 %, issue slots 45 %, the shared-memory pipe 21 %). Half the code, or scalar instead of
-// packed subtractions, changes nothing. One 128 x BN tile per CTA, or one segment of its K:
+// Bound by the chain of a chunk - its place free, operands cut, products, sums read -, 3220 cycles for a 128 x 128 tile, of which the
+// tensor cores are busy 1610; no unit is full. With h and m by truncation, all products in one accumulator and two of those for every width it
+// took 2880 cycles (24 instead of 26 MMAs, the next chunk's begun before the sums were read), but its sums were too small by 1.1e-7 on numbers of one sign.
+// Rounding costs nothing: truncation of h, other subtractions or loads further ahead leave the times as they are.
+// One 128 x BN tile per CTA, or one segment of its K:
 //   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
 //   warp 1    : TMEM allocation, MMA issue. The parts of A are operands in TMEM - from shared memory both operands of a
 //               128 x 128 tile would take its whole bandwidth -, those of Wt in shared memory.
 //   warps 2-17: the parts of a chunk, the two groups of eight warps taking chunks in turn: 32 numbers of a row of A per thread, to
 //               TMEM, and whole 16-byte pieces of the parts of Wt, to shared memory. And all of them, for every chunk, its
-//               sums (32 rows, a quarter of the columns per warp) from TMEM into registers. TMEM accumulators and parts are
-//               double-buffered.
+//               sums (32 rows, a quarter of the columns per warp) from TMEM into registers. Parts are double-buffered, the two
+//               accumulators too where tensor memory has room (up to 64 columns).
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
 // An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by FP32 multiply-adds (computeAgain), unless one
-// of them is NaN: then it comes out as that. So is a sum near the smallest numbers (sumIsInexact).
+// of them is NaN: then it comes out as that. So is a sum that sumIsInexact names.
 template <int BN, bool kHold>
 __global__ void __launch_bounds__(kThreadsF32, 1)
     fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ FcF32TcArgs p)
@@ -241,7 +277,8 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     using L = FcF32Smem<BN>;
     constexpr uint32_t kIdesc = makeInstrDesc(1u, 1u, 0u, 0u, 128u, static_cast<uint32_t>(BN));
     constexpr int kCols = BN / 4; // accumulator columns per worker thread
-    constexpr uint32_t kPartsCol = 2 * BN;
+    constexpr uint32_t kIdescMinus = kIdesc | 1u << 13; // minus A
+    constexpr uint32_t kPartsCol = L::kAccCols;
 
     extern __shared__ uint8_t smemRaw[];
     uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -339,21 +376,29 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int c = 0; c < count && ok; ++c)
         {
             uint32_t const s = c & 1, round = c >> 1;
-            ok = (c < 2 || mbarWaitWarp(&accFree[s], (round - 1) & 1u, abortFlag, kWaitAccFree))
+            uint32_t const slot = c % L::kAccs;
+            ok = (c < L::kAccs || mbarWaitWarp(&accFree[slot], (c / L::kAccs - 1) & 1u, abortFlag, kWaitAccFree))
                 && mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
             tcFenceAfter();
             if (ok && electOne())
             {
                 // parts (A, Wt), the smallest products first
-                constexpr int kOrder[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+                constexpr int kOrder[5][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
                 uint32_t const a = tmemBase + kPartsCol + s * 96;
                 uint32_t const w = wLo + s * (3 * L::kPlaneBytes >> 4);
+                uint32_t const sumP = tmemBase + slot * 2 * BN, sumQ = sumP + BN;
 #pragma unroll
-                for (int i = 0; i < 6; ++i)
+                for (int i = 0; i < 5; ++i)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        mmaF16TmemA(tmemBase + s * BN, a + kOrder[i][0] * 32 + k * 8, w + kOrder[i][1] * (L::kPlaneBytes >> 4) + k * 2, descHi,
-                            kIdesc, i != 0 || k != 0);
+                        mmaF16TmemA(sumQ, a + kOrder[i][0] * 32 + k * 8, w + kOrder[i][1] * (L::kPlaneBytes >> 4) + k * 2, descHi, kIdesc,
+                            i != 0 || k != 0);
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    mmaF16TmemA(sumP, a + k * 8, w + k * 2, descHi, kIdesc, k != 0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    mmaF16TmemA(sumQ, a + k * 8, w + k * 2, descHi, k < 2 ? kIdescMinus : kIdesc, true);
                 tcCommit(&done[s]);
             }
             __syncwarp();
@@ -370,7 +415,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         uint32_t const tRow = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
         // Sums of the segments before: touched once per segment and kept out of the registers, which are all taken in the loop
         // (spilled by the compiler they cost 14 us of 1024 x 2304 x 768: beside so much shared memory the L1 holds little). What does
-        // not fit tensor memory is in local memory on purpose. (All of them there: 31.5 us instead of 28.9 us.)
+        // not fit tensor memory is in local memory on purpose (all of them there: 2.6 us more).
         uint32_t const tHeld = tRow + kPartsCol + kParts * 96 + cols * L::kHeldCols;
         volatile uint64_t rest[kHold && kCols > L::kHeldCols ? (kCols - L::kHeldCols) / 2 : 1];
         int segment = 0;
@@ -382,16 +427,17 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             tcFenceAfter();
             if (hasRows)
             {
-                uint32_t x[kCols];
-                tmemLoadCols(tRow + (c & 1) * BN + cols * kCols, x);
+                uint32_t const t = tRow + (c % L::kAccs) * 2 * BN + cols * kCols;
 #pragma unroll
-                for (int i = 0; i < kCols / 2; ++i)
-                    acc[i] = add2(acc[i], pack2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])));
+                for (int g = 0; g + 16 <= kCols; g += 16)
+                    addSums<16>(t + g, t + BN + g, acc + g / 2);
+                if constexpr (kCols % 16 != 0)
+                    addSums<8>(t + kCols - 8, t + BN + kCols - 8, acc + (kCols - 8) / 2);
             }
             tcFenceBefore();
             __syncwarp();
             if (lane == 0)
-                mbarArrive(&accFree[c & 1]);
+                mbarArrive(&accFree[c % L::kAccs]);
             if constexpr (kHold)
                 if (c + 1 == segmentEnd)
                 {
@@ -404,7 +450,8 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                         for (int g = 0; g < L::kHeldCols / 8; ++g)
                         {
                             uint32_t x[8];
-                            tmemLoadCols(tHeld + g * 8, x);
+                            tmemLoad8(tHeld + g * 8, x);
+                            tmemLoadWait8(x);
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
                                 acc[g * 4 + i] = add2(pack2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), acc[g * 4 + i]);
@@ -443,11 +490,6 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     }
                 }
         };
-        auto flag = [&](uint32_t* at, bool nan) {
-            atomicOr(at, nan ? 2u : 1u);
-            if (!nan)
-                *flagAny = 1;
-        };
         int stage = 0;
         uint32_t phase = 0;
         for (int c = 0; c < count; ++c)
@@ -484,13 +526,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                         tmemStore8(t + g * 8 + 64, l);
                     }
                     if ((lost & 0xffffu) != 0)
-                    {
-                        bool nan = false;
-#pragma unroll 1
-                        for (int i = 0; i < 8; ++i)
-                            nan = nan || hasNan(src[i]);
-                        flag(flagA + row, nan);
-                    }
+                        flagA[row] = *flagAny = 1;
                 }
                 // eight numbers of a row of Wt: 16 bytes of each part
                 uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
@@ -522,7 +558,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                         *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
                         *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
                         if ((lost & 0xffffu) != 0)
-                            flag(flagW + row, hasNan(v[i][0]) || hasNan(v[i][1]));
+                            flagW[row] = *flagAny = 1;
                     }
                 }
                 fenceProxyAsync();
@@ -581,22 +617,27 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         clusterBarrier();
         for (int s = 0; s < p.ctas; ++s)
             exact = exact && ldSharedCluster(flagAny, s) == 0;
-        if (!exact)
-        {
-            uint32_t merged = 0; // flags of a row over all of K
-            if (threadIdx.x < kTileM + BN)
-                for (int s = 0; s < p.ctas; ++s)
-                    merged |= ldSharedCluster(flagA + threadIdx.x, s);
-            clusterBarrier();
-            if (threadIdx.x < kTileM + BN)
-                flagA[threadIdx.x] = merged;
-            __syncthreads();
-        }
     }
     else
     {
         __syncthreads();
         exact = *flagAny == 0;
+    }
+    if (!exact)
+    {
+        uint32_t merged = 0; // a row's flag over all of K
+        if (threadIdx.x < kTileM + BN)
+            for (int s = 0; s < p.ctas; ++s)
+                merged |= p.ctas > 1 ? ldSharedCluster(flagA + threadIdx.x, s) : flagA[threadIdx.x];
+        if (p.ctas > 1)
+            clusterBarrier();
+        if (threadIdx.x < kTileM + BN)
+            flagA[threadIdx.x] = merged;
+        __syncthreads();
+        for (int r = warp; r < kTileM + BN; r += kThreadsF32 / 32)
+            if (flagA[r] != 0 && hasNan(r < kTileM ? p.A + (m0 + r) * p.lda : p.Wt + (n0 + r - kTileM) * p.K, p.K))
+                flagA[r] = 2;
+        __syncthreads();
     }
     constexpr int kPieces = BN / 4;
     bool any = false;
@@ -631,7 +672,10 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             bits |= sumIsInexact(o[j]) ? 1u << j : 0u;
         if (!exact)
             for (int j = 0; j < 4; ++j)
-                bits |= (flagA[r] | flagW[c + j]) == 1 ? 1u << j : 0u;
+            {
+                uint32_t const flags = flagA[r] | flagW[c + j];
+                bits = (bits | (flags & 1u) << j) & ~((flags >> 1) << j);
+            }
         if (inside < 4)
             bits &= (1u << inside) - 1u;
         if (bits != 0)
@@ -681,11 +725,17 @@ int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaSt
 
 } // namespace
 
-// From K = 384 on. Error against 64 bits (2-norm, normal inputs) here / of the FP32 multiply-adds of fcF32Simt: K = 384 1.31e-7 / 1.34e-7,
-// 768 1.34e-7 / 1.40e-7, 1024 1.36e-7 / 1.57e-7, 3072 1.44e-7 / 2.56e-7, 4096 1.47e-7 / 2.94e-7; below, the truncation of the tensor core
-// shows (K = 36 1.12e-7 / 0.81e-7) and the multiply-adds stay. They also take what the TMA unit does not: rows that are no
-// multiple of 16 bytes apart, sizes beyond its coordinates. Time, same order: 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 10.9 / 14.9 us, 128 x 768 x
-// 3072 13.9 / 44.6 us, 1024 x 2304 x 768 28.9 / 95.7 us, 4096 x 1024 x 4096 205 / 843 us.
+// From K = 384 on. Error against 64 bits (2-norm) here / of the FP32 multiply-adds of fcF32Simt, in 1e-7:
+//   K                        384          768          1024         3072         4096
+//   normal                   0.83 / 1.34  0.89 / 1.40  0.91 / 1.58  1.03 / 2.56  1.07 / 2.93
+//   rectified x normal       0.81 / 1.05  0.85 / 1.10  0.88 / 1.21  1.00 / 1.88  1.03 / 2.10
+//   uniform, 0 ... 1         0.40 / 0.56  0.44 / 0.55  0.45 / 0.56  0.50 / 0.71  0.50 / 0.73
+//   normal, 1 +- 0.2         0.43 / 0.55  0.48 / 0.55  0.49 / 0.55  0.54 / 0.71  0.54 / 0.72
+// (mean error on the third and fourth -0.06 and +0.22; parts by truncation and 64 products in one accumulator: 1.2 and 1.0, the mean -1.1 and
+// -0.9). A shorter K has not been measured in this form and stays with the multiply-adds. They also take what the TMA unit does not: rows that are no
+// multiple of 16 bytes apart, sizes beyond its coordinates. GPU time, same order: 1 x 64 x 384 6.3 / 8.5 us, 1 x 768 x 768 8.0 / 8.6 us, 37 x 768 x 768
+// 8.4 / 8.9 us, 37 x 2304 x 768 11.2 / 14.9 us, 300 x 768 x 512 9.9 / 18.5 us, 128 x 768 x 3072 14.0 / 44.9 us, 1024 x 2304 x 768 33.2 / 96.9 us,
+// 4096 x 1024 x 4096 232 / 843 us. The two tensor maps cost a call 1 us of the host: 10.1 instead of 9.5 us where the host is what bounds it.
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
     constexpr int64_t kMax = 1ll << 31;
@@ -698,8 +748,10 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
     int const segments = kChunks >= 24 ? 8 : kChunks >= 12 ? 4 : 2;
     // Width of the tiles, and whether a CTA takes all segments: what the measured cycles per chunk and per CTA, times the waves of CTAs,
     // make shortest. Clusters find fewer places than there are SMs. Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768
-    // 29.1 / 42.5 / 36.0 / 55.0 us, 1024 x 3072 x 768 55.1 / 42.9 / 52.2 / 80.4 us, 1024 x 768 x 768 27.6 / 21.2 / 17.6 / 27.0 us; one segment per
-    // CTA, 128 / 64 columns: 1024 x 768 x 3072 73.4 / 94.5 us (64 columns in one CTA 51.9 us), 128 x 768 x 3072 17.9 / 13.8 us (50.1 us).
+    // 33.6 / 49.9 / 39.0 / 56.5 us, 1024 x 3072 x 768 64.1 / 50.3 / 57.1 / 83.0 us, 1024 x 768 x 768 32.2 / 25.4 / 19.6 / 28.1 us; one segment per
+    // CTA, 128 / 64 columns: 1024 x 768 x 3072 75.4 / 97.7 us (64 columns in one CTA 56.0 us), 128 x 768 x 3072 19.4 / 14.6 us (54.0 us).
+    static constexpr int kCycles[4] = {1480, 1990, 2700, 3220}; // per chunk, of 32, 64, 96 and 128 columns
+    static constexpr int kFixed[2][4] = {{12500, 13000, 16500, 26000}, {12500, 14500, 16300, 17500}}; // per CTA with all segments, with one
     int bestN = 128, bestCtas = 1;
     int64_t best = 0;
     for (int bn = 128; bn >= 32; bn -= 32)
@@ -707,8 +759,8 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
         {
             int64_t const slots = smCount() * (ctas == 1 ? 148 : ctas == 2 ? 140 : ctas == 4 ? 128 : 112) / 148;
             int64_t const waves = (mTiles * ((p.n + bn - 1) / bn) * ctas + slots - 1) / slots;
-            int64_t const fixed = ctas == 1 ? 9000 + 700 * (segments - 1) : 10000 + 700 * ctas;
-            int64_t const cost = waves * ((kChunks + ctas - 1) / ctas * (bn == 128 ? 2880 : bn == 96 ? 2330 : bn == 64 ? 1880 : 1400) + fixed);
+            int const fixed = kFixed[ctas > 1][bn / 32 - 1] - (bn == 128 && segments == 2 && ctas == 1 ? 6000 : 0); // little to hold
+            int64_t const cost = waves * ((kChunks + ctas - 1) / ctas * kCycles[bn / 32 - 1] + fixed);
             if (best == 0 || cost < best)
             {
                 best = cost;

@@ -272,6 +272,46 @@ def test_fc_fp32_outputs_computed_again(cuda, m, k, n):
     assert float((T.fc(a, w).double() - ref).norm()) <= float((T.fc(_off_by_four_bytes(a), w).double() - ref).norm())
 
 
+# K from where the tensor cores take it on (a tail included), tiles of few and many columns
+@pytest.mark.parametrize("m,k,n", [(200, 384, 130), (200, 772, 130), (1030, 768, 2304), (300, 1024, 770), (200, 3072, 768), (520, 4096, 1024)])
+@pytest.mark.parametrize("values", ["normal", "rectified", "one sign", "around one"])
+def test_fc_fp32_error_against_float64(cuda, values, m, k, n):
+    """No further from float64 (2-norm over m n outputs) than the multiply-add kernel on the same numbers, whatever their signs; on numbers of
+    one sign the mean error is below half a unit of the last place too (2^-24)."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    if values == "rectified":
+        a = torch.clamp(a, min=0.0)
+    elif values == "one sign":
+        a, w = torch.rand(m, k, device=cuda, generator=gen), torch.rand(n, k, device=cuda, generator=gen)
+    elif values == "around one":
+        a, w = 1 + 0.2 * a, 1 + 0.2 * w
+    st = _status(cuda)
+    ref, out, plain = a.double() @ w.double().T, T.fc(a, w, status=st).double(), T.fc(_off_by_four_bytes(a), w).double()
+    assert int(st[0]) == 0
+    assert float((out - ref).norm()) <= float((plain - ref).norm())
+    if values in ("one sign", "around one"):
+        assert abs(float(((out - ref) / ref).mean())) <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("m,k,n", [(130, 384, 142), (1030, 768, 770)])
+def test_fc_fp32_sums_near_the_largest_numbers(cuda, m, k, n):
+    """Sums of 2^127 on the way to a small result, and the largest number itself, whose BF16 rounding is infinity: exact in any order."""
+    import tensorrt_b200 as T
+
+    a, w = torch.full((m, k), 2.0 ** 122, device=cuda), torch.ones(n, k, device=cuda)
+    a.view(m, k // 64, 64)[:, :, 32:] = -2.0 ** 122
+    a[:, k - 1] = 0.0
+    w[:, 0] = 0.5
+    a[5] = 0.0
+    a[5, 7] = torch.finfo(torch.float32).max
+    w[3] = 0.5
+    ref, out = a.double() @ w.double().T, T.fc(a, w)
+    assert torch.equal(out.double(), ref)
+
+
 # products around the smallest normal number, a row of zeros among them
 @pytest.mark.parametrize("exponent", [-50, -56, -63, -66, -70])
 @pytest.mark.parametrize("m,k,n", [(130, 384, 142), (1030, 768, 770), (70, 4096, 130)])
