@@ -173,7 +173,8 @@ def test_fc_fp32_tile_edges(cuda, m, k, n, epi):
     assert bool((out[m] == 7.0).all())   # nothing written past the last row
 
 
-# K in one, two, four and eight segments; rows for which a tile's segments go to one CTA each and to one CTA (148 SMs)
+# K in one, two, four and eight segments. K below 384 or no multiple of four: multiply-adds, rows for which a tile's segments go to one CTA each
+# and to one CTA (`one_wave`, of 64 x 64 tiles on 148 SMs); K = 400, 768 and 3072: tensor cores, with these rows 32 to 128 columns, clusters and single CTAs
 @pytest.mark.parametrize("k,n", [(80, 96), (192, 200), (400, 768), (768, 768), (3072, 768), (1001, 130)])
 def test_fc_fp32_rows_do_not_depend_on_m(cuda, k, n):
     """The same bits for a row whatever it is multiplied with."""
@@ -310,6 +311,43 @@ def test_fc_fp32_sums_near_the_largest_numbers(cuda, m, k, n):
     w[3] = 0.5
     ref, out = a.double() @ w.double().T, T.fc(a, w)
     assert torch.equal(out.double(), ref)
+
+
+# each width of the tiles, with all segments of K (two, four, eight) in a CTA and with one each, as fcF32 chooses them on 148 SMs; rows, columns and K that
+# fill neither a tile nor a chunk
+@pytest.mark.parametrize("m,k,n", [
+    (4547, 388, 65), (4163, 708, 33), (67, 1540, 1793), (67, 388, 33), (67, 708, 33), (67, 1540, 33),              # 32 columns: 2, 4, 8 held; 2, 4, 8 CTAs
+    (6339, 388, 65), (6339, 708, 65), (6339, 1540, 65), (4547, 388, 33), (67, 708, 1025), (67, 1540, 449),         # 64
+    (6339, 388, 129), (6339, 708, 129), (6339, 1540, 129), (6339, 452, 65), (67, 708, 2049), (67, 1540, 897),      # 96
+    (6339, 388, 193), (6339, 708, 193), (6339, 1540, 193), (2115, 708, 97), (67, 1540, 1345), (1024, 768, 2304)])  # 128 (no two CTAs)
+def test_fc_fp32_every_width_and_division_of_k(cuda, m, k, n):
+    """No further from float64 than the multiply-add kernel, the bits of fewer rows, outputs computed again, the epilogue, and nothing written beyond."""
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + k + n)
+    a, w, bias = (torch.randn(*s, device=cuda, generator=gen) for s in ((m, k), (n, k), (n,)))
+    st = _status(cuda)
+    out = torch.full((m + 1, n), 7.0, device=cuda)
+    T.fc(a, w, status=st, out=out[:m])
+    ref = a.double() @ w.double().T
+    assert float((out[:m].double() - ref).norm()) <= float((T.fc(_off_by_four_bytes(a), w).double() - ref).norm())
+    assert torch.equal(T.fc(a[-38:], w), out[m - 38:m])
+    # erff is good to 2 units of the last place, the sum to half of one of its terms' magnitudes
+    want = torch.nn.functional.gelu(out[:m].double() * 0.5 + bias.double())
+    assert bool(((T.fc(a, w, bias, T.ACT_GELU_ERF, alpha=0.5).double() - want).abs() <= 2.0 ** -21 * torch.clamp(out[:m].abs() + bias.abs(), min=1.0)).all())
+    a[m - 2] *= 2.0 ** -120
+    w[n - 1] *= 2.0 ** -120
+    a[1, k - 1] = float("nan")
+    w[1, 0] = -float("inf")
+    again = T.fc(a, w, status=st, out=out[:m])
+    ref = a.double() @ w.double().T
+    assert int(st[0]) == 0 and bool((out[m] == 7.0).all())
+    assert torch.equal(torch.isnan(ref), torch.isnan(again)) and torch.equal(torch.isinf(ref), torch.isinf(again))
+    finite = torch.isfinite(ref)
+    # the 2-norm of the error is below 2^-23 of the result's for normal values, a result |a| |w| k^-0.5 on average: eight times that for the largest of
+    # a million; 2^-140 for what lies below the smallest numbers
+    size = torch.nan_to_num(a.double() ** 2, 0, 0, 0).sum(1, keepdim=True).sqrt() * torch.nan_to_num(w.double() ** 2, 0, 0, 0).sum(1).sqrt()
+    assert bool(((again.double() - ref).abs()[finite] <= (2.0 ** -20 * k ** -0.5 * size + 2.0 ** -140)[finite]).all())
 
 
 # products around the smallest normal number, a row of zeros among them
