@@ -193,7 +193,13 @@ enum
  * C[m,n] = epilogue( sum_k A[m,k] * Wt[n,k] ).
  *  type_id 1: A, Wt FP16, FP32 accumulation (tcgen05 kind::f16);   out_type_id 1.
  *  type_id 2: A, Wt INT8, INT32 accumulation (tcgen05 kind::i8);   out_type_id 1 or 2.
- *  type_id 0: A, Wt FP32, FP32 SIMT kernel;                        out_type_id 0.
+ *  type_id 0: A, Wt FP32, full FP32 precision;                     out_type_id 0.
+ *    k >= 384, k % 4 == 0, lda % 4 == 0, A and Wt 16-byte aligned: tensor cores (three BF16 parts per number, six products,
+ *    sums of 64 products in the tensor core, the rest in FP32); otherwise FP32 multiply-adds. The two round differently, so
+ *    the same numbers may differ in the last bits where one call is aligned and another is not. Both are within 2e-7
+ *    of the exact result (2-norm) for normal inputs up to k = 1024; the tensor cores are the closer ones. Infinities, NaN, the
+ *    smallest and the largest numbers come out as multiply-adds give them, at up to ten times the time when a whole
+ *    input consists of infinities or of numbers below 2^-110.
  * epilogue(acc) = quant( act( acc * alpha + bias[n] ) ), bias FP32 or NULL, act per `activation`,
  * quant = sat8(rni(x * out_scale)) when out_type_id == 2, identity otherwise.
  * Wt is the weight matrix stored [n][k] (K contiguous); the reference plugin holds W as [k][n]

@@ -31,8 +31,6 @@
 //                         the next tile.
 //               The passes loop over the key blocks (not unrolled): unrolled, the kernel was bound by instruction
 //               fetch (122 KB of text, 77 % instruction-cache hits).
-// The kernel template also takes FP16 tensors (exact-maximum two-sweep form, P in shared memory); that instantiation
-// is not built.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM, reports through the status word.
 #include "mha_items.h"
 #include "sm100.cuh"
@@ -54,7 +52,7 @@ constexpr int kQTile = 128;
 constexpr int kKeyBlock = 128;
 constexpr int kHeadSize = 64;
 constexpr int kMaxBlocks = 4; // S <= 512
-constexpr int kMhaThreads = 608;     // TMA warp, MMA warp, 16 softmax warps, second MMA warp (FP16)
+constexpr int kMhaThreads = 608;     // TMA warp, MMA warp, 16 softmax warps, second MMA warp
 constexpr int kSoftmaxThreads = 512;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kOColumn = 384;   // context accumulator when the scores need at most 384 columns
@@ -81,13 +79,10 @@ struct alignas(1024) ItemTable
     int32_t lengths[kItemOrder];
 };
 
-template <typename T>
 struct MhaSmem
 {
-    static constexpr int kElem = sizeof(T);
-    static constexpr int kRowBytes = kHeadSize * kElem;           // 128 (FP16) or 64 (INT8)
-    static constexpr int kTileBytes = kQTile * kRowBytes;         // Q tile, one K block, one V block
-    static constexpr int kPBytes = kQTile * kKeyBlock * kElem;    // one P block: 32 KB (FP16) or 16 KB (INT8)
+    static constexpr int kTileBytes = kQTile * kHeadSize; // Q tile, one K block, one V block
+    static constexpr int kPBytes = kQTile * kKeyBlock;    // one P block
     // [ Q ][ K blocks ][ V blocks ][ P slots ][ barriers, reduction scratch ]
     static __host__ __device__ constexpr int kOffset()
     {
@@ -145,17 +140,11 @@ __device__ __forceinline__ uint32_t packProb4(float a, float b, float c, float d
     return __byte_perm(__byte_perm(ua, ub, 0x0040), __byte_perm(uc, ud, 0x0040), 0x5410);
 }
 
-// The row reductions only join the four warps that own the columns of the same 32 query rows (one TMEM lane
-// quadrant). FP16: one named barrier per quadrant, so that the quadrants drift apart instead of waiting for the
-// slowest (+6 % at S = 384). INT8: all sixteen warps in step - its per-key-block hand-overs to the MMA warps need
-// every warp's arrival anyway, and drifting quadrants delay them (per-quadrant barriers: -4 %).
-template <bool kPerQuadrant>
-__device__ __forceinline__ void softmaxBarrier(int quad)
+// All sixteen softmax warps in step: the row reductions only join the four that own the columns of the same 32 query rows, but the
+// per-key-block hand-overs to the MMA warps need every warp's arrival anyway (a barrier per four warps: -4 %).
+__device__ __forceinline__ void softmaxBarrier()
 {
-    if (kPerQuadrant)
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory");
-    else
-        asm volatile("bar.sync 1, 512;" ::: "memory");
+    asm volatile("bar.sync 1, 512;" ::: "memory");
 }
 
 __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[32])
@@ -171,28 +160,26 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
         : "memory");
 }
 
-// IL (INT8 only): CHW32-interleaved tensors. Q, K and V tiles then arrive as two 32-channel sub-tiles of
+// IL: CHW32-interleaved tensors. Q, K and V tiles then arrive as two 32-channel sub-tiles of
 // [128 tokens][32 B] (32-byte swizzle); the head dimension is covered by one MMA per sub-tile.
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
 // ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h).
-template <typename T, bool IL, bool BNSD, bool ORDERED>
+template <bool IL, bool BNSD, bool ORDERED>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
 {
     static_assert(!BNSD || !IL, "separate Q / K / V tensors: linear layout");
-    using L = MhaSmem<T>;
-    constexpr bool kInt8 = sizeof(T) == 1;
-    static_assert(!IL || kInt8, "the interleaved layout is INT8 only");
-    // Q, K, V rows are 128 B (FP16), 64 B (INT8) or 32 B (interleaved INT8 sub-tiles)
-    constexpr uint64_t kSwz = IL ? kSwizzle32B : (kInt8 ? kSwizzle64B : kSwizzle128B);
-    constexpr uint32_t kAtomBytes = IL ? 256u : 8 * L::kRowBytes; // 8 rows of a swizzle atom: SBO
-    constexpr uint32_t kSubTile = L::kTileBytes / 2;              // interleaved: bytes of one 32-channel sub-tile
-    constexpr int kQkMmas = kInt8 ? 2 : 4;                        // head size 64 = 2 x 32 (INT8) or 4 x 16 (FP16)
-    constexpr int kPvMmas = kInt8 ? 4 : 8;                        // 128 keys = 4 x 32 or 8 x 16
-    constexpr uint32_t kIdescQk = makeInstrDesc(kInt8 ? 2u : 1u, kInt8 ? 1u : 0u, 0u, 0u, 128u, 128u);
-    constexpr uint32_t kIdescPv = makeInstrDesc(kInt8 ? 2u : 1u, kInt8 ? 1u : 0u, 0u, 1u, 128u, 64u);
+    using L = MhaSmem;
+    // Q, K, V rows are 64 B or 32 B (interleaved sub-tiles)
+    constexpr uint64_t kSwz = IL ? kSwizzle32B : kSwizzle64B;
+    constexpr uint32_t kAtomBytes = IL ? 256u : 8 * kHeadSize; // 8 rows of a swizzle atom: SBO
+    constexpr uint32_t kSubTile = L::kTileBytes / 2;           // interleaved: bytes of one 32-channel sub-tile
+    constexpr int kQkMmas = 2;                                 // head size 64 = 2 x 32
+    constexpr int kPvMmas = 4;                                 // 128 keys = 4 x 32
+    constexpr uint32_t kIdescQk = makeInstrDesc(2u, 1u, 0u, 0u, 128u, 128u);
+    constexpr uint32_t kIdescPv = makeInstrDesc(2u, 1u, 0u, 1u, 128u, 64u);
 
     int const warp = threadIdx.x >> 5;
     int const lane = threadIdx.x & 31;
@@ -443,9 +430,9 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             constexpr bool kDoContext = decltype(doContextTag)::value;
             bool ok = true;
             uint64_t const dQk = makeSmemDesc(0, 16, kAtomBytes, kSwz);
-            // P: K-major, 128-byte rows, 128-byte swizzle. FP16 holds the block as two 64-key tiles.
+            // P: K-major, 128-byte rows, 128-byte swizzle.
             uint64_t const dP = makeSmemDesc(0, 16, 1024, kSwizzle128B);
-            // V: MN-major (head dimension contiguous), one MMA consumes 16 (FP16) / 32 (INT8) key rows.
+            // V: MN-major (head dimension contiguous), one MMA consumes 32 key rows.
             // Interleaved: the two 32-channel sub-tiles are LBO apart, 32 key rows are 1024 bytes.
             uint64_t const dV = IL ? makeSmemDesc(0, kSubTile, kAtomBytes, kSwz) : makeSmemDesc(0, kAtomBytes, kAtomBytes, kSwz);
             uint32_t const hiQk = static_cast<uint32_t>(dQk >> 32), hiP = static_cast<uint32_t>(dP >> 32),
@@ -467,7 +454,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     for (int k = 0; k < kQkMmas; ++k)
                     {
                         uint32_t const off = (IL ? k * kSubTile : k * 32) >> 4; // next 32 bytes of the head dimension
-                        mmaLoHi<kInt8>(tmemBase + j * kKeyBlock, qLo + off, hiQk, kLo + j * kTile16 + off, hiQk, kIdescQk, k != 0);
+                        mmaLoHi<true>(tmemBase + j * kKeyBlock, qLo + off, hiQk, kLo + j * kTile16 + off, hiQk, kIdescQk, k != 0);
                     }
                     tcCommit(&sFull[j]);
                     if (j == nbOf - 1)
@@ -556,8 +543,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                                         for (int k = 0; k < kPvMmas; ++k)
                                         {
                                             constexpr uint32_t kVStep = (IL ? 1024u : 2048u) >> 4;
-                                            uint32_t const pOff = (kInt8 ? k * 32 : (k / 4) * (kQTile * 128) + (k % 4) * 32) >> 4;
-                                            mmaLoHi<kInt8>(tmemBase + oCol, a + pOff, hiP, b + k * kVStep, hiV, kIdescPv, (j | k) != 0);
+                                            mmaLoHi<true>(tmemBase + oCol, a + k * 2, hiP, b + k * kVStep, hiV, kIdescPv, (j | k) != 0);
                                         }
                                         if (oAliasesScores) // otherwise every tile has its own P slots, released with oFull
                                             tcCommit(&pFree[slotOf(j)]);
@@ -659,9 +645,9 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             slotFilled |= 1u << slot;
             return got;
         };
-        // Reads 16 of the 64 context values of this row (tile number `tileNo` of the CTA), normalises / requantises
+        // Reads 16 of the 64 context values of this row (tile number `tileNo` of the CTA), requantises
         // and stores them to `dst` (null: row beyond the sequence).
-        auto epilogue = [&](uint32_t tileNo, T* dst, float inv) {
+        auto epilogue = [&](uint32_t tileNo, int8_t* dst) {
             if (ok)
                 ok = mbarWait(oFull, tileNo & 1, abortFlag, kWaitAccFull);
             if (!ok)
@@ -674,31 +660,16 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             mbarArrive(oFree);
             if (dst == nullptr)
                 return;
-            if (kInt8)
-            {
-                float const s2 = args.scaleBmm2;
-                uint4 o;
-                uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+            float const s2 = args.scaleBmm2;
+            uint4 o;
+            uint32_t* w = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    w[i] = packChar4(static_cast<float>(static_cast<int32_t>(x[4 * i])) * s2,
-                        static_cast<float>(static_cast<int32_t>(x[4 * i + 1])) * s2,
-                        static_cast<float>(static_cast<int32_t>(x[4 * i + 2])) * s2,
-                        static_cast<float>(static_cast<int32_t>(x[4 * i + 3])) * s2);
-                *reinterpret_cast<uint4*>(dst) = o;
-            }
-            else
-            {
-#pragma unroll
-                for (int g = 0; g < 2; ++g)
-                {
-                    float f[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        f[i] = __uint_as_float(x[g * 8 + i]) * inv;
-                    reinterpret_cast<uint4*>(dst)[g] = packHalf8(f);
-                }
-            }
+            for (int i = 0; i < 4; ++i)
+                w[i] = packChar4(static_cast<float>(static_cast<int32_t>(x[4 * i])) * s2,
+                    static_cast<float>(static_cast<int32_t>(x[4 * i + 1])) * s2,
+                    static_cast<float>(static_cast<int32_t>(x[4 * i + 2])) * s2,
+                    static_cast<float>(static_cast<int32_t>(x[4 * i + 3])) * s2);
+            *reinterpret_cast<uint4*>(dst) = o;
         };
 
         // The epilogue of a tile runs after pass A of the CTA's next tile (of the same or the next item): the last PV
@@ -706,31 +677,30 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         // shares columns with the scores.
         bool const deferEpilogue = !oAliasesScores;
         bool pending = false;
-        T* pendDst = nullptr;
-        float pendInv = 0.f;
+        int8_t* pendDst = nullptr;
 
         Item it;
         for (int item = firstItem; item < numItems; item += itemStep)
         {
             bool const work = getItem(item, it);
             int64_t const outRowStride = static_cast<int64_t>(args.N) * args.d; // elements
-            T* const outBase = static_cast<T*>(args.out) + static_cast<int64_t>(it.head) * args.d;
+            int8_t* const out = static_cast<int8_t*>(args.out);
+            int8_t* const outBase = out + static_cast<int64_t>(it.head) * args.d;
             // linear layouts: the d values of (token, head) are contiguous
-            auto outRow = [&](int q) -> T* {
+            auto outRow = [&](int q) -> int8_t* {
                 if (BNSD)
-                    return static_cast<T*>(args.out) + ((static_cast<int64_t>(it.b) * args.N + it.head) * args.S + q) * args.d;
+                    return out + ((static_cast<int64_t>(it.b) * args.N + it.head) * args.S + q) * args.d;
                 int64_t const rr = args.fixedLayout ? static_cast<int64_t>(q) * args.B + it.b : static_cast<int64_t>(it.rowBase) + q;
                 return outBase + rr * outRowStride;
             };
             // interleaved output [N][d/32][total][32]: 32-channel group `grp` of (token, head)
-            auto outPtrIl = [&](int q, int grp) -> T* {
-                return static_cast<T*>(args.out)
-                    + ((static_cast<int64_t>(it.head) * (args.d / 32) + grp) * args.total + it.rowBase + q) * 32;
+            auto outPtrIl = [&](int q, int grp) -> int8_t* {
+                return out + ((static_cast<int64_t>(it.head) * (args.d / 32) + grp) * args.total + it.rowBase + q) * 32;
             };
             if (!work)
             {
                 // no valid key: every probability is zero and so is the context row
-                int const kChunks = args.d * L::kElem / 16;
+                int const kChunks = args.d / 16;
                 int const q0 = it.tBegin * kQTile, q1 = min(it.rows, it.tEnd * kQTile);
                 for (int i = threadIdx.x - 64; i < (q1 - q0) * kChunks; i += kSoftmaxThreads)
                 {
@@ -749,184 +719,125 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             {
                 uint32_t x[32];
 
-                // ---- pass A: row maximum (INT8: integer maximum, no conversions) ----
-                float mx = -INFINITY;
+                // ---- pass A: row maximum (integers, no conversions) ----
                 int32_t mxi = INT32_MIN;
 #pragma unroll 1
                 for (int j = 0; j < nb; ++j)
                 {
-                    if (j < nb)
+                    ok = ok && mbarWait(&sFull[j], (sBits >> j) & 1u, abortFlag, kWaitSoftmax);
+                    tcFenceAfter();
+                    tmemLoad32(tRow + colOf(j), x);
+                    tmemLoadWait32(x);
+                    int const limit = len - colOf(j);
+                    if (limit >= 32)
                     {
-                        ok = ok && mbarWait(&sFull[j], (sBits >> j) & 1u, abortFlag, kWaitSoftmax);
-                        tcFenceAfter();
-                        tmemLoad32(tRow + colOf(j), x);
-                        tmemLoadWait32(x);
-                        int const limit = len - colOf(j);
-                        if (limit >= 32)
-                        {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                            {
-                                if (kInt8)
-                                    mxi = max(mxi, static_cast<int32_t>(x[i]));
-                                else
-                                    mx = fmaxf(mx, __uint_as_float(x[i]));
-                            }
-                        }
-                        else
-                        {
+                        for (int i = 0; i < 32; ++i)
+                            mxi = max(mxi, static_cast<int32_t>(x[i]));
+                    }
+                    else
+                    {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                            {
-                                if (i < limit)
-                                {
-                                    if (kInt8)
-                                        mxi = max(mxi, static_cast<int32_t>(x[i]));
-                                    else
-                                        mx = fmaxf(mx, __uint_as_float(x[i]));
-                                }
-                            }
-                        }
+                        for (int i = 0; i < 32; ++i)
+                            if (i < limit)
+                                mxi = max(mxi, static_cast<int32_t>(x[i]));
                     }
                 }
-                if (kInt8)
-                    mx = mxi == INT32_MIN ? -INFINITY : static_cast<float>(mxi);
+                float mx = mxi == INT32_MIN ? -INFINITY : static_cast<float>(mxi);
                 if (pending)
                 {
-                    epilogue(tiles - 1, pendDst, pendInv);
+                    epilogue(tiles - 1, pendDst);
                     pending = false;
                 }
                 rowRed[sub * kQTile + r] = mx;
-                softmaxBarrier<!kInt8>(quad);
+                softmaxBarrier();
                 mx = fmaxf(fmaxf(rowRed[r], rowRed[kQTile + r]), fmaxf(rowRed[2 * kQTile + r], rowRed[3 * kQTile + r]));
-                float const mOff = mx * sl2;
                 float const mxMagic = kMagic + mx; // exact: both are integers below 2^24
 
-                // ---- pass B: exponentials, row sum; FP16 writes P here, INT8 parks exp values in TMEM ----
+                // ---- pass B: exponentials, back to where the scores were, and the row sum ----
                 float sum = 0.f;
 #pragma unroll 1
                 for (int j = 0; j < nb; ++j)
                 {
-                    if (j < nb)
+                    tmemLoad32(tRow + colOf(j), x);
+                    tmemLoadWait32(x);
+                    int const limit = len - colOf(j);
+                    // (acc - max) is formed exactly (integers through the 2^23 trick, no conversion unit), so the exponent carries a
+                    // single rounding
+                    auto expOf = [&](uint32_t v) { return ex2Approx((__uint_as_float(v + kMagicBits) - mxMagic) * sl2); };
+                    if (limit >= 32) // all 32 keys valid: no per-element select
                     {
-                        tmemLoad32(tRow + colOf(j), x);
-                        tmemLoadWait32(x);
-                        if (!kInt8)
-                        {
-                            // the scores are in registers: their TMEM columns may take the next tile's scores
-                            tcFenceBefore();
-                            mbarArrive(&sFree[j]);
-                        }
-                        int const limit = len - colOf(j);
-                        // INT8: (acc - max) is formed exactly (integers through the 2^23 trick, no conversion unit),
-                        // so the exponent carries a single rounding; FP16: one fused multiply-add.
-                        auto expOf = [&](uint32_t v) {
-                            return kInt8 ? ex2Approx((__uint_as_float(v + kMagicBits) - mxMagic) * sl2)
-                                         : ex2Approx(fmaf(__uint_as_float(v), sl2, -mOff));
-                        };
-                        if (limit >= 32) // all 32 keys valid: no per-element select
-                        {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                            {
-                                float const e = expOf(x[i]);
-                                sum += e;
-                                x[i] = __float_as_uint(e);
-                            }
-                        }
-                        else
+                        for (int i = 0; i < 32; ++i)
                         {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                            {
-                                float const e = i < limit ? expOf(x[i]) : 0.f;
-                                sum += e;
-                                x[i] = __float_as_uint(e);
-                            }
-                        }
-                        if (kInt8)
-                        {
-                            tmemStore32(tRow + colOf(j), x);
-                        }
-                        else
-                        {
-                            ok = acquireP(j) && ok;
-                            // FP16 P block = two [128 rows][64 keys] tiles of 128-byte rows; this thread owns 4 chunks of a row
-                            uint8_t* pRow = sP + slotOf(j) * L::kPBytes + (sub >> 1) * (kQTile * 128) + r * 128;
-#pragma unroll
-                            for (int g = 0; g < 4; ++g)
-                            {
-                                float f[8];
-#pragma unroll
-                                for (int i = 0; i < 8; ++i)
-                                    f[i] = __uint_as_float(x[g * 8 + i]);
-                                int const chunk = (sub & 1) * 4 + g;
-                                *reinterpret_cast<uint4*>(pRow + ((chunk ^ (r & 7)) << 4)) = packHalf8(f);
-                            }
-                            fenceProxyAsync();
-                            tcFenceBefore();
-                            mbarArrive(&pReady[j]);
+                            float const e = expOf(x[i]);
+                            sum += e;
+                            x[i] = __float_as_uint(e);
                         }
                     }
+                    else
+                    {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                        {
+                            float const e = i < limit ? expOf(x[i]) : 0.f;
+                            sum += e;
+                            x[i] = __float_as_uint(e);
+                        }
+                    }
+                    tmemStore32(tRow + colOf(j), x);
                 }
-                if (kInt8)
-                    tmemStoreWait();
+                tmemStoreWait();
                 rowRed[4 * kQTile + sub * kQTile + r] = sum;
-                softmaxBarrier<!kInt8>(quad);
+                softmaxBarrier();
                 sum = (rowRed[4 * kQTile + r] + rowRed[5 * kQTile + r]) + (rowRed[6 * kQTile + r] + rowRed[7 * kQTile + r]);
                 float const inv = 1.f / sum;
 
-                if (kInt8)
-                {
-                    // ---- pass C (INT8): P_q = rni(p / sum * scale_softmax) ----
-                    float const pq = inv * args.scaleSoftmax;
+                // ---- pass C: P_q = rni(p / sum * scale_softmax) ----
+                float const pq = inv * args.scaleSoftmax;
 #pragma unroll 1
-                    for (int j = 0; j < nb; ++j)
+                for (int j = 0; j < nb; ++j)
+                {
+                    tmemLoad32(tRow + colOf(j), x);
+                    tmemLoadWait32(x);
+                    tcFenceBefore();
+                    mbarArrive(&sFree[j]); // the parked exponentials are in registers: columns free for new scores
+                    ok = acquireP(j) && ok;
+                    uint8_t* pRow = sP + slotOf(j) * L::kPBytes + r * 128; // P block: [128 rows][128 keys]
+#pragma unroll
+                    for (int g = 0; g < 2; ++g)
                     {
-                        if (j < nb)
+                        uint4 o;
+                        uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+                        // p / sum <= 1 (the sum contains p; a rounded-up reciprocal adds a few ulp at most), so
+                        // with scale_softmax <= 127 nothing can round beyond 127 and the clamp is left out
+                        if (args.scaleSoftmax <= 127.f)
                         {
-                            tmemLoad32(tRow + colOf(j), x);
-                            tmemLoadWait32(x);
-                            tcFenceBefore();
-                            mbarArrive(&sFree[j]); // the parked exponentials are in registers: columns free for new scores
-                            ok = acquireP(j) && ok;
-                            uint8_t* pRow = sP + slotOf(j) * L::kPBytes + r * 128; // INT8 P block: [128 rows][128 keys]
 #pragma unroll
-                            for (int g = 0; g < 2; ++g)
-                            {
-                                uint4 o;
-                                uint32_t* w = reinterpret_cast<uint32_t*>(&o);
-                                // p / sum <= 1 (the sum contains p; a rounded-up reciprocal adds a few ulp at most), so
-                                // with scale_softmax <= 127 nothing can round beyond 127 and the clamp is left out
-                                if (args.scaleSoftmax <= 127.f)
-                                {
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i)
-                                        w[i] = packProb4<false>(__uint_as_float(x[g * 16 + 4 * i]) * pq,
-                                            __uint_as_float(x[g * 16 + 4 * i + 1]) * pq, __uint_as_float(x[g * 16 + 4 * i + 2]) * pq,
-                                            __uint_as_float(x[g * 16 + 4 * i + 3]) * pq);
-                                }
-                                else
-                                {
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i)
-                                        w[i] = packProb4<true>(__uint_as_float(x[g * 16 + 4 * i]) * pq,
-                                            __uint_as_float(x[g * 16 + 4 * i + 1]) * pq, __uint_as_float(x[g * 16 + 4 * i + 2]) * pq,
-                                            __uint_as_float(x[g * 16 + 4 * i + 3]) * pq);
-                                }
-                                int const chunk = sub * 2 + g; // 16 keys per 16-byte chunk
-                                *reinterpret_cast<uint4*>(pRow + ((chunk ^ (r & 7)) << 4)) = o;
-                            }
-                            fenceProxyAsync();
-                            tcFenceBefore();
-                            mbarArrive(&pReady[j]);
+                            for (int i = 0; i < 4; ++i)
+                                w[i] = packProb4<false>(__uint_as_float(x[g * 16 + 4 * i]) * pq,
+                                    __uint_as_float(x[g * 16 + 4 * i + 1]) * pq, __uint_as_float(x[g * 16 + 4 * i + 2]) * pq,
+                                    __uint_as_float(x[g * 16 + 4 * i + 3]) * pq);
                         }
+                        else
+                        {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                w[i] = packProb4<true>(__uint_as_float(x[g * 16 + 4 * i]) * pq,
+                                    __uint_as_float(x[g * 16 + 4 * i + 1]) * pq, __uint_as_float(x[g * 16 + 4 * i + 2]) * pq,
+                                    __uint_as_float(x[g * 16 + 4 * i + 3]) * pq);
+                        }
+                        int const chunk = sub * 2 + g; // 16 keys per 16-byte chunk
+                        *reinterpret_cast<uint4*>(pRow + ((chunk ^ (r & 7)) << 4)) = o;
                     }
+                    fenceProxyAsync();
+                    tcFenceBefore();
+                    mbarArrive(&pReady[j]);
                 }
                 sBits ^= (1u << nb) - 1u; // every block of this tile used its sFull / pReady phase
                 int const q = t * kQTile + r;
                 // this thread's 16 of the 64 context columns; columns >= d are the zero padding
-                T* const dst = q >= it.rows || sub * 16 >= args.d
+                int8_t* const dst = q >= it.rows || sub * 16 >= args.d
                     ? nullptr
                     : (IL ? outPtrIl(q, sub >> 1) + (sub & 1) * 16 : outRow(q) + sub * 16);
                 ++tiles;
@@ -934,14 +845,13 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 {
                     pending = true;
                     pendDst = dst;
-                    pendInv = inv;
                 }
                 else
-                    epilogue(tiles - 1, dst, inv);
+                    epilogue(tiles - 1, dst);
             }
         }
         if (pending)
-            epilogue(tiles - 1, pendDst, pendInv);
+            epilogue(tiles - 1, pendDst);
         tcFenceBefore();
     }
 
@@ -966,16 +876,16 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
 
 // Sequences of at most one key block: one CTA per (sequence, head), four warps that do everything in turn, a thread per query row.
 //
-// Bound by the exponentials' unit (1024 cycles per pair) where there are many pairs, by a pair's chain of latencies (lengths, loads,
-// scores, softmax, product, store) where there are few. The persistent kernel works on one tile at a time: its sixteen warps
-// pass through the same phase together, so the exponentials' unit waits for the maximum and the quantisation and the other way
-// round, and two barriers per tile keep them in step. Here four CTAs share an SM (128 columns of tensor memory each, the context
-// in the first ones once the exponentials there have been read), each in a phase of its own, no row is shared between threads, and the
-// code is small: loops over pieces of 32 columns. The arithmetic is that of the persistent kernel, to the bit, the row sum's order included.
-// Measured (persistent kernel in brackets): 1 x 37 tokens, 12 heads 4.2 us (5.2 us), 32 x 64 ... 128, 12 heads 9.0 us (11.0 us), 64 x 128, 16
-// heads 13.8 us (21.8 us), 128 x 16, 16 heads 16.7 us (40.8 us). Two threads per row: 4.4, 9.0, 14.7 and 20.1 us. The same for two key
-// blocks (256 columns, two CTAs per SM) is no clear gain: 9 x 256, 16 heads 8.3 us (10.0 us), 64 x 256 49.5 us (53.4 us), but 2 x 256 7.1
-// us (6.3 us), 37 interleaved sequences of 100 ... 256 28.4 us (26.5 us).
+// Bound by a pair's chain of latencies (lengths, loads, scores, softmax, product, store), with many pairs too: 64 x 128 tokens, 16 heads take 13.3
+// us, the exponentials' unit (1024 cycles per pair, 3.7 us) is busy for 27 % of it and the issue slots for 40 %, with 16 warps on an SM. The persistent
+// kernel works on one tile at a time: its sixteen warps pass through the same phase together, so one unit after the other waits, and two
+// barriers per tile keep them in step. Here four CTAs share an SM (128 columns of tensor memory each, the context in the first ones once
+// the exponentials there have been read), each in a phase of its own, no row is shared between threads, and the code is small: loops over
+// pieces of 32 columns. The arithmetic is that of the persistent kernel, to the bit, the row sum's order included.
+// Measured, GPU time (persistent kernel in brackets): 1 x 37 tokens, 12 heads 4.1 us (4.9 us), 32 x 64 ... 128, 12 heads 8.3 us (10.9 us), 64 x 128,
+// 16 heads 13.3 us (21.2 us), 128 x 16, 16 heads 15.9 us (39.5 us), 1024 x 128, 16 heads 172 us (307 us). Two threads per row are 0 ... 20 % slower. The
+// same for two key blocks (256 columns, two CTAs per SM) is no clear gain: 9 x 256, 16 heads 8.3 us (10.0 us), 64 x 256 49.5 us (53.4 us),
+// but 2 x 256 7.1 us (6.3 us), 37 interleaved sequences of 100 ... 256 28.4 us (26.5 us).
 constexpr int kShortThreads = 128;
 constexpr int kShortTile = kQTile * kHeadSize;  // bytes of the Q, K or V tile
 constexpr int kShortP = 3 * kShortTile;         // after Q, K and V
@@ -1274,7 +1184,7 @@ __global__ void __launch_bounds__(kShortThreads, 4) mhaShortInt8Kernel(const __g
 }
 
 // Sets the work items and launches: one persistent CTA per SM (512 TMEM columns and most of the shared memory each).
-template <typename T, bool IL, bool BNSD>
+template <bool IL, bool BNSD>
 int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t stream)
 {
     static_assert(kItemTile == kQTile, "tiles of the plan");
@@ -1295,9 +1205,9 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     int64_t const items = static_cast<int64_t>(args.B) * args.N * plan.chunks;
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
-    int const smem = MhaSmem<T>::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (plan.longestFirst ? static_cast<int>(sizeof(ItemTable)) : 0);
+    int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (plan.longestFirst ? static_cast<int>(sizeof(ItemTable)) : 0);
     static SmemOptIn optIn[2];
-    auto const kernel = plan.longestFirst ? mhaTcgen05Kernel<T, IL, BNSD, true> : mhaTcgen05Kernel<T, IL, BNSD, false>;
+    auto const kernel = plan.longestFirst ? mhaTcgen05Kernel<IL, BNSD, true> : mhaTcgen05Kernel<IL, BNSD, false>;
     cudaError_t const e = launchDependentCluster(
         &optIn[plan.longestFirst], kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
     if (e != cudaSuccess)
@@ -1305,7 +1215,7 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     return checkLaunch("mhaTcgen05Kernel");
 }
 
-template <typename T, bool IL>
+template <bool IL>
 int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
 {
     bool const fixedLayout = p.cu_seqlens == nullptr;
@@ -1332,11 +1242,10 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
         // dim3: sequence position / packed row
         uint64_t const dims[4] = {d, 3ull * static_cast<uint64_t>(p.num_heads), fixedLayout ? static_cast<uint64_t>(p.B) : 1ull,
             fixedLayout ? static_cast<uint64_t>(p.S) : static_cast<uint64_t>(p.total)};
-        uint64_t const strides[3] = {d * sizeof(T), rowElems * sizeof(T),
-            (fixedLayout ? static_cast<uint64_t>(p.B) : 1ull) * rowElems * sizeof(T)};
+        uint64_t const strides[3] = {d, rowElems, (fixedLayout ? static_cast<uint64_t>(p.B) : 1ull) * rowElems};
         uint32_t const box[4] = {kHeadSize, 1, 1, kKeyBlock};
-        int32_t const st = makeTensorMap(&map, sizeof(T) == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-            4, p.qkv, dims, strides, box, sizeof(T) == 1 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+        int32_t const st = makeTensorMap(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, p.qkv, dims, strides, box,
+            CU_TENSOR_MAP_SWIZZLE_64B);
         if (st != BERT_B200_OK)
             return st;
     }
@@ -1344,12 +1253,11 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
     maps[2] = map;
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
         p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1};
-    return launchItems<T, IL, false>(args, maps, stream);
+    return launchItems<IL, false>(args, maps, stream);
 }
 
 // Separate Q, K, V tensors of shape [B][N][S][d] (the operand layout of TensorRT's attention layer), output
 // [B][N][S][d]: three tensor maps, the same kernel.
-template <typename T>
 int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t stream)
 {
     uint64_t const d = static_cast<uint64_t>(p.head_size), S = static_cast<uint64_t>(p.S), N = static_cast<uint64_t>(p.num_heads);
@@ -1359,16 +1267,16 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
     {
         // dim0: channel (box 64 wide, zero-filled beyond d); dim1: position; dim2: head; dim3: sequence
         uint64_t const dims[4] = {d, S, N, static_cast<uint64_t>(p.B)};
-        uint64_t const strides[3] = {d * sizeof(T), S * d * sizeof(T), N * S * d * sizeof(T)};
+        uint64_t const strides[3] = {d, S * d, N * S * d};
         uint32_t const box[4] = {kHeadSize, kKeyBlock, 1, 1};
-        int32_t const st = makeTensorMap(&maps[i], sizeof(T) == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-            base[i], dims, strides, box, sizeof(T) == 1 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+        int32_t const st = makeTensorMap(&maps[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base[i], dims, strides, box,
+            CU_TENSOR_MAP_SWIZZLE_64B);
         if (st != BERT_B200_OK)
             return st;
     }
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
         p.scale_bmm2, p.status_word, 1, 1, 1};
-    return launchItems<T, false, true>(args, maps, stream);
+    return launchItems<false, true>(args, maps, stream);
 }
 
 } // namespace
@@ -1400,7 +1308,7 @@ extern "C" int32_t bert_b200_attention_bnsd(bert_b200_attention_bnsd_params cons
         B200_REQUIRE(p.scale_bmm1 > 0.f, "attention_bnsd: scale_bmm1 must be positive");
         return mhaOnlineF16Bnsd(p, s);
     }
-    return launchMhaBnsd<int8_t>(p, s);
+    return launchMhaBnsd(p, s);
 }
 
 extern "C" int32_t bert_b200_mha(bert_b200_mha_params const* params, void* stream)
@@ -1438,8 +1346,8 @@ extern "C" int32_t bert_b200_mha(bert_b200_mha_params const* params, void* strea
         B200_FAIL(BERT_B200_NOT_SUPPORTED, "mha: INT8 takes S <= %d, got %d", kMaxBlocks * kKeyBlock, p.S);
     B200_REQUIRE(aligned16(p.qkv) && aligned16(p.out), "mha: qkv and out must be 16-byte aligned");
     if (p.interleaved)
-        return launchMha<int8_t, true>(p, s);
-    return launchMha<int8_t, false>(p, s);
+        return launchMha<true>(p, s);
+    return launchMha<false>(p, s);
 }
 
 extern "C" int64_t bert_b200_mha_workspace_size(bert_b200_mha_params const* params)
