@@ -196,10 +196,12 @@ enum
  *  type_id 0: A, Wt FP32, full FP32 precision;                     out_type_id 0.
  *    k >= 384, k % 4 == 0, lda % 4 == 0, A and Wt 16-byte aligned: tensor cores (three BF16 parts per number, six products,
  *    sums of 64 products in the tensor core, the rest in FP32); otherwise FP32 multiply-adds. The two round differently, so
- *    the same numbers may differ in the last bits where one call is aligned and another is not. Both are within 2e-7
- *    of the exact result (2-norm) for normal inputs up to k = 1024; the tensor cores are the closer ones. Infinities, NaN, the
- *    smallest and the largest numbers come out as multiply-adds give them, at up to ten times the time when a whole
- *    input consists of infinities or of numbers below 2^-110.
+ *    the same numbers may differ in the last bits where one call is aligned and another is not. Error (2-norm) for normal inputs,
+ *    k = 384 ... 4096: tensor cores 0.8e-7 ... 1.1e-7, multiply-adds 1.3e-7 ... 2.9e-7; for uniform ones of one sign 0.4e-7 ... 0.5e-7 and
+ *    0.6e-7 ... 0.7e-7. The multiply-adds are closer only where both operands have one sign and spread over orders of magnitude
+ *    (softmax of 3 N(0, 1) times uniform: 2e-7 and 0.8e-7 ... 1.1e-7; exp(2 N(0, 1)) on both sides: 3e-7 ... 4e-7 and 1e-7 ... 1.8e-7).
+ *    Infinities, NaN, the smallest and the largest numbers come out as multiply-adds give them, at up to ten times the time
+ *    when a whole input consists of infinities or of numbers below 2^-110.
  * epilogue(acc) = quant( act( acc * alpha + bias[n] ) ), bias FP32 or NULL, act per `activation`,
  * quant = sat8(rni(x * out_scale)) when out_type_id == 2, identity otherwise.
  * Wt is the weight matrix stored [n][k] (K contiguous); the reference plugin holds W as [k][n]

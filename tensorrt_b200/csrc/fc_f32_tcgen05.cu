@@ -732,10 +732,13 @@ int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaSt
 //   uniform, 0 ... 1         0.40 / 0.56  0.44 / 0.55  0.45 / 0.56  0.50 / 0.71  0.50 / 0.73
 //   normal, 1 +- 0.2         0.43 / 0.55  0.48 / 0.55  0.49 / 0.55  0.54 / 0.71  0.54 / 0.72
 // (mean error on the third and fourth -0.06 and +0.22; parts by truncation and 64 products in one accumulator: 1.2 and 1.0, the mean -1.1 and
-// -0.9). A shorter K has not been measured in this form and stays with the multiply-adds. They also take what the TMA unit does not: rows that are no
-// multiple of 16 bytes apart, sizes beyond its coordinates. GPU time, same order: 1 x 64 x 384 6.3 / 8.5 us, 1 x 768 x 768 8.0 / 8.6 us, 37 x 768 x 768
-// 8.4 / 8.9 us, 37 x 2304 x 768 11.2 / 14.9 us, 300 x 768 x 512 9.9 / 18.5 us, 128 x 768 x 3072 14.0 / 44.9 us, 1024 x 2304 x 768 33.2 / 96.9 us,
-// 4096 x 1024 x 4096 232 / 843 us. The two tensor maps cost a call 1 us of the host: 10.1 instead of 9.5 us where the host is what bounds it.
+// -0.9). The multiply-adds are closer where both operands have one sign and spread over orders of magnitude, since small products are cut off beside a
+// large sum: softmax of 3 N(0, 1) x uniform 1.8e-7 ... 2.1e-7 / 0.8e-7 ... 1.1e-7 (before 3.0e-7 ... 3.3e-7), exp(2 N(0, 1)) on both sides 3.1e-7 ... 3.8e-7 /
+// 1.0e-7 ... 1.8e-7 (before 4.1e-7 ... 5.4e-7); with normal weights they are not. A shorter K has not been measured in this form and stays with
+// the multiply-adds. They also take what the TMA unit does not: rows that are no multiple of 16 bytes apart, sizes beyond its coordinates. GPU time,
+// same order: 1 x 64 x 384 6.3 / 8.5 us, 1 x 768 x 768 8.0 / 8.6 us, 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 11.2 / 14.9 us, 300 x 768 x 512 9.9 /
+// 18.5 us, 128 x 768 x 3072 14.0 / 44.9 us, 1024 x 2304 x 768 33.2 / 96.9 us, 4096 x 1024 x 4096 232 / 843 us. The two tensor maps cost a call 1 us
+// of the host: 10.1 instead of 9.5 us where the host is what bounds it.
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
     constexpr int64_t kMax = 1ll << 31;

@@ -179,7 +179,7 @@ def mha(qkv, B, S, num_heads, head_size=64, cu_seqlens=None, mask_idx=None, scal
         scale_bmm2=1.0, status=None, interleaved=False, workspace=None, use_workspace=True, out=None):
     """Fused attention. qkv: fixed [S, B, 3*N*d] (cu_seqlens None), packed [total, 3*N*d], or with
     interleaved=True the INT8 CHW32 form [3*N*d/32, total, 32] (output [N*d/32, total, 32]). `out`: a tensor of the
-    output's shape and type to write into instead of a new one."""
+    output's shape and type to write into instead of a new one. No kernel needs a workspace: `use_workspace` changes nothing."""
     E = num_heads * head_size
     if interleaved:
         total = qkv.shape[1]
