@@ -173,8 +173,8 @@ __device__ __forceinline__ bool hasNan(float const* row, int64_t k)
 // of K, even and odd ones apart, and their sums are added as a tree, so an output has the same bits wherever its tile lies. The chains are a
 // quarter or less as long as those of fcF32Simt (error on normal values K = 768 0.9e-7 / 1.4e-7, 4096 1.6e-7 / 2.9e-7). Bound by the loads' latency for a
 // few outputs, by what the L2 brings for all (4 x 4 outputs are read by 8 rows). 1024 x 2304 x 768, nothing to compute again / an infinity in A / a number
-// below 2^-110 in Wt / A full of them: 29.6 / 39.6 / 39.5 / 285 us; a thread per output and all of K in one chain 29.6 / 140 / 169 / 10 100 us;
-// fcF32Simt 97 us.
+// below 2^-110 in Wt / A full of them: 33.2 / 45.9 / 46.2 / 335 us (a NaN 34.9 us); a thread per output and all of K in one chain, in the kernel
+// of that time, 29.6 / 140 / 169 / 10 100 us; fcF32Simt 97 us.
 template <int BN>
 __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* again, uint32_t* list, int64_t m0, int64_t n0)
 {
@@ -635,8 +635,11 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             flagA[threadIdx.x] = merged;
         __syncthreads();
         for (int r = warp; r < kTileM + BN; r += kThreadsF32 / 32)
-            if (flagA[r] != 0 && hasNan(r < kTileM ? p.A + (m0 + r) * p.lda : p.Wt + (n0 + r - kTileM) * p.K, p.K))
+        {
+            bool const inside = r < kTileM ? m0 + r < p.M : n0 + r - kTileM < p.N; // after an expired wait any row may be flagged
+            if (inside && flagA[r] != 0 && hasNan(r < kTileM ? p.A + (m0 + r) * p.lda : p.Wt + (n0 + r - kTileM) * p.K, p.K))
                 flagA[r] = 2;
+        }
         __syncthreads();
     }
     constexpr int kPieces = BN / 4;
