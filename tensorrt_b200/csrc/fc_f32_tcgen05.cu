@@ -54,14 +54,15 @@ struct FcF32Smem
     static constexpr int kPlaneBytes = BN * kChunk * 2; // one BF16 part of the Wt tile
     static constexpr int kPlanesOff = kStages * kStageBytes;
     static constexpr int kBarrierOff = kPlanesOff + kParts * 3 * kPlaneBytes;
-    // stFull[stages] stFree[stages] ready[parts] done[parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
+    static constexpr int kAccs = BN <= 64 ? 2 : 1;      // chunks whose sums are in tensor memory, two accumulators each
+    static constexpr int kHalves = kAccs == 1 ? 2 : 1; // of the columns, whose products are formed one after the other
+    // stFull[stages] stFree[2][stages] ready[parts] done[halves][parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
     // whether any is set
-    static constexpr int kFlagsOff = kBarrierOff + (2 * kStages + 2 * kParts + 2) * 8 + 16;
+    static constexpr int kFlagsOff = kBarrierOff + (3 * kStages + (1 + kHalves) * kParts + 2) * 8 + 16;
     static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
     static constexpr int kDynamic = kTotal + 1024;
     static constexpr int kPitch = BN + 4; // floats: sums of a tile over the drained FP32 tiles
     static constexpr int kTmem = 512;
-    static constexpr int kAccs = BN <= 64 ? 2 : 1; // chunks whose sums are in tensor memory, two accumulators each
     static constexpr int kAccCols = kAccs * 2 * BN;
     // Columns that a worker's sums of the segments before take in tensor memory: all of them but for the 128-wide tile (half).
     static constexpr int kHeldCols = BN / 4 < (kTmem - kAccCols - kParts * 96) / 4 ? BN / 4 : (kTmem - kAccCols - kParts * 96) / 4;
@@ -140,9 +141,9 @@ __device__ __forceinline__ void addSums(uint32_t tP, uint32_t tQ, uint64_t* sums
                                     pack2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1]))));
 }
 
-__device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, int64_t n)
+__device__ __forceinline__ float finishF32(FcF32TcArgs const& p, float v, float bias)
 {
-    v = v * p.alpha + (p.bias ? __ldg(p.bias + n) : 0.f);
+    v = v * p.alpha + bias;
     return p.act == BERT_B200_ACT_GELU_ERF ? geluErfF32(v) : v;
 }
 
@@ -173,7 +174,7 @@ __device__ __forceinline__ bool hasNan(float const* row, int64_t k)
 // of K, even and odd ones apart, and their sums are added as a tree, so an output has the same bits wherever its tile lies. The chains are a
 // quarter or less as long as those of fcF32Simt (error on normal values K = 768 0.9e-7 / 1.4e-7, 4096 1.6e-7 / 2.9e-7). Bound by the loads' latency for a
 // few outputs, by what the L2 brings for all (4 x 4 outputs are read by 8 rows). 1024 x 2304 x 768, nothing to compute again / an infinity in A / a number
-// below 2^-110 in Wt / A full of them: 33.2 / 45.9 / 46.2 / 335 us (a NaN 34.9 us); a thread per output and all of K in one chain, in the kernel
+// below 2^-110 in Wt / A full of them, in the form of that time: 33.2 / 45.9 / 46.2 / 335 us (a NaN 34.9 us); a thread per output and all of K in one chain, in the kernel
 // of that time, 29.6 / 140 / 169 / 10 100 us; fcF32Simt 97 us.
 template <int BN>
 __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* again, uint32_t* list, int64_t m0, int64_t n0)
@@ -249,23 +250,26 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
         if ((lane & 1) == 0 && (mask >> j & 1u) != 0)
         {
             int64_t const n = n0 + c + (j & 3);
-            p.C[(m0 + r + (j >> 2)) * p.ldc + n] = finishF32(p, v[0], n);
+            p.C[(m0 + r + (j >> 2)) * p.ldc + n] = finishF32(p, v[0], p.bias ? __ldg(p.bias + n) : 0.f);
         }
     }
 }
 
-// Bound by the chain of a chunk - its place free, operands cut, products, sums read -, 3220 cycles for a 128 x 128 tile, of which the
-// tensor cores are busy 1610; no unit is full. With h and m by truncation, all products in one accumulator and two of those for every width it
-// took 2880 cycles (24 instead of 26 MMAs, the next chunk's begun before the sums were read), but its sums were too small by 1.1e-7 on numbers of one sign.
+// Bound by the warps that cut operands, and by shared memory behind them: a chunk of a 128 x 128 tile takes 2900 cycles, of which the
+// tensor cores are busy 1750 and shared memory 2240 (tiles written and read, parts of Wt written and read by 26 products), of a 64-wide one 1870
+// (830, 1380). The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are
+// multiplied in two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk (with two groups
+// taking chunks in turn the sums waited for the group that was cutting); a chunk's three barriers are asked at once (an answer takes 120 ... 150
+// cycles); and a tile's place in the ring is handed back as soon as its numbers are in registers. Before / after: 3400 / 2900 cycles
+// per chunk; 1024 x 2304 x 768 32.7 / 28.3 us, 2000 x 3072 x 1024 113.1 / 98.7 us, 4096 x 3072 x 1024 210.9 / 195.4 us, 37 x 2304 x 768 11.1 / 10.6 us.
 // Rounding costs nothing: truncation of h, other subtractions or loads further ahead leave the times as they are.
 // One 128 x BN tile per CTA, or one segment of its K:
 //   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
 //   warp 1    : TMEM allocation, MMA issue. The parts of A are operands in TMEM - from shared memory both operands of a
 //               128 x 128 tile would take its whole bandwidth -, those of Wt in shared memory.
-//   warps 2-17: the parts of a chunk, the two groups of eight warps taking chunks in turn: 32 numbers of a row of A per thread, to
-//               TMEM, and whole 16-byte pieces of the parts of Wt, to shared memory. And all of them, for every chunk, its
-//               sums (32 rows, a quarter of the columns per warp) from TMEM into registers. Parts are double-buffered, the two
-//               accumulators too where tensor memory has room (up to 64 columns).
+//   warps 2-17: the parts of every chunk: 16 numbers of a row of A per thread, to TMEM, and whole 16-byte pieces of the parts of
+//               Wt, to shared memory. And its sums (32 rows, a quarter of the columns per warp) from TMEM into registers. Parts are
+//               double-buffered, the two accumulators too where tensor memory has room (up to 64 columns).
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
 // An output whose row of A or Wt holds numbers without exact parts (splitPair) is computed again by FP32 multiply-adds (computeAgain), unless one
@@ -275,7 +279,8 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     fcF32TcKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ FcF32TcArgs p)
 {
     using L = FcF32Smem<BN>;
-    constexpr uint32_t kIdesc = makeInstrDesc(1u, 1u, 0u, 0u, 128u, static_cast<uint32_t>(BN));
+    constexpr int kWidth = BN / L::kHalves; // columns of a product
+    constexpr uint32_t kIdesc = makeInstrDesc(1u, 1u, 0u, 0u, 128u, static_cast<uint32_t>(kWidth));
     constexpr int kCols = BN / 4; // accumulator columns per worker thread
     constexpr uint32_t kIdescMinus = kIdesc | 1u << 13; // minus A
     constexpr uint32_t kPartsCol = L::kAccCols;
@@ -284,9 +289,9 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* const stFull = reinterpret_cast<uint64_t*>(smem + L::kBarrierOff);
     uint64_t* const stFree = stFull + L::kStages;
-    uint64_t* const ready = stFree + L::kStages; // parts of a chunk in place
-    uint64_t* const done = ready + kParts;       // their products complete
-    uint64_t* const accFree = done + kParts;     // an accumulator has been read
+    uint64_t* const ready = stFree + 2 * L::kStages; // parts of a chunk in place
+    uint64_t* const done = ready + kParts;       // [halves][parts] their products complete
+    uint64_t* const accFree = done + L::kHalves * kParts; // an accumulator (or its half) has been read
     uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(accFree + 2);
     volatile uint32_t* const abortFlag = tmemSlot + 1;
     uint32_t* const flagA = reinterpret_cast<uint32_t*>(smem + L::kFlagsOff);
@@ -312,15 +317,15 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int i = 0; i < L::kStages; ++i)
         {
             mbarInit(&stFull[i], 1);
-            mbarInit(&stFree[i], kWorkers / 2);
+            mbarInit(&stFree[i], kWorkers);               // A
+            mbarInit(&stFree[L::kStages + i], kWorkers); // Wt
         }
         for (int i = 0; i < kParts; ++i)
-        {
-            mbarInit(&ready[i], kWorkers / 2);
+            mbarInit(&ready[i], kWorkers);
+        for (int i = 0; i < L::kHalves * kParts; ++i)
             mbarInit(&done[i], 1);
-        }
         for (int i = 0; i < 2; ++i)
-            mbarInit(&accFree[i], kWorkers);
+            mbarInit(&accFree[i], kWorkers / L::kHalves);
         *abortFlag = 0;
         fenceBarrierInit();
         prefetchTensorMap(&mapA);
@@ -345,19 +350,24 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         uint32_t phase = 1;
         for (int c = 0; c < count && ok; ++c)
         {
+            uint32_t const bar = smemAddr(&stFull[stage]);
+            uint32_t const a = smemAddr(smem) + stage * L::kStageBytes;
+            int32_t const k = (first + c) * kChunk;
             ok = mbarWaitWarp(&stFree[stage], phase, abortFlag, kWaitStageFree);
             if (ok && electOne())
             {
-                uint32_t const bar = smemAddr(&stFull[stage]);
-                uint32_t const a = smemAddr(smem) + stage * L::kStageBytes;
-                int32_t const k = (first + c) * kChunk;
                 mbarArriveExpectTxAddr(bar, L::kStageBytes);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                {
                     tmaLoad2dAddr(a + h * (L::kABytes / 2), &mapA, bar, k + h * 32, static_cast<int32_t>(m0));
+            }
+            __syncwarp();
+            ok = ok && mbarWaitWarp(&stFree[L::kStages + stage], phase, abortFlag, kWaitStageFree);
+            if (ok && electOne())
+            {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
                     tmaLoad2dAddr(a + L::kABytes + h * (L::kWBytes / 2), &mapW, bar, k + h * 32, static_cast<int32_t>(n0));
-                }
             }
             __syncwarp();
             if (++stage == L::kStages)
@@ -377,40 +387,44 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         {
             uint32_t const s = c & 1, round = c >> 1;
             uint32_t const slot = c % L::kAccs;
-            ok = (c < L::kAccs || mbarWaitWarp(&accFree[slot], (c / L::kAccs - 1) & 1u, abortFlag, kWaitAccFree))
-                && mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
-            tcFenceAfter();
-            if (ok && electOne())
-            {
-                // parts (A, Wt), the smallest products first
-                constexpr int kOrder[5][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
-                uint32_t const a = tmemBase + kPartsCol + s * 96;
-                uint32_t const w = wLo + s * (3 * L::kPlaneBytes >> 4);
-                uint32_t const sumP = tmemBase + slot * 2 * BN, sumQ = sumP + BN;
+            ok = mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
 #pragma unroll
-                for (int i = 0; i < 5; ++i)
+            for (int h = 0; h < L::kHalves; ++h)
+            {
+                ok = ok && (c < L::kAccs || mbarWaitWarp(&accFree[slot + h], (c / L::kAccs - 1) & 1u, abortFlag, kWaitAccFree));
+                tcFenceAfter();
+                if (ok && electOne())
+                {
+                    // parts (A, Wt), the smallest products first
+                    constexpr int kOrder[5][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
+                    uint32_t const a = tmemBase + kPartsCol + s * 96;
+                    uint32_t const w = wLo + s * (3 * L::kPlaneBytes >> 4) + h * (kWidth * 128 >> 4);
+                    uint32_t const sumP = tmemBase + slot * 2 * BN + h * kWidth, sumQ = sumP + BN;
+#pragma unroll
+                    for (int i = 0; i < 5; ++i)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            mmaF16TmemA(sumQ, a + kOrder[i][0] * 32 + k * 8, w + kOrder[i][1] * (L::kPlaneBytes >> 4) + k * 2, descHi, kIdesc,
+                                i != 0 || k != 0);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        mmaF16TmemA(sumP, a + k * 8, w + k * 2, descHi, kIdesc, k != 0);
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        mmaF16TmemA(sumQ, a + kOrder[i][0] * 32 + k * 8, w + kOrder[i][1] * (L::kPlaneBytes >> 4) + k * 2, descHi, kIdesc,
-                            i != 0 || k != 0);
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    mmaF16TmemA(sumP, a + k * 8, w + k * 2, descHi, kIdesc, k != 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    mmaF16TmemA(sumQ, a + k * 8, w + k * 2, descHi, k < 2 ? kIdescMinus : kIdesc, true);
-                tcCommit(&done[s]);
+                        mmaF16TmemA(sumQ, a + k * 8, w + k * 2, descHi, k < 2 ? kIdescMinus : kIdesc, true);
+                    tcCommit(&done[h * kParts + s]);
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
     }
     else
     {
         int const quad = warp & 3;
-        int const group = (warp - 2) >> 3; // takes every second chunk
-        int const w = (warp - 2) & 7;
-        int const half = w >> 2;           // which 32 of a chunk's K of A
-        int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns
+        int const group = (warp - 2) >> 3; // takes every second 32 rows of Wt
+        int const w = (warp - 2) & 7;      // which 8 of a chunk's K of Wt
+        int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns, and which 16 of a chunk's K of A
+        int const part = L::kHalves == 2 ? group : 0;
         bool const hasRows = m0 + quad * 32 < p.M; // warp-uniform; products of the other rows are never read
         uint32_t const tRow = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
         // Sums of the segments before: touched once per segment and kept out of the registers, which are all taken in the loop
@@ -422,8 +436,10 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         int segmentEnd = segmentBegin(1);
         bool ok = true;
         // the sums of chunk c
-        auto promote = [&](int c) {
-            ok = ok && mbarWaitWarp(&done[c & 1], (c >> 1) & 1u, abortFlag, kWaitAccFull);
+        // (`ready`: they are known to be complete)
+        auto promote = [&](int c, bool ready) {
+            if (!__all_sync(0xffffffffu, ready))
+                ok = ok && mbarWaitWarp(&done[part * kParts + (c & 1)], (c >> 1) & 1u, abortFlag, kWaitAccFull);
             tcFenceAfter();
             if (hasRows)
             {
@@ -437,7 +453,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             tcFenceBefore();
             __syncwarp();
             if (lane == 0)
-                mbarArrive(&accFree[c % L::kAccs]);
+                mbarArrive(&accFree[c % L::kAccs + part]);
             if constexpr (kHold)
                 if (c + 1 == segmentEnd)
                 {
@@ -495,81 +511,81 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int c = 0; c < count; ++c)
         {
             uint32_t const s = c & 1;
+            // A barrier answers after 120 ... 150 cycles: all are asked at once.
+            bool const landed = mbarTryWaitAddr(smemAddr(&stFull[stage]), phase);
             if (c >= 2)
-                promote(c - 2); // its products are complete: so is what they read where this chunk's parts go
-            if (static_cast<int>(s) == group)
             {
+                uint32_t const parity = ((c - 2) >> 1) & 1u;
+                bool const summed = mbarTryWaitAddr(smemAddr(&done[part * kParts + s]), parity);
+                bool const complete = L::kHalves == 1 || part == 1 || mbarTryWaitAddr(smemAddr(&done[kParts + s]), parity);
+                promote(c - 2, summed);
+                // all its products are complete: so is what they read where this chunk's parts go
+                if (L::kHalves == 2 && part == 0 && !__all_sync(0xffffffffu, complete))
+                    ok = ok && mbarWaitWarp(&done[kParts + s], parity, abortFlag, kWaitAccFull);
+            }
+            if (!__all_sync(0xffffffffu, landed))
                 ok = ok && mbarWaitWarp(&stFull[stage], phase, abortFlag, kWaitTmaFull);
-                uint8_t const* const fp = smem + stage * L::kStageBytes;
-                if (hasRows)
-                {
-                    int const row = quad * 32 + lane;
-                    float4 const* const src = reinterpret_cast<float4 const*>(fp + half * (L::kABytes / 2) + row * 128);
-                    uint32_t const t = tRow + kPartsCol + s * 96 + half * 16;
-                    uint32_t lost = 0;
+            uint8_t const* const fp = smem + stage * L::kStageBytes;
+            if (hasRows)
+            {
+                int const row = quad * 32 + lane;
+                float4 const* const src = reinterpret_cast<float4 const*>(fp + (cols >> 1) * (L::kABytes / 2) + row * 128);
+                uint32_t const t = tRow + kPartsCol + s * 96 + cols * 8;
+                uint32_t lost = 0;
+                float4 v[4];
 #pragma unroll
-                    for (int g = 0; g < 2; ++g)
-                    {
-                        float4 v[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            v[i] = src[(4 * g + i) ^ (row & 7)];
-                        uint32_t h[8], m[8], l[8];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                        {
-                            splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], lost);
-                            splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], lost);
-                        }
-                        tmemStore8(t + g * 8, h);
-                        tmemStore8(t + g * 8 + 32, m);
-                        tmemStore8(t + g * 8 + 64, l);
-                    }
-                    if ((lost & 0xffffu) != 0)
-                        flagA[row] = *flagAny = 1;
-                }
-                // eight numbers of a row of Wt: 16 bytes of each part
-                uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
-                constexpr int kAhead = BN == 32 ? 1 : BN == 96 ? 3 : 2; // rows on their way before the first is cut
-#pragma unroll
-                for (int r0 = 0; r0 < BN / 32; r0 += kAhead)
-                {
-                    float4 v[kAhead][2];
-#pragma unroll
-                    for (int i = 0; i < kAhead; ++i)
-                    {
-                        int const row = (r0 + i) * 32 + lane;
-                        float4 const* const src = reinterpret_cast<float4 const*>(fp + L::kABytes + (w >> 2) * (L::kWBytes / 2) + row * 128);
-                        v[i][0] = src[(2 * (w & 3)) ^ (row & 7)];
-                        v[i][1] = src[(2 * (w & 3) + 1) ^ (row & 7)];
-                    }
-#pragma unroll
-                    for (int i = 0; i < kAhead; ++i)
-                    {
-                        int const row = (r0 + i) * 32 + lane;
-                        uint4 h, m, l;
-                        uint32_t lost = 0;
-                        splitPair(v[i][0].x, v[i][0].y, h.x, m.x, l.x, lost);
-                        splitPair(v[i][0].z, v[i][0].w, h.y, m.y, l.y, lost);
-                        splitPair(v[i][1].x, v[i][1].y, h.z, m.z, l.z, lost);
-                        splitPair(v[i][1].z, v[i][1].w, h.w, m.w, l.w, lost);
-                        uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
-                        *reinterpret_cast<uint4*>(dst) = h;
-                        *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
-                        *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
-                        if ((lost & 0xffffu) != 0)
-                            flagW[row] = *flagAny = 1;
-                    }
-                }
-                fenceProxyAsync();
-                tmemStoreWait();
-                tcFenceBefore();
+                for (int i = 0; i < 4; ++i)
+                    v[i] = src[((cols & 1) * 4 + i) ^ (row & 7)];
                 __syncwarp();
                 if (lane == 0)
-                {
-                    mbarArrive(&ready[s]);
                     mbarArrive(&stFree[stage]);
+                uint32_t h[8], m[8], l[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                    splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], lost);
+                    splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], lost);
                 }
+                tmemStore8(t, h);
+                tmemStore8(t + 32, m);
+                tmemStore8(t + 64, l);
+                if ((lost & 0xffffu) != 0)
+                    flagA[row] = *flagAny = 1;
+            }
+            else if (lane == 0)
+                mbarArrive(&stFree[stage]);
+            // eight numbers of a row of Wt: 16 bytes of each part; an odd number of 32 rows is dealt to the groups by turns
+            uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
+#pragma unroll
+            for (int i = 0; i < (BN + 32) / 64; ++i)
+            {
+                int const block = 2 * i + (BN % 64 == 0 ? group : (group + c) & 1);
+                if (BN % 64 != 0 && block >= BN / 32)
+                    break;
+                int const row = block * 32 + lane;
+                float4 const* const src = reinterpret_cast<float4 const*>(fp + L::kABytes + (w >> 2) * (L::kWBytes / 2) + row * 128);
+                float4 const v0 = src[(2 * (w & 3)) ^ (row & 7)], v1 = src[(2 * (w & 3) + 1) ^ (row & 7)];
+                uint4 h, m, l;
+                uint32_t lost = 0;
+                splitPair(v0.x, v0.y, h.x, m.x, l.x, lost);
+                splitPair(v0.z, v0.w, h.y, m.y, l.y, lost);
+                splitPair(v1.x, v1.y, h.z, m.z, l.z, lost);
+                splitPair(v1.z, v1.w, h.w, m.w, l.w, lost);
+                uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
+                *reinterpret_cast<uint4*>(dst) = h;
+                *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
+                *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
+                if ((lost & 0xffffu) != 0)
+                    flagW[row] = *flagAny = 1;
+            }
+            fenceProxyAsync();
+            tmemStoreWait();
+            tcFenceBefore();
+            __syncwarp();
+            if (lane == 0)
+            {
+                mbarArrive(&ready[s]);
+                mbarArrive(&stFree[L::kStages + stage]);
             }
             if (++stage == L::kStages)
             {
@@ -578,7 +594,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
             }
         }
         for (int c = count < 2 ? 0 : count - 2; c < count; ++c)
-            promote(c);
+            promote(c, false);
     }
 
     __syncthreads(); // the ring is drained
@@ -642,60 +658,73 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         }
         __syncthreads();
     }
-    constexpr int kPieces = BN / 4;
+    // A thread keeps its four columns and goes down the rows, so what depends on the columns is formed once.
+    constexpr int kPieces = BN / 4, kRows = kThreadsF32 / kPieces; // rows at a time of a CTA
     bool any = false;
-    for (int i = rank * kThreadsF32 + threadIdx.x; i < kTileM * kPieces && !aborted; i += p.ctas * kThreadsF32)
+    int const column = static_cast<int>(threadIdx.x % kPieces) * 4;
+    int64_t const n = n0 + column;
+    if (threadIdx.x < kRows * kPieces && n < p.N && !aborted)
     {
-        int const r = i / kPieces, c = i % kPieces * 4;
-        int64_t const m = m0 + r, n = n0 + c;
-        if (m >= p.M || n >= p.N)
-            continue;
-        float const* const at = sums + r * L::kPitch + c;
-        float4 v;
-        if (p.ctas > 1)
-        {
-            float4 x[kMaxSegments];
-#pragma unroll
-            for (int s = 0; s < kMaxSegments; ++s) // all on their way before the first is added
-                if (s < p.ctas)
-                    x[s] = ldSharedCluster4(at, s);
-            v = x[0];
-#pragma unroll
-            for (int s = 1; s < kMaxSegments; ++s)
-                if (s < p.ctas)
-                    v = make_float4(v.x + x[s].x, v.y + x[s].y, v.z + x[s].z, v.w + x[s].w);
-        }
-        else
-            v = *reinterpret_cast<float4 const*>(at);
-        float o[4] = {v.x, v.y, v.z, v.w};
         int const inside = p.N - n < 4 ? static_cast<int>(p.N - n) : 4;
-        uint32_t bits = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            bits |= sumIsInexact(o[j]) ? 1u << j : 0u;
-        if (!exact)
-            for (int j = 0; j < 4; ++j)
-            {
-                uint32_t const flags = flagA[r] | flagW[c + j];
-                bits = (bits | (flags & 1u) << j) & ~((flags >> 1) << j);
-            }
-        if (inside < 4)
-            bits &= (1u << inside) - 1u;
-        if (bits != 0)
+        int const rows = p.M - m0 < kTileM ? static_cast<int>(p.M - m0) : kTileM;
+        bool const whole = p.wide && inside == 4;
+        float bias[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p.bias)
         {
-            atomicOr(again + r * (BN / 32) + c / 32, bits << (c % 32));
-            any = true;
-        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j < inside)
-                o[j] = finishF32(p, o[j], n + j);
-        float* const dst = p.C + m * p.ldc + n;
-        if (p.wide && inside == 4)
-            *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
-        else
-            for (int j = 0; j < inside; ++j)
-                dst[j] = o[j];
+            for (int j = 0; j < 4; ++j)
+                if (j < inside)
+                    bias[j] = __ldg(p.bias + n + j);
+        }
+        int r = rank * kRows + static_cast<int>(threadIdx.x) / kPieces;
+        float* dst = p.C + (m0 + r) * p.ldc + n;
+        int64_t const step = static_cast<int64_t>(p.ctas) * kRows * p.ldc;
+        for (; r < rows; r += p.ctas * kRows, dst += step)
+        {
+            float const* const at = sums + r * L::kPitch + column;
+            float4 v;
+            if (p.ctas > 1)
+            {
+                float4 x[kMaxSegments];
+#pragma unroll
+                for (int s = 0; s < kMaxSegments; ++s) // all on their way before the first is added
+                    if (s < p.ctas)
+                        x[s] = ldSharedCluster4(at, s);
+                v = x[0];
+#pragma unroll
+                for (int s = 1; s < kMaxSegments; ++s)
+                    if (s < p.ctas)
+                        v = make_float4(v.x + x[s].x, v.y + x[s].y, v.z + x[s].z, v.w + x[s].w);
+            }
+            else
+                v = *reinterpret_cast<float4 const*>(at);
+            float o[4] = {v.x, v.y, v.z, v.w};
+            uint32_t bits = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                bits |= sumIsInexact(o[j]) ? 1u << j : 0u;
+            if (!exact)
+                for (int j = 0; j < 4; ++j)
+                {
+                    uint32_t const flags = flagA[r] | flagW[column + j];
+                    bits = (bits | (flags & 1u) << j) & ~((flags >> 1) << j);
+                }
+            if (inside < 4)
+                bits &= (1u << inside) - 1u;
+            if (bits != 0)
+            {
+                atomicOr(again + r * (BN / 32) + column / 32, bits << (column % 32));
+                any = true;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                o[j] = finishF32(p, o[j], bias[j]);
+            if (whole)
+                *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+            else
+                for (int j = 0; j < inside; ++j)
+                    dst[j] = o[j];
+        }
     }
     if (__syncthreads_or(any))
         computeAgain<BN>(p, again, list, m0, n0);
@@ -740,7 +769,7 @@ int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaSt
 // 1.0e-7 ... 1.8e-7 (before 4.1e-7 ... 5.4e-7); with normal weights they are not. A shorter K has not been measured in this form and stays with
 // the multiply-adds. They also take what the TMA unit does not: rows that are no multiple of 16 bytes apart, sizes beyond its coordinates. GPU time,
 // same order: 1 x 64 x 384 6.3 / 8.5 us, 1 x 768 x 768 8.0 / 8.6 us, 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 11.2 / 14.9 us, 300 x 768 x 512 9.9 /
-// 18.5 us, 128 x 768 x 3072 14.0 / 44.9 us, 1024 x 2304 x 768 33.2 / 96.9 us, 4096 x 1024 x 4096 232 / 843 us. The two tensor maps cost a call 1 us
+// 18.5 us, 128 x 768 x 3072 13.6 / 44.9 us, 1024 x 2304 x 768 28.3 / 96.9 us, 4096 x 1024 x 4096 217 / 843 us. The two tensor maps cost a call 1 us
 // of the host: 10.1 instead of 9.5 us where the host is what bounds it.
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
@@ -753,9 +782,10 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
     int64_t const kChunks = (p.k + kChunk - 1) / kChunk;
     int const segments = kChunks >= 24 ? 8 : kChunks >= 12 ? 4 : 2;
     // Width of the tiles, and whether a CTA takes all segments: what the measured cycles per chunk and per CTA, times the waves of CTAs,
-    // make shortest. Clusters find fewer places than there are SMs. Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768
-    // 33.6 / 49.9 / 39.0 / 56.5 us, 1024 x 3072 x 768 64.1 / 50.3 / 57.1 / 83.0 us, 1024 x 768 x 768 32.2 / 25.4 / 19.6 / 28.1 us; one segment per
-    // CTA, 128 / 64 columns: 1024 x 768 x 3072 75.4 / 97.7 us (64 columns in one CTA 56.0 us), 128 x 768 x 3072 19.4 / 14.6 us (54.0 us).
+    // make shortest (of an earlier form of the kernel, whose order is still the right one). Clusters find fewer places than there are SMs.
+    // Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768 29.1 / 46.0 / 36.7 / 58.2 us, 1024 x 3072 x 768 54.5 / 46.8 /
+    // 53.4 / 85.6 us, 1024 x 768 x 768 27.3 / 23.2 / 18.4 / 28.9 us; one segment per CTA, 128 / 64 columns: 1024 x 768 x 3072 72.0 / 93.2 us (64
+    // columns in one CTA 55.5 us), 128 x 768 x 3072 17.8 / 13.8 us (52.9 us).
     static constexpr int kCycles[4] = {1480, 1990, 2700, 3220}; // per chunk, of 32, 64, 96 and 128 columns
     static constexpr int kFixed[2][4] = {{12500, 13000, 16500, 26000}, {12500, 14500, 16300, 17500}}; // per CTA with all segments, with one
     int bestN = 128, bestCtas = 1;
