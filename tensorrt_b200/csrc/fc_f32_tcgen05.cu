@@ -512,12 +512,12 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         {
             uint32_t const s = c & 1;
             // A barrier answers after 120 ... 150 cycles: all are asked at once.
-            bool const landed = mbarTryWaitAddr(smemAddr(&stFull[stage]), phase);
+            bool const landed = mbarTestAddr(smemAddr(&stFull[stage]), phase);
             if (c >= 2)
             {
                 uint32_t const parity = ((c - 2) >> 1) & 1u;
-                bool const summed = mbarTryWaitAddr(smemAddr(&done[part * kParts + s]), parity);
-                bool const complete = L::kHalves == 1 || part == 1 || mbarTryWaitAddr(smemAddr(&done[kParts + s]), parity);
+                bool const summed = mbarTestAddr(smemAddr(&done[part * kParts + s]), parity);
+                bool const complete = L::kHalves == 1 || part == 1 || mbarTestAddr(smemAddr(&done[kParts + s]), parity);
                 promote(c - 2, summed);
                 // all its products are complete: so is what they read where this chunk's parts go
                 if (L::kHalves == 2 && part == 0 && !__all_sync(0xffffffffu, complete))

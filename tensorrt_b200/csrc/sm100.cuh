@@ -90,6 +90,23 @@ __device__ __forceinline__ bool mbarTryWaitAddr(uint32_t barAddr, uint32_t parit
     return ok != 0;
 }
 
+// The same without waiting: try_wait may hold the thread back for microseconds while the phase is incomplete, so a barrier that is only asked
+// ahead of its use (an answer takes 120 to 150 cycles, in which a warp can do something else) is asked by this one.
+__device__ __forceinline__ bool mbarTestAddr(uint32_t barAddr, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(ok)
+        : "r"(barAddr), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Every spin in these kernels is bounded: after kWaitLimitNs without progress the waiter records
 // `code` in *abortFlag (shared memory; every later wait in the CTA returns immediately) and
 // returns false. The kernel then drains, frees its TMEM and exits; the host sees the status word.
