@@ -19,7 +19,7 @@
 //               (swizzled shared-memory tiles, one mbarrier each).
 //   warp 1    : TMEM allocation (512 columns); issues the context products (an elected lane does)
 //                 O  += P_j V_j           (128 x 64, accumulator in TMEM columns 384..447; for S > 384 it re-uses
-//                                          the columns of S_0, which serialises consecutive tiles)
+//                                          the columns of S_0: the next tile's scores of that block wait for them)
 //   warp 18   : issues the scores of the following tile, per key block as soon as the softmax warps hold
 //               the current S_j in registers:
 //                 S_j = Q K_j^T           (128 x 128 per key block, accumulators in TMEM columns 128j..)
@@ -30,7 +30,10 @@
 //                 epilogue O * scale_bmm2, round, saturate -> 128-bit global stores, deferred until after pass A of
 //                         the next tile.
 //               The passes loop over the key blocks (not unrolled): unrolled, the kernel was bound by instruction
-//               fetch (122 KB of text, 77 % instruction-cache hits).
+//               fetch (122 KB of text, 77 % instruction-cache hits). For the same reason what differs at four key blocks (the context
+//               shares columns with scores, blocks of P share slots) is decided when the kernel is compiled: 64 x 384 tokens, 16 heads
+//               101 -> 94 us, 64 x 256 53.4 -> 49.2 us, 64 x 512 180 -> 170 us. Of these last 10, 7 us come from the scores of key blocks 1 ... 3, which
+//               are formed while the context of the tile before is finished and read: only those of block 0 wait for its columns.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM, reports through the status word.
 #include "mha_items.h"
 #include "sm100.cuh"
@@ -165,7 +168,9 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
 // ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h).
-template <bool IL, bool BNSD, bool ORDERED>
+// FOUR: the longest sequence has four key blocks, not up to three. The context accumulator then has to share TMEM columns with the scores of key block 0, and four
+// blocks of P share two slots.
+template <bool IL, bool BNSD, bool ORDERED, bool FOUR>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
@@ -247,10 +252,9 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
 
     // The layout of shared memory and TMEM follows the longest sequence the launch admits.
     int const nbMax = (args.S + kKeyBlock - 1) / kKeyBlock;
-    // S > 384: the context accumulator has to share TMEM columns with the scores of key block 0
-    bool const oAliasesScores = nbMax > 3;
-    uint32_t const oCol = oAliasesScores ? 0u : kOColumn;
-    auto slotOf = [&](int j) { return nbMax <= 3 ? j : (j & 1); };
+    constexpr bool oAliasesScores = FOUR;
+    constexpr uint32_t oCol = oAliasesScores ? 0u : kOColumn;
+    auto slotOf = [&](int j) { return oAliasesScores ? (j & 1) : j; };
 
     uint8_t* sQ = smem;                          // kTileBytes
     uint8_t* sK = smem + L::kOffset();           // nbMax x kTileBytes
@@ -441,13 +445,13 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             uint32_t const kLo = static_cast<uint32_t>(dQk) + (smemAddr(sK) >> 4);
             uint32_t const vLo = static_cast<uint32_t>(dV) + (smemAddr(sV) >> 4);
             uint32_t const pLo = static_cast<uint32_t>(dP) + (smemAddr(sP) >> 4);
-            uint32_t const pPairStep = nbMax <= 3 ? 2u * (L::kPBytes >> 4) : 0u; // slotOf(j) = (j & 1) + (j >> 1) * (2 or 0)
+            constexpr uint32_t pPairStep = oAliasesScores ? 0u : 2u * (L::kPBytes >> 4); // slotOf(j) = (j & 1) + (j >> 1) * (2 or 0)
             constexpr uint32_t kTile16 = L::kTileBytes >> 4;
             uint32_t qkTiles = 0;  // tiles whose scores have been issued
             uint32_t pvTiles = 0;  // tiles of this CTA that the loop below has passed (= whose context has been issued)
             uint32_t kBits = 0, vBits = 0, pBits = 0, fBits = 0; // parity per key block: K landed, V landed, P written, S read
             // scores of key block j for the query tile whose Q is in shared memory; nbOf = key blocks of that tile's item
-            auto issueScores = [&](int j, int nbOf) {
+            auto issueScores = [&](int j, bool last) {
                 if (electOne())
                 {
 #pragma unroll
@@ -457,7 +461,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                         mmaLoHi<true>(tmemBase + j * kKeyBlock, qLo + off, hiQk, kLo + j * kTile16 + off, hiQk, kIdescQk, k != 0);
                     }
                     tcCommit(&sFull[j]);
-                    if (j == nbOf - 1)
+                    if (last)
                         tcCommit(qFree);
                 }
                 __syncwarp();
@@ -468,6 +472,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 kBits ^= 1u << j;
                 return got;
             };
+            constexpr int firstBlock = oAliasesScores ? 1 : 0; // key blocks whose scores do not wait for the context
             Item cur, nxt;
             int item = nextWork(firstItem, cur);
             if (kDoScores && item < numItems)
@@ -482,7 +487,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                         if (ok)
                         {
                             tcFenceAfter();
-                            issueScores(j, cur.nb);
+                            issueScores(j, j == cur.nb - 1);
                         }
                     }
                 }
@@ -507,17 +512,17 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                             // Scores of the following tile for this key block first: they only need the softmax warps
                             // to hold this tile's S_j in registers (sFree), not the finished P_j, and the next pass A
                             // waits for them, while this tile's context is not read before the pass after.
-                            if (kDoScores && j < nbFollow && !oAliasesScores)
+                            if (kDoScores && j == 0 && nbFollow > 0)
+                                ok = mbarWaitWarp(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
+                            if (kDoScores && j < nbFollow && j >= firstBlock)
                             {
-                                if (j == 0)
-                                    ok = mbarWaitWarp(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
                                 if (ok && lastT)
                                     ok = waitK(j);
                                 ok = ok && mbarWaitWarp(&sFree[j], (fBits >> j) & 1u, abortFlag, kWaitSoftmax);
                                 if (ok)
                                 {
                                     tcFenceAfter();
-                                    issueScores(j, nbFollow);
+                                    issueScores(j, j == nbFollow - 1 && !oAliasesScores);
                                 }
                             }
                             fBits ^= 1u << j; // the softmax warps complete this phase in every tile that uses block j
@@ -559,7 +564,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                             }
                         }
                     }
-                    if (kDoScores && ok && !oAliasesScores)
+                    if (kDoScores && ok)
                     {
                         // key blocks the next item has beyond this one's: their score columns are idle
 #pragma unroll 1
@@ -571,28 +576,19 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                                 if (ok)
                                 {
                                     tcFenceAfter();
-                                    issueScores(j, nbFollow);
+                                    issueScores(j, j == nbFollow - 1 && !oAliasesScores);
                                 }
                             }
                         }
                     }
                     if (kDoScores && ok && nbFollow > 0 && oAliasesScores)
                     {
-                        // the context accumulator occupies score columns: wait until the epilogue has read it
-                        ok = mbarWaitWarp(oFree, pvTiles & 1, abortFlag, kWaitAccFree) && mbarWaitWarp(qFull, qkTiles & 1, abortFlag, kWaitTmaFull);
-#pragma unroll 1
-                        for (int j = 0; j < kMaxBlocks; ++j)
+                        // the context accumulator occupies the columns of key block 0: wait until the epilogue has read it
+                        ok = (!lastT || waitK(0)) && mbarWaitWarp(oFree, pvTiles & 1, abortFlag, kWaitAccFree);
+                        if (ok)
                         {
-                            if (j < nbFollow && ok)
-                            {
-                                if (lastT)
-                                    ok = waitK(j);
-                                if (ok)
-                                {
-                                    tcFenceAfter();
-                                    issueScores(j, nbFollow);
-                                }
-                            }
+                            tcFenceAfter();
+                            issueScores(0, true);
                         }
                     }
                     if (nbFollow > 0)
@@ -646,8 +642,11 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             return got;
         };
         // Reads 16 of the 64 context values of this row (tile number `tileNo` of the CTA), requantises
-        // and stores them to `dst` (null: row beyond the sequence).
-        auto epilogue = [&](uint32_t tileNo, int8_t* dst) {
+        // and stores them to `pendDst` (null: row beyond the sequence).
+        bool pending = false;
+        int8_t* pendDst = nullptr;
+        auto epilogue = [&](uint32_t tileNo) {
+            pending = false;
             if (ok)
                 ok = mbarWait(oFull, tileNo & 1, abortFlag, kWaitAccFull);
             if (!ok)
@@ -658,7 +657,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             tmemLoadWait16(x);
             tcFenceBefore();
             mbarArrive(oFree);
-            if (dst == nullptr)
+            if (pendDst == nullptr)
                 return;
             float const s2 = args.scaleBmm2;
             uint4 o;
@@ -669,15 +668,13 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     static_cast<float>(static_cast<int32_t>(x[4 * i + 1])) * s2,
                     static_cast<float>(static_cast<int32_t>(x[4 * i + 2])) * s2,
                     static_cast<float>(static_cast<int32_t>(x[4 * i + 3])) * s2);
-            *reinterpret_cast<uint4*>(dst) = o;
+            *reinterpret_cast<uint4*>(pendDst) = o;
         };
 
-        // The epilogue of a tile runs after pass A of the CTA's next tile (of the same or the next item): the last PV
-        // product then completes under useful work instead of a stall. Not possible when the context accumulator
-        // shares columns with the scores.
-        bool const deferEpilogue = !oAliasesScores;
-        bool pending = false;
-        int8_t* pendDst = nullptr;
+        // The epilogue of a tile runs after pass A of the CTA's next tile (of the same or the next item): the last PV product then completes
+        // under useful work instead of a stall. Where the context accumulator shares columns with the scores of key block 0, it runs
+        // before the maximum over that block, which comes last.
+        constexpr int firstBlock = oAliasesScores ? 1 : 0;
 
         Item it;
         for (int item = firstItem; item < numItems; item += itemStep)
@@ -721,9 +718,16 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
 
                 // ---- pass A: row maximum (integers, no conversions) ----
                 int32_t mxi = INT32_MIN;
+                // the block whose columns hold the context of the tile before comes last
 #pragma unroll 1
-                for (int j = 0; j < nb; ++j)
+                for (int i = firstBlock; i < nb + firstBlock; ++i)
                 {
+                    int const j = i < nb ? i : 0;
+                    if constexpr (FOUR)
+                    {
+                        if (pending && j == 0)
+                            epilogue(tiles - 1);
+                    }
                     ok = ok && mbarWait(&sFull[j], (sBits >> j) & 1u, abortFlag, kWaitSoftmax);
                     tcFenceAfter();
                     tmemLoad32(tRow + colOf(j), x);
@@ -732,22 +736,22 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     if (limit >= 32)
                     {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            mxi = max(mxi, static_cast<int32_t>(x[i]));
+                        for (int k = 0; k < 32; ++k)
+                            mxi = max(mxi, static_cast<int32_t>(x[k]));
                     }
                     else
                     {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (i < limit)
-                                mxi = max(mxi, static_cast<int32_t>(x[i]));
+                        for (int k = 0; k < 32; ++k)
+                            if (k < limit)
+                                mxi = max(mxi, static_cast<int32_t>(x[k]));
                     }
                 }
                 float mx = mxi == INT32_MIN ? -INFINITY : static_cast<float>(mxi);
-                if (pending)
+                if constexpr (!FOUR)
                 {
-                    epilogue(tiles - 1, pendDst);
-                    pending = false;
+                    if (pending)
+                        epilogue(tiles - 1);
                 }
                 rowRed[sub * kQTile + r] = mx;
                 softmaxBarrier();
@@ -841,17 +845,12 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     ? nullptr
                     : (IL ? outPtrIl(q, sub >> 1) + (sub & 1) * 16 : outRow(q) + sub * 16);
                 ++tiles;
-                if (deferEpilogue)
-                {
-                    pending = true;
-                    pendDst = dst;
-                }
-                else
-                    epilogue(tiles - 1, dst);
+                pending = true;
+                pendDst = dst;
             }
         }
         if (pending)
-            epilogue(tiles - 1, pendDst);
+            epilogue(tiles - 1);
         tcFenceBefore();
     }
 
@@ -1206,10 +1205,13 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
     int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (plan.longestFirst ? static_cast<int>(sizeof(ItemTable)) : 0);
-    static SmemOptIn optIn[2];
-    auto const kernel = plan.longestFirst ? mhaTcgen05Kernel<IL, BNSD, true> : mhaTcgen05Kernel<IL, BNSD, false>;
+    static SmemOptIn optIn[4];
+    int const form = (plan.longestFirst ? 1 : 0) + (args.S > 3 * kKeyBlock ? 2 : 0);
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
+    static constexpr Kernel kForms[4] = {mhaTcgen05Kernel<IL, BNSD, false, false>, mhaTcgen05Kernel<IL, BNSD, true, false>,
+        mhaTcgen05Kernel<IL, BNSD, false, true>, mhaTcgen05Kernel<IL, BNSD, true, true>};
     cudaError_t const e = launchDependentCluster(
-        &optIn[plan.longestFirst], kernel, dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
+        &optIn[form], kForms[form], dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(e));
     return checkLaunch("mhaTcgen05Kernel");
