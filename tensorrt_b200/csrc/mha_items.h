@@ -56,6 +56,24 @@ inline ItemPlan planItems(int32_t B, int32_t N, int32_t S, int64_t missing, int6
     return plan;
 }
 
+// Ragged packed batches of no more pairs than CTAs, which planItems leaves whole because full sequences would be: their tiles, one by one, in the order
+// of the sequences' lengths. The longest pair then no longer holds up the launch, at the price of K and V for each tile. In the units above a tile
+// costs up to four per key block and a whole pair 3 tiles + 1, so the cut is shorter while the rounds of tiles are fewer than that over four. How
+// many tiles there are follows from the tokens, taking half a tile per sequence for its last one and a sixteenth on top. Over 40 000 random batches of this
+// model the cut is never longer, and half as long on average. Measured (whole pairs in brackets): 8 sequences of 90 ... 384 tokens, 16 heads 12.3 us
+// (16.0 us), 12 of 32 ... 384, 12 heads 12.5 us
+// (15.9 us).
+// Returns the most tiles that there can be, or 0: not cut. tokens: of the batch.
+inline int64_t cutTiles(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t ctas)
+{
+    int64_t const pairs = static_cast<int64_t>(B) * N, nq = (S + kItemTile - 1) / kItemTile;
+    if (pairs > ctas || B > kItemOrder || tokens > pairs / N * S - (S - (nq - 1) * kItemTile))
+        return 0;
+    int64_t const about = N * (tokens / kItemTile + (B + 1) / 2), rounds = (about + about / 16 + ctas - 1) / ctas;
+    int64_t const most = N * (tokens / kItemTile + B);
+    return 4 * rounds < 3 * nq + 1 && most <= kItemRounds * ctas ? (most < pairs * nq ? most : pairs * nq) : 0;
+}
+
 // The item that CTA `cta` takes in its `round`-th turn, the items being in the order of their lengths: every second round runs
 // backwards, so that who had the longest of a round gets the shortest of the next. May lie beyond the last item in the last round.
 B200_HOST_DEVICE inline int32_t itemOfRound(int32_t round, int32_t cta, int32_t ctas)

@@ -71,14 +71,14 @@ struct MhaArgs
     float scaleBmm1, scaleSoftmax, scaleBmm2;
     uint32_t* statusWord;
     int32_t tilesPerItem, chunks; // a work item = (sequence, head, chunk of tilesPerItem query tiles)
-    int32_t rounds;               // ORDERED: items per CTA
+    int32_t rounds, cut;          // ORDERED: items per CTA; whether they are tiles, not pairs
 };
 
 // Sequences by length and the items of a CTA (ORDERED, see the kernel).
 struct alignas(1024) ItemTable
 {
     int4 ordered[kItemOrder]; // number, first row, length
-    int4 items[kItemRounds];  // sequence (-1: none), head, first row, length
+    int4 items[kItemRounds];  // sequence (-1: none), head and first tile (above 16 bits), first row, length
     int32_t lengths[kItemOrder];
 };
 
@@ -224,11 +224,11 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         {
             int4 const q = table->items[i];
             it.b = q.x;
-            it.head = q.y;
+            it.head = q.y & 0xffff;
             it.rowBase = q.z;
             it.len = q.w;
             it.rows = args.fixedLayout && q.x >= 0 ? args.S : it.len;
-            it.tBegin = 0;
+            it.tBegin = q.y >> 16;
         }
         else
         {
@@ -340,12 +340,27 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             if (b < args.rounds)
             {
                 int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
-                int const place = item / args.N;
                 int4 q = make_int4(-1, 0, 0, 0);
-                if (place < args.B)
+                if (args.cut) // the tiles of a pair one by one: a longer sequence has more of them
                 {
-                    int4 const o = table->ordered[place];
-                    q = make_int4(o.x, item - place * args.N, o.y, o.z);
+                    int left = item;
+                    for (int place = 0; place < args.B; ++place)
+                    {
+                        int4 const o = table->ordered[place];
+                        int const tiles = (o.z + kQTile - 1) / kQTile;
+                        if (left < tiles * args.N)
+                        {
+                            int const head = left / tiles;
+                            q = make_int4(o.x, head | (left - head * tiles) << 16, o.y, o.z);
+                            break;
+                        }
+                        left -= tiles * args.N;
+                    }
+                }
+                else if (item / args.N < args.B)
+                {
+                    int4 const o = table->ordered[item / args.N];
+                    q = make_int4(o.x, item % args.N, o.y, o.z);
                 }
                 table->items[b] = q;
             }
@@ -1199,14 +1214,17 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     }
     int64_t const missing = !args.fixedLayout ? static_cast<int64_t>(args.B) * args.S - args.total : (args.maskIdx ? INT64_MAX : 0);
     ItemPlan const plan = planItems(args.B, args.N, args.S, missing, smCount());
-    args.tilesPerItem = plan.tilesPerItem;
+    int64_t const cut = args.fixedLayout || plan.chunks > 1 ? 0 : cutTiles(args.B, args.N, args.S, args.total, smCount());
+    args.cut = cut > 0 ? 1 : 0;
+    args.tilesPerItem = cut > 0 ? 1 : plan.tilesPerItem;
     args.chunks = plan.chunks;
-    int64_t const items = static_cast<int64_t>(args.B) * args.N * plan.chunks;
+    int64_t const items = cut > 0 ? cut : static_cast<int64_t>(args.B) * args.N * plan.chunks;
+    bool const ordered = plan.longestFirst || cut > 0;
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
-    int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (plan.longestFirst ? static_cast<int>(sizeof(ItemTable)) : 0);
+    int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (ordered ? static_cast<int>(sizeof(ItemTable)) : 0);
     static SmemOptIn optIn[4];
-    int const form = (plan.longestFirst ? 1 : 0) + (args.S > 3 * kKeyBlock ? 2 : 0);
+    int const form = (ordered ? 1 : 0) + (args.S > 3 * kKeyBlock ? 2 : 0);
     using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
     static constexpr Kernel kForms[4] = {mhaTcgen05Kernel<IL, BNSD, false, false>, mhaTcgen05Kernel<IL, BNSD, true, false>,
         mhaTcgen05Kernel<IL, BNSD, false, true>, mhaTcgen05Kernel<IL, BNSD, true, true>};
@@ -1254,7 +1272,7 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
     maps[1] = map;
     maps[2] = map;
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
-        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1};
+        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1, 0};
     return launchItems<IL, false>(args, maps, stream);
 }
 
@@ -1277,7 +1295,7 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
             return st;
     }
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
-        p.scale_bmm2, p.status_word, 1, 1, 1};
+        p.scale_bmm2, p.status_word, 1, 1, 1, 0};
     return launchItems<false, true>(args, maps, stream);
 }
 

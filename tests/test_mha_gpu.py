@@ -627,6 +627,29 @@ def test_mha_int8_longest_first(cuda, B, N, smax, layout):
     _assert_int8_attention(out, ref)
 
 
+# Few ragged sequences, whose tiles are dealt one by one: as many pairs as SMs, empty sequences, lengths at the edges of tiles, one long one
+@pytest.mark.parametrize("lengths,N", [([384, 97, 279, 90, 195, 241, 267, 119], 16), ([1, 0, 512, 129, 128, 127, 257, 0, 385], 16), ([300, 1, 1], 37),
+                                       ([0, 500, 3], 49), ([511, 384, 256, 255, 40], 12), ([260] + [16] * 147, 1)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_mha_int8_few_ragged_pairs(cuda, lengths, N, interleaved):
+    import tensorrt_b200 as T
+
+    d, B, smax = 32, len(lengths), max(lengths)
+    cu = O.cu_seqlens(np.array(lengths, dtype=np.int32))
+    x = np.random.default_rng(N).integers(-127, 128, size=(int(cu[-1]), 3 * N * d)).astype(np.int8)
+    s1, s2 = float((4.0 / 127) ** 2 / np.sqrt(d)), 2.0 / 127
+    ref = O.mha_int8(x, B, smax, N, d, s1, 127.0, s2, cu=cu)
+    st = _status(cuda)
+    scales = {"scale_bmm1": s1, "scale_softmax": 127.0, "scale_bmm2": s2, "cu_seqlens": _t(cu, cuda), "status": st}
+    if interleaved:
+        il = x.reshape(-1, N, 3, d).transpose(0, 2, 1, 3).reshape(-1, 3 * N * d)   # [3][N][d / 32][total][32]
+        out = O.from_chw32(T.mha(_t(O.to_chw32(il), cuda), B, smax, N, d, interleaved=True, **scales).cpu().numpy())
+    else:
+        out = T.mha(_t(x, cuda), B, smax, N, d, **scales).cpu().numpy()
+    assert int(st[0]) == 0
+    _assert_int8_attention(out, ref)
+
+
 @pytest.mark.parametrize("d", [16, 48, 64])
 @pytest.mark.parametrize("lengths", [[37], [1, 16, 17, 32, 33, 0, 64, 65, 96, 97, 127, 128], [5] * 150])
 def test_mha_fp16_single_key_block(cuda, d, lengths):

@@ -19,9 +19,12 @@ def lib(tmp_path_factory):
     (d / "items.cpp").write_text('#include "mha_items.h"\n'
                                  'extern "C" void plan(int32_t B, int32_t N, int32_t S, int64_t missing, int64_t ctas, int32_t* out)'
                                  "{ auto p = b200::planItems(B, N, S, missing, ctas); out[0] = p.tilesPerItem; out[1] = p.chunks; out[2] = p.longestFirst; }\n"
+                                 'extern "C" int64_t cut(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t ctas) { return b200::cutTiles(B, N, S, tokens, ctas); }\n'
                                  'extern "C" int32_t item(int32_t round, int32_t cta, int32_t ctas) { return b200::itemOfRound(round, cta, ctas); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", str(d / "items.cpp"), "-o", str(d / "items.so")], check=True)
-    return ctypes.CDLL(str(d / "items.so"))
+    so = ctypes.CDLL(str(d / "items.so"))
+    so.cut.restype = ctypes.c_int64
+    return so
 
 
 def _plan(lib, b, heads, s, missing):
@@ -68,6 +71,35 @@ def test_ragged_batches_are_not_slower_than_whole_pairs_as_they_come(lib, heads,
                      / _time(lengths, s, heads, nq, 1, padded))
     assert max(ratio) <= 1.13 and sum(r > 1.03 for r in ratio) <= 3, sorted(ratio)[-5:]
     assert sum(ratio) / len(ratio) < 0.9
+
+
+@pytest.mark.parametrize("heads", [1, 12, 16])
+def test_few_ragged_pairs_are_cut_into_tiles_where_that_is_shorter(lib, heads):
+    """Tiles dealt longest first against whole pairs: never a longer list, all tiles inside the bound that the launch is made for."""
+    rng = random.Random(heads)
+    ratio = []
+    for _ in range(3000):
+        s, b = rng.randint(1, 512), rng.randint(1, CTAS // heads)
+        lengths = [rng.randint(s // rng.choice([1, 2, 4, 12]), s) for _ in range(b)]
+        lengths[rng.randrange(b)] = s
+        most = lib.cut(b, heads, s, ctypes.c_int64(sum(lengths)), ctypes.c_int64(CTAS))
+        if most == 0 or _plan(lib, b, heads, s, b * s - sum(lengths))[1] > 1:
+            continue
+        blocks = sorted((-(-n // TILE) for n in lengths), reverse=True)
+        tiles = [4 * n for n in blocks for _ in range(heads * n)]
+        assert len(tiles) <= most <= 64 * CTAS
+        ctas = min(CTAS, most)
+        load = [0] * ctas
+        seen = set()
+        for r in range(-(-most // ctas)):
+            for cta in range(ctas):
+                i = lib.item(r, cta, ctas)
+                seen.add(i)
+                load[cta] += tiles[i] if i < len(tiles) else 0
+        assert seen >= set(range(len(tiles)))
+        ratio.append(max(load) / max((3 * n + 1) * n for n in blocks))
+    assert not ratio or (max(ratio) <= 1.0 and sum(ratio) / len(ratio) < 0.75), max(ratio)
+    assert ratio or heads == 1
 
 
 def test_equal_lengths_are_cut_where_that_is_shorter(lib):
