@@ -73,14 +73,24 @@ __device__ __forceinline__ float tokSum(float v, float* slot, int wInRow, int la
 __device__ __forceinline__ void maskIdxOfSequence(int32_t const S, int32_t const B, int32_t const b, int const lane,
     int32_t const* __restrict__ mask, int32_t* __restrict__ maskIdx)
 {
+    constexpr int kAhead = 8; // reads of 32 positions on their way (one at a time: 8 x 384 tokens, embedding and mask index, 8.8 us instead of 7.0 us)
     int first = S;
-    for (int base = 0; base < S && first == S; base += 32)
+    for (int base = 0; base < S && first == S; base += 32 * kAhead)
     {
-        int const s = base + lane;
-        bool const zero = s < S && mask[static_cast<int64_t>(s) * B + b] == 0;
-        uint32_t const ballot = __ballot_sync(0xffffffffu, zero);
-        if (ballot)
-            first = base + __ffs(ballot) - 1;
+        bool zero[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+        {
+            int const s = base + i * 32 + lane;
+            zero[i] = s < S && __ldg(mask + static_cast<int64_t>(s) * B + b) == 0;
+        }
+#pragma unroll
+        for (int i = kAhead - 1; i >= 0; --i)
+        {
+            uint32_t const ballot = __ballot_sync(0xffffffffu, zero[i]);
+            if (ballot)
+                first = base + i * 32 + __ffs(ballot) - 1;
+        }
     }
     if (lane == 0)
         maskIdx[b] = first;

@@ -103,6 +103,20 @@ def test_mask_idx_bit_exact(cuda, S, B):
     assert np.array_equal(out, lengths.astype(np.int32))
 
 
+# Masks are read 256 positions at a time: the first masked position at the edges of that and beyond, zeros behind it that are not the first
+@pytest.mark.parametrize("S", [255, 256, 257, 511, 512, 700])
+def test_mask_idx_edges(cuda, S):
+    import tensorrt_b200 as T
+
+    first = [0, 1, 31, 32, 33, 254, 255, 256, 257, 287, 288, 510, 511, 512, 513, S - 1, S]
+    first = [f for f in first if f <= S]
+    mask = np.ones((S, len(first)), np.int32)
+    for b, f in enumerate(first):
+        mask[f::3, b] = 0
+    out = T.compute_mask_idx(_t(mask, cuda)).cpu().numpy()
+    assert np.array_equal(out, np.array(first))
+
+
 @pytest.mark.parametrize("S,B,E,dtype", [(1, 1, 128, np.float32), (20, 5, 100, np.float32), (128, 32, 768, np.float16),
                                          (384, 64, 1024, np.float16), (3, 700, 1024, np.float16)])
 def test_mask_idx_from_the_embedding_launch(cuda, S, B, E, dtype):
