@@ -72,6 +72,7 @@ struct OnlineArgs : ShareArgs
     void* out;
     float scaleBmm1;
     uint32_t* statusWord;
+    uint32_t shortCols; // tensor memory that a CTA of the short kernel takes
 };
 
 // [ Q slots ][ K/V stages ][ barriers ][ shares ]
@@ -730,16 +731,18 @@ __global__ void __maxnreg__(168)
 // A launch of few such tiles is a chain of latencies: lengths, loads, scores, softmax, product, store. The persistent kernel adds
 // to them what its division of the work and the hand-overs between its twelve warps take, and the fetch of 80 KB of code, of
 // which a tile runs through a small part: a forward's other kernels have replaced it in the instruction caches since the layer
-// before. Here the code is a few KB and a tile 50 KB of shared memory and half of the tensor memory, so that two CTAs share an
-// SM. The arithmetic is that of the persistent kernel, to the bit. Measured, 16 heads (persistent kernel in brackets): 1 x 37
-// tokens 3.4 us (5.1 us), 8 x 128 4.4 us (6.4 us), 36 x 64 7.1 us (12.6 us), 148 x 128 39.4 us (42.8 us).
+// before. Here the code is a few KB, and a tile takes 50 KB of shared memory, 128 columns of tensor memory (P and the context lie where the scores
+// were) and 150 registers a thread, so that three CTAs can share an SM. The arithmetic is that of the persistent kernel, to the bit. Measured, 16 heads
+// (persistent kernel in brackets): 1 x 37 tokens 3.4 us (5.1 us), 8 x 128 4.4 us (6.4 us), 36 x 64 7.1 us (12.6 us), 148 x 128 34.0 us (42.8 us).
+// Two or three: see launchOnline.
 constexpr int kShortThreads = 128;
 constexpr int kShortBars = 3 * kStageBytes; // after Q, K and V
 constexpr int kShortSmemBytes = kShortBars + 64 + 1024;
-constexpr uint32_t kShortTmemCols = 256; // scores 0 ..., P 128 ..., context 192 ...
+constexpr int kShortSmemTwo = 80 * 1024; // asked for where two CTAs are to share an SM
+constexpr uint32_t kShortTmemCols = 128; // scores; once they are in registers, P in the first 64 columns and the context in the others
 
 template <bool BNSD>
-__global__ void __launch_bounds__(kShortThreads, 2) mhaShortF16Kernel(const __grid_constant__ CUtensorMap mapQ,
+__global__ void __launch_bounds__(kShortThreads, 3) mhaShortF16Kernel(const __grid_constant__ CUtensorMap mapQ,
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, OnlineArgs const args)
 {
     constexpr uint32_t kIdescQk = makeInstrDesc(1u, 0u, 0u, 0u, 128u, 128u);
@@ -772,7 +775,7 @@ __global__ void __launch_bounds__(kShortThreads, 2) mhaShortF16Kernel(const __gr
     }
     __syncwarp();
     if (warp == 0)
-        tmemAlloc(tmemSlot, kShortTmemCols);
+        tmemAlloc(tmemSlot, args.shortCols);
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
@@ -828,7 +831,7 @@ __global__ void __launch_bounds__(kShortThreads, 2) mhaShortF16Kernel(const __gr
             __syncwarp();
         }
         uint32_t const tRow = tmemBase + (static_cast<uint32_t>(warp * 32) << 16);
-        uint32_t const tP = tRow + 128, tO = tRow + 192;
+        uint32_t const tP = tRow, tO = tRow + 64;
         float const sl2 = args.scaleBmm1 * 1.4426950408889634f;
         ok = ok && mbarWait(sFull, 0, abortFlag, kWaitSoftmax);
         __syncwarp();
@@ -895,7 +898,7 @@ __global__ void __launch_bounds__(kShortThreads, 2) mhaShortF16Kernel(const __gr
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                     if (k * 16 < g.len)
-                        mmaF16TmemA(tmemBase + 192, tmemBase + 128 + 8 * k, lo + k * 128u, hi, kIdescPv, k != 0);
+                        mmaF16TmemA(tmemBase + 64, tmemBase + 8 * k, lo + k * 128u, hi, kIdescPv, k != 0);
                 tcCommit(oFull);
             }
             __syncwarp();
@@ -950,7 +953,7 @@ __global__ void __launch_bounds__(kShortThreads, 2) mhaShortF16Kernel(const __gr
     {
         __syncwarp();
         tcFenceAfter();
-        tmemFree(tmemBase, kShortTmemCols);
+        tmemFree(tmemBase, args.shortCols);
     }
 }
 
@@ -960,9 +963,18 @@ int32_t launchOnline(CUtensorMap const (&maps)[3], OnlineArgs args, cudaStream_t
     int64_t const pairs = static_cast<int64_t>(args.B) * args.N;
     if (args.S <= kTile && pairs <= INT32_MAX) // one key block: the short kernel is ahead from one pair to thousands (see there)
     {
+        // How many CTAs share an SM. Three where that takes fewer rounds than two: 32 x 64 ... 128 tokens, 12 heads 7.1 us (two: 8.9 us), 64 x 128, 16
+        // heads 14.4 us (16.1 us), 1000 x 20 ... 60, 12 heads 107 us (121 us); in as many rounds they hinder each other: 40 x 64 ... 128, 12 heads
+        // 9.4 us (9.0 us). Two by their tensor memory, which the placement of CTAs knows nothing of: a third one waits for it, but has been set up
+        // when it gets it. That is ahead where a CTA per SM does - 8 x 128, 16 heads 4.4 us, limited by shared memory 5.3 us -, and behind where a
+        // round has more of them: 24 x 64 ... 128, 12 heads 7.1 us, by shared memory 6.2 us.
+        int64_t const sms = smCount(), two = (pairs + 2 * sms - 1) / (2 * sms), three = (pairs + 3 * sms - 1) / (3 * sms);
+        bool const bySmem = three == two && pairs > sms && pairs <= 2 * sms;
+        args.shortCols = three < two || bySmem ? kShortTmemCols : 2 * kShortTmemCols;
+        int const smem = bySmem ? kShortSmemTwo : kShortSmemBytes;
         static SmemOptIn optIn;
         cudaError_t const e = launchDependentCluster(&optIn, mhaShortF16Kernel<BNSD>, dim3(static_cast<unsigned>(pairs)), dim3(kShortThreads),
-            kShortSmemBytes, stream, 1, maps[0], maps[1], maps[2], args);
+            smem, stream, 1, maps[0], maps[1], maps[2], args);
         if (e != cudaSuccess)
             B200_FAIL(BERT_B200_CUDA_ERROR, "mhaShortF16Kernel: %s", cudaGetErrorString(e));
         return checkLaunch("mhaShortF16Kernel");
@@ -996,7 +1008,7 @@ int32_t mhaOnlineF16(bert_b200_mha_params const& p, cudaStream_t stream)
         return st;
     maps[1] = maps[0];
     maps[2] = maps[0];
-    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, p.cu_seqlens, p.mask_idx), p.head_size, p.out, p.scale_bmm1, p.status_word};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, p.cu_seqlens, p.mask_idx), p.head_size, p.out, p.scale_bmm1, p.status_word, 0};
     return launchOnline<false>(maps, args, stream);
 }
 
@@ -1016,7 +1028,7 @@ int32_t mhaOnlineF16Bnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t 
         if (st != BERT_B200_OK)
             return st;
     }
-    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, nullptr, p.kv_lengths), p.head_size, p.out, p.scale_bmm1, p.status_word};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, nullptr, p.kv_lengths), p.head_size, p.out, p.scale_bmm1, p.status_word, 0};
     return launchOnline<true>(maps, args, stream);
 }
 

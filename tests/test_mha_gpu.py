@@ -627,6 +627,21 @@ def test_mha_int8_longest_first(cuda, B, N, smax, layout):
     _assert_int8_attention(out, ref)
 
 
+# One, two or three CTAs of the short kernel per SM: pairs at the edges of the rounds that decide it (148 SMs), against the persistent
+# kernel, which an S of more than 128 (an upper bound only, in the packed layout) selects. Same bits.
+@pytest.mark.parametrize("B", [148, 149, 296, 297, 444, 445, 592, 593, 889])
+def test_mha_fp16_short_kernel_residency(cuda, B):
+    import tensorrt_b200 as T
+
+    lengths = np.array([(37 * i) % 129 for i in range(B)], dtype=np.int32)
+    lengths[B // 2] = 128
+    cu = _t(O.cu_seqlens(lengths), cuda)
+    x = torch.randn((int(lengths.sum()), 3 * 64), device=cuda, generator=torch.Generator(device=cuda).manual_seed(B)).half()
+    st = _status(cuda)
+    short, persistent = (T.mha(x, B, S, 1, 64, cu_seqlens=cu, status=st) for S in (128, 129))
+    assert int(st[0]) == 0 and torch.equal(short, persistent)
+
+
 # Few ragged sequences, whose tiles are dealt one by one: as many pairs as SMs, empty sequences, lengths at the edges of tiles, one long one
 @pytest.mark.parametrize("lengths,N", [([384, 97, 279, 90, 195, 241, 267, 119], 16), ([1, 0, 512, 129, 128, 127, 257, 0, 385], 16), ([300, 1, 1], 37),
                                        ([0, 500, 3], 49), ([511, 384, 256, 255, 40], 12), ([260] + [16] * 147, 1)])
