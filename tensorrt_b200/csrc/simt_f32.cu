@@ -322,32 +322,57 @@ __device__ __forceinline__ void store4(__half* p, float4 v)
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t const*>(&lo), *reinterpret_cast<uint32_t const*>(&hi));
 }
 
-// 64 queries of one (sequence, head) per CTA against blocks of 64 keys, running maximum and sum per row.
+// 16 bytes into shared memory, or zeros.
+__device__ __forceinline__ void copy16(void* to, void const* from, bool ok)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(to))), "l"(from), "r"(ok ? 16u : 0u)
+                 : "memory");
+}
+__device__ __forceinline__ void copyGroup()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N> // groups that may still be on their way
+__device__ __forceinline__ void copyWait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// 64 or 32 queries of one (sequence, head) per CTA against blocks of 64 keys, running maximum and sum per row.
 //
 // Bound by the FP32 pipes and the shared-memory loads that feed them. Every warp owns 16 query rows, so its scores,
 // probabilities and row sums are its own business (a warp-level sync between the two products); a thread computes 4 rows x
 // 8 keys of the scores with 16-byte loads along d (packed FMAs, even and odd channels apart, as in the FC above), and 4
-// rows x D / 8 columns of the context. Rows are padded by 4 floats against bank conflicts. Measured: 8 sequences of 128
-// tokens, 12 heads of 64 channels in 26 us (a warp per query row, keys and values from global memory: 509 us).
-constexpr int kAttRows = 64;
+// rows x D / 8 columns of the context. Rows are padded by 4 floats against bank conflicts. The next keys are fetched during the softmax and the
+// second product, the next values during the scores (see kAttAsync; with one barrier less each, values during scores and softmax, keys during the second product:
+// 16 x 128, 12 heads 31.7 us instead of 27.5 us). Measured, heads of 64 channels: 8 sequences of 128
+// tokens, 12 heads 21.4 us (a warp per query row, keys and values from global memory: 509 us).
 constexpr int kAttKeys = 64;
-constexpr int kAttThreads = 128;
 
-template <int D> // head size rounded up to 32, 64, 96 or 128; channels beyond d are zero
+template <int D, int WARPS> // head size rounded up to 32, 64, 96 or 128; channels beyond d are zero
 struct AttSmem
 {
+    static constexpr int kAttRows = 16 * WARPS;
     float q[kAttRows][D + 4];
     float k[kAttKeys][D + 4];
     float v[kAttKeys][D];
     float p[kAttRows][kAttKeys + 4];
 };
 
+// Asynchronous copies: FP32 heads of up to 64 channels. FP16 has to be converted on the way, and with wider heads fewer CTAs share an SM: the two
+// barriers more per block cost more than the copies' time (2 x 1100 tokens, 8 heads of 128 channels, FP32 327 -> 387 us).
 template <typename T, int D>
-__global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
+constexpr bool kAttAsync = sizeof(T) == 4 && D <= 64;
+
+template <typename T, int D, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
     T const* __restrict__ qkv, T* __restrict__ out, int32_t const* __restrict__ cu, int32_t const* __restrict__ maskIdx, float const scale)
 {
     extern __shared__ float smRaw[];
-    AttSmem<D>& sm = *reinterpret_cast<AttSmem<D>*>(smRaw);
+    using Smem = AttSmem<D, WARPS>;
+    Smem& sm = *reinterpret_cast<Smem*>(smRaw);
+    constexpr int kAttRows = Smem::kAttRows, kAttThreads = 32 * WARPS;
+    constexpr bool kAsync = kAttAsync<T, D>;
     constexpr int kVecs = D / 4;
     constexpr int kCols = D / 32; // float4 columns of the context per thread
     int const lane = threadIdx.x & 31;
@@ -371,7 +396,41 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
     {
         int const r = i / kVecs, c = i % kVecs * 4;
         bool const ok = q0 + r < seq.rows && c < d;
-        *reinterpret_cast<float4*>(&sm.q[r][c]) = ok ? load4(base + (q0 + r) * rowStep + c) : zero;
+        if constexpr (kAsync)
+            copy16(&sm.q[r][c], ok ? base + (q0 + r) * rowStep + c : base, ok);
+        else
+            *reinterpret_cast<float4*>(&sm.q[r][c]) = ok ? load4(base + (q0 + r) * rowStep + c) : zero;
+    }
+    // Scores of keys beyond the sequence are never looked at, so such rows are left as they are; a value row with them has to be a number.
+    [[maybe_unused]] auto fetchKeys = [&](int k0) {
+        if constexpr (sizeof(T) != 4)
+            return;
+        int const rows = min(kAttKeys, seq.len - k0);
+#pragma unroll 2
+        for (int i = threadIdx.x; i < rows * kVecs; i += kAttThreads)
+        {
+            int const r = i / kVecs, c = i % kVecs * 4;
+            copy16(&sm.k[r][c], c < d ? base + (k0 + r) * rowStep + c + d : base, c < d);
+        }
+        copyGroup();
+    };
+    [[maybe_unused]] auto fetchValues = [&](int k0) {
+        if constexpr (sizeof(T) != 4)
+            return;
+        int const rows = min(kAttKeys, (seq.len - k0 + 3) & ~3);
+#pragma unroll 2
+        for (int i = threadIdx.x; i < rows * kVecs; i += kAttThreads)
+        {
+            int const r = i / kVecs, c = i % kVecs * 4;
+            bool const ok = k0 + r < seq.len && c < d;
+            copy16(&sm.v[r][c], ok ? base + (k0 + r) * rowStep + c + 2 * d : base, ok);
+        }
+        copyGroup();
+    };
+    if constexpr (kAsync)
+    {
+        fetchKeys(0); // and the queries
+        fetchValues(0);
     }
     float4 o[4][kCols];
     float mx[4], sum[4];
@@ -386,15 +445,20 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
     }
     for (int k0 = 0; k0 < seq.len; k0 += kAttKeys)
     {
-        __syncthreads(); // the previous block of keys is done with
-#pragma unroll 4
-        for (int i = threadIdx.x; i < kAttKeys * kVecs; i += kAttThreads)
+        if constexpr (kAsync)
+            copyWait<1>(); // keys
+        else
         {
-            int const r = i / kVecs, c = i % kVecs * 4;
-            bool const ok = k0 + r < seq.len && c < d;
-            T const* const src = base + (k0 + r) * rowStep + c;
-            *reinterpret_cast<float4*>(&sm.k[r][c]) = ok ? load4(src + d) : zero;
-            *reinterpret_cast<float4*>(&sm.v[r][c]) = ok ? load4(src + 2 * d) : zero;
+            __syncthreads(); // the previous block of keys is done with
+#pragma unroll 4
+            for (int i = threadIdx.x; i < kAttKeys * kVecs; i += kAttThreads)
+            {
+                int const r = i / kVecs, c = i % kVecs * 4;
+                bool const ok = k0 + r < seq.len && c < d;
+                T const* const src = base + (k0 + r) * rowStep + c;
+                *reinterpret_cast<float4*>(&sm.k[r][c]) = ok ? load4(src + d) : zero;
+                *reinterpret_cast<float4*>(&sm.v[r][c]) = ok ? load4(src + 2 * d) : zero;
+            }
         }
         __syncthreads();
         uint64_t acc[4][8] = {};
@@ -416,6 +480,11 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
                     acc[i][j] = fma2(a[i].y, b.y, acc[i][j]);
                 }
             }
+        }
+        if constexpr (kAsync)
+        {
+            __syncthreads();
+            fetchKeys(k0 + kAttKeys);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -452,32 +521,81 @@ __global__ void __launch_bounds__(kAttThreads) mhaTiledKernel(int32_t const B, i
                 sm.p[row0 + 4 * i][tx + 8 * j] = e;
             }
         }
-        __syncwarp();
-#pragma unroll 2
-        for (int c = 0; c < kAttKeys; c += 4)
+        if constexpr (kAsync)
         {
-            float4 pr[4];
+            copyWait<1>(); // values
+            __syncthreads();
+        }
+        else
+            __syncwarp();
+        if constexpr (!kAsync)
+        {
+#pragma unroll 2
+            for (int c = 0; c < kAttKeys; c += 4)
+            {
+                float4 pr[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
+                for (int i = 0; i < 4; ++i)
+                    pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+                for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int j = 0; j < kCols; ++j)
+                    for (int j = 0; j < kCols; ++j)
+                    {
+                        float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                        {
+                            float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
+                            o[i][j].x = fmaf(w, v.x, o[i][j].x);
+                            o[i][j].y = fmaf(w, v.y, o[i][j].y);
+                            o[i][j].z = fmaf(w, v.z, o[i][j].z);
+                            o[i][j].w = fmaf(w, v.w, o[i][j].w);
+                        }
+                    }
+            }
+        }
+        else
+        {
+            auto product = [&](int const keys) {
+#pragma unroll 2
+                for (int c = 0; c < keys; c += 4)
                 {
-                    float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
+                    float4 pr[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                    {
-                        float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
-                        o[i][j].x = fmaf(w, v.x, o[i][j].x);
-                        o[i][j].y = fmaf(w, v.y, o[i][j].y);
-                        o[i][j].z = fmaf(w, v.z, o[i][j].z);
-                        o[i][j].w = fmaf(w, v.w, o[i][j].w);
-                    }
+                        pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int j = 0; j < kCols; ++j)
+                        {
+                            float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                            {
+                                float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
+                                o[i][j].x = fmaf(w, v.x, o[i][j].x);
+                                o[i][j].y = fmaf(w, v.y, o[i][j].y);
+                                o[i][j].z = fmaf(w, v.z, o[i][j].z);
+                                o[i][j].w = fmaf(w, v.w, o[i][j].w);
+                            }
+                        }
                 }
+            };
+            if (seq.len - k0 >= kAttKeys) // a loop of its own: with a variable end it is 2.5 % slower
+                product(kAttKeys);
+            else
+                product(seq.len - k0);
+        }
+        if constexpr (kAsync)
+        {
+            __syncthreads();
+            fetchValues(k0 + kAttKeys);
         }
     }
+    if constexpr (kAsync)
+        copyWait<0>();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
     {
@@ -605,18 +723,33 @@ int32_t fcF32Simt(bert_b200_fc_params const& p, cudaStream_t stream)
 namespace
 {
 
-template <typename T, int D>
+template <typename T, int D, int WARPS>
 int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 {
-    int32_t const rowBlocks = (p.S - 1) / kAttRows + 1;
+    int32_t const rowBlocks = (p.S - 1) / (16 * WARPS) + 1;
     B200_REQUIRE(rowBlocks <= 65535, "mha (SIMT): S=%d too large", p.S); // the grid's third dimension
     static SmemOptIn optIn;
-    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D>, dim3(p.num_heads, p.B, rowBlocks),
-        dim3(kAttThreads), sizeof(AttSmem<D>), stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
+    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D, WARPS>, dim3(p.num_heads, p.B, rowBlocks),
+        dim3(32 * WARPS), sizeof(AttSmem<D, WARPS>), stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
         static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTiledKernel: %s", cudaGetErrorString(e));
     return checkLaunch("mhaTiledKernel");
+}
+
+template <typename T, int D>
+int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
+{
+    int64_t const ctas = static_cast<int64_t>(p.num_heads) * p.B * ((p.S - 1) / 64 + 1);
+    // 32 rows where the 64-row CTAs are no more than two per SM: twice as many CTAs even out better, each with its own copies on the way.
+    // 8 x 128 tokens, 12 heads 24.4 -> 21.4 us, 10 x 128 26.9 -> 21.7 us, 5 x 200 49.1 -> 36.0 us, 16 heads 16 x 40 15.0 -> 10.4 us, 2 x 512 95.8 -> 77.5 us. With
+    // more of them 64: 13 x 128, 12 heads 27.3 us (31.0 us), 19 x 40, 16 heads 13.2 us (16.9 us); and where even 32-row ones would leave SMs
+    // without, 1 x 128, 16 heads 13.3 us (14.3 us).
+    [[maybe_unused]] bool const few = ctas <= 2 * smCount() && (2 * ctas > smCount() || p.S <= 64);
+    if constexpr (kAttAsync<T, D>)
+        if (few)
+            return launchMhaTiled<T, D, 2>(p, stream);
+    return launchMhaTiled<T, D, 4>(p, stream);
 }
 
 template <typename T>

@@ -428,6 +428,26 @@ def test_mha_simt_tile_edges(cuda, d, half):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, tol, tol)[0]
 
 
+# FP32 on CTAs of 32 and of 64 query rows: as many 64-row CTAs as make the difference (148 SMs: 74, 75 ... 296, 297; any number up to 64 tokens), lengths
+# at the edges of both, keys ending at and beside fours, padded and packed
+@pytest.mark.parametrize("S,B,N", [(31, 1, 1), (33, 3, 2), (64, 2, 2), (65, 37, 1), (66, 38, 1), (97, 10, 6), (128, 37, 4), (127, 25, 6), (259, 15, 4)])
+@pytest.mark.parametrize("d", [64, 20])
+def test_mha_fp32_rows_per_cta(cuda, S, B, N, d):
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(S + d)
+    lengths = np.array([S - 7 * i % S for i in range(B)], dtype=np.int32)
+    qkv = rng.standard_normal((S, B, 3 * N * d)).astype(np.float32)
+    ref = O.mha(qkv, B, S, N, d, lengths=lengths)
+    out = T.mha(_t(qkv, cuda), B, S, N, head_size=d, mask_idx=_t(lengths, cuda))
+    assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
+    cu = O.cu_seqlens(lengths)
+    packed = rng.standard_normal((int(cu[-1]), 3 * N * d)).astype(np.float32)
+    ref = O.mha(packed, B, S, N, d, cu=cu)
+    out = T.mha(_t(packed, cuda), B, S, N, head_size=d, cu_seqlens=_t(cu, cuda))
+    assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
+
+
 @pytest.mark.parametrize("d", [32, 64, 128])
 @pytest.mark.parametrize("block", [0, 64])
 def test_mha_fp32_scores_that_overflow(cuda, block, d):
