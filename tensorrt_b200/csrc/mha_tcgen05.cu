@@ -31,9 +31,10 @@
 //                         the next tile.
 //               The passes loop over the key blocks (not unrolled): unrolled, the kernel was bound by instruction
 //               fetch (122 KB of text, 77 % instruction-cache hits). For the same reason what differs at four key blocks (the context
-//               shares columns with scores, blocks of P share slots) is decided when the kernel is compiled: 64 x 384 tokens, 16 heads
-//               101 -> 94 us, 64 x 256 53.4 -> 49.2 us, 64 x 512 180 -> 170 us. Of these last 10, 7 us come from the scores of key blocks 1 ... 3, which
-//               are formed while the context of the tile before is finished and read: only those of block 0 wait for its columns.
+//               shares columns with scores, blocks of P share slots), and the layout, is decided when the kernel is compiled: 64 x 384
+//               tokens, 16 heads 101 -> 94 us, the layout too 93.5 us, 64 x 256 53.4 -> 49.2 -> 48.2 us, 64 x 512 180 -> 170 -> 168 us. Of these
+//               first 10, 7 us come from the scores of key blocks 1 ... 3, which are formed while the context of the tile before is finished
+//               and read: only those of block 0 wait for its columns.
 // Every wait is bounded (sm100.cuh); on expiry the CTA drains, frees TMEM, reports through the status word.
 #include "mha_items.h"
 #include "sm100.cuh"
@@ -168,9 +169,10 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
 // ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h).
+// FIXED: the fixed layout (or separate tensors), not the packed one.
 // FOUR: the longest sequence has four key blocks, not up to three. The context accumulator then has to share TMEM columns with the scores of key block 0, and four
 // blocks of P share two slots.
-template <bool IL, bool BNSD, bool ORDERED, bool FOUR>
+template <bool IL, bool BNSD, bool FIXED, bool ORDERED, bool FOUR>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     int const itemStep = ORDERED ? 1 : static_cast<int>(gridDim.x);
     // first row and valid keys of sequence b
     auto sequence = [&](int b, int32_t& rowBase, int32_t& len) {
-        if (args.fixedLayout)
+        if (FIXED)
         {
             rowBase = 0;
             len = args.maskIdx ? min(max(__ldg(args.maskIdx + b), 0), args.S) : args.S;
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             it.head = q.y & 0xffff;
             it.rowBase = q.z;
             it.len = q.w;
-            it.rows = args.fixedLayout && q.x >= 0 ? args.S : it.len;
+            it.rows = FIXED && q.x >= 0 ? args.S : it.len;
             it.tBegin = q.y >> 16;
         }
         else
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             it.head = pair - it.b * args.N;
             it.tBegin = (i - pair * args.chunks) * args.tilesPerItem;
             sequence(it.b, it.rowBase, it.len);
-            it.rows = args.fixedLayout ? args.S : it.len;
+            it.rows = FIXED ? args.S : it.len;
         }
         it.nb = (it.len + kKeyBlock - 1) / kKeyBlock; // key blocks
         it.tEnd = min((it.rows + kQTile - 1) / kQTile, it.tBegin + args.tilesPerItem);
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         bool ok = true;
         for (int item = nextWork(firstItem, it); item < numItems && ok; item = nextWork(item + itemStep, it))
         {
-            int32_t const rowK = args.fixedLayout ? 0 : it.rowBase;
+            int32_t const rowK = FIXED ? 0 : it.rowBase;
             int32_t const rowKv = rowK; // first key of this item
             // linear: (channel, which of [N][3], batch, row). interleaved: (channel, row, 32-channel group, which of [3][N])
             auto load = [&](uint8_t* dst, uint64_t* bar, int which, int32_t row) {
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                 else if (IL)
                     tmaLoad4d(dst, &mapQkv, bar, 0, row, 0, which * args.N + it.head);
                 else
-                    tmaLoad4d(dst, &mapQkv, bar, 0, it.head * 3 + which, args.fixedLayout ? it.b : 0, row);
+                    tmaLoad4d(dst, &mapQkv, bar, 0, it.head * 3 + which, FIXED ? it.b : 0, row);
             };
             for (int t = it.tBegin; t < it.tEnd && ok; ++t)
             {
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             auto outRow = [&](int q) -> int8_t* {
                 if (BNSD)
                     return out + ((static_cast<int64_t>(it.b) * args.N + it.head) * args.S + q) * args.d;
-                int64_t const rr = args.fixedLayout ? static_cast<int64_t>(q) * args.B + it.b : static_cast<int64_t>(it.rowBase) + q;
+                int64_t const rr = FIXED ? static_cast<int64_t>(q) * args.B + it.b : static_cast<int64_t>(it.rowBase) + q;
                 return outBase + rr * outRowStride;
             };
             // interleaved output [N][d/32][total][32]: 32-channel group `grp` of (token, head)
@@ -1223,13 +1225,17 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
     int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (ordered ? static_cast<int>(sizeof(ItemTable)) : 0);
-    static SmemOptIn optIn[4];
     int const form = (ordered ? 1 : 0) + (args.S > 3 * kKeyBlock ? 2 : 0);
     using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
-    static constexpr Kernel kForms[4] = {mhaTcgen05Kernel<IL, BNSD, false, false>, mhaTcgen05Kernel<IL, BNSD, true, false>,
-        mhaTcgen05Kernel<IL, BNSD, false, true>, mhaTcgen05Kernel<IL, BNSD, true, true>};
+    // BNSD is always fixed, interleaved always packed
+    static constexpr Kernel kForms[2][4] = {{mhaTcgen05Kernel<IL, BNSD, BNSD, false, false>, mhaTcgen05Kernel<IL, BNSD, BNSD, true, false>,
+                                                mhaTcgen05Kernel<IL, BNSD, BNSD, false, true>, mhaTcgen05Kernel<IL, BNSD, BNSD, true, true>},
+        {mhaTcgen05Kernel<IL, BNSD, !IL, false, false>, mhaTcgen05Kernel<IL, BNSD, !IL, true, false>, mhaTcgen05Kernel<IL, BNSD, !IL, false, true>,
+            mhaTcgen05Kernel<IL, BNSD, !IL, true, true>}};
+    static SmemOptIn optIn[2][4];
+    int const fixed = args.fixedLayout ? 1 : 0;
     cudaError_t const e = launchDependentCluster(
-        &optIn[form], kForms[form], dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
+        &optIn[fixed][form], kForms[fixed][form], dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(e));
     return checkLaunch("mhaTcgen05Kernel");
