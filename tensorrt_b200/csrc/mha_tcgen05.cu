@@ -172,7 +172,9 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
 // FIXED: the fixed layout (or separate tensors), not the packed one.
 // FOUR: the longest sequence has four key blocks, not up to three. The context accumulator then has to share TMEM columns with the scores of key block 0, and four
 // blocks of P share two slots.
-template <bool IL, bool BNSD, bool FIXED, bool ORDERED, bool FOUR>
+// CLAMP: with FOUR, whether scale_softmax is above 127 (64 x 512 tokens, 16 heads 168.7 -> 165.1 us); the form for shorter sequences finds out (decided when it is
+// compiled, it is 2 % slower).
+template <bool IL, bool BNSD, bool FIXED, bool ORDERED, bool FOUR, bool CLAMP>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                         uint32_t* w = reinterpret_cast<uint32_t*>(&o);
                         // p / sum <= 1 (the sum contains p; a rounded-up reciprocal adds a few ulp at most), so
                         // with scale_softmax <= 127 nothing can round beyond 127 and the clamp is left out
-                        if (args.scaleSoftmax <= 127.f)
+                        if (FOUR ? !CLAMP : args.scaleSoftmax <= 127.f)
                         {
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
@@ -1225,14 +1227,18 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
     int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (ordered ? static_cast<int>(sizeof(ItemTable)) : 0);
-    int const form = (ordered ? 1 : 0) + (args.S > 3 * kKeyBlock ? 2 : 0);
+    int const form = (ordered ? 1 : 0) + (args.S <= 3 * kKeyBlock ? 0 : args.scaleSoftmax <= 127.f ? 2 : 4);
     using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
     // BNSD is always fixed, interleaved always packed
-    static constexpr Kernel kForms[2][4] = {{mhaTcgen05Kernel<IL, BNSD, BNSD, false, false>, mhaTcgen05Kernel<IL, BNSD, BNSD, true, false>,
-                                                mhaTcgen05Kernel<IL, BNSD, BNSD, false, true>, mhaTcgen05Kernel<IL, BNSD, BNSD, true, true>},
-        {mhaTcgen05Kernel<IL, BNSD, !IL, false, false>, mhaTcgen05Kernel<IL, BNSD, !IL, true, false>, mhaTcgen05Kernel<IL, BNSD, !IL, false, true>,
-            mhaTcgen05Kernel<IL, BNSD, !IL, true, true>}};
-    static SmemOptIn optIn[2][4];
+    constexpr bool kPacked = BNSD, kFixed = !IL;
+    static constexpr Kernel kForms[2][6] = {
+        {mhaTcgen05Kernel<IL, BNSD, kPacked, false, false, false>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, false, false>,
+            mhaTcgen05Kernel<IL, BNSD, kPacked, false, true, false>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, true, false>,
+            mhaTcgen05Kernel<IL, BNSD, kPacked, false, true, true>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, true, true>},
+        {mhaTcgen05Kernel<IL, BNSD, kFixed, false, false, false>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, false, false>,
+            mhaTcgen05Kernel<IL, BNSD, kFixed, false, true, false>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, true, false>,
+            mhaTcgen05Kernel<IL, BNSD, kFixed, false, true, true>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, true, true>}};
+    static SmemOptIn optIn[2][6];
     int const fixed = args.fixedLayout ? 1 : 0;
     cudaError_t const e = launchDependentCluster(
         &optIn[fixed][form], kForms[fixed][form], dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);

@@ -157,6 +157,31 @@ def test_mha_int8_saturating_probabilities(cuda):
     _assert_int8_attention(out.cpu().numpy(), ref)
 
 
+# With four key blocks the clamp is part of the kernel's form: on both sides of 127, few pairs and more than SMs, packed and fixed
+@pytest.mark.parametrize("scale_softmax", [127.0, 200.0])
+@pytest.mark.parametrize("N", [3, 40])
+@pytest.mark.parametrize("packed", [True, False])
+def test_mha_int8_clamp_at_four_key_blocks(cuda, scale_softmax, N, packed):
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(N)
+    lengths, S, d = np.array([400, 3, 1, 130], dtype=np.int32), 400, 64   # short sequences have probabilities close to 1
+    cu = O.cu_seqlens(lengths)
+    q8, s_qkv = _int8_case(rng, int(cu[-1]) if packed else S * len(lengths), N, d)
+    s1, s2 = float(np.float32(s_qkv) * np.float32(s_qkv) * np.float32(0.125)), 0.4 / scale_softmax
+    st = _status(cuda)
+    scales = {"scale_bmm1": s1, "scale_softmax": scale_softmax, "scale_bmm2": s2, "status": st}
+    if packed:
+        ref = O.mha_int8(q8, len(lengths), S, N, d, s1, scale_softmax, s2, cu=cu)
+        out = T.mha(_t(q8, cuda), len(lengths), S, N, cu_seqlens=_t(cu, cuda), **scales)
+    else:
+        q8 = q8.reshape(S, len(lengths), -1)
+        ref = O.mha_int8(q8, len(lengths), S, N, d, s1, scale_softmax, s2, lengths=lengths)
+        out = T.mha(_t(q8, cuda), len(lengths), S, N, mask_idx=_t(lengths, cuda), **scales)
+    assert int(st[0]) == 0
+    _assert_int8_attention(out.cpu().numpy(), ref)
+
+
 @pytest.mark.parametrize("S,B,N", [(128, 4, 12), (384, 2, 16)])
 def test_mha_fixed_int8(cuda, S, B, N):
     import tensorrt_b200 as T
