@@ -521,7 +521,10 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                 promote(c - 2, summed);
                 // all its products are complete: so is what they read where this chunk's parts go
                 if (L::kHalves == 2 && part == 0 && !__all_sync(0xffffffffu, complete))
+                {
                     ok = ok && mbarWaitWarp(&done[kParts + s], parity, abortFlag, kWaitAccFull);
+                    tcFenceAfter(); // that of promote() came before this wait
+                }
             }
             if (!__all_sync(0xffffffffu, landed))
                 ok = ok && mbarWaitWarp(&stFull[stage], phase, abortFlag, kWaitTmaFull);

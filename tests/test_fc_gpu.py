@@ -313,6 +313,29 @@ def test_fc_fp32_sums_near_the_largest_numbers(cuda, m, k, n):
     assert torch.equal(out.double(), ref)
 
 
+# 96 and 128 columns: the products of a chunk are waited for in two halves, the second by warps that have read the sums of the first. Another stream keeps the
+# SMs busy beside them, so that the barriers are asked early and late
+@pytest.mark.parametrize("m,k,n", [(6339, 1540, 129), (2115, 3072, 97), (1024, 768, 2304)])
+def test_fc_fp32_halves_of_a_tile_beside_other_work(cuda, m, k, n):
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    x, y = torch.randn(512, 1024, device=cuda, generator=gen).half(), torch.randn(1024, 1024, device=cuda, generator=gen).half()
+    st = _status(cuda)
+    first = T.fc(a, w, status=st)
+    ref = a.double() @ w.double().T
+    assert float((first.double() - ref).norm()) <= 2.0 ** -22 * float(ref.norm())   # two units of the last place on average
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for _ in range(20):
+        with torch.cuda.stream(side):
+            T.fc(x, y)
+        assert torch.equal(T.fc(a, w, status=st), first)
+    torch.cuda.synchronize()
+    assert int(st[0]) == 0
+
+
 # each width of the tiles, with all segments of K (two, four, eight) in a CTA and with one each, as fcF32 chooses them on 148 SMs; rows, columns and K that
 # fill neither a tile nor a chunk
 @pytest.mark.parametrize("m,k,n", [
