@@ -56,6 +56,10 @@ struct FcF32Smem
     static constexpr int kBarrierOff = kPlanesOff + kParts * 3 * kPlaneBytes;
     static constexpr int kAccs = BN <= 64 ? 2 : 1;      // chunks whose sums are in tensor memory, two accumulators each
     static constexpr int kHalves = kAccs == 1 ? 2 : 1; // of the columns, whose products are formed one after the other
+    // Groups of warps that take chunks in turn. 32 columns: eight warps cut a chunk as fast as 16 (Wt has 32 rows, eight warps' work), and with the other
+    // eight a chunk ahead the sums wait less: 512 x 1024 x 4096 53.8 us (all 16: 58.5 us), 129 x 2304 x 768 13.8 us (14.4 us).
+    static constexpr int kTurns = BN == 32 ? 2 : 1;
+    static constexpr int kCutters = kWorkers / kTurns; // warps that cut a chunk
     // stFull[stages] stFree[2][stages] ready[parts] done[halves][parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
     // whether any is set
     static constexpr int kFlagsOff = kBarrierOff + (3 * kStages + (1 + kHalves) * kParts + 2) * 8 + 16;
@@ -258,7 +262,7 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
 // Bound by the warps that cut operands, and by shared memory behind them: a chunk of a 128 x 128 tile takes 2900 cycles, of which the
 // tensor cores are busy 1750 and shared memory 2240 (tiles written and read, parts of Wt written and read by 26 products), of a 64-wide one 1870
 // (830, 1380). The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are
-// multiplied in two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk (with two groups
+// multiplied in two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk beyond 32 columns (with two groups
 // taking chunks in turn the sums waited for the group that was cutting); a chunk's three barriers are asked at once (an answer takes 120 ... 150
 // cycles); and a tile's place in the ring is handed back as soon as its numbers are in registers. Before / after: 3400 / 2900 cycles
 // per chunk; 1024 x 2304 x 768 32.7 / 28.3 us, 2000 x 3072 x 1024 113.1 / 98.7 us, 4096 x 3072 x 1024 210.9 / 195.4 us, 37 x 2304 x 768 11.1 / 10.6 us.
@@ -267,8 +271,8 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
 //   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
 //   warp 1    : TMEM allocation, MMA issue. The parts of A are operands in TMEM - from shared memory both operands of a
 //               128 x 128 tile would take its whole bandwidth -, those of Wt in shared memory.
-//   warps 2-17: the parts of every chunk: 16 numbers of a row of A per thread, to TMEM, and whole 16-byte pieces of the parts of
-//               Wt, to shared memory. And its sums (32 rows, a quarter of the columns per warp) from TMEM into registers. Parts are
+//   warps 2-17: the parts of every chunk (32 columns: two groups of eight, chunks in turn): 16 numbers of a row of A per thread, to TMEM, and whole
+//               16-byte pieces of the parts of Wt, to shared memory. And its sums (32 rows, a quarter of the columns per warp) from TMEM into registers. Parts are
 //               double-buffered, the two accumulators too where tensor memory has room (up to 64 columns).
 // K is cut into segments by K alone and the segments' sums are added in order, so a row has the same bits whatever M: a CTA takes
 // all segments in turn (kHold), or a cluster one per CTA, exchanging the sums through distributed shared memory.
@@ -317,11 +321,11 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int i = 0; i < L::kStages; ++i)
         {
             mbarInit(&stFull[i], 1);
-            mbarInit(&stFree[i], kWorkers);               // A
-            mbarInit(&stFree[L::kStages + i], kWorkers); // Wt
+            mbarInit(&stFree[i], L::kCutters);               // A
+            mbarInit(&stFree[L::kStages + i], L::kCutters); // Wt
         }
         for (int i = 0; i < kParts; ++i)
-            mbarInit(&ready[i], kWorkers);
+            mbarInit(&ready[i], L::kCutters);
         for (int i = 0; i < L::kHalves * kParts; ++i)
             mbarInit(&done[i], 1);
         for (int i = 0; i < 2; ++i)
@@ -387,11 +391,15 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         {
             uint32_t const s = c & 1, round = c >> 1;
             uint32_t const slot = c % L::kAccs;
-            ok = mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
+            // What is there first is asked first, so that an answer is not waited for when the last one has come: two accumulators have been read before
+            // a chunk's parts are ready, a single one after it (512 x 1024 x 4096, 32 columns: the other way round 55.2 us).
+            bool const freeFirst = L::kAccs == 2 && c >= L::kAccs;
+            ok = (!freeFirst || mbarWaitWarp(&accFree[slot], (c / L::kAccs - 1) & 1u, abortFlag, kWaitAccFree))
+                && mbarWaitWarp(&ready[s], round & 1u, abortFlag, kWaitSoftmax);
 #pragma unroll
             for (int h = 0; h < L::kHalves; ++h)
             {
-                ok = ok && (c < L::kAccs || mbarWaitWarp(&accFree[slot + h], (c / L::kAccs - 1) & 1u, abortFlag, kWaitAccFree));
+                ok = ok && (L::kAccs == 2 || c == 0 || mbarWaitWarp(&accFree[h], (c - 1) & 1u, abortFlag, kWaitAccFree));
                 tcFenceAfter();
                 if (ok && electOne())
                 {
@@ -421,9 +429,9 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     else
     {
         int const quad = warp & 3;
-        int const group = (warp - 2) >> 3; // takes every second 32 rows of Wt
+        int const group = (warp - 2) >> 3; // takes every second 32 rows of Wt (32 columns: every second chunk)
         int const w = (warp - 2) & 7;      // which 8 of a chunk's K of Wt
-        int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns, and which 16 of a chunk's K of A
+        int const cols = (warp - 2) >> 2;  // which quarter of the accumulator columns, and which 16 of a chunk's K of A (32 columns: two of these)
         int const part = L::kHalves == 2 ? group : 0;
         bool const hasRows = m0 + quad * 32 < p.M; // warp-uniform; products of the other rows are never read
         uint32_t const tRow = tmemBase + (static_cast<uint32_t>(quad * 32) << 16);
@@ -511,8 +519,9 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int c = 0; c < count; ++c)
         {
             uint32_t const s = c & 1;
+            bool const cuts = L::kTurns == 1 || static_cast<int>(s) == group;
             // A barrier answers after 120 ... 150 cycles: all are asked at once.
-            bool const landed = mbarTestAddr(smemAddr(&stFull[stage]), phase);
+            bool const landed = !cuts || mbarTestAddr(smemAddr(&stFull[stage]), phase);
             if (c >= 2)
             {
                 uint32_t const parity = ((c - 2) >> 1) & 1u;
@@ -526,69 +535,80 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     tcFenceAfter(); // that of promote() came before this wait
                 }
             }
-            if (!__all_sync(0xffffffffu, landed))
-                ok = ok && mbarWaitWarp(&stFull[stage], phase, abortFlag, kWaitTmaFull);
-            uint8_t const* const fp = smem + stage * L::kStageBytes;
-            if (hasRows)
+            if (cuts)
             {
-                int const row = quad * 32 + lane;
-                float4 const* const src = reinterpret_cast<float4 const*>(fp + (cols >> 1) * (L::kABytes / 2) + row * 128);
-                uint32_t const t = tRow + kPartsCol + s * 96 + cols * 8;
-                uint32_t lost = 0;
-                float4 v[4];
+                if (!__all_sync(0xffffffffu, landed))
+                    ok = ok && mbarWaitWarp(&stFull[stage], phase, abortFlag, kWaitTmaFull);
+                uint8_t const* const fp = smem + stage * L::kStageBytes;
+                if (hasRows)
+                {
+                    int const row = quad * 32 + lane;
+                    uint32_t lost = 0;
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    v[i] = src[((cols & 1) * 4 + i) ^ (row & 7)];
+                    for (int g = 0; g < L::kTurns; ++g)
+                    {
+                        int const at = L::kTurns == 1 ? cols : 2 * (w >> 2) + g; // which 16 of the chunk's K
+                        float4 const* const src = reinterpret_cast<float4 const*>(fp + (at >> 1) * (L::kABytes / 2) + row * 128);
+                        uint32_t const t = tRow + kPartsCol + s * 96 + at * 8;
+                        float4 v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            v[i] = src[((at & 1) * 4 + i) ^ (row & 7)];
+                        if (g == L::kTurns - 1)
+                        {
+                            __syncwarp();
+                            if (lane == 0)
+                                mbarArrive(&stFree[stage]);
+                        }
+                        uint32_t h[8], m[8], l[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                        {
+                            splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], lost);
+                            splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], lost);
+                        }
+                        tmemStore8(t, h);
+                        tmemStore8(t + 32, m);
+                        tmemStore8(t + 64, l);
+                    }
+                    if ((lost & 0xffffu) != 0)
+                        flagA[row] = *flagAny = 1;
+                }
+                else if (lane == 0)
+                    mbarArrive(&stFree[stage]);
+                // eight numbers of a row of Wt: 16 bytes of each part; an odd number of 32 rows is dealt to the groups by turns
+                uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
+#pragma unroll
+                for (int i = 0; i < (BN + 32) / 64; ++i)
+                {
+                    int const block = L::kTurns == 2 ? 0 : 2 * i + (BN % 64 == 0 ? group : (group + c) & 1);
+                    if (BN % 64 != 0 && block >= BN / 32)
+                        break;
+                    int const row = block * 32 + lane;
+                    float4 const* const src = reinterpret_cast<float4 const*>(fp + L::kABytes + (w >> 2) * (L::kWBytes / 2) + row * 128);
+                    float4 const v0 = src[(2 * (w & 3)) ^ (row & 7)], v1 = src[(2 * (w & 3) + 1) ^ (row & 7)];
+                    uint4 h, m, l;
+                    uint32_t lost = 0;
+                    splitPair(v0.x, v0.y, h.x, m.x, l.x, lost);
+                    splitPair(v0.z, v0.w, h.y, m.y, l.y, lost);
+                    splitPair(v1.x, v1.y, h.z, m.z, l.z, lost);
+                    splitPair(v1.z, v1.w, h.w, m.w, l.w, lost);
+                    uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
+                    *reinterpret_cast<uint4*>(dst) = h;
+                    *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
+                    *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
+                    if ((lost & 0xffffu) != 0)
+                        flagW[row] = *flagAny = 1;
+                }
+                fenceProxyAsync();
+                tmemStoreWait();
+                tcFenceBefore();
                 __syncwarp();
                 if (lane == 0)
-                    mbarArrive(&stFree[stage]);
-                uint32_t h[8], m[8], l[8];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
                 {
-                    splitPair(v[i].x, v[i].y, h[2 * i], m[2 * i], l[2 * i], lost);
-                    splitPair(v[i].z, v[i].w, h[2 * i + 1], m[2 * i + 1], l[2 * i + 1], lost);
+                    mbarArrive(&ready[s]);
+                    mbarArrive(&stFree[L::kStages + stage]);
                 }
-                tmemStore8(t, h);
-                tmemStore8(t + 32, m);
-                tmemStore8(t + 64, l);
-                if ((lost & 0xffffu) != 0)
-                    flagA[row] = *flagAny = 1;
-            }
-            else if (lane == 0)
-                mbarArrive(&stFree[stage]);
-            // eight numbers of a row of Wt: 16 bytes of each part; an odd number of 32 rows is dealt to the groups by turns
-            uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
-#pragma unroll
-            for (int i = 0; i < (BN + 32) / 64; ++i)
-            {
-                int const block = 2 * i + (BN % 64 == 0 ? group : (group + c) & 1);
-                if (BN % 64 != 0 && block >= BN / 32)
-                    break;
-                int const row = block * 32 + lane;
-                float4 const* const src = reinterpret_cast<float4 const*>(fp + L::kABytes + (w >> 2) * (L::kWBytes / 2) + row * 128);
-                float4 const v0 = src[(2 * (w & 3)) ^ (row & 7)], v1 = src[(2 * (w & 3) + 1) ^ (row & 7)];
-                uint4 h, m, l;
-                uint32_t lost = 0;
-                splitPair(v0.x, v0.y, h.x, m.x, l.x, lost);
-                splitPair(v0.z, v0.w, h.y, m.y, l.y, lost);
-                splitPair(v1.x, v1.y, h.z, m.z, l.z, lost);
-                splitPair(v1.z, v1.w, h.w, m.w, l.w, lost);
-                uint8_t* const dst = planes + row * 128 + ((w ^ (row & 7)) << 4);
-                *reinterpret_cast<uint4*>(dst) = h;
-                *reinterpret_cast<uint4*>(dst + L::kPlaneBytes) = m;
-                *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneBytes) = l;
-                if ((lost & 0xffffu) != 0)
-                    flagW[row] = *flagAny = 1;
-            }
-            fenceProxyAsync();
-            tmemStoreWait();
-            tcFenceBefore();
-            __syncwarp();
-            if (lane == 0)
-            {
-                mbarArrive(&ready[s]);
-                mbarArrive(&stFree[L::kStages + stage]);
             }
             if (++stage == L::kStages)
             {
