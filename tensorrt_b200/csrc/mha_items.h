@@ -25,7 +25,7 @@ struct ItemPlan
 // when that shortens the longest CTA's list. Measured (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
 // us), 4 x 256 6.5 us (10.2 us), 12 x 384 22.5 us (31.8 us); 8 x 384 whole, 16.7 us.
 // The lengths are on the device; what the host knows is how many tokens the batch has less than B * S (`missing`; INT64_MAX: unknown).
-// With no more pairs than CTAs a cut is never the longer way, whatever they are. With more, pairs are cut only when every sequence is
+// With no more pairs than CTAs a cut into equal items is never the longer way, whatever they are. With more, pairs are cut only when every sequence is
 // known to have the same number of tiles: whether halves or whole pairs even out better depends on where the long ones lie. Ragged
 // batches keep whole pairs, and every CTA puts the sequences in the order of their lengths first (0.3 us) and takes a long pair, then a
 // short one. Measured, packed, longest first / halves as they come / whole pairs as they come: 14 sequences of 87 ... 338 tokens, 12
@@ -58,11 +58,12 @@ inline ItemPlan planItems(int32_t B, int32_t N, int32_t S, int64_t missing, int6
 
 // Ragged packed batches of no more pairs than CTAs, which planItems leaves whole because full sequences would be: their tiles, one by one, in the order
 // of the sequences' lengths. The longest pair then no longer holds up the launch, at the price of K and V for each tile. In the units above a tile
-// costs up to four per key block and a whole pair 3 tiles + 1, so the cut is shorter while the rounds of tiles are fewer than that over four. How
-// many tiles there are follows from the tokens, taking half a tile per sequence for its last one and a sixteenth on top. Over 40 000 random batches of this
-// model the cut is never longer, and half as long on average. Measured (whole pairs in brackets): 8 sequences of 90 ... 384 tokens, 16 heads 12.3 us
-// (16.0 us), 12 of 32 ... 384, 12 heads 12.5 us
-// (15.9 us).
+// costs up to four per key block and a whole pair 3 tiles + 1, so the cut is shorter while the rounds of tiles are fewer than that over four.
+// The host knows the tokens only and guesses, half a tile per sequence for its last one and a sixteenth on top, whether that can be; then the CTAs, which
+// read the lengths anyway, count the tiles and decide (cutIsShorter). The cut alone by the guess was up to 1.2 times as long (lengths just beyond a multiple
+// of 128), and wherever S is far above the lengths. Measured (whole pairs / cut by the guess / as it is): 8 sequences of 90 ... 384 tokens, 16 heads
+// 16.9 / 11.7 / 11.9 us, 12 of 32 ... 384, 12 heads 16.9 / 12.1 / 12.1 us; 5 of 133 ... 160, 16 heads 9.8 / 10.2 / 9.7 us (in the form of the kernel that
+// always keeps them whole 9.3 us), 92 of 129, one of 256, one head 9.9 / 15.8 / 9.7 us, 12 of up to 128 with S = 512, 12 heads 5.2 / 6.3 / 5.7 us.
 // Returns the most tiles that there can be, or 0: not cut. tokens: of the batch.
 inline int64_t cutTiles(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t ctas)
 {
@@ -72,6 +73,13 @@ inline int64_t cutTiles(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t
     int64_t const about = N * (tokens / kItemTile + (B + 1) / 2), rounds = (about + about / 16 + ctas - 1) / ctas;
     int64_t const most = N * (tokens / kItemTile + B);
     return 4 * rounds < 3 * nq + 1 && most <= kItemRounds * ctas ? (most < pairs * nq ? most : pairs * nq) : 0;
+}
+
+// Whether `tiles` tiles, dealt one by one to `ctas` CTAs, are shorter than whole pairs, one to a CTA: 4 * rounds < 3 * longest + 1, so at most
+// 3 / 4 * longest rounds. longest: tiles of the longest sequence.
+B200_HOST_DEVICE inline bool cutIsShorter(int32_t tiles, int32_t longest, int32_t ctas)
+{
+    return tiles <= 3 * longest / 4 * ctas;
 }
 
 // The item that CTA `cta` takes in its `round`-th turn, the items being in the order of their lengths: every second round runs

@@ -72,14 +72,14 @@ struct MhaArgs
     float scaleBmm1, scaleSoftmax, scaleBmm2;
     uint32_t* statusWord;
     int32_t tilesPerItem, chunks; // a work item = (sequence, head, chunk of tilesPerItem query tiles)
-    int32_t rounds, cut;          // ORDERED: items per CTA; whether they are tiles, not pairs
+    int32_t rounds, cut;          // ORDERED: items per CTA (at most); whether they are tiles, not pairs, where that is shorter
 };
 
 // Sequences by length and the items of a CTA (ORDERED, see the kernel).
 struct alignas(1024) ItemTable
 {
     int4 ordered[kItemOrder]; // number, first row, length
-    int4 items[kItemRounds];  // sequence (-1: none), head and first tile (above 16 bits), first row, length
+    int4 items[kItemRounds];  // sequence (-1: none), head | first tile << 16 | tiles (at most) << 24, first row, length
     int32_t lengths[kItemOrder];
 };
 
@@ -164,11 +164,99 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, uint32_t const (&r)[
         : "memory");
 }
 
+// First row and valid keys of sequence b.
+template <bool FIXED>
+__device__ __forceinline__ void sequenceOf(
+    int32_t const S, int32_t const* __restrict__ cu, int32_t const* __restrict__ maskIdx, int const b, int32_t& rowBase, int32_t& len)
+{
+    if (FIXED)
+    {
+        rowBase = 0;
+        len = maskIdx ? min(max(__ldg(maskIdx + b), 0), S) : S;
+    }
+    else
+    {
+        rowBase = __ldg(cu + b);
+        len = min(max(__ldg(cu + b + 1) - rowBase, 0), S);
+    }
+}
+
+// The sequences in the order of their lengths, by the first kItemOrder threads, each with one of them (len -1: beyond the batch); lengths are in place.
+__device__ __forceinline__ void orderSequences(ItemTable* const table, int32_t const B, int const b, int32_t const rowBase, int32_t const len)
+{
+    // a sequence's place is the number of longer ones, and of equal ones before it
+    if (b < B)
+    {
+        int place = 0;
+        for (int u = 0; u < B; u += 4)
+        {
+            int4 const v = *reinterpret_cast<int4 const*>(table->lengths + u);
+            place += (v.x > len || (v.x == len && u < b)) + (v.y > len || (v.y == len && u + 1 < b))
+                + (v.z > len || (v.z == len && u + 2 < b)) + (v.w > len || (v.w == len && u + 3 < b));
+        }
+        table->ordered[place] = make_int4(b, rowBase, len, 0);
+    }
+    asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
+}
+
+// Items of this CTA where pairs may be cut into tiles (packed layout), by the first kItemOrder threads. Not inlined: in the way of those that are not
+// (instruction fetch), it costs each launch that deals whole pairs 0.2 us.
+__device__ __noinline__ void listTiles(ItemTable* const table, int32_t const B, int32_t const S, int32_t const N, int32_t const* const cu, int32_t const rounds)
+{
+    int const b = static_cast<int>(threadIdx.x), warp = b >> 5, lane = b & 31;
+    int32_t rowBase = 0, len = -1;
+    if (b < B)
+        sequenceOf<false>(S, cu, nullptr, b, rowBase, len);
+    table->lengths[b] = len;
+    // tiles of the batch and of its longest sequence; the warps' sums go where so few rounds list no item
+    unsigned const tiles = (max(len, 0) + kQTile - 1) / kQTile;
+    int sum = static_cast<int>(__reduce_add_sync(0xffffffffu, tiles)), most = static_cast<int>(__reduce_max_sync(0xffffffffu, tiles));
+    if (lane == 0)
+        table->items[kItemRounds - 1 - warp] = make_int4(sum, most, 0, 0);
+    asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
+    sum = 0;
+    for (int w = 0; w * 32 < B; ++w)
+    {
+        int4 const v = table->items[kItemRounds - 1 - w];
+        sum += v.x;
+        most = max(most, v.y);
+    }
+    if (!cutIsShorter(sum * N, most, static_cast<int>(gridDim.x))) // a pair per CTA, as they come
+    {
+        int const pair = static_cast<int>(blockIdx.x);
+        bool const one = pair < B * N;
+        if (b >= (one ? 1 : 0) && b < rounds)
+            table->items[b] = make_int4(-1, 0, 0, 0);
+        if (one && b == pair / N)
+            table->items[0] = make_int4(b, pair % N | kMaxBlocks << 24, rowBase, len);
+        return;
+    }
+    orderSequences(table, B, b, rowBase, len);
+    if (b < rounds)
+    {
+        int left = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)); // a longer sequence has more tiles
+        int4 q = make_int4(-1, 0, 0, 0);
+        for (int place = 0; place < B; ++place)
+        {
+            int4 const o = table->ordered[place];
+            int const ofPair = (o.z + kQTile - 1) / kQTile;
+            if (left < ofPair * N)
+            {
+                int const head = left / ofPair;
+                q = make_int4(o.x, head | (left - head * ofPair) << 16 | 1 << 24, o.y, o.z);
+                break;
+            }
+            left -= ofPair * N;
+        }
+        table->items[b] = q;
+    }
+}
+
 // IL: CHW32-interleaved tensors. Q, K and V tiles then arrive as two 32-channel sub-tiles of
 // [128 tokens][32 B] (32-byte swizzle); the head dimension is covered by one MMA per sub-tile.
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
-// ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h).
+// ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items, pairs or tiles (see mha_items.h).
 // FIXED: the fixed layout (or separate tensors), not the packed one.
 // FOUR: the longest sequence has four key blocks, not up to three. The context accumulator then has to share TMEM columns with the scores of key block 0, and four
 // blocks of P share two slots.
@@ -200,7 +288,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
         smem += sizeof(ItemTable);
 
     // ---- work items: some or all query tiles of a (sequence, head), item = (b * N + head) * chunks + chunk, dealt round-robin
-    //      to the persistent CTAs; or whole (sequence, head) pairs as the CTA has listed them ----
+    //      to the persistent CTAs; or whole (sequence, head) pairs, or single tiles, as the CTA has listed them ----
     struct Item
     {
         int32_t b, head, rowBase, rows, len, nb, tBegin, tEnd;
@@ -208,31 +296,21 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
     int const numItems = ORDERED ? args.rounds : args.B * args.N * args.chunks;
     int const firstItem = ORDERED ? 0 : static_cast<int>(blockIdx.x);
     int const itemStep = ORDERED ? 1 : static_cast<int>(gridDim.x);
-    // first row and valid keys of sequence b
-    auto sequence = [&](int b, int32_t& rowBase, int32_t& len) {
-        if (FIXED)
-        {
-            rowBase = 0;
-            len = args.maskIdx ? min(max(__ldg(args.maskIdx + b), 0), args.S) : args.S;
-        }
-        else
-        {
-            rowBase = __ldg(args.cu + b);
-            len = min(max(__ldg(args.cu + b + 1) - rowBase, 0), args.S);
-        }
-    };
+    auto sequence = [&](int b, int32_t& rowBase, int32_t& len) { sequenceOf<FIXED>(args.S, args.cu, args.maskIdx, b, rowBase, len); };
     // Geometry of item i (uniform over the CTA; every role derives the same values). Returns whether the item has
     // work for the tensor pipeline (at least one query row and one valid key).
     auto getItem = [&](int i, Item& it) -> bool {
+        int tiles = args.tilesPerItem;
         if (ORDERED)
         {
             int4 const q = table->items[i];
             it.b = q.x;
             it.head = q.y & 0xffff;
+            it.tBegin = q.y >> 16 & 0xff;
+            tiles = q.y >> 24;
             it.rowBase = q.z;
             it.len = q.w;
             it.rows = FIXED && q.x >= 0 ? args.S : it.len;
-            it.tBegin = q.y >> 16;
         }
         else
         {
@@ -244,7 +322,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             it.rows = FIXED ? args.S : it.len;
         }
         it.nb = (it.len + kKeyBlock - 1) / kKeyBlock; // key blocks
-        it.tEnd = min((it.rows + kQTile - 1) / kQTile, it.tBegin + args.tilesPerItem);
+        it.tEnd = min((it.rows + kQTile - 1) / kQTile, it.tBegin + tiles);
         return it.len > 0 && it.tBegin < it.tEnd;
     };
     // first item >= i of this CTA's sequence that has pipeline work; numItems or more if there is none
@@ -320,51 +398,25 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
 
     if (ORDERED)
     {
-        // a sequence's place is the number of longer ones, and of equal ones before it (those beyond the batch count as -1)
         int const b = static_cast<int>(threadIdx.x);
-        if (b < kItemOrder)
+        if (!FIXED && args.cut && b < kItemOrder)
+            listTiles(table, args.B, args.S, args.N, args.cu, args.rounds);
+        else if (b < kItemOrder)
         {
             int32_t rowBase = 0, len = -1;
             if (b < args.B)
                 sequence(b, rowBase, len);
             table->lengths[b] = len;
             asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
-            if (b < args.B)
-            {
-                int place = 0;
-                for (int u = 0; u < args.B; u += 4)
-                {
-                    int4 const v = *reinterpret_cast<int4 const*>(table->lengths + u);
-                    place += (v.x > len || (v.x == len && u < b)) + (v.y > len || (v.y == len && u + 1 < b))
-                        + (v.z > len || (v.z == len && u + 2 < b)) + (v.w > len || (v.w == len && u + 3 < b));
-                }
-                table->ordered[place] = make_int4(b, rowBase, len, 0);
-            }
-            asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
+            orderSequences(table, args.B, b, rowBase, len);
             if (b < args.rounds)
             {
-                int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+                int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)), place = item / args.N;
                 int4 q = make_int4(-1, 0, 0, 0);
-                if (args.cut) // the tiles of a pair one by one: a longer sequence has more of them
+                if (place < args.B)
                 {
-                    int left = item;
-                    for (int place = 0; place < args.B; ++place)
-                    {
-                        int4 const o = table->ordered[place];
-                        int const tiles = (o.z + kQTile - 1) / kQTile;
-                        if (left < tiles * args.N)
-                        {
-                            int const head = left / tiles;
-                            q = make_int4(o.x, head | (left - head * tiles) << 16, o.y, o.z);
-                            break;
-                        }
-                        left -= tiles * args.N;
-                    }
-                }
-                else if (item / args.N < args.B)
-                {
-                    int4 const o = table->ordered[item / args.N];
-                    q = make_int4(o.x, item % args.N, o.y, o.z);
+                    int4 const o = table->ordered[place];
+                    q = make_int4(o.x, (item - place * args.N) | kMaxBlocks << 24, o.y, o.z);
                 }
                 table->items[b] = q;
             }
@@ -469,7 +521,7 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
             uint32_t qkTiles = 0;  // tiles whose scores have been issued
             uint32_t pvTiles = 0;  // tiles of this CTA that the loop below has passed (= whose context has been issued)
             uint32_t kBits = 0, vBits = 0, pBits = 0, fBits = 0; // parity per key block: K landed, V landed, P written, S read
-            // scores of key block j for the query tile whose Q is in shared memory; nbOf = key blocks of that tile's item
+            // scores of key block j for the query tile whose Q is in shared memory; last: of that tile's, Q is free after them
             auto issueScores = [&](int j, bool last) {
                 if (electOne())
                 {
@@ -1220,12 +1272,12 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     ItemPlan const plan = planItems(args.B, args.N, args.S, missing, smCount());
     int64_t const cut = args.fixedLayout || plan.chunks > 1 ? 0 : cutTiles(args.B, args.N, args.S, args.total, smCount());
     args.cut = cut > 0 ? 1 : 0;
-    args.tilesPerItem = cut > 0 ? 1 : plan.tilesPerItem;
+    args.tilesPerItem = plan.tilesPerItem;
     args.chunks = plan.chunks;
     int64_t const items = cut > 0 ? cut : static_cast<int64_t>(args.B) * args.N * plan.chunks;
     bool const ordered = plan.longestFirst || cut > 0;
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
-    args.rounds = static_cast<int32_t>((items + grid - 1) / grid);
+    args.rounds = cut > 0 ? 3 * plan.tilesPerItem / 4 : static_cast<int32_t>((items + grid - 1) / grid); // cut: see cutIsShorter
     int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (ordered ? static_cast<int>(sizeof(ItemTable)) : 0);
     int const form = (ordered ? 1 : 0) + (args.S <= 3 * kKeyBlock ? 0 : args.scaleSoftmax <= 127.f ? 2 : 4);
     using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);

@@ -687,14 +687,17 @@ def test_mha_fp16_short_kernel_residency(cuda, B):
     assert int(st[0]) == 0 and torch.equal(short, persistent)
 
 
-# Few ragged sequences, whose tiles are dealt one by one: as many pairs as SMs, empty sequences, lengths at the edges of tiles, one long one
-@pytest.mark.parametrize("lengths,N", [([384, 97, 279, 90, 195, 241, 267, 119], 16), ([1, 0, 512, 129, 128, 127, 257, 0, 385], 16), ([300, 1, 1], 37),
-                                       ([0, 500, 3], 49), ([511, 384, 256, 255, 40], 12), ([260] + [16] * 147, 1)])
+# Few ragged sequences, whose tiles are dealt one by one: as many pairs as SMs, empty sequences, lengths at the edges of tiles, one long one. Then such as
+# the host takes for shorter when cut, but the CTAs, counting tiles, keep whole: lengths just beyond a tile, S far above the lengths
+@pytest.mark.parametrize("lengths,N,S", [([384, 97, 279, 90, 195, 241, 267, 119], 16, 384), ([1, 0, 512, 129, 128, 127, 257, 0, 385], 16, 512), ([300, 1, 1], 37, 300),
+                                         ([0, 500, 3], 49, 500), ([511, 384, 256, 255, 40], 12, 511), ([260] + [16] * 147, 1, 260),
+                                         ([160, 153, 160, 133, 160], 16, 160), ([130] + [129] * 6, 12, 130), ([256] + [129] * 91, 1, 256),
+                                         ([128] + [100] * 11, 12, 512), ([0, 0, 1, 0], 12, 400), ([300, 5, 260, 129], 37, 512)])
 @pytest.mark.parametrize("interleaved", [False, True])
-def test_mha_int8_few_ragged_pairs(cuda, lengths, N, interleaved):
+def test_mha_int8_few_ragged_pairs(cuda, lengths, N, S, interleaved):
     import tensorrt_b200 as T
 
-    d, B, smax = 32, len(lengths), max(lengths)
+    d, B, smax = 32, len(lengths), S
     cu = O.cu_seqlens(np.array(lengths, dtype=np.int32))
     x = np.random.default_rng(N).integers(-127, 128, size=(int(cu[-1]), 3 * N * d)).astype(np.int8)
     s1, s2 = float((4.0 / 127) ** 2 / np.sqrt(d)), 2.0 / 127

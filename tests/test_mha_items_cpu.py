@@ -20,6 +20,7 @@ def lib(tmp_path_factory):
                                  'extern "C" void plan(int32_t B, int32_t N, int32_t S, int64_t missing, int64_t ctas, int32_t* out)'
                                  "{ auto p = b200::planItems(B, N, S, missing, ctas); out[0] = p.tilesPerItem; out[1] = p.chunks; out[2] = p.longestFirst; }\n"
                                  'extern "C" int64_t cut(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t ctas) { return b200::cutTiles(B, N, S, tokens, ctas); }\n'
+                                 'extern "C" int32_t shorter(int32_t tiles, int32_t longest, int32_t ctas) { return b200::cutIsShorter(tiles, longest, ctas); }\n'
                                  'extern "C" int32_t item(int32_t round, int32_t cta, int32_t ctas) { return b200::itemOfRound(round, cta, ctas); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", str(d / "items.cpp"), "-o", str(d / "items.so")], check=True)
     so = ctypes.CDLL(str(d / "items.so"))
@@ -73,33 +74,61 @@ def test_ragged_batches_are_not_slower_than_whole_pairs_as_they_come(lib, heads,
     assert sum(ratio) / len(ratio) < 0.9
 
 
+def _cut(lib, heads, s, lengths):
+    """Units of the longest CTA's list over those of whole pairs: of the tiles as the CTAs deal them, 1 where they decide on whole pairs, None where the host does."""
+    b = len(lengths)
+    most = lib.cut(b, heads, s, ctypes.c_int64(sum(lengths)), ctypes.c_int64(CTAS))
+    if most == 0 or _plan(lib, b, heads, s, b * s - sum(lengths))[1] > 1:
+        return None
+    blocks = sorted((-(-n // TILE) for n in lengths), reverse=True)
+    tiles = [4 * n for n in blocks for _ in range(heads * n)]
+    ctas = min(CTAS, most)
+    assert len(tiles) <= most and b * heads <= ctas   # a CTA for each pair, should they stay whole
+    if not lib.shorter(len(tiles), blocks[0], ctas):
+        return 1.0
+    rounds = -(-len(tiles) // ctas)
+    assert rounds <= 3 * -(-s // TILE) // 4           # what the launch has room for
+    load, seen = [0] * ctas, set()
+    for r in range(rounds):
+        for cta in range(ctas):
+            i = lib.item(r, cta, ctas)
+            seen.add(i)
+            load[cta] += tiles[i] if i < len(tiles) else 0
+    assert seen >= set(range(len(tiles)))
+    return max(load) / max((3 * n + 1) * n for n in blocks)
+
+
 @pytest.mark.parametrize("heads", [1, 12, 16])
-def test_few_ragged_pairs_are_cut_into_tiles_where_that_is_shorter(lib, heads):
+@pytest.mark.parametrize("seed", range(4))
+def test_few_ragged_pairs_are_cut_into_tiles_where_that_is_shorter(lib, heads, seed):
     """Tiles dealt longest first against whole pairs: never a longer list, all tiles inside the bound that the launch is made for."""
-    rng = random.Random(heads)
+    rng = random.Random(100 * seed + heads)
     ratio = []
     for _ in range(3000):
-        s, b = rng.randint(1, 512), rng.randint(1, CTAS // heads)
+        s, b = rng.randint(129, 512), rng.randint(1, CTAS // heads)
         lengths = [rng.randint(s // rng.choice([1, 2, 4, 12]), s) for _ in range(b)]
         lengths[rng.randrange(b)] = s
-        most = lib.cut(b, heads, s, ctypes.c_int64(sum(lengths)), ctypes.c_int64(CTAS))
-        if most == 0 or _plan(lib, b, heads, s, b * s - sum(lengths))[1] > 1:
-            continue
-        blocks = sorted((-(-n // TILE) for n in lengths), reverse=True)
-        tiles = [4 * n for n in blocks for _ in range(heads * n)]
-        assert len(tiles) <= most <= 64 * CTAS
-        ctas = min(CTAS, most)
-        load = [0] * ctas
-        seen = set()
-        for r in range(-(-most // ctas)):
-            for cta in range(ctas):
-                i = lib.item(r, cta, ctas)
-                seen.add(i)
-                load[cta] += tiles[i] if i < len(tiles) else 0
-        assert seen >= set(range(len(tiles)))
-        ratio.append(max(load) / max((3 * n + 1) * n for n in blocks))
-    assert not ratio or (max(ratio) <= 1.0 and sum(ratio) / len(ratio) < 0.75), max(ratio)
-    assert ratio or heads == 1
+        ratio.append(_cut(lib, heads, s, lengths))
+    ratio = [r for r in ratio if r is not None]
+    assert len(ratio) > 100 and max(ratio) <= 1.0 and sum(ratio) / len(ratio) < 0.8, (len(ratio), max(ratio), sum(ratio) / len(ratio))
+
+
+@pytest.mark.parametrize("heads", [1, 12, 16])
+def test_lengths_just_beyond_a_tile_are_not_cut_where_that_is_longer(lib, heads):
+    """Lengths at the edges of tiles, S up to 512 above them: the host guesses that a cut is shorter, the CTAs count."""
+    kept = 0
+    for s in (130, 200, 256, 257, 300, 385, 400, 512):
+        for b in range(1, CTAS // heads + 1):
+            for n in (1, 2, 128, 129, 130, 133, 160, 256, 257, 273, 384, 385):
+                for first in {s, n, 1}:
+                    if max(n, first) <= s:
+                        r = _cut(lib, heads, s, [first] + [n] * (b - 1))
+                        assert r is None or r <= 1.0, (s, b, n, first)
+                        kept += r == 1.0
+    assert kept > 100
+    for s, lengths, h in [(160, [160, 153, 160, 133, 160], 16), (130, [130] + [129] * 6, 12), (256, [256] + [129] * 91, 1),
+                          (273, [257, 273, 260, 259, 257, 270, 265, 261, 258, 1], 12), (512, [128] + [100] * 11, 12)]:
+        assert _cut(lib, h, s, lengths) == 1.0   # the guess alone cuts these
 
 
 def test_equal_lengths_are_cut_where_that_is_shorter(lib):
