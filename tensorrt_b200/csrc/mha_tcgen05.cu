@@ -637,7 +637,9 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
                     }
                     if (kDoScores && ok)
                     {
-                        // key blocks the next item has beyond this one's: their score columns are idle
+                        // key blocks the next item has beyond this one's: their score columns are idle, since all softmax threads are done with the
+                        // tile before, the last that can have used them. Up to three key blocks: they have arrived at sFree[0] for this tile. Four:
+                        // at oFree for the tile before, which this tile's scores of block 0 waited for
 #pragma unroll 1
                         for (int j = 1; j < kMaxBlocks; ++j)
                         {

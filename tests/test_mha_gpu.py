@@ -687,6 +687,42 @@ def test_mha_fp16_short_kernel_residency(cuda, B):
     assert int(st[0]) == 0 and torch.equal(short, persistent)
 
 
+# Four key blocks in the order in which the sequences come: a CTA's tiles go from one key block to four and back, so that scores of blocks 1 to 3 are formed
+# beside a tile that has none of them. 9 x 12 pairs of four tiles (432 items), and more sequences than a CTA puts in order; some without keys between
+@pytest.mark.parametrize("B,N,S,layout", [(9, 12, 512, "fixed"), (9, 12, 512, "separate"), (9, 12, 400, "fixed"), (260, 1, 512, "packed"), (260, 1, 400, "interleaved")])
+@pytest.mark.parametrize("scale_softmax", [127.0, 200.0])
+def test_mha_int8_four_key_blocks_as_they_come(cuda, B, N, S, layout, scale_softmax):
+    import tensorrt_b200 as T
+
+    rng = np.random.default_rng(B + S)
+    d = 32
+    lengths = np.array([(20, S, 1, S - 3, 130, 0, 128, 385)[(i + i // 8) % 8] for i in range(B)], dtype=np.int32)
+    lengths[1] = S
+    cu = O.cu_seqlens(lengths)
+    packed = layout in ("packed", "interleaved")
+    x = rng.integers(-127, 128, size=(int(cu[-1]) if packed else S * B, 3 * N * d)).astype(np.int8)
+    s1, s2 = float((4.0 / 127) ** 2 / np.sqrt(d)), 2.0 / 127
+    st = _status(cuda)
+    scales = {"scale_bmm1": s1, "scale_softmax": scale_softmax, "scale_bmm2": s2, "status": st}
+    if packed:
+        ref = O.mha_int8(x, B, S, N, d, s1, scale_softmax, s2, cu=cu)
+    else:
+        x = x.reshape(S, B, 3 * N * d)
+        ref = O.mha_int8(x, B, S, N, d, s1, scale_softmax, s2, lengths=lengths)
+    if layout == "packed":
+        out = T.mha(_t(x, cuda), B, S, N, d, cu_seqlens=_t(cu, cuda), **scales).cpu().numpy()
+    elif layout == "fixed":
+        out = T.mha(_t(x, cuda), B, S, N, d, mask_idx=_t(lengths, cuda), **scales).cpu().numpy()
+    elif layout == "separate":
+        q, k, v = (_t(a, cuda) for a in x.reshape(S, B, N, 3, d).transpose(3, 1, 2, 0, 4))
+        out = T.attention_bnsd(q, k, v, kv_lengths=_t(lengths, cuda), **scales).cpu().numpy().transpose(2, 0, 1, 3).reshape(S, B, N * d)
+    else:
+        il = x.reshape(-1, N, 3, d).transpose(0, 2, 1, 3).reshape(-1, 3 * N * d)   # [3][N][d / 32][total][32]
+        out = O.from_chw32(T.mha(_t(O.to_chw32(il), cuda), B, S, N, d, cu_seqlens=_t(cu, cuda), interleaved=True, **scales).cpu().numpy())
+    assert int(st[0]) == 0
+    _assert_int8_attention(out, ref)
+
+
 # Few ragged sequences, whose tiles are dealt one by one: as many pairs as SMs, empty sequences, lengths at the edges of tiles, one long one. Then such as
 # the host takes for shorter when cut, but the CTAs, counting tiles, keep whole: lengths just beyond a tile, S far above the lengths
 @pytest.mark.parametrize("lengths,N,S", [([384, 97, 279, 90, 195, 241, 267, 119], 16, 384), ([1, 0, 512, 129, 128, 127, 257, 0, 385], 16, 512), ([300, 1, 1], 37, 300),
