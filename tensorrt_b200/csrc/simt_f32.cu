@@ -8,6 +8,7 @@
 // (plugin/bertQKVToContextPlugin/mhaRunner.cu:533-601) and the FP32 cublasLtMatmul of the FC plugin
 // (plugin/fcPlugin/fcPlugin.cpp:551-610).
 #include "common.cuh"
+#include "mha_f32_plan.h"
 
 namespace b200
 {
@@ -341,12 +342,10 @@ __device__ __forceinline__ void copyWait()
 // 64 or 32 queries of one (sequence, head) per CTA against blocks of 64 keys, running maximum and sum per row.
 //
 // Bound by the FP32 pipes and the shared-memory loads that feed them. Every warp owns 16 query rows, so its scores,
-// probabilities and row sums are its own business (a warp-level sync between the two products); a thread computes 4 rows x
+// probabilities and row sums are its own business; a thread computes 4 rows x
 // 8 keys of the scores with 16-byte loads along d (packed FMAs, even and odd channels apart, as in the FC above), and 4
-// rows x D / 8 columns of the context. Rows are padded by 4 floats against bank conflicts. The next keys are fetched during the softmax and the
-// second product, the next values during the scores (see kAttAsync; with one barrier less each, values during scores and softmax, keys during the second product:
-// 16 x 128, 12 heads 31.7 us instead of 27.5 us). Measured, heads of 64 channels: 8 sequences of 128
-// tokens, 12 heads 21.4 us (a warp per query row, keys and values from global memory: 509 us).
+// rows x D / 8 columns of the context. Rows are padded by 4 floats against bank conflicts. Which form, and how many CTAs share an SM: see planAtt.
+// Measured, heads of 64 channels: 8 sequences of 128 tokens, 12 heads 19.6 us (a warp per query row, keys and values from global memory: 509 us).
 constexpr int kAttKeys = 64;
 
 template <int D, int WARPS> // head size rounded up to 32, 64, 96 or 128; channels beyond d are zero
@@ -359,20 +358,44 @@ struct AttSmem
     float p[kAttRows][kAttKeys + 4];
 };
 
-// Asynchronous copies: FP32 heads of up to 64 channels. FP16 has to be converted on the way, and with wider heads fewer CTAs share an SM: the two
-// barriers more per block cost more than the copies' time (2 x 1100 tokens, 8 heads of 128 channels, FP32 327 -> 387 us).
-template <typename T, int D>
-constexpr bool kAttAsync = sizeof(T) == 4 && D <= 64;
+// Context of rows row0 + 4 i: keys c ... c + 3 of the block.
+template <typename Smem, int COLS>
+__device__ __forceinline__ void addFourKeys(Smem const& sm, int const row0, int const tx, int const c, float4 (&o)[4][COLS])
+{
+    float4 pr[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+        {
+            float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
+                o[i][j].x = fmaf(w, v.x, o[i][j].x);
+                o[i][j].y = fmaf(w, v.y, o[i][j].y);
+                o[i][j].z = fmaf(w, v.z, o[i][j].z);
+                o[i][j].w = fmaf(w, v.w, o[i][j].w);
+            }
+        }
+}
 
-template <typename T, int D, int WARPS>
+// ASYNC: FP32 keys and values come by asynchronous copies, the next keys during the softmax and the second product, the next values during the scores (with one
+// barrier less each, values during scores and softmax, keys during the second product: 16 x 128, 12 heads 31.7 us instead of 27.5 us). That takes four
+// barriers per block of keys instead of two.
+template <typename T, int D, int WARPS, bool ASYNC>
 __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
     T const* __restrict__ qkv, T* __restrict__ out, int32_t const* __restrict__ cu, int32_t const* __restrict__ maskIdx, float const scale)
 {
+    static_assert(!ASYNC || sizeof(T) == 4, "FP16 is converted on the way");
     extern __shared__ float smRaw[];
     using Smem = AttSmem<D, WARPS>;
     Smem& sm = *reinterpret_cast<Smem*>(smRaw);
     constexpr int kAttRows = Smem::kAttRows, kAttThreads = 32 * WARPS;
-    constexpr bool kAsync = kAttAsync<T, D>;
     constexpr int kVecs = D / 4;
     constexpr int kCols = D / 32; // float4 columns of the context per thread
     int const lane = threadIdx.x & 31;
@@ -396,7 +419,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
     {
         int const r = i / kVecs, c = i % kVecs * 4;
         bool const ok = q0 + r < seq.rows && c < d;
-        if constexpr (kAsync)
+        if constexpr (ASYNC)
             copy16(&sm.q[r][c], ok ? base + (q0 + r) * rowStep + c : base, ok);
         else
             *reinterpret_cast<float4*>(&sm.q[r][c]) = ok ? load4(base + (q0 + r) * rowStep + c) : zero;
@@ -427,7 +450,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
         }
         copyGroup();
     };
-    if constexpr (kAsync)
+    if constexpr (ASYNC)
     {
         fetchKeys(0); // and the queries
         fetchValues(0);
@@ -445,7 +468,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
     }
     for (int k0 = 0; k0 < seq.len; k0 += kAttKeys)
     {
-        if constexpr (kAsync)
+        if constexpr (ASYNC)
             copyWait<1>(); // keys
         else
         {
@@ -481,7 +504,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
                 }
             }
         }
-        if constexpr (kAsync)
+        if constexpr (ASYNC)
         {
             __syncthreads();
             fetchKeys(k0 + kAttKeys);
@@ -521,14 +544,37 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
                 sm.p[row0 + 4 * i][tx + 8 * j] = e;
             }
         }
-        if constexpr (kAsync)
+        if constexpr (ASYNC)
         {
             copyWait<1>(); // values
             __syncthreads();
         }
         else
             __syncwarp();
-        if constexpr (!kAsync)
+        // Keys beyond the sequence have no weight and are left out, four or eight at a time (the scores' product takes all 64), but for FP16 and wide heads.
+        if constexpr (ASYNC)
+        {
+            auto product = [&](int const keys) {
+#pragma unroll 2
+                for (int c = 0; c < keys; c += 4)
+                    addFourKeys(sm, row0, tx, c, o);
+            };
+            if (seq.len - k0 >= kAttKeys) // a loop of its own: with a variable end it is 2.5 % slower
+                product(kAttKeys);
+            else
+                product(seq.len - k0);
+        }
+        else if constexpr (sizeof(T) == 4 && D <= 64)
+        {
+            int const keys = min(kAttKeys, seq.len - k0);
+#pragma unroll 1
+            for (int c = 0; c < keys; c += 8)
+            {
+                addFourKeys(sm, row0, tx, c, o);
+                addFourKeys(sm, row0, tx, c + 4, o);
+            }
+        }
+        else // addFourKeys written out: called, heads of 128 channels are 2.5 % slower
         {
 #pragma unroll 2
             for (int c = 0; c < kAttKeys; c += 4)
@@ -555,46 +601,13 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
                     }
             }
         }
-        else
-        {
-            auto product = [&](int const keys) {
-#pragma unroll 2
-                for (int c = 0; c < keys; c += 4)
-                {
-                    float4 pr[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        pr[i] = *reinterpret_cast<float4 const*>(&sm.p[row0 + 4 * i][c]);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int j = 0; j < kCols; ++j)
-                        {
-                            float4 const v = *reinterpret_cast<float4 const*>(&sm.v[c + k][tx * 4 + 32 * j]);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                            {
-                                float const w = k == 0 ? pr[i].x : k == 1 ? pr[i].y : k == 2 ? pr[i].z : pr[i].w;
-                                o[i][j].x = fmaf(w, v.x, o[i][j].x);
-                                o[i][j].y = fmaf(w, v.y, o[i][j].y);
-                                o[i][j].z = fmaf(w, v.z, o[i][j].z);
-                                o[i][j].w = fmaf(w, v.w, o[i][j].w);
-                            }
-                        }
-                }
-            };
-            if (seq.len - k0 >= kAttKeys) // a loop of its own: with a variable end it is 2.5 % slower
-                product(kAttKeys);
-            else
-                product(seq.len - k0);
-        }
-        if constexpr (kAsync)
+        if constexpr (ASYNC)
         {
             __syncthreads();
             fetchValues(k0 + kAttKeys);
         }
     }
-    if constexpr (kAsync)
+    if constexpr (ASYNC)
         copyWait<0>();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -723,14 +736,17 @@ int32_t fcF32Simt(bert_b200_fc_params const& p, cudaStream_t stream)
 namespace
 {
 
-template <typename T, int D, int WARPS>
-int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
+// perSm: how many CTAs may share an SM (0: as many as fit), by the shared memory that is asked for.
+template <typename T, int D, int WARPS, bool ASYNC>
+int32_t launchMhaTiled(bert_b200_mha_params const& p, int perSm, cudaStream_t stream)
 {
     int32_t const rowBlocks = (p.S - 1) / (16 * WARPS) + 1;
     B200_REQUIRE(rowBlocks <= 65535, "mha (SIMT): S=%d too large", p.S); // the grid's third dimension
+    constexpr size_t kSmem = sizeof(AttSmem<D, WARPS>), kSm = 227 * 1024;
+    size_t const share = perSm > 0 ? kSm / perSm - 2048 : 0;
     static SmemOptIn optIn;
-    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D, WARPS>, dim3(p.num_heads, p.B, rowBlocks),
-        dim3(32 * WARPS), sizeof(AttSmem<D, WARPS>), stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
+    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D, WARPS, ASYNC>, dim3(p.num_heads, p.B, rowBlocks),
+        dim3(32 * WARPS), share > kSmem ? share : kSmem, stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
         static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTiledKernel: %s", cudaGetErrorString(e));
@@ -740,16 +756,18 @@ int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 template <typename T, int D>
 int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 {
-    int64_t const ctas = static_cast<int64_t>(p.num_heads) * p.B * ((p.S - 1) / 64 + 1);
-    // 32 rows where the 64-row CTAs are no more than two per SM: twice as many CTAs even out better, each with its own copies on the way.
-    // 8 x 128 tokens, 12 heads 24.4 -> 21.4 us, 10 x 128 26.9 -> 21.7 us, 5 x 200 49.1 -> 36.0 us, 16 heads 16 x 40 15.0 -> 10.4 us, 2 x 512 95.8 -> 77.5 us. With
-    // more of them 64: 13 x 128, 12 heads 27.3 us (31.0 us), 19 x 40, 16 heads 13.2 us (16.9 us); and where even 32-row ones would leave SMs
-    // without, 1 x 128, 16 heads 13.3 us (14.3 us).
-    [[maybe_unused]] bool const few = ctas <= 2 * smCount() && (2 * ctas > smCount() || p.S <= 64);
-    if constexpr (kAttAsync<T, D>)
-        if (few)
-            return launchMhaTiled<T, D, 2>(p, stream);
-    return launchMhaTiled<T, D, 4>(p, stream);
+    if constexpr (sizeof(T) == 4 && D <= 64)
+    {
+        AttPlan const plan = planAtt(p.B, p.num_heads, p.S, D, smCount());
+        if (plan.rows == 32)
+            return launchMhaTiled<T, D, 2, true>(p, plan.perSm, stream);
+        if constexpr (D == 64)
+            if (plan.async)
+                return launchMhaTiled<T, D, 4, true>(p, plan.perSm, stream);
+        return launchMhaTiled<T, D, 4, false>(p, plan.perSm, stream);
+    }
+    else
+        return launchMhaTiled<T, D, 4, false>(p, 0, stream);
 }
 
 template <typename T>

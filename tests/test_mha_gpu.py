@@ -453,9 +453,13 @@ def test_mha_simt_tile_edges(cuda, d, half):
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, tol, tol)[0]
 
 
-# FP32 on CTAs of 32 and of 64 query rows: as many 64-row CTAs as make the difference (148 SMs: 74, 75 ... 296, 297; any number up to 64 tokens), lengths
-# at the edges of both, keys ending at and beside fours, padded and packed
-@pytest.mark.parametrize("S,B,N", [(31, 1, 1), (33, 3, 2), (64, 2, 2), (65, 37, 1), (66, 38, 1), (97, 10, 6), (128, 37, 4), (127, 25, 6), (259, 15, 4)])
+# FP32, every form of the launch on 148 SMs (csrc/mha_f32_plan.h), lengths at the edges of rows and blocks of keys, keys ending at and beside fours and eights,
+# padded and packed
+@pytest.mark.parametrize("S,B,N", [
+    (31, 1, 1), (33, 3, 2), (64, 2, 2), (128, 74, 1), (64, 148, 1),               # 64 rows, one CTA per SM, asynchronous copies (64 channels)
+    (64, 149, 1), (97, 10, 12), (128, 37, 4), (127, 25, 6), (64, 297, 1),         # two and more
+    (129, 3, 2), (192, 49, 1), (257, 7, 4), (259, 15, 4), (192, 149, 1),          # 64 rows, copies between barriers: one, two and more
+    (31, 40, 5), (65, 75, 1), (200, 40, 1), (17, 150, 2), (65, 149, 1), (9, 500, 2)])  # 32 rows: two, three and more
 @pytest.mark.parametrize("d", [64, 20])
 def test_mha_fp32_rows_per_cta(cuda, S, B, N, d):
     import tensorrt_b200 as T
