@@ -72,7 +72,6 @@ struct OnlineArgs : ShareArgs
     void* out;
     float scaleBmm1;
     uint32_t* statusWord;
-    uint32_t shortCols; // tensor memory that a CTA of the short kernel takes
 };
 
 // [ Q slots ][ K/V stages ][ barriers ][ shares ]
@@ -741,7 +740,8 @@ constexpr int kShortSmemBytes = kShortBars + 64 + 1024;
 constexpr int kShortSmemTwo = 80 * 1024; // asked for where two CTAs are to share an SM
 constexpr uint32_t kShortTmemCols = 128; // scores; once they are in registers, P in the first 64 columns and the context in the others
 
-template <bool BNSD>
+// COLS: tensor memory of a CTA, 128 or 256 columns (an argument instead has to arrive before the allocation: 1 x 37 ... 8 x 128 tokens alone on the GPU 0.1 us)
+template <bool BNSD, uint32_t COLS>
 __global__ void __launch_bounds__(kShortThreads, 3) mhaShortF16Kernel(const __grid_constant__ CUtensorMap mapQ,
     const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, OnlineArgs const args)
 {
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kShortThreads, 3) mhaShortF16Kernel(const __gr
     }
     __syncwarp();
     if (warp == 0)
-        tmemAlloc(tmemSlot, args.shortCols);
+        tmemAlloc(tmemSlot, COLS);
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(kShortThreads, 3) mhaShortF16Kernel(const __gr
     {
         __syncwarp();
         tcFenceAfter();
-        tmemFree(tmemBase, args.shortCols);
+        tmemFree(tmemBase, COLS);
     }
 }
 
@@ -966,14 +966,16 @@ int32_t launchOnline(CUtensorMap const (&maps)[3], OnlineArgs args, cudaStream_t
         // How many CTAs share an SM. Three where that takes fewer rounds than two: 32 x 64 ... 128 tokens, 12 heads 7.1 us (two: 8.9 us), 64 x 128, 16
         // heads 14.4 us (16.1 us), 1000 x 20 ... 60, 12 heads 107 us (121 us); in as many rounds they hinder each other: 40 x 64 ... 128, 12 heads
         // 9.4 us (9.0 us). Two by their tensor memory, which the placement of CTAs knows nothing of: a third one waits for it, but has been set up
-        // when it gets it. That is ahead where a CTA per SM does - 8 x 128, 16 heads 4.4 us, limited by shared memory 5.3 us -, and behind where a
-        // round has more of them: 24 x 64 ... 128, 12 heads 7.1 us, by shared memory 6.2 us.
+        // when it gets it. That is ahead where attention follows attention and a CTA per SM does - 8 x 128, 16 heads 4.4 us, limited by shared memory
+        // 5.3 us -, and behind where a round has more of them, as placement puts three on the SMs that the kernel before leaves first: behind a fully
+        // connected layer of 4.7 us and with it, pairs of 128 tokens, by tensor memory / by shared memory: 149 12.6 / 9.8 us, 296 12.9 / 10.4 us; attention after
+        // attention 149 5.4 / 5.6 us, 222 5.8 / 6.0 us, 240 7.5 / 5.9 us, 296 7.4 / 5.7 us.
         int64_t const sms = smCount(), two = (pairs + 2 * sms - 1) / (2 * sms), three = (pairs + 3 * sms - 1) / (3 * sms);
-        bool const bySmem = three == two && pairs > sms && pairs <= 2 * sms;
-        args.shortCols = three < two || bySmem ? kShortTmemCols : 2 * kShortTmemCols;
+        bool const bySmem = three == two && pairs > sms && pairs <= 2 * sms, few = three < two || bySmem;
         int const smem = bySmem ? kShortSmemTwo : kShortSmemBytes;
-        static SmemOptIn optIn;
-        cudaError_t const e = launchDependentCluster(&optIn, mhaShortF16Kernel<BNSD>, dim3(static_cast<unsigned>(pairs)), dim3(kShortThreads),
+        static SmemOptIn optIn[2];
+        auto const kernel = few ? mhaShortF16Kernel<BNSD, kShortTmemCols> : mhaShortF16Kernel<BNSD, 2 * kShortTmemCols>;
+        cudaError_t const e = launchDependentCluster(&optIn[few], kernel, dim3(static_cast<unsigned>(pairs)), dim3(kShortThreads),
             smem, stream, 1, maps[0], maps[1], maps[2], args);
         if (e != cudaSuccess)
             B200_FAIL(BERT_B200_CUDA_ERROR, "mhaShortF16Kernel: %s", cudaGetErrorString(e));
@@ -1008,7 +1010,7 @@ int32_t mhaOnlineF16(bert_b200_mha_params const& p, cudaStream_t stream)
         return st;
     maps[1] = maps[0];
     maps[2] = maps[0];
-    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, p.cu_seqlens, p.mask_idx), p.head_size, p.out, p.scale_bmm1, p.status_word, 0};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, p.cu_seqlens, p.mask_idx), p.head_size, p.out, p.scale_bmm1, p.status_word};
     return launchOnline<false>(maps, args, stream);
 }
 
@@ -1028,7 +1030,7 @@ int32_t mhaOnlineF16Bnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t 
         if (st != BERT_B200_OK)
             return st;
     }
-    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, nullptr, p.kv_lengths), p.head_size, p.out, p.scale_bmm1, p.status_word, 0};
+    OnlineArgs const args{shareArgs(p.B, p.S, p.num_heads, nullptr, p.kv_lengths), p.head_size, p.out, p.scale_bmm1, p.status_word};
     return launchOnline<true>(maps, args, stream);
 }
 
