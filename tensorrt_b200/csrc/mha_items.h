@@ -60,10 +60,10 @@ inline ItemPlan planItems(int32_t B, int32_t N, int32_t S, int64_t missing, int6
 // of the sequences' lengths. The longest pair then no longer holds up the launch, at the price of K and V for each tile. In the units above a tile
 // costs up to four per key block and a whole pair 3 tiles + 1, so the cut is shorter while the rounds of tiles are fewer than that over four.
 // The host knows the tokens only and guesses, half a tile per sequence for its last one and a sixteenth on top, whether that can be; then the CTAs, which
-// read the lengths anyway, count the tiles and decide (cutIsShorter). The cut alone by the guess was up to 1.2 times as long (lengths just beyond a multiple
+// put the lengths in order anyway, count the tiles and decide (cutIsShorter). The cut alone by the guess was up to 1.2 times as long (lengths just beyond a multiple
 // of 128), and wherever S is far above the lengths. Measured (whole pairs / cut by the guess / as it is): 8 sequences of 90 ... 384 tokens, 16 heads
-// 16.9 / 11.7 / 11.9 us, 12 of 32 ... 384, 12 heads 16.9 / 12.1 / 12.1 us; 5 of 133 ... 160, 16 heads 9.8 / 10.2 / 9.7 us (in the form of the kernel that
-// always keeps them whole 9.3 us), 92 of 129, one of 256, one head 9.9 / 15.8 / 9.7 us, 12 of up to 128 with S = 512, 12 heads 5.2 / 6.3 / 5.7 us.
+// 17.0 / 11.7 / 11.6 us, 12 of 32 ... 384, 12 heads 17.0 / 12.1 / 11.8 us; 5 of 133 ... 160, 16 heads 9.9 / 10.3 / 9.8 us (a launch that the host keeps whole
+// 9.3 us), 92 of 129, one of 256, one head 9.9 / 15.9 / 10.8 us, 12 of up to 128 with S = 512, 12 heads 5.2 / 6.4 / 5.8 us (5.0 us).
 // Returns the most tiles that there can be, or 0: not cut. tokens: of the batch.
 inline int64_t cutTiles(int32_t B, int32_t N, int32_t S, int64_t tokens, int64_t ctas)
 {

@@ -72,10 +72,17 @@ struct MhaArgs
     float scaleBmm1, scaleSoftmax, scaleBmm2;
     uint32_t* statusWord;
     int32_t tilesPerItem, chunks; // a work item = (sequence, head, chunk of tilesPerItem query tiles)
-    int32_t rounds, cut;          // ORDERED: items per CTA (at most); whether they are tiles, not pairs, where that is shorter
+    int32_t rounds;               // listed items per CTA, at most
 };
 
-// Sequences by length and the items of a CTA (ORDERED, see the kernel).
+enum class Order
+{
+    kNone,
+    kPairs,
+    kTiles,
+};
+
+// Sequences by length and the items of a CTA (see ORDER).
 struct alignas(1024) ItemTable
 {
     int4 ordered[kItemOrder]; // number, first row, length
@@ -181,93 +188,26 @@ __device__ __forceinline__ void sequenceOf(
     }
 }
 
-// The sequences in the order of their lengths, by the first kItemOrder threads, each with one of them (len -1: beyond the batch); lengths are in place.
-__device__ __forceinline__ void orderSequences(ItemTable* const table, int32_t const B, int const b, int32_t const rowBase, int32_t const len)
-{
-    // a sequence's place is the number of longer ones, and of equal ones before it
-    if (b < B)
-    {
-        int place = 0;
-        for (int u = 0; u < B; u += 4)
-        {
-            int4 const v = *reinterpret_cast<int4 const*>(table->lengths + u);
-            place += (v.x > len || (v.x == len && u < b)) + (v.y > len || (v.y == len && u + 1 < b))
-                + (v.z > len || (v.z == len && u + 2 < b)) + (v.w > len || (v.w == len && u + 3 < b));
-        }
-        table->ordered[place] = make_int4(b, rowBase, len, 0);
-    }
-    asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
-}
-
-// Items of this CTA where pairs may be cut into tiles (packed layout), by the first kItemOrder threads. Not inlined: in the way of those that are not
-// (instruction fetch), it costs each launch that deals whole pairs 0.2 us.
-__device__ __noinline__ void listTiles(ItemTable* const table, int32_t const B, int32_t const S, int32_t const N, int32_t const* const cu, int32_t const rounds)
-{
-    int const b = static_cast<int>(threadIdx.x), warp = b >> 5, lane = b & 31;
-    int32_t rowBase = 0, len = -1;
-    if (b < B)
-        sequenceOf<false>(S, cu, nullptr, b, rowBase, len);
-    table->lengths[b] = len;
-    // tiles of the batch and of its longest sequence; the warps' sums go where so few rounds list no item
-    unsigned const tiles = (max(len, 0) + kQTile - 1) / kQTile;
-    int sum = static_cast<int>(__reduce_add_sync(0xffffffffu, tiles)), most = static_cast<int>(__reduce_max_sync(0xffffffffu, tiles));
-    if (lane == 0)
-        table->items[kItemRounds - 1 - warp] = make_int4(sum, most, 0, 0);
-    asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
-    sum = 0;
-    for (int w = 0; w * 32 < B; ++w)
-    {
-        int4 const v = table->items[kItemRounds - 1 - w];
-        sum += v.x;
-        most = max(most, v.y);
-    }
-    if (!cutIsShorter(sum * N, most, static_cast<int>(gridDim.x))) // a pair per CTA, as they come
-    {
-        int const pair = static_cast<int>(blockIdx.x);
-        bool const one = pair < B * N;
-        if (b >= (one ? 1 : 0) && b < rounds)
-            table->items[b] = make_int4(-1, 0, 0, 0);
-        if (one && b == pair / N)
-            table->items[0] = make_int4(b, pair % N | kMaxBlocks << 24, rowBase, len);
-        return;
-    }
-    orderSequences(table, B, b, rowBase, len);
-    if (b < rounds)
-    {
-        int left = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)); // a longer sequence has more tiles
-        int4 q = make_int4(-1, 0, 0, 0);
-        for (int place = 0; place < B; ++place)
-        {
-            int4 const o = table->ordered[place];
-            int const ofPair = (o.z + kQTile - 1) / kQTile;
-            if (left < ofPair * N)
-            {
-                int const head = left / ofPair;
-                q = make_int4(o.x, head | (left - head * ofPair) << 16 | 1 << 24, o.y, o.z);
-                break;
-            }
-            left -= ofPair * N;
-        }
-        table->items[b] = q;
-    }
-}
-
 // IL: CHW32-interleaved tensors. Q, K and V tiles then arrive as two 32-channel sub-tiles of
 // [128 tokens][32 B] (32-byte swizzle); the head dimension is covered by one MMA per sub-tile.
 // BNSD: Q, K and V are three separate [B][N][S][d] tensors (mapQkv, mapK, mapV) and the output is [B][N][S][d];
 // otherwise mapQkv covers the fused tensor and the other two maps are not used.
-// ORDERED: the CTA first puts the sequences in the order of their lengths and lists its items, pairs or tiles (see mha_items.h).
+// ORDER: items as they come; or the CTA first puts the sequences in the order of their lengths and lists its items (see mha_items.h), whole pairs, or tiles where
+// these, counted, are shorter. The last is a form of its own: with its code beside the other's, launches that deal pairs were 1 ... 2 % slower, and with it in a
+// function of its own the launches that deal tiles 0.4 us.
 // FIXED: the fixed layout (or separate tensors), not the packed one.
 // FOUR: the longest sequence has four key blocks, not up to three. The context accumulator then has to share TMEM columns with the scores of key block 0, and four
 // blocks of P share two slots.
 // CLAMP: with FOUR, whether scale_softmax is above 127 (64 x 512 tokens, 16 heads 168.7 -> 165.1 us); the form for shorter sequences finds out (decided when it is
 // compiled, it is 2 % slower).
-template <bool IL, bool BNSD, bool FIXED, bool ORDERED, bool FOUR, bool CLAMP>
+template <bool IL, bool BNSD, bool FIXED, Order ORDER, bool FOUR, bool CLAMP>
 __global__ void __launch_bounds__(kMhaThreads, 1)
     mhaTcgen05Kernel(const __grid_constant__ CUtensorMap mapQkv, const __grid_constant__ CUtensorMap mapK,
         const __grid_constant__ CUtensorMap mapV, MhaArgs const args)
 {
     static_assert(!BNSD || !IL, "separate Q / K / V tensors: linear layout");
+    static_assert(!FIXED || ORDER != Order::kTiles, "packed layout");
+    constexpr bool ORDERED = ORDER != Order::kNone, kCut = ORDER == Order::kTiles;
     using L = MhaSmem;
     // Q, K, V rows are 64 B or 32 B (interleaved sub-tiles)
     constexpr uint64_t kSwz = IL ? kSwizzle32B : kSwizzle64B;
@@ -398,25 +338,64 @@ __global__ void __launch_bounds__(kMhaThreads, 1)
 
     if (ORDERED)
     {
+        // a sequence's place is the number of longer ones, and of equal ones before it (those beyond the batch count as -1)
         int const b = static_cast<int>(threadIdx.x);
-        if (!FIXED && args.cut && b < kItemOrder)
-            listTiles(table, args.B, args.S, args.N, args.cu, args.rounds);
-        else if (b < kItemOrder)
+        if (b < kItemOrder)
         {
             int32_t rowBase = 0, len = -1;
             if (b < args.B)
                 sequence(b, rowBase, len);
             table->lengths[b] = len;
             asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
-            orderSequences(table, args.B, b, rowBase, len);
+            [[maybe_unused]] int total = 0, most = 0; // tiles of the batch and of its longest sequence (threads with a sequence or an item)
+            if (b < args.B || (kCut && b < args.rounds))
+            {
+                int place = 0;
+                for (int u = 0; u < args.B; u += 4)
+                {
+                    int4 const v = *reinterpret_cast<int4 const*>(table->lengths + u);
+                    place += (v.x > len || (v.x == len && u < b)) + (v.y > len || (v.y == len && u + 1 < b))
+                        + (v.z > len || (v.z == len && u + 2 < b)) + (v.w > len || (v.w == len && u + 3 < b));
+                    if (kCut)
+                    {
+                        total += (v.x + kQTile - 1) / kQTile + (v.y + kQTile - 1) / kQTile + (v.z + kQTile - 1) / kQTile + (v.w + kQTile - 1) / kQTile;
+                        most = max(max(max(most, v.x), max(v.y, v.z)), v.w);
+                    }
+                }
+                if (!kCut || b < args.B)
+                    table->ordered[place] = make_int4(b, rowBase, len, 0);
+            }
+            asm volatile("bar.sync 8, %0;" ::"n"(kItemOrder) : "memory");
             if (b < args.rounds)
             {
-                int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)), place = item / args.N;
+                int const item = itemOfRound(b, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+                int place = item / args.N, what = (item - place * args.N) | kMaxBlocks << 24;
+                if (kCut)
+                {
+                    if (cutIsShorter(total * args.N, (most + kQTile - 1) / kQTile, static_cast<int>(gridDim.x)))
+                    {
+                        // the tiles of a pair one by one: a longer sequence has more of them
+                        int left = item;
+                        for (place = 0; place < args.B; ++place)
+                        {
+                            int const tiles = (table->ordered[place].z + kQTile - 1) / kQTile;
+                            if (left < tiles * args.N)
+                            {
+                                int const head = left / tiles;
+                                what = head | (left - head * tiles) << 16 | 1 << 24;
+                                break;
+                            }
+                            left -= tiles * args.N;
+                        }
+                    }
+                    else if (b > 0)
+                        place = args.B; // whole pairs: one round
+                }
                 int4 q = make_int4(-1, 0, 0, 0);
                 if (place < args.B)
                 {
                     int4 const o = table->ordered[place];
-                    q = make_int4(o.x, (item - place * args.N) | kMaxBlocks << 24, o.y, o.z);
+                    q = make_int4(o.x, what, o.y, o.z);
                 }
                 table->items[b] = q;
             }
@@ -1256,6 +1235,17 @@ __global__ void __launch_bounds__(kShortThreads, 4) mhaShortInt8Kernel(const __g
     }
 }
 
+using MhaKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
+
+// form: up to three key blocks; four; four with the clamp of the probabilities
+template <bool IL, bool BNSD, bool FIXED, Order ORDER>
+MhaKernel mhaForm(int form)
+{
+    static constexpr MhaKernel kForms[3] = {mhaTcgen05Kernel<IL, BNSD, FIXED, ORDER, false, false>, mhaTcgen05Kernel<IL, BNSD, FIXED, ORDER, true, false>,
+        mhaTcgen05Kernel<IL, BNSD, FIXED, ORDER, true, true>};
+    return kForms[form];
+}
+
 // Sets the work items and launches: one persistent CTA per SM (512 TMEM columns and most of the shared memory each).
 template <bool IL, bool BNSD>
 int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t stream)
@@ -1274,29 +1264,29 @@ int32_t launchItems(MhaArgs& args, CUtensorMap const (&maps)[3], cudaStream_t st
     int64_t const missing = !args.fixedLayout ? static_cast<int64_t>(args.B) * args.S - args.total : (args.maskIdx ? INT64_MAX : 0);
     ItemPlan const plan = planItems(args.B, args.N, args.S, missing, smCount());
     int64_t const cut = args.fixedLayout || plan.chunks > 1 ? 0 : cutTiles(args.B, args.N, args.S, args.total, smCount());
-    args.cut = cut > 0 ? 1 : 0;
     args.tilesPerItem = plan.tilesPerItem;
     args.chunks = plan.chunks;
     int64_t const items = cut > 0 ? cut : static_cast<int64_t>(args.B) * args.N * plan.chunks;
-    bool const ordered = plan.longestFirst || cut > 0;
+    Order const order = cut > 0 ? Order::kTiles : plan.longestFirst ? Order::kPairs : Order::kNone;
     int const grid = static_cast<int>(items < smCount() ? items : smCount());
     args.rounds = cut > 0 ? 3 * plan.tilesPerItem / 4 : static_cast<int32_t>((items + grid - 1) / grid); // cut: see cutIsShorter
-    int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (ordered ? static_cast<int>(sizeof(ItemTable)) : 0);
-    int const form = (ordered ? 1 : 0) + (args.S <= 3 * kKeyBlock ? 0 : args.scaleSoftmax <= 127.f ? 2 : 4);
-    using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, MhaArgs);
-    // BNSD is always fixed, interleaved always packed
-    constexpr bool kPacked = BNSD, kFixed = !IL;
-    static constexpr Kernel kForms[2][6] = {
-        {mhaTcgen05Kernel<IL, BNSD, kPacked, false, false, false>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, false, false>,
-            mhaTcgen05Kernel<IL, BNSD, kPacked, false, true, false>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, true, false>,
-            mhaTcgen05Kernel<IL, BNSD, kPacked, false, true, true>, mhaTcgen05Kernel<IL, BNSD, kPacked, true, true, true>},
-        {mhaTcgen05Kernel<IL, BNSD, kFixed, false, false, false>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, false, false>,
-            mhaTcgen05Kernel<IL, BNSD, kFixed, false, true, false>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, true, false>,
-            mhaTcgen05Kernel<IL, BNSD, kFixed, false, true, true>, mhaTcgen05Kernel<IL, BNSD, kFixed, true, true, true>}};
-    static SmemOptIn optIn[2][6];
-    int const fixed = args.fixedLayout ? 1 : 0;
-    cudaError_t const e = launchDependentCluster(
-        &optIn[fixed][form], kForms[fixed][form], dim3(grid), dim3(kMhaThreads), smem, stream, 1, maps[0], maps[1], maps[2], args);
+    int const smem = MhaSmem::dynamicBytes((args.S + kKeyBlock - 1) / kKeyBlock) + (order != Order::kNone ? static_cast<int>(sizeof(ItemTable)) : 0);
+    int const form = args.S <= 3 * kKeyBlock ? 0 : args.scaleSoftmax <= 127.f ? 1 : 2;
+    MhaKernel kernel;
+    if constexpr (BNSD) // always fixed
+        kernel = order == Order::kPairs ? mhaForm<IL, BNSD, true, Order::kPairs>(form) : mhaForm<IL, BNSD, true, Order::kNone>(form);
+    else
+    {
+        kernel = order == Order::kTiles ? mhaForm<IL, BNSD, false, Order::kTiles>(form)
+            : order == Order::kPairs    ? mhaForm<IL, BNSD, false, Order::kPairs>(form)
+                                        : mhaForm<IL, BNSD, false, Order::kNone>(form);
+        if constexpr (!IL) // interleaved: always packed
+            if (args.fixedLayout)
+                kernel = order == Order::kPairs ? mhaForm<IL, BNSD, true, Order::kPairs>(form) : mhaForm<IL, BNSD, true, Order::kNone>(form);
+    }
+    static SmemOptIn optIn[2][3][3];
+    cudaError_t const e = launchDependentCluster(&optIn[args.fixedLayout ? 1 : 0][static_cast<int>(order)][form], kernel, dim3(grid), dim3(kMhaThreads), smem,
+        stream, 1, maps[0], maps[1], maps[2], args);
     if (e != cudaSuccess)
         B200_FAIL(BERT_B200_CUDA_ERROR, "mhaTcgen05Kernel: %s", cudaGetErrorString(e));
     return checkLaunch("mhaTcgen05Kernel");
@@ -1339,7 +1329,7 @@ int32_t launchMha(bert_b200_mha_params const& p, cudaStream_t stream)
     maps[1] = map;
     maps[2] = map;
     MhaArgs args{p.B, p.S, p.num_heads, p.total, p.head_size, fixedLayout ? 1 : 0, p.out, p.cu_seqlens, p.mask_idx, p.scale_bmm1,
-        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1, 0};
+        p.scale_softmax, p.scale_bmm2, p.status_word, 1, 1, 1};
     return launchItems<IL, false>(args, maps, stream);
 }
 
@@ -1362,7 +1352,7 @@ int32_t launchMhaBnsd(bert_b200_attention_bnsd_params const& p, cudaStream_t str
             return st;
     }
     MhaArgs args{p.B, p.S, p.num_heads, 0, p.head_size, 1, p.out, nullptr, p.kv_lengths, p.scale_bmm1, p.scale_softmax,
-        p.scale_bmm2, p.status_word, 1, 1, 1, 0};
+        p.scale_bmm2, p.status_word, 1, 1, 1};
     return launchItems<false, true>(args, maps, stream);
 }
 
