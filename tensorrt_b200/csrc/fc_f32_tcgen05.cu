@@ -259,13 +259,12 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
     }
 }
 
-// Bound by the warps that cut operands, and by shared memory behind them: a chunk of a 128 x 128 tile takes 2900 cycles, of which the
-// tensor cores are busy 1750 and shared memory 2240 (tiles written and read, parts of Wt written and read by 26 products), of a 64-wide one 1870
-// (830, 1380). The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are
+// Bound by the warps that cut operands, and by shared memory behind them: a chunk of a 128 x 128 tile takes 2900 cycles (stamps), of which the
+// tensor cores are busy 1620 and shared memory serves the warps for 1130 and the products for 840 (counters, the tile's end included); of a 64-wide one 1870. The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are
 // multiplied in two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk beyond 32 columns (with two groups
 // taking chunks in turn the sums waited for the group that was cutting); a chunk's three barriers are asked at once (an answer takes 120 ... 150
 // cycles); and a tile's place in the ring is handed back as soon as its numbers are in registers. Before / after: 3400 / 2900 cycles
-// per chunk; 1024 x 2304 x 768 32.7 / 28.3 us, 2000 x 3072 x 1024 113.1 / 98.7 us, 4096 x 3072 x 1024 210.9 / 195.4 us, 37 x 2304 x 768 11.1 / 10.6 us.
+// per chunk; 1024 x 2304 x 768 32.7 / 28.3 us, 2000 x 3072 x 1024 113.1 / 98.7 us, 4096 x 3072 x 1024 210.9 / 195.4 us, 37 x 2304 x 768 11.3 / 10.7 us.
 // Rounding costs nothing: truncation of h, other subtractions or loads further ahead leave the times as they are.
 // One 128 x BN tile per CTA, or one segment of its K:
 //   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
@@ -443,10 +442,9 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         int segment = 0;
         int segmentEnd = segmentBegin(1);
         bool ok = true;
-        // the sums of chunk c
-        // (`ready`: they are known to be complete)
-        auto promote = [&](int c, bool ready) {
-            if (!__all_sync(0xffffffffu, ready))
+        // the sums of chunk c (`summed`: they are known to be complete)
+        auto promote = [&](int c, bool summed) {
+            if (!__all_sync(0xffffffffu, summed))
                 ok = ok && mbarWaitWarp(&done[part * kParts + (c & 1)], (c >> 1) & 1u, abortFlag, kWaitAccFull);
             tcFenceAfter();
             if (hasRows)
@@ -791,8 +789,8 @@ int32_t launchF32Tc(bert_b200_fc_params const& p, int segments, int ctas, cudaSt
 // large sum: softmax of 3 N(0, 1) x uniform 1.8e-7 ... 2.1e-7 / 0.8e-7 ... 1.1e-7 (before 3.0e-7 ... 3.3e-7), exp(2 N(0, 1)) on both sides 3.1e-7 ... 3.8e-7 /
 // 1.0e-7 ... 1.8e-7 (before 4.1e-7 ... 5.4e-7); with normal weights they are not. A shorter K has not been measured in this form and stays with
 // the multiply-adds. They also take what the TMA unit does not: rows that are no multiple of 16 bytes apart, sizes beyond its coordinates. GPU time,
-// same order: 1 x 64 x 384 6.3 / 8.5 us, 1 x 768 x 768 8.0 / 8.6 us, 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 11.2 / 14.9 us, 300 x 768 x 512 9.9 /
-// 18.5 us, 128 x 768 x 3072 13.6 / 44.9 us, 1024 x 2304 x 768 28.3 / 96.9 us, 4096 x 1024 x 4096 217 / 843 us. The two tensor maps cost a call 1 us
+// same order: 1 x 64 x 384 6.1 / 8.5 us, 1 x 768 x 768 8.2 / 8.6 us, 37 x 768 x 768 8.4 / 8.9 us, 37 x 2304 x 768 10.7 / 14.9 us, 300 x 768 x 512 9.4 /
+// 18.5 us, 128 x 768 x 3072 13.5 / 44.9 us, 1024 x 2304 x 768 28.3 / 96.9 us, 4096 x 1024 x 4096 226 ... 249 / 843 us. The two tensor maps cost a call 1 us
 // of the host: 10.1 instead of 9.5 us where the host is what bounds it.
 int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
 {
@@ -805,10 +803,12 @@ int32_t fcF32(bert_b200_fc_params const& p, cudaStream_t stream)
     int64_t const kChunks = (p.k + kChunk - 1) / kChunk;
     int const segments = kChunks >= 24 ? 8 : kChunks >= 12 ? 4 : 2;
     // Width of the tiles, and whether a CTA takes all segments: what the measured cycles per chunk and per CTA, times the waves of CTAs,
-    // make shortest (of an earlier form of the kernel, whose order is still the right one). Clusters find fewer places than there are SMs.
-    // Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768 29.1 / 46.0 / 36.7 / 58.2 us, 1024 x 3072 x 768 54.5 / 46.8 /
-    // 53.4 / 85.6 us, 1024 x 768 x 768 27.3 / 23.2 / 18.4 / 28.9 us; one segment per CTA, 128 / 64 columns: 1024 x 768 x 3072 72.0 / 93.2 us (64
-    // columns in one CTA 55.5 us), 128 x 768 x 3072 17.8 / 13.8 us (52.9 us).
+    // make shortest: cycles of the kernel before its columns were multiplied in halves, which is now 10 % faster with 128 and 6 % with 64 columns. Over 190
+    // shapes (M 1 ... 4096, N and K of encoders) the choice is still 0.3 % behind the best of the eight forms in the mean, more than 2 % behind in 13 of
+    // them and 14 % at most (640 x 768 x 3072 42.5 us, 128 columns and a segment per CTA 37.4 us; 1300 x 4096 x 1024 106 us, 128 columns 99.5 us). Clusters find
+    // fewer places than there are SMs. Measured with 128 / 96 / 64 / 32 columns, all segments in one CTA: 1024 x 2304 x 768 29.1 / 46.0 / 36.7 / 58.2 us, 1024 x
+    // 3072 x 768 54.5 / 46.8 / 53.4 / 85.6 us, 1024 x 768 x 768 27.3 / 23.2 / 18.4 / 28.9 us; one segment per CTA, 128 / 64 columns: 1024 x 768 x 3072 72.0 /
+    // 93.2 us (64 columns in one CTA 55.5 us), 128 x 768 x 3072 17.8 / 13.8 us (52.9 us).
     static constexpr int kCycles[4] = {1480, 1990, 2700, 3220}; // per chunk, of 32, 64, 96 and 128 columns
     static constexpr int kFixed[2][4] = {{12500, 13000, 16500, 26000}, {12500, 14500, 16300, 17500}}; // per CTA with all segments, with one
     int bestN = 128, bestCtas = 1;

@@ -22,7 +22,7 @@ struct ItemPlan
 };
 
 // All tiles of a pair share one load of K and V, which an item waits for at about a third of a tile's time; items are cut smaller only
-// when that shortens the longest CTA's list. Measured (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
+// when that shortens the longest CTA's list. Measured in an earlier form of the kernel, 8 % slower (16 heads; whole pairs in brackets): 2 x 512 tokens 9.4 us (30.2 us), 3 x 384 7.8 us (17.5
 // us), 4 x 256 6.5 us (10.2 us), 12 x 384 22.5 us (31.8 us); 8 x 384 whole, 16.7 us.
 // The lengths are on the device; what the host knows is how many tokens the batch has less than B * S (`missing`; INT64_MAX: unknown).
 // With no more pairs than CTAs a cut into equal items is never the longer way, whatever they are. With more, pairs are cut only when every sequence is
