@@ -60,9 +60,9 @@ struct FcF32Smem
     // eight a chunk ahead the sums wait less: 512 x 1024 x 4096 53.8 us (all 16: 58.5 us), 129 x 2304 x 768 13.8 us (14.4 us).
     static constexpr int kTurns = BN == 32 ? 2 : 1;
     static constexpr int kCutters = kWorkers / kTurns; // warps that cut a chunk
-    // stFull[stages] stFree[2][stages] ready[parts] done[halves][parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
+    // stFull[stages] stFree[stages] ready[parts] done[halves][parts] accFree[2], tmem slot, abort flag, flags of rows of A and Wt (1: a number without exact parts, 2: NaN),
     // whether any is set
-    static constexpr int kFlagsOff = kBarrierOff + (3 * kStages + (1 + kHalves) * kParts + 2) * 8 + 16;
+    static constexpr int kFlagsOff = kBarrierOff + (2 * kStages + (1 + kHalves) * kParts + 2) * 8 + 16;
     static constexpr int kTotal = kFlagsOff + (kTileM + BN + 4) * 4;
     static constexpr int kDynamic = kTotal + 1024;
     static constexpr int kPitch = BN + 4; // floats: sums of a tile over the drained FP32 tiles
@@ -260,11 +260,13 @@ __device__ __noinline__ void computeAgain(FcF32TcArgs const& p, uint32_t const* 
 }
 
 // Bound by the warps that cut operands, and by shared memory behind them: a chunk of a 128 x 128 tile takes 2900 cycles (stamps), of which the
-// tensor cores are busy 1620 and shared memory serves the warps for 1130 and the products for 840 (counters, the tile's end included); of a 64-wide one 1870. The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are
-// multiplied in two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk beyond 32 columns (with two groups
-// taking chunks in turn the sums waited for the group that was cutting); a chunk's three barriers are asked at once (an answer takes 120 ... 150
-// cycles); and a tile's place in the ring is handed back as soon as its numbers are in registers. Before / after: 3400 / 2900 cycles
-// per chunk; 1024 x 2304 x 768 32.7 / 28.3 us, 2000 x 3072 x 1024 113.1 / 98.7 us, 4096 x 3072 x 1024 210.9 / 195.4 us, 37 x 2304 x 768 11.3 / 10.7 us.
+// tensor cores are busy 1620 and shared memory serves the warps for 1130 and the products for 840 (counters, the tile's end included); of a 64-wide
+// one 1870. The warps take turns with nothing any more: the columns of a 128- or 96-wide tile, whose accumulators fit tensor memory only once, are multiplied in
+// two halves, so that the sums of one are read while the other's products run; all 16 warps cut every chunk beyond 32 columns (with two groups
+// taking chunks in turn the sums waited for the group that was cutting); and a chunk's three barriers are asked at once (an answer takes 120 ... 150
+// cycles). A chunk's place in the ring is handed back behind the stores of its parts and a proxy fence: an arrival right behind the loads does not wait
+// for them, so that now and then numbers of the next tile came into the registers instead (and it saved no time). Before / after: 3400 / 2900 cycles
+// per chunk; 1024 x 2304 x 768 32.7 / 28.2 us, 2000 x 3072 x 1024 117 / 101 us, 4096 x 3072 x 1024 215 / 209 us, 37 x 2304 x 768 11.3 / 10.7 us.
 // Rounding costs nothing: truncation of h, other subtractions or loads further ahead leave the times as they are.
 // One 128 x BN tile per CTA, or one segment of its K:
 //   warp 0    : FP32 tiles of A and Wt by TMA (128-byte swizzle) into a ring.
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
     uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* const stFull = reinterpret_cast<uint64_t*>(smem + L::kBarrierOff);
     uint64_t* const stFree = stFull + L::kStages;
-    uint64_t* const ready = stFree + 2 * L::kStages; // parts of a chunk in place
+    uint64_t* const ready = stFree + L::kStages; // parts of a chunk in place
     uint64_t* const done = ready + kParts;       // [halves][parts] their products complete
     uint64_t* const accFree = done + L::kHalves * kParts; // an accumulator (or its half) has been read
     uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(accFree + 2);
@@ -320,8 +322,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
         for (int i = 0; i < L::kStages; ++i)
         {
             mbarInit(&stFull[i], 1);
-            mbarInit(&stFree[i], L::kCutters);               // A
-            mbarInit(&stFree[L::kStages + i], L::kCutters); // Wt
+            mbarInit(&stFree[i], L::kCutters);
         }
         for (int i = 0; i < kParts; ++i)
             mbarInit(&ready[i], L::kCutters);
@@ -362,15 +363,10 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                 mbarArriveExpectTxAddr(bar, L::kStageBytes);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
+                {
                     tmaLoad2dAddr(a + h * (L::kABytes / 2), &mapA, bar, k + h * 32, static_cast<int32_t>(m0));
-            }
-            __syncwarp();
-            ok = ok && mbarWaitWarp(&stFree[L::kStages + stage], phase, abortFlag, kWaitStageFree);
-            if (ok && electOne())
-            {
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
                     tmaLoad2dAddr(a + L::kABytes + h * (L::kWBytes / 2), &mapW, bar, k + h * 32, static_cast<int32_t>(n0));
+                }
             }
             __syncwarp();
             if (++stage == L::kStages)
@@ -552,12 +548,6 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                             v[i] = src[((at & 1) * 4 + i) ^ (row & 7)];
-                        if (g == L::kTurns - 1)
-                        {
-                            __syncwarp();
-                            if (lane == 0)
-                                mbarArrive(&stFree[stage]);
-                        }
                         uint32_t h[8], m[8], l[8];
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
@@ -572,8 +562,6 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                     if ((lost & 0xffffu) != 0)
                         flagA[row] = *flagAny = 1;
                 }
-                else if (lane == 0)
-                    mbarArrive(&stFree[stage]);
                 // eight numbers of a row of Wt: 16 bytes of each part; an odd number of 32 rows is dealt to the groups by turns
                 uint8_t* const planes = smem + L::kPlanesOff + s * 3 * L::kPlaneBytes;
 #pragma unroll
@@ -605,7 +593,7 @@ __global__ void __launch_bounds__(kThreadsF32, 1)
                 if (lane == 0)
                 {
                     mbarArrive(&ready[s]);
-                    mbarArrive(&stFree[L::kStages + stage]);
+                    mbarArrive(&stFree[stage]);
                 }
             }
             if (++stage == L::kStages)

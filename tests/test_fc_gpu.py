@@ -313,6 +313,28 @@ def test_fc_fp32_sums_near_the_largest_numbers(cuda, m, k, n):
     assert torch.equal(out.double(), ref)
 
 
+# A tile's place in the ring must not be filled again before all of its numbers have been read: when it was, one launch in some 1500 of 2296 x 3072 x 768 had rows
+# that were off. 128, 96, 64 and 32 columns, launch after launch with another shape between, so that the loads find the memory system in all states
+@pytest.mark.parametrize("m,k,n", [(2296, 768, 3072), (1024, 768, 3072), (2296, 768, 768), (512, 4096, 1024)])
+def test_fc_fp32_same_bits_every_time(cuda, m, k, n):
+    import tensorrt_b200 as T
+
+    gen = torch.Generator(device=cuda).manual_seed(m + n)
+    a, w = torch.randn(m, k, device=cuda, generator=gen), torch.randn(n, k, device=cuda, generator=gen)
+    x, y = torch.randn(700, 1536, device=cuda, generator=gen), torch.randn(768, 1536, device=cuda, generator=gen)
+    first = T.fc(a, w)
+    ref = a.double() @ w.double().T
+    assert float((first.double() - ref).norm()) <= 2.0 ** -22 * float(ref.norm())
+    out = torch.empty_like(first)
+    wrong = torch.zeros((), dtype=torch.int64, device=cuda)
+    for i in range(2500):
+        if i % 2:
+            T.fc(x, y)
+        T.fc(a, w, out=out)
+        wrong += (out.view(torch.int32) != first.view(torch.int32)).sum()
+    assert int(wrong) == 0
+
+
 # 96 and 128 columns: the products of a chunk are waited for in two halves, the second by warps that have read the sums of the first. Another stream keeps the
 # SMs busy beside them, so that the barriers are asked early and late
 @pytest.mark.parametrize("m,k,n", [(6339, 1540, 129), (2115, 3072, 97), (1024, 768, 2304)])
