@@ -10,6 +10,7 @@ struct AttPlan
     int32_t rows;  // query rows of a CTA: 64 or 32
     int32_t perSm; // CTAs that may share an SM, 0: as many as fit
     bool async;    // keys and values by asynchronous copies (always with 32 rows)
+    bool skip;     // keys beyond a sequence are left out
 };
 
 // FP32, heads of up to 64 channels (headSize: 32 or 64).
@@ -25,13 +26,16 @@ struct AttPlan
 // Copies. With one or two blocks of keys asynchronous ones hide most of the loads (4 x 64 tokens, 16 heads 9.2 us instead of 10.1 us). With more, the two
 // barriers that they need on top cost 1 ... 2 % more than they bring (16 x 256, 12 heads 100.8 us instead of 99.6 us), since other CTAs' work hides the loads; with
 // 32 channels, whose products are half as long, from one block on (12 heads, 8 x 384 7 %).
-inline AttPlan planAtt(int32_t B, int32_t N, int32_t S, int32_t headSize, int64_t sms)
+// Keys beyond a sequence. The loop that leaves them out is 1 ... 1.5 % slower (64 channels, 16 x 256, 12 heads), so it is not taken where there are none (`full`: all
+// sequences have S tokens).
+inline AttPlan planAtt(int32_t B, int32_t N, int32_t S, int32_t headSize, bool full, int64_t sms)
 {
     int64_t const pairs = static_cast<int64_t>(B) * N;
     int64_t const n64 = (pairs * ((S - 1) / 64 + 1) + sms - 1) / sms, n32 = (pairs * ((S - 1) / 32 + 1) + sms - 1) / sms;
     if (n32 <= 2 * (n64 - 1) && (n64 <= 6 || S <= 32))
-        return {32, n32 <= 3 ? static_cast<int32_t>(n32) : 0, true};
-    return {64, n64 <= 2 ? static_cast<int32_t>(n64) : 0, headSize == 64 && S <= 128};
+        return {32, n32 <= 3 ? static_cast<int32_t>(n32) : 0, true, true};
+    bool const async = headSize == 64 && S <= 128;
+    return {64, n64 <= 2 ? static_cast<int32_t>(n64) : 0, async, async || headSize != 64 || !full || S % 64 != 0};
 }
 
 } // namespace b200

@@ -387,11 +387,12 @@ __device__ __forceinline__ void addFourKeys(Smem const& sm, int const row0, int 
 // ASYNC: FP32 keys and values come by asynchronous copies, the next keys during the softmax and the second product, the next values during the scores (with one
 // barrier less each, values during scores and softmax, keys during the second product: 16 x 128, 12 heads 31.7 us instead of 27.5 us). That takes four
 // barriers per block of keys instead of two.
-template <typename T, int D, int WARPS, bool ASYNC>
+// SKIP: keys beyond the sequence, which have no weight, are left out of the second product, four or eight at a time (the scores' product takes all 64).
+template <typename T, int D, int WARPS, bool ASYNC, bool SKIP>
 __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, int32_t const S, int32_t const N, int32_t const d,
     T const* __restrict__ qkv, T* __restrict__ out, int32_t const* __restrict__ cu, int32_t const* __restrict__ maskIdx, float const scale)
 {
-    static_assert(!ASYNC || sizeof(T) == 4, "FP16 is converted on the way");
+    static_assert(!ASYNC || (sizeof(T) == 4 && SKIP), "FP16 is converted on the way");
     extern __shared__ float smRaw[];
     using Smem = AttSmem<D, WARPS>;
     Smem& sm = *reinterpret_cast<Smem*>(smRaw);
@@ -551,7 +552,6 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
         }
         else
             __syncwarp();
-        // Keys beyond the sequence have no weight and are left out, four or eight at a time (the scores' product takes all 64), but for FP16 and wide heads.
         if constexpr (ASYNC)
         {
             auto product = [&](int const keys) {
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhaTiledKernel(int32_t const B, in
             else
                 product(seq.len - k0);
         }
-        else if constexpr (sizeof(T) == 4 && D <= 64)
+        else if constexpr (SKIP)
         {
             int const keys = min(kAttKeys, seq.len - k0);
 #pragma unroll 1
@@ -737,7 +737,7 @@ namespace
 {
 
 // perSm: how many CTAs may share an SM (0: as many as fit), by the shared memory that is asked for.
-template <typename T, int D, int WARPS, bool ASYNC>
+template <typename T, int D, int WARPS, bool ASYNC, bool SKIP>
 int32_t launchMhaTiled(bert_b200_mha_params const& p, int perSm, cudaStream_t stream)
 {
     int32_t const rowBlocks = (p.S - 1) / (16 * WARPS) + 1;
@@ -745,7 +745,7 @@ int32_t launchMhaTiled(bert_b200_mha_params const& p, int perSm, cudaStream_t st
     constexpr size_t kSmem = sizeof(AttSmem<D, WARPS>), kSm = 227 * 1024;
     size_t const share = perSm > 0 ? kSm / perSm - 2048 : 0;
     static SmemOptIn optIn;
-    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D, WARPS, ASYNC>, dim3(p.num_heads, p.B, rowBlocks),
+    cudaError_t const e = launchDependentCluster(&optIn, mhaTiledKernel<T, D, WARPS, ASYNC, SKIP>, dim3(p.num_heads, p.B, rowBlocks),
         dim3(32 * WARPS), share > kSmem ? share : kSmem, stream, 1, p.B, p.S, p.num_heads, p.head_size, static_cast<T const*>(p.qkv),
         static_cast<T*>(p.out), p.cu_seqlens, p.mask_idx, p.scale_bmm1);
     if (e != cudaSuccess)
@@ -758,16 +758,21 @@ int32_t launchMhaTiled(bert_b200_mha_params const& p, cudaStream_t stream)
 {
     if constexpr (sizeof(T) == 4 && D <= 64)
     {
-        AttPlan const plan = planAtt(p.B, p.num_heads, p.S, D, smCount());
+        bool const full = p.cu_seqlens != nullptr ? p.total == static_cast<int64_t>(p.B) * p.S : p.mask_idx == nullptr;
+        AttPlan const plan = planAtt(p.B, p.num_heads, p.S, D, full, smCount());
         if (plan.rows == 32)
-            return launchMhaTiled<T, D, 2, true>(p, plan.perSm, stream);
+            return launchMhaTiled<T, D, 2, true, true>(p, plan.perSm, stream);
         if constexpr (D == 64)
+        {
             if (plan.async)
-                return launchMhaTiled<T, D, 4, true>(p, plan.perSm, stream);
-        return launchMhaTiled<T, D, 4, false>(p, plan.perSm, stream);
+                return launchMhaTiled<T, D, 4, true, true>(p, plan.perSm, stream);
+            if (!plan.skip)
+                return launchMhaTiled<T, D, 4, false, false>(p, plan.perSm, stream);
+        }
+        return launchMhaTiled<T, D, 4, false, true>(p, plan.perSm, stream);
     }
     else
-        return launchMhaTiled<T, D, 4, false>(p, 0, stream);
+        return launchMhaTiled<T, D, 4, false, false>(p, 0, stream);
 }
 
 template <typename T>

@@ -13,14 +13,15 @@ SMS = 148
 def plan(tmp_path_factory):
     d = tmp_path_factory.mktemp("f32plan")
     (d / "plan.cpp").write_text('#include "mha_f32_plan.h"\n'
-                                'extern "C" void plan(int32_t B, int32_t N, int32_t S, int32_t d, int64_t sms, int32_t* out)'
-                                "{ auto p = b200::planAtt(B, N, S, d, sms); out[0] = p.rows; out[1] = p.perSm; out[2] = p.async; }\n")
+                                'extern "C" void plan(int32_t B, int32_t N, int32_t S, int32_t d, int32_t full, int64_t sms, int32_t* out)'
+                                "{ auto p = b200::planAtt(B, N, S, d, full, sms); out[0] = p.rows; out[1] = p.perSm; out[2] = p.async; out[3] = p.skip; }\n")
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", str(d / "plan.cpp"), "-o", str(d / "plan.so")], check=True)
     so = ctypes.CDLL(str(d / "plan.so"))
 
-    def call(b, n, s, d=64):
-        out = (ctypes.c_int32 * 3)()
-        so.plan(b, n, s, d, ctypes.c_int64(SMS), out)
+    def call(b, n, s, d=64, full=0):
+        out = (ctypes.c_int32 * 4)()
+        so.plan(b, n, s, d, full, ctypes.c_int64(SMS), out)
+        assert out[3] or (full and s % 64 == 0 and out[0] == 64 and not out[2])   # keys are only kept where there are none to leave out
         return out[0], out[1], bool(out[2])
 
     return call
@@ -36,6 +37,7 @@ def test_every_launch_fits_the_residency_it_asks_for(plan, head_size):
     for pairs in list(range(1, 320)) + [444, 445, 592, 600, 888, 1000, 1776, 5000]:
         for s in (1, 16, 32, 33, 64, 65, 96, 97, 128, 129, 192, 193, 200, 256, 257, 400, 512, 1000):
             rows, per_sm, asynchronous = plan(pairs, 1, s, head_size)
+            assert plan(pairs, 1, s, head_size, 1) == (rows, per_sm, asynchronous)
             n64, n32 = _rounds(pairs, s, 64), _rounds(pairs, s, 32)
             assert rows in (32, 64) and per_sm in (0, 1, 2, 3)
             if per_sm:

@@ -470,6 +470,8 @@ def test_mha_fp32_rows_per_cta(cuda, S, B, N, d):
     ref = O.mha(qkv, B, S, N, d, lengths=lengths)
     out = T.mha(_t(qkv, cuda), B, S, N, head_size=d, mask_idx=_t(lengths, cuda))
     assert O.close_abs_or_rel(out.cpu().numpy(), ref, 1e-5, 1e-5)[0]
+    out = T.mha(_t(qkv, cuda), B, S, N, head_size=d)   # all lengths S: nothing is left out where S is a multiple of 64
+    assert O.close_abs_or_rel(out.cpu().numpy(), O.mha(qkv, B, S, N, d), 1e-5, 1e-5)[0]
     cu = O.cu_seqlens(lengths)
     packed = rng.standard_normal((int(cu[-1]), 3 * N * d)).astype(np.float32)
     ref = O.mha(packed, B, S, N, d, cu=cu)
